@@ -64,6 +64,12 @@ enum WindowFlags : uint8_t {
  * them per site. */
 constexpr int kDeepSlots = 256;
 
+/* the short FP32 form (lean.cuh): record groups per adjusted-quality table row
+ * (distinct keys of a base group, at most the record slots of a bin that uses
+ * it), and the unit of its gaps (in log10) */
+constexpr int kLeanG = 64;
+constexpr float kLeanGapUnit = 0x1p-5f;
+
 /* tiles a warp of the persistent FP32 kernel takes per counter increment */
 constexpr int kStreamChunk = 2;
 
@@ -95,7 +101,7 @@ struct CallArgs {
     const int32_t* pos;
     const int32_t* lenhit;       /* (read_len << 16) | hit */
     const uint8_t* strand;       /* '+' or '-' */
-    const uint16_t* bq;          /* [n_reads][L]: base char | quality char << 8 */
+    const uint16_t* bq;          /* [n_reads][L]: bases and qualities (make_elem) */
     int64_t n_reads;
     int64_t read_lo;             /* reads [read_lo, n_reads) are on the device (0 unless streamed) */
     int L;                       /* -L: read pitch and coordinate bound */
@@ -112,6 +118,8 @@ struct CallArgs {
     const float* lik32;          /* same, rounded to FP32: [qa_rows][L][4][8] columns 0-7 */
     const float* lik32b;         /* [qa_rows][L][4][2] columns 8-9 */
     int qa_rows;
+    const uint32_t* lean_q;      /* [16][kLeanG][64] the short form's q_adj table (lean.cuh), or null: no short form */
+    const float* lean4;          /* [4][1 + qa_rows * L][4] its terms: base o's records, genotypes (o, 0..3) */
     const uint8_t* qadj;         /* [tmax][gmax][65] adjusted quality */
     int tmax, gmax;
     const double* p_prior;       /* [8][16] */
@@ -134,7 +142,6 @@ struct CallArgs {
     int64_t* tile_rng;           /* [n_tiles][2]: reads starting in [s0 - L + 1, s0 + kTile) of each tile */
     int64_t* warp_rng;           /* [n_tiles][2]: reads that can cover each tile's sites */
     int bin_limit[kNumBins];     /* deepest column each depth bin takes (at most its record slots) */
-    uint32_t* deep_recs;         /* record columns of the deep bins' CTAs, [CTA][SLOTS][kTile] */
     /* the call of a site without records or counts, by site code (16 entries;
      * empty_valid[code] = 0 where it is not a fixed homozygous call) */
     const SiteCall* empty_calls;

@@ -1,0 +1,1090 @@
+/*
+ * calling_fast.cu - the FP32 calling kernels: the tile kernels in the short
+ * form (lean.cuh) and the general one, the persistent kernel over a segment's
+ * tiles, and the warp-per-site kernel of the deepest bin.
+ */
+#include <cuda_runtime.h>
+
+#include "calling.cuh"
+#include "lean.cuh"
+#include "site_math.cuh"
+#include "tile.cuh"
+#include "tma.cuh"
+
+namespace gsnp {
+
+namespace {
+
+/* resident CTAs per SM the kernels are compiled for; this caps their
+ * registers at 64 (32 warps per SM; a few spilled words cost less than the
+ * latency the extra warps hide) */
+constexpr int kFastCtasPerSm = 32 * 32 / kTile;
+
+/* The reads of a tile staged in shared memory by the persistent kernel: per
+ * read its start, (len << 16) | hit with the strand in bit 31, and the byte
+ * offset in `rows` that column 0 of its row would have; the bulk copy of the
+ * read holds the columns that cover the tile. */
+struct StagedReads {
+    const int32_t* pos;
+    const uint32_t* lhs;
+    const int32_t* rbase;
+    const uint8_t* rows;
+    int n;
+};
+
+/* warp_pileup over staged reads: the same records and counts, read from
+ * shared memory (broadcast loads of the per-read values, one 16-bit load
+ * per covering read and lane). */
+template <int SLOTS>
+__device__ __forceinline__ PackedPileup warp_pileup_staged(const CallArgs& a, const StagedReads& sr, int64_t site,
+                                                          bool active, uint32_t* recs, bool* report_overflow) {
+    PileupAcc acc;
+    for (int k = 0; k < sr.n; ++k) {
+        const int32_t start = sr.pos[k];
+        const uint32_t lhs = sr.lhs[k];
+        const int coord = (int)(site - start);
+        const uint32_t lh = lhs & 0x7fffffffu;
+        if (active && coord >= 0 && coord < (int)(lh >> 16)) {
+            const uint32_t bq = *reinterpret_cast<const uint16_t*>(sr.rows + sr.rbase[k] + 2 * coord);
+            acc.take<SLOTS>(bq, lh, coord, (int)(lhs >> 31), recs);
+        }
+    }
+    return acc.finish(a, report_overflow);
+}
+
+}  // namespace
+
+/* ------------------------------------------------------------------------ */
+/* the fast calling kernel                                                   */
+/* ------------------------------------------------------------------------ */
+
+/* The end of a site's FP32 call: prove(&call) decides it from its sums, or the
+ * site is appended to the deferred pool with its counts p and sorted records
+ * (record() gives a column word as a record word of occurrence 1).  Every lane of the warp calls it (the
+ * appends are warp-aggregated). */
+template <class Prove, class Record>
+__device__ __forceinline__ void finish_fast_site(const CallArgs& a, int64_t site, bool active, uint8_t ori,
+                                                 uint8_t wflags, int32_t snp_row, const SitePileup& p,
+                                                 const uint32_t* recs, Prove&& prove, Record&& record) {
+    const int lane = threadIdx.x & 31;
+    uint8_t dflags = 0;
+    if (active) {
+        if (wflags & kWinKeepCounts) store_counts(a, site, p);
+        CallWords call;
+        if ((site & 4095) == 0 && a.stats) dflags = kCallSampled;
+        const bool empty = p.num == 0 && (p.ca[0] | p.ca[1] | p.ca[2] | p.ca[3]) == 0 && a.empty_valid[ori];
+        if (empty) {
+            /* no record and no count: the call depends on the site code only */
+            const uint4* src = reinterpret_cast<const uint4*>(a.empty_calls + ori);
+            call.a = __ldg(src);
+            call.b = __ldg(src + 1);
+            call.b.x = p.depth;
+            call.b.y = p.repeat;
+        } else if (!prove(&call)) {
+            call.a = call.b = make_uint4(0u, 0u, 0u, 0u);
+            dflags |= kCallPending;
+        }
+        call.a.y |= (uint32_t)dflags << 16;
+        uint4* dst = reinterpret_cast<uint4*>(a.out + site);
+        dst[0] = call.a;
+        dst[1] = call.b;
+    }
+    /* append the deferred sites of the warp */
+    const unsigned m = __ballot_sync(kFull, dflags != 0);
+    if (m == 0) return;
+    unsigned long long base = 0;
+    const int leader = __ffs(m) - 1;
+    if (lane == leader) base = atomicAdd(a.dcount, (unsigned long long)__popc(m));
+    base = __shfl_sync(kFull, base, leader);
+    if (!dflags) return;
+    const unsigned long long slot = base + __popc(m & ((1u << lane) - 1u));
+    const unsigned long long off = atomicAdd(a.dcount + 1, (unsigned long long)p.num);
+    if ((int64_t)slot >= a.dsite_cap || (int64_t)(off + p.num) > a.dpool_cap) return;
+    DeferredSite d;
+    d.site = site;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        d.cu[i] = (uint16_t)p.cu[i];
+        d.qs[i] = (uint16_t)p.qs[i];
+        d.ca[i] = p.ca[i];
+    }
+    d.depth = p.depth;
+    d.repeat = p.repeat;
+    d.rec_off = (uint32_t)off;
+    d.num = (uint16_t)p.num;
+    d.dep_uni = (uint16_t)p.dep_uni;
+    d.snp_row = snp_row;
+    d.flags = dflags;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) d.pad[i] = 0;
+    a.dsites[slot] = d;
+    uint32_t* dst = a.dpool + off;
+    for (int i = 0; i < p.num; ++i) dst[i] = record(recs[i * kTile]);
+}
+
+/* The FP32 work on one site of a tile after its pileup and sort, in the
+ * general form: the dependency walk, the compensated sums and the FP32
+ * posterior.  Every lane of the warp calls it. */
+template <int SLOTS>
+__device__ __forceinline__ void fast_site(const CallArgs& a, int64_t site, bool active, uint8_t ori, uint8_t wflags,
+                                          int32_t snp_row, const SitePileup& p, uint32_t* recs, uint32_t* seen) {
+    Kahan10 k;
+    k.init();
+    if (active) {
+        /* adjusted quality of each record, written over its occurrence byte */
+        walk_records<true, kPcrBits(SLOTS, true)>(a, recs, seen, kTile, p.num, [&](int i, int qa, int, int) {
+            recs[i * kTile] = (recs[i * kTile] & ~0xffu) | (uint32_t)qa;
+        });
+        /* FP32 sums, four records per compensated step (the grouping of
+         * likelihood_fp32) */
+        for (int i = 0; i < p.num; i += 4) {
+            float x[10], y[10];
+            uint32_t w = recs[i * kTile];
+            lik32_row(a, (int)(w & 0xffu), rec_coord(w), rec_base(w), x);
+            if (i + 1 < p.num) {
+                w = recs[(i + 1) * kTile];
+                lik32_row(a, (int)(w & 0xffu), rec_coord(w), rec_base(w), y);
+#pragma unroll
+                for (int v = 0; v < 10; ++v) x[v] = __fadd_rn(x[v], y[v]);
+            }
+            if (i + 2 < p.num) {
+                float z[10];
+                w = recs[(i + 2) * kTile];
+                lik32_row(a, (int)(w & 0xffu), rec_coord(w), rec_base(w), y);
+                if (i + 3 < p.num) {
+                    w = recs[(i + 3) * kTile];
+                    lik32_row(a, (int)(w & 0xffu), rec_coord(w), rec_base(w), z);
+#pragma unroll
+                    for (int v = 0; v < 10; ++v) y[v] = __fadd_rn(y[v], z[v]);
+                }
+#pragma unroll
+                for (int v = 0; v < 10; ++v) x[v] = __fadd_rn(x[v], y[v]);
+            }
+            k.add(x);
+        }
+    }
+    finish_fast_site(a, site, active, ori, wflags, snp_row, p, recs,
+                     [&](CallWords* call) {
+                         SiteCall c;
+                         if (!fast_posterior(a, snp_row, ori, p, k.s, p.num, &c)) return false;
+                         *call = call_words(c);
+                         return true;
+                     },
+                     [](uint32_t w) { return (w & ~0xffu) | 1u; });
+}
+
+/* ------------------------------------------------------------------------ */
+/* the short form (lean.cuh) of a tile                                        */
+/* ------------------------------------------------------------------------ */
+
+/* Per-warp shared memory of the short form: the tile's unique reads as the
+ * pileup broadcasts them, and a 16-bit entry per (strand, start or end) that
+ * a covering read can have in a tile: its reads in the low byte, the number of
+ * their group in the high one. */
+struct LeanRead {
+    int32_t c0;        /* column of the read at the tile's first site */
+    int32_t off;       /* its element there, from the first read's row */
+    uint32_t low;      /* bits 23:0 of its lean record there: cycle, strand, 4 * group */
+    int32_t len;       /* bits 7:0; while the groups are formed, its table entry above */
+};
+/* record slots of the short form in a bin of that many: whole chunks of 16 */
+__host__ __device__ constexpr int lean_slots(int slots) { return (slots + 15) & ~15; }
+/* unique reads that a tile of the short form holds, with room to pad both lists */
+__host__ __device__ constexpr int lean_reads(int slots) { return 2 * lean_slots(slots); }
+__host__ __device__ constexpr int lean_table_words(int L) { return L + kTile; }
+__host__ __device__ constexpr size_t lean_smem_bytes(int slots, int L) {
+    /* the table is done with before the first record is written, and lies in
+     * the records' place */
+    return ((size_t)lean_slots(slots) * kTile > (size_t)lean_table_words(L) ? (size_t)lean_slots(slots) * kTile
+                                                                           : (size_t)lean_table_words(L)) * 4 +
+           (size_t)lean_reads(slots) * sizeof(LeanRead);
+}
+constexpr int kLeanGroups = 15;   /* most groups, and most reads of one (a 4-bit count each) */
+
+/* The pileup of a warp's tile (as warp_pileup) in the short form: false, for
+ * the whole warp, when the tile needs the general one - a site deeper than
+ * SLOTS records, more reads than the lists hold, a quality outside 1 .. 63, or
+ * more repeated keys than the walk's counts hold.
+ *
+ * What bounds it is the number of instructions per read, since every lane
+ * looks at every read of the tile.  What depends on the read only is worked
+ * out once, by one lane, and broadcast with one 128-bit shared load; a lane
+ * then needs its column, the element's address, and two additions for the
+ * record word: the element is the word's top byte, and the cycle runs up
+ * (forward reads) or down (reverse ones) with the site.  The records are
+ * sorted afterwards and no site reaches the 255-record cap, so the reads may be
+ * taken in any order: forward ones from a list at the front, reverse ones from
+ * one at the back, and the few reads of several hits, which leave no record,
+ * as they are met. */
+template <int SLOTS>
+__device__ __forceinline__ bool lean_pileup(const CallArgs& a, int64_t s0, int64_t r_lo, int64_t r_hi,
+                                            uint32_t* recs_all, LeanRead* reads, LeanPile* out) {
+    constexpr int kReads = lean_reads(SLOTS);
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const int L = a.L;
+    uint32_t* const recs = recs_all + lane;
+    uint32_t* const table = recs_all;
+    if (r_hi - r_lo > kReads - 8) return false;
+    const int n = (int)(r_hi - r_lo);
+    for (int i = lane; i < lean_table_words(L); i += 32) table[i] = 0u;
+    __syncwarp();
+    const uint16_t* row = a.bq + r_lo * L + lane;
+    uint32_t depth = 0, extra_hits = 0;
+    uint64_t extra4 = 0;
+    int groups = 0, fwd = 0, rev = 0;
+    bool bad = false;
+#pragma unroll 1
+    for (int c = 0; c < n; c += 32) {
+        bool uni = false, minus = false, second = false;
+        int c0 = 0, len = 0, at = 0;
+        uint32_t hit = 0;
+        if (c + lane < n) {
+            const int64_t r = r_lo + c + lane;
+            c0 = (int)(s0 - __ldg(a.pos + r));
+            const uint32_t lh = (uint32_t)__ldg(a.lenhit + r);
+            len = (int)(lh >> 16);
+            if (c0 < len) {   /* it covers a site of the tile */
+                hit = lh & 0xffffu;
+                uni = hit == 1u;
+                minus = __ldg(a.strand + r) != '+';
+            }
+        }
+        const unsigned covers = __ballot_sync(kFull, c0 < len);
+        unsigned multi = covers & ~__ballot_sync(kFull, uni);
+        const unsigned mr = __ballot_sync(kFull, uni && minus), mf = __ballot_sync(kFull, uni && !minus);
+        if (uni) {
+            /* entry of the read in the table: starts s0 - L + 1 .. s0 + 31 of the
+             * forward reads, then ends s0 + 1 .. s0 + 31 + L of the reverse ones */
+            at = minus ? L + kTile + (len - c0) - 1 : L - 1 - c0;
+            const int sh = (at & 1) * 16;
+            const uint32_t before = (atomicAdd(table + (at >> 1), 1u << sh) >> sh) & 0xffu;
+            second = before == 1u;
+            bad |= before >= (uint32_t)kLeanGroups;
+            LeanRead m;
+            m.c0 = c0;
+            m.off = (c + lane) * L + c0;
+            m.low = ((uint32_t)(minus ? len - 1 - c0 : c0) << 16) + (minus ? 0x8000u : 0u);
+            m.len = len | at << 8;
+            reads[minus ? kReads - 1 - rev - __popc(mr & lt) : fwd + __popc(mf & lt)] = m;
+        }
+        const unsigned b = __ballot_sync(kFull, second);
+        if (second) reinterpret_cast<uint8_t*>(table)[at * 2 + 1] = (uint8_t)(groups + __popc(b & lt) + 1);
+        groups += __popc(b);
+        fwd += __popc(mf);
+        rev += __popc(mr);
+        for (; multi; multi &= multi - 1) {
+            const int src = __ffs(multi) - 1;
+            const int x = __shfl_sync(kFull, c0, src) + lane;
+            const uint32_t h = __shfl_sync(kFull, hit, src);
+            if ((uint32_t)x < (uint32_t)__shfl_sync(kFull, len, src)) {
+                const uint32_t e = __ldg(a.bq + (r_lo + c + src) * L + x);
+                depth += 1;
+                extra_hits += h - 1u;
+                if (elem_valid(e)) extra4 += 1ull << (elem_base(e) * 16);
+            }
+        }
+        __syncwarp();
+    }
+    if (__any_sync(kFull, bad) || groups > kLeanGroups) return false;
+    /* each read's group; both lists are padded to whole steps of four */
+    if (lane < 4) {
+        reads[fwd + lane].len = 0;
+        reads[kReads - 1 - rev - lane].len = 0;
+    }
+    for (int i = lane; i < fwd + rev; i += 32) {
+        LeanRead* m = reads + (i < fwd ? i : kReads - 1 - (i - fwd));
+        const int x = m->len;
+        m->low |= (uint32_t)reinterpret_cast<const uint8_t*>(table)[(x >> 8) * 2 + 1] << 2;
+        m->len = x & 0xff;
+    }
+    __syncwarp();
+    uint32_t seen_bits = 0;
+    int num = 0;
+#pragma unroll 1
+    for (int strand = 0; strand < 2; ++strand) {
+        const int cnt = strand ? rev : fwd;
+        const uint32_t step = strand ? 0u - ((uint32_t)lane << 16) : (uint32_t)lane << 16;
+        const int4* list = reinterpret_cast<const int4*>(strand ? reads + (kReads - ((rev + 3) & ~3)) : reads);
+#pragma unroll 1
+        for (int k0 = 0; k0 < cnt; k0 += 4) {
+            uint32_t e[4], low[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int4 rd = list[k0 + u];
+                const bool cov = (uint32_t)(rd.x + lane) < (uint32_t)rd.w;
+                low[u] = (uint32_t)rd.z + step;
+                e[u] = kElemInvalid;
+                if (cov) {
+                    e[u] = __ldg(row + rd.y);
+                    depth += 1;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                seen_bits |= e[u];
+                if (e[u] < kElemWide) {
+                    if (num < SLOTS) recs[num * kTile] = (e[u] << 24) + low[u];
+                    num += 1;
+                }
+            }
+        }
+    }
+    if (__any_sync(kFull, num > SLOTS || (seen_bits & kElemWide))) return false;
+    out->depth = depth;
+    out->repeat = depth + extra_hits;
+    out->extra4 = extra4;
+    out->num = num;
+    return true;
+}
+
+/* A tile in the short form; every lane of the warp calls it.  False (for the
+ * warp, nothing written) when lean_pileup leaves it. */
+template <int SLOTS>
+__device__ __forceinline__ bool lean_tile(const CallArgs& a, int64_t tile, int64_t r_lo, int64_t r_hi, uint8_t wflags,
+                                          uint32_t* recs_all, uint32_t* scratch) {
+    static_assert(SLOTS <= kLeanG && SLOTS % 16 == 0, "a walk counts at most kLeanG distinct keys; chunks of 16");
+    const int t = threadIdx.x & 31;
+    const int64_t s0 = tile * kTile, site = s0 + t;
+    const bool active = site < a.chr_len;
+    LeanRead* reads = reinterpret_cast<LeanRead*>(scratch);
+    uint32_t* recs = recs_all + t;
+    LeanPile pile;
+    /* a read's columns end before the chromosome does, so sites past the end
+     * have no covering read */
+    if (!lean_pileup<SLOTS>(a, s0, r_lo, r_hi, recs_all, reads, &pile))
+        return false;
+    const uint8_t ori = active ? __ldg(a.ori + site) : 0;
+    const int32_t snp_row = tile_snp_row(a, tile, (ori & 8) != 0);
+    const int most = __reduce_max_sync(kFull, pile.num);
+    for (int i = pile.num; i < ((most + 15) & ~15); ++i) recs[i * kTile] = kLeanPad;
+    lean_sort<kTile>(recs, pile.num, most);
+    LeanSums z;
+    lean_walk<kTile>(a, recs, pile.num, ori & 3, &z);
+    const SitePileup p = lean_counts(pile, z);
+    finish_fast_site(a, site, active, ori, wflags, snp_row, p, recs,
+                     [&](CallWords* call) { return lean_posterior(a, snp_row, ori, pile, z, call); },
+                     [](uint32_t w) { return lean_to_record(w); });
+    return true;
+}
+
+/* Sites whose call is not proven in FP32 (and every 4096th site, sampled for
+ * the FP32 accuracy figure) are appended to the deferred pool: counts and the
+ * sorted records with their occurrence byte restored.  The append counters
+ * keep counting past the capacities so that the host can size the pool and
+ * run the pass again. */
+template <int SLOTS>
+__device__ __forceinline__ void fast_tile(const CallArgs& a, int64_t tile, uint32_t* recs_all, uint32_t* seen_all) {
+    const int t = threadIdx.x;
+    const int64_t s0 = tile * kTile;
+    const int win = (int)(s0 / kWin);
+    const uint8_t wflags = a.win_flags[win];
+    const int64_t r_lo = a.warp_rng[tile * 2];
+    const int64_t r_hi = a.warp_rng[tile * 2 + 1];
+    if constexpr (SLOTS <= kLeanG) {
+        if (a.lean_q && lean_tile<lean_slots(SLOTS)>(a, tile, r_lo, r_hi, wflags, recs_all,
+                                                     recs_all + lean_slots(SLOTS) * kTile))
+            return;
+        __syncwarp();
+    }
+    const int64_t site = s0 + t;
+    const bool active = site < a.chr_len;
+    const uint8_t ori = active ? __ldg(a.ori + site) : 0;
+    const int32_t snp_row = tile_snp_row(a, tile, (ori & 8) != 0);
+    const SitePileup p = warp_pileup<SLOTS>(a, r_lo, r_hi, site, active, recs_all + t).unpack();
+    uint32_t* recs = recs_all + t;
+    uint32_t* seen = seen_all + t;
+    if (active) sort_column<SLOTS>(recs, p.num);
+
+    fast_site<SLOTS>(a, site, active, ori, wflags, snp_row, p, recs, seen);
+}
+
+/* The tiles of one depth bin, as call_tiles_kernel takes them. */
+template <int SLOTS>
+__global__ void __launch_bounds__(kTile, kFastCtasPerSm) call_fast_kernel(CallArgs a, const int32_t* __restrict__ tiles,
+                                                                          const int* __restrict__ count, int* next) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint32_t* recs_all = reinterpret_cast<uint32_t*>(smem);
+    uint32_t* seen_all = recs_all + SLOTS * kTile;
+    if (!count) {
+        fast_tile<SLOTS>(a, tiles[blockIdx.x], recs_all, seen_all);
+        return;
+    }
+    for_each_listed(count, next, [&](int i) { fast_tile<SLOTS>(a, tiles[i], recs_all, seen_all); });
+}
+
+/* ------------------------------------------------------------------------ */
+/* the deep bins of the FP32 form: one warp per site                          */
+/* ------------------------------------------------------------------------ */
+
+/* Tiles with a site of more than 64 records (hotspots of hundreds of reads)
+ * are called by a CTA of 32 warps, warp w calling site w of the tile, so that
+ * a site's hundreds of records are spread over 32 lanes instead of walked by
+ * one.  Per warp, in shared memory: the site's record column (at most 255
+ * records) and a byte counter per (base, strand, cycle) key. */
+constexpr int kDeepThreads = 32 * kTile;
+constexpr int kDeepCap = 256;
+constexpr int kDeepKeys = 4 * 2 * 256;
+constexpr size_t kDeepSmem = (size_t)kTile * (kDeepCap * 4 + kDeepKeys);
+
+/* The pileup of one site by its warp (kernel/update_kernel.cu:260-325, as
+ * PileupAcc::take): the reads [r_lo, r_hi) 32 at a time, in order.  A
+ * covering read counts in depth and repeat; one that is not N and reaches
+ * q_min is taken while the site has fewer than 255 unique records, and a
+ * unique one (hit 1) adds a record.  Whether the cap still admits a read
+ * depends only on the unique valid reads before it, which a ballot gives, so
+ * the 32 reads of a step are decided together with the reference's result.
+ * Once the cap is reached a read can only add to depth and repeat, which
+ * need no base or quality; the scan ends at the first step whose reads all
+ * start past the site.
+ *
+ * The scan is bound by load latency (each step's base and quality load
+ * depends on the read's start), so its loads run ahead of the decisions: an
+ * iteration loads the starts and lengths of its kDeepAhead steps' reads in
+ * the iteration before, and their bases, qualities and strands all at its
+ * start (for every covering read, when the site was below the cap as the
+ * iteration began; a step that finds the site capped leaves its loads
+ * unused).  The steps are then decided in order, as above. */
+constexpr int kDeepAhead = 2;
+
+__device__ __forceinline__ SitePileup deep_pileup(const CallArgs& a, int64_t r_lo, int64_t r_hi, int64_t site,
+                                                  uint32_t* recs) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const int L = a.L;
+    SitePileup p;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        p.cu[b] = 0;
+        p.qs[b] = 0;
+        p.ca[b] = 0;
+    }
+    p.depth = 0;
+    p.repeat = 0;
+    p.dep_uni = 0;
+    p.num = 0;
+    /* repeat and the quality sums per lane, added over the warp after the
+     * scan (the same sums, modulo 2^32 as before) */
+    uint32_t rep_l = 0, qs_l[4] = {0u, 0u, 0u, 0u};
+    int32_t nst[kDeepAhead];
+    uint32_t nlh[kDeepAhead];
+#pragma unroll
+    for (int u = 0; u < kDeepAhead; ++u) {
+        const int64_t r = r_lo + 32 * u + lane;
+        nst[u] = r < r_hi ? __ldg(a.pos + r) : 0;
+        nlh[u] = r < r_hi ? (uint32_t)__ldg(a.lenhit + r) : 0u;
+    }
+    for (int64_t rb = r_lo; rb < r_hi; rb += 32 * kDeepAhead) {
+        int coord[kDeepAhead];
+        uint32_t lh[kDeepAhead], bq[kDeepAhead];
+        bool cov[kDeepAhead], minus[kDeepAhead];
+        const bool capped_at_start = p.dep_uni >= 0xFF;
+#pragma unroll
+        for (int u = 0; u < kDeepAhead; ++u) {
+            const int64_t r = rb + 32 * u + lane;
+            const bool in = r < r_hi;
+            coord[u] = in ? (int)(site - nst[u]) : -1;
+            lh[u] = nlh[u];
+            cov[u] = in && coord[u] >= 0 && coord[u] < (int)(lh[u] >> 16);
+            bq[u] = 0;
+            minus[u] = false;
+            if (cov[u] && !capped_at_start) {
+                bq[u] = __ldg(a.bq + r * L + coord[u]);
+                minus[u] = __ldg(a.strand + r) != '+';
+            }
+            const int64_t rn = r + 32 * kDeepAhead;
+            nst[u] = rn < r_hi ? __ldg(a.pos + rn) : 0;
+            nlh[u] = rn < r_hi ? (uint32_t)__ldg(a.lenhit + rn) : 0u;
+        }
+        bool past = false;
+#pragma unroll
+        for (int u = 0; u < kDeepAhead; ++u) {
+            if (__all_sync(kFull, coord[u] < 0)) {   /* every read from here on starts past the site */
+                past = true;
+                break;
+            }
+            const unsigned mc = __ballot_sync(kFull, cov[u]);
+            if (mc == 0) continue;
+            const uint32_t hit = lh[u] & 0xffffu;
+            p.depth += (uint32_t)__popc(mc);
+            rep_l += cov[u] ? hit : 0u;
+            if (p.dep_uni >= 0xFF) continue;
+            const bool valid = cov[u] && elem_valid(bq[u]);
+            const int bi = elem_base(bq[u]), q = elem_q(bq[u]);
+            const bool uni = valid && hit == 1;
+            const int uni_before = p.dep_uni + __popc(__ballot_sync(kFull, uni) & lt);
+            const bool acc = valid && uni_before < 0xFF;
+            const bool rec = acc && uni;
+            const unsigned mr = __ballot_sync(kFull, rec);
+            if (rec) {
+                const uint32_t cv =
+                    minus[u] ? (uint32_t)((int)(lh[u] >> 16) - 1 - coord[u]) : (uint32_t)coord[u];
+                recs[p.num + __popc(mr & lt)] = make_record_of((uint32_t)bi, q, cv, (uint32_t)minus[u]);
+            }
+            p.num += __popc(mr);
+            p.dep_uni += __popc(mr);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                p.cu[b] += __popc(__ballot_sync(kFull, rec && bi == b));
+                qs_l[b] += (rec && bi == b) ? (uint32_t)q : 0u;
+                p.ca[b] += (uint32_t)__popc(__ballot_sync(kFull, acc && bi == b));
+            }
+        }
+        if (past) break;
+    }
+    p.repeat = __reduce_add_sync(kFull, rep_l);
+#pragma unroll
+    for (int b = 0; b < 4; ++b) p.qs[b] = (int)__reduce_add_sync(kFull, qs_l[b]);
+    return p;
+}
+
+/* Ascending bitonic sort of v[0, n), n <= kDeepCap = 256, by the lanes of a
+ * warp in registers: lane l holds elements 8l .. 8l+7 (padded with
+ * 0xFFFFFFFF, which no record word equals).  The network's stages of
+ * distance j < 8 are compare-exchanges within a lane; those of distance
+ * j >= 8 pair lane l with lane l ^ (j / 8), which keeps the smaller or the
+ * larger of each of its eight elements.  Every loop bound is a constant, so
+ * the 36 stages unroll into straight code with no index arithmetic and no
+ * shared-memory traffic between them. */
+__device__ __forceinline__ void deep_sort(uint32_t* v, int n) {
+    static_assert(kDeepCap == 256, "eight elements a lane");
+    const int lane = threadIdx.x & 31;
+    uint32_t x[8];
+    const uint4 lo4 = reinterpret_cast<const uint4*>(v)[lane * 2];
+    const uint4 hi4 = reinterpret_cast<const uint4*>(v)[lane * 2 + 1];
+    x[0] = lo4.x, x[1] = lo4.y, x[2] = lo4.z, x[3] = lo4.w;
+    x[4] = hi4.x, x[5] = hi4.y, x[6] = hi4.z, x[7] = hi4.w;
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        if (lane * 8 + e >= n) x[e] = 0xFFFFFFFFu;
+#pragma unroll
+    for (int k = 2; k <= 256; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j >= 8) {
+                const int d = j >> 3;
+                const bool keep_min = (((lane * 8) & k) == 0) == ((lane & d) == 0);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const uint32_t y = __shfl_xor_sync(kFull, x[e], d);
+                    x[e] = keep_min ? min(x[e], y) : max(x[e], y);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    if (e & j) continue;
+                    const int f = e | j;
+                    const bool asc = ((lane * 8 + e) & k) == 0;
+                    const uint32_t a = min(x[e], x[f]), b = max(x[e], x[f]);
+                    x[e] = asc ? a : b;
+                    x[f] = asc ? b : a;
+                }
+            }
+        }
+    }
+    __syncwarp();
+    reinterpret_cast<uint4*>(v)[lane * 2] = make_uint4(x[0], x[1], x[2], x[3]);
+    reinterpret_cast<uint4*>(v)[lane * 2 + 1] = make_uint4(x[4], x[5], x[6], x[7]);
+    __syncwarp();
+}
+
+/* The dependency walk and the FP32 sums of a sorted column by its warp,
+ * 32 records a step, record c0 + lane on that lane.  The walk's two counts
+ * (walk_records) come from the whole step at once:
+ *   - tmp, the earlier records of the same (base, strand, cycle) key: the
+ *     key's counter from the steps before plus the lower lanes with that key
+ *     (match-any); the highest of them then stores the new count;
+ *   - gdc, the first occurrences of a key (tmp = 0) so far in the record's
+ *     base group, less one: a ballot prefix, from the lane where the base
+ *     group starts, or carried over from the step before.
+ * Each lane sums its records' rows with compensation; the 32 sums are then
+ * added in a tree (the bound of fast_posterior's k_units 9). */
+__device__ __forceinline__ void deep_walk_sums(const CallArgs& a, const uint32_t* recs, uint8_t* cnt, int num,
+                                               float* s) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u, le = (lt << 1) | 1u;
+    for (int i = lane; i < kDeepKeys / 4; i += 32) reinterpret_cast<uint32_t*>(cnt)[i] = 0u;
+    __syncwarp();
+    Kahan10 k;
+    k.init();
+    int carry_firsts = 0, carry_base = -1;
+    for (int c0 = 0; c0 < num; c0 += 32) {
+        const int i = c0 + lane;
+        const bool valid = i < num;
+        const uint32_t w = valid ? recs[i] : 0u;
+        const int o = rec_base(w), coord = rec_coord(w);
+        const int key = valid ? (o << 9) | (rec_strand(w) << 8) | coord : kDeepKeys + lane;
+        const unsigned peers = __match_any_sync(kFull, key);
+        const int seen = valid ? (int)cnt[key] : 0;
+        __syncwarp();
+        const int tmp = seen + __popc(peers & lt);
+        if (valid && (peers >> lane) == 1u) cnt[key] = (uint8_t)(seen + __popc(peers));
+        __syncwarp();
+        const int prev_o = __shfl_up_sync(kFull, o, 1);
+        const bool brk = valid && o != (lane == 0 ? carry_base : prev_o);
+        const unsigned bm = __ballot_sync(kFull, brk) & le;
+        const unsigned fm = __ballot_sync(kFull, valid && tmp == 0) & le;
+        const int firsts = bm ? __popc(fm & ~((1u << (31 - __clz(bm))) - 1u)) : carry_firsts + __popc(fm);
+        carry_firsts = __shfl_sync(kFull, firsts, 31);
+        carry_base = __shfl_sync(kFull, o, 31);
+        if (valid) {
+            const int gdc = firsts - 1, t1 = tmp + 1;
+            const int qa = (t1 < a.tmax && gdc < a.gmax)
+                               ? (int)__ldg(a.qadj + ((size_t)t1 * a.gmax + gdc) * 65 + rec_q(w))
+                               : 1;
+            float x[10];
+            lik32_row(a, qa, coord, o, x);
+            k.add(x);
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < 10; ++v) {
+        float t = k.s[v];
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) t = __fadd_rn(t, __shfl_xor_sync(kFull, t, d));
+        s[v] = t;
+    }
+}
+
+/* Site w of a deep tile, called by one warp (as fast_site: counts kept for
+ * later gap windows, the FP32 posterior, or the site deferred with its
+ * records). */
+__device__ __forceinline__ void deep_tile(const CallArgs& a, int64_t tile, int w, uint32_t* recs, uint8_t* cnt) {
+    const int lane = threadIdx.x & 31;
+    const int64_t s0 = tile * kTile, site = s0 + w;
+    const int64_t sl = s0 + lane;
+    const uint8_t ori_l = sl < a.chr_len ? __ldg(a.ori + sl) : 0;
+    const unsigned flagged = __ballot_sync(kFull, (ori_l & 8) != 0);
+    if (site >= a.chr_len) return;
+    const uint8_t ori = (uint8_t)__shfl_sync(kFull, ori_l, w);
+    const int32_t snp_row = (ori & 8) ? a.tile_snp[tile] + __popc(flagged & ((1u << w) - 1u)) : -1;
+    const uint8_t wflags = a.win_flags[s0 / kWin];
+    const SitePileup p = deep_pileup(a, a.warp_rng[tile * 2], a.warp_rng[tile * 2 + 1], site, recs);
+    __syncwarp();
+    deep_sort(recs, p.num);
+    float s[10];
+    deep_walk_sums(a, recs, cnt, p.num, s);
+    uint8_t dflags = 0;
+    if (lane == 0) {
+        if (p.depth > 0xffff) atomicExch(a.error, 1);
+        if (wflags & kWinKeepCounts) store_counts(a, site, p);
+        SiteCall call;
+        if ((site & 4095) == 0 && a.stats) dflags = kCallSampled;
+        const bool empty = p.num == 0 && (p.ca[0] | p.ca[1] | p.ca[2] | p.ca[3]) == 0 && a.empty_valid[ori];
+        if (empty) {
+            call = a.empty_calls[ori];
+            call.depth = p.depth;
+            call.repeat_time = p.repeat;
+            call.flags |= dflags;
+        } else if (fast_posterior(a, snp_row, ori, p, s, p.num, &call, 9.0f)) {
+            call.flags |= dflags;
+        } else {
+            call = SiteCall{};
+            dflags |= kCallPending;
+            call.flags = dflags;
+        }
+        a.out[site] = call;
+    }
+    dflags = (uint8_t)__shfl_sync(kFull, dflags, 0);
+    if (!dflags) return;
+    /* the site and its sorted records to the deferred pool */
+    unsigned long long slot = 0, off = 0;
+    if (lane == 0) {
+        slot = atomicAdd(a.dcount, 1ull);
+        off = atomicAdd(a.dcount + 1, (unsigned long long)p.num);
+    }
+    slot = __shfl_sync(kFull, slot, 0);
+    off = __shfl_sync(kFull, off, 0);
+    if ((int64_t)slot >= a.dsite_cap || (int64_t)(off + p.num) > a.dpool_cap) return;
+    for (int i = lane; i < p.num; i += 32) a.dpool[off + i] = recs[i];
+    if (lane == 0) {
+        DeferredSite d;
+        d.site = site;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            d.cu[b] = (uint16_t)p.cu[b];
+            d.qs[b] = (uint16_t)p.qs[b];
+            d.ca[b] = p.ca[b];
+        }
+        d.depth = p.depth;
+        d.repeat = p.repeat;
+        d.rec_off = (uint32_t)off;
+        d.num = (uint16_t)p.num;
+        d.dep_uni = (uint16_t)p.dep_uni;
+        d.snp_row = snp_row;
+        d.flags = dflags;
+#pragma unroll
+        for (int b = 0; b < 3; ++b) d.pad[b] = 0;
+        a.dsites[slot] = d;
+    }
+}
+
+/* The tiles of a deep FP32 bin: tiles[blockIdx.x] with count == nullptr, warp
+ * w calling its site w; else the sites of the first *count tiles of the list,
+ * handed out one at a time to each warp from *next (zero before the launch),
+ * so that no warp waits for the deepest site of a tile. */
+__global__ void __launch_bounds__(kDeepThreads, 1) call_deep_kernel(CallArgs a, const int32_t* __restrict__ tiles,
+                                                                    const int* __restrict__ count, int* next) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t* recs = reinterpret_cast<uint32_t*>(smem) + (size_t)w * kDeepCap;
+    uint8_t* cnt = smem + (size_t)kTile * kDeepCap * 4 + (size_t)w * kDeepKeys;
+    if (!count) {
+        deep_tile(a, tiles[blockIdx.x], w, recs, cnt);
+        return;
+    }
+    const unsigned items = (unsigned)*count * kTile;   /* tile-list index * kTile + site */
+    unsigned item = blockIdx.x * kTile + w;
+    while (item < items) {
+        deep_tile(a, tiles[item / kTile], (int)(item % kTile), recs, cnt);
+        unsigned nx = 0;
+        if (lane == 0) nx = (unsigned)atomicAdd(next, 1) + gridDim.x * kTile;
+        item = __shfl_sync(kFull, nx, 0);
+    }
+}
+
+/* ------------------------------------------------------------------------ */
+/* the persistent FP32 calling kernel                                        */
+/* ------------------------------------------------------------------------ */
+
+/* Reads of a tile staged in shared memory by the persistent kernel, and the
+ * bytes of each read's row window (32 columns of 16-bit base|quality plus up
+ * to 14 bytes before them, to start the copy on a 16-byte boundary).  A tile
+ * with more reads than this (deep pileups) reads its rows from global memory
+ * instead. */
+constexpr int kStageReads = 56;
+constexpr int kStageSlot = 80;
+constexpr uint64_t kStageWaitNs = 1000000000ull;   /* bound on one wait for a tile's bulk copies */
+constexpr int kStageHeader = 16 + kStageReads * 12;
+/* how the persistent kernel fetches a tile's reads */
+constexpr int kStreamPlain = 0;      /* loads from global memory (through L1/L2) */
+constexpr int kStreamPrefetch = 1;   /* the same, after a bulk prefetch of the rows into L2 */
+constexpr int kStreamStaged = 2;     /* bulk copies into shared memory, one tile ahead */
+static_assert(kStageHeader % 16 == 0 && kStageSlot % 16 == 0, "staging buffers are 16-byte aligned");
+
+/* warps of a CTA of the persistent kernel: each works by itself; several share
+ * the CTA's reserved shared memory */
+constexpr int kStreamWarps = 4;
+
+/* records [slots][kTile] and the pcr state of the general form; the bins that
+ * try the short form first: its records and scratch in the same place */
+__host__ __device__ constexpr size_t call_smem_bytes(int slots, int L) {
+    const size_t general = ((size_t)slots * kTile + (size_t)pcr_smem_words(slots, L, true)) * 4;
+    const size_t lean = slots <= kLeanG ? lean_smem_bytes(slots, L) : 0;
+    return general > lean ? general : lean;
+}
+
+/* shared memory of one warp of the persistent kernel (a multiple of 16) */
+__host__ __device__ constexpr size_t stream_warp_smem(int slots, int L, int mode) {
+    const size_t n = mode != kStreamStaged ? lean_smem_bytes(slots, L)
+                                           : call_smem_bytes(slots, L) + (size_t)kStageHeader + (size_t)kStageReads * kStageSlot;
+    return (n + 15) & ~(size_t)15;
+}
+
+/* One launch over the FP32 windows' tiles of a segment: each warp takes
+ * kStreamChunk consecutive tiles at a time from a counter, so the tiles in
+ * flight are neighbours and the read rows they share are fetched from DRAM
+ * about once and then served by L2.  The grid is sized to the resident CTAs,
+ * whatever the segment's length.  A tile whose window needs the FP64 form
+ * (its likelihood is kept for, or taken from, another window), or one with a
+ * site of more than SLOTS records, is appended to the leftover list for the
+ * binned kernels instead.
+ *
+ * MODE kStreamPrefetch: as soon as a warp takes a tile, it asks the
+ * bulk-copy unit to prefetch the next tile's read rows into L2
+ * (cp.async.bulk.prefetch), which costs no shared memory.
+ * MODE kStreamStaged: as soon as a tile's pileup is done, the warp stages the
+ * next tile's reads in shared memory - their start, length and strand with plain
+ * loads, and each covering read's 32-column row window with one bulk copy
+ * (cp.async.bulk) completing on the warp's mbarrier - so that the copies run
+ * while the current tile is sorted, walked and summed, and the next pileup
+ * reads only shared memory.  A wait for the copies that does not complete
+ * within kStageWaitNs sets error code 5 and ends the warp. */
+template <int SLOTS, int MODE>
+__global__ void __launch_bounds__(32 * kStreamWarps, kFastCtasPerSm / kStreamWarps) call_stream_kernel(CallArgs a, StreamQueue q) {
+    constexpr bool STAGED = MODE == kStreamStaged;
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int t = threadIdx.x & 31;
+    uint8_t* base = smem + (threadIdx.x >> 5) * stream_warp_smem(SLOTS, a.L, MODE);
+    uint64_t* bar = nullptr;
+    int32_t* s_pos = nullptr;
+    uint32_t* s_lhs = nullptr;
+    int32_t* s_rbase = nullptr;
+    uint8_t* s_rows = nullptr;
+    if (STAGED) {
+        bar = reinterpret_cast<uint64_t*>(base);
+        s_pos = reinterpret_cast<int32_t*>(base + 16);
+        s_lhs = reinterpret_cast<uint32_t*>(s_pos + kStageReads);
+        s_rbase = reinterpret_cast<int32_t*>(s_lhs + kStageReads);
+        s_rows = base + kStageHeader;
+        base = s_rows + kStageReads * kStageSlot;
+    }
+    uint32_t* recs_all = reinterpret_cast<uint32_t*>(base);
+    uint32_t* seen_all = recs_all + SLOTS * kTile;
+    uint32_t* recs = recs_all + t;
+    uint32_t* seen = seen_all + t;
+    const int64_t n = q.t_end - q.t_begin;
+
+    /* tiles in order: kStreamChunk at a time from the counter; -1 at the end */
+    int64_t chunk_next = 0, chunk_end = 0;
+    auto next_tile = [&]() -> int64_t {
+        if (chunk_next >= chunk_end) {
+            unsigned long long first = 0;
+            if (t == 0) first = atomicAdd(q.next, (unsigned long long)kStreamChunk);
+            first = __shfl_sync(kFull, first, 0);
+            chunk_next = (int64_t)first;
+            chunk_end = min(chunk_next + (int64_t)kStreamChunk, n);
+            if (chunk_next >= n) {
+                chunk_end = 0;
+                return -1;
+            }
+        }
+        return q.t_begin + chunk_next++;
+    };
+    auto fp64_window = [&](int64_t tile) {
+        return (a.win_flags[(int)(tile * kTile / kWin)] & (kWinKeepLik | kWinExternalLik)) != 0;
+    };
+    /* stage the reads of `tile` (see above); their count, or -1 when the
+     * tile is not staged.  Every lane calls it, after its last read of the
+     * buffers. */
+    auto stage = [&](int64_t tile) -> int {
+        if (!STAGED || tile < 0 || fp64_window(tile)) return -1;
+        const int64_t r_lo = a.tile_rng[tile * 2], r_hi = a.tile_rng[tile * 2 + 1];
+        const int64_t nr = r_hi - r_lo;
+        if (nr > kStageReads) return -1;
+        const int64_t s0 = tile * kTile;
+        uint32_t bytes[2] = {0u, 0u}, total = 0;
+        const uint8_t* src[2] = {nullptr, nullptr};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int k = t + 32 * j;
+            if (k >= nr) continue;
+            const int64_t r = r_lo + k;
+            const int32_t pos = __ldg(a.pos + r);
+            const uint32_t lh = (uint32_t)__ldg(a.lenhit + r);
+            const uint32_t minus = __ldg(a.strand + r) != '+';
+            const int len = (int)(lh >> 16);
+            const int c_lo = max(0, (int)(s0 - pos));
+            const int c_hi = min(len, (int)(s0 + kTile - pos));
+            const int64_t e_lo = (r * a.L + c_lo) * 2;   /* byte offset of column c_lo in the rows */
+            const int m = (int)(e_lo & 15);
+            if (c_hi > c_lo) {
+                bytes[j] = (uint32_t)((m + 2 * (c_hi - c_lo) + 15) & ~15);
+                src[j] = reinterpret_cast<const uint8_t*>(a.bq) + (e_lo - m);
+            }
+            s_pos[k] = pos;
+            s_lhs[k] = lh | (minus << 31);
+            s_rbase[k] = k * kStageSlot + m - 2 * c_lo;
+            total += bytes[j];
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(kFull, total, off);
+        /* this lane's reads of the rows are done before the copies overwrite them */
+        fence_proxy_async_smem();
+        if (t == 0) mbar_arrive_expect_tx(bar, total);
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            if (bytes[j]) bulk_copy_g2s(s_rows + (t + 32 * j) * kStageSlot, src[j], bytes[j], bar);
+        return (int)nr;
+    };
+
+    /* the read rows of `tile` into L2 (the rows of a tile's reads are one
+     * contiguous block; the bulk unit wants 16-byte bounds, and the row
+     * array has slack past its end for the rounding) */
+    auto prefetch_l2 = [&](int64_t tile) {
+        if (MODE != kStreamPrefetch || tile < 0 || t != 0) return;
+        const int64_t r_lo = a.tile_rng[tile * 2], r_hi = a.tile_rng[tile * 2 + 1];
+        if (r_hi <= r_lo) return;
+        const uintptr_t lo = reinterpret_cast<uintptr_t>(a.bq + r_lo * a.L) & ~(uintptr_t)15;
+        const uintptr_t hi = (reinterpret_cast<uintptr_t>(a.bq + r_hi * a.L) + 15) & ~(uintptr_t)15;
+        bulk_prefetch_l2(reinterpret_cast<const void*>(lo), (uint32_t)(hi - lo));
+    };
+
+    uint32_t phase = 0;
+    if (STAGED) {
+        if (t == 0) mbar_init(bar, 1);
+        __syncwarp();
+    }
+    int64_t tile = next_tile();
+    int staged_n = stage(tile);
+    while (tile >= 0) {
+        const int64_t s0 = tile * kTile;
+        const int win = (int)(s0 / kWin);
+        const uint8_t wflags = a.win_flags[win];
+        const int64_t nxt = next_tile();
+        prefetch_l2(nxt);
+        if (wflags & (kWinKeepLik | kWinExternalLik)) {
+            if (t == 0) q.leftover[atomicAdd(q.n_leftover, 1)] = (int32_t)tile;
+            tile = nxt;
+            staged_n = stage(tile);
+            continue;
+        }
+        int staged_next = -1;
+        bool called;
+        if (STAGED) {
+            const int64_t site = s0 + t;
+            const bool active = site < a.chr_len;
+            const uint8_t ori = active ? __ldg(a.ori + site) : 0;
+            const int32_t snp_row = tile_snp_row(a, tile, (ori & 8) != 0);
+            bool overflow = false;
+            SitePileup p;
+            if (staged_n >= 0) {
+                if (!mbar_wait_bounded(bar, phase, kStageWaitNs)) {
+                    if (t == 0) atomicExch(a.error, 5);
+                    (void)mbar_wait_bounded(bar, phase, kStageWaitNs);
+                    return;
+                }
+                phase ^= 1u;
+                const StagedReads sr{s_pos, s_lhs, s_rbase, s_rows, staged_n};
+                p = warp_pileup_staged<SLOTS>(a, sr, site, active, recs, &overflow).unpack();
+            } else {
+                p = warp_pileup<SLOTS>(a, a.tile_rng[tile * 2], a.tile_rng[tile * 2 + 1], site, active, recs, &overflow)
+                        .unpack();
+            }
+            /* the staging buffers are free: stage the next tile now, so that its
+             * copies run while this one is sorted, walked and summed */
+            staged_next = stage(nxt);
+            called = !__any_sync(kFull, overflow);
+            if (called) {
+                /* one sort network for every tile: specialised networks per
+                 * tile depth made the kernel's code larger and it ran slower */
+                if (active) sort_column<SLOTS>(recs, p.num);
+                fast_site<SLOTS>(a, site, active, ori, wflags, snp_row, p, recs, seen);
+            }
+        } else {
+            called = lean_tile<SLOTS>(a, tile, a.tile_rng[tile * 2], a.tile_rng[tile * 2 + 1], wflags, recs_all, seen_all);
+        }
+        if (!called && t == 0) q.leftover[atomicAdd(q.n_leftover, 1)] = (int32_t)tile;
+        tile = nxt;
+        staged_n = staged_next;
+        __syncwarp();
+    }
+}
+
+/* ------------------------------------------------------------------------ */
+/* launchers                                                                 */
+/* ------------------------------------------------------------------------ */
+
+template <int SLOTS, int MODE>
+static cudaError_t stream_attr(int L, int* ctas_per_sm, int carveout = 0) {
+    const int smem = (int)(kStreamWarps * stream_warp_smem(SLOTS, L, MODE));
+    cudaError_t e =
+        cudaFuncSetAttribute(call_stream_kernel<SLOTS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    /* a preferred shared-memory carveout (percent; 0 leaves the default) is a
+     * hint: a refusal only costs speed, and its error is cleared */
+    if (e == cudaSuccess && carveout > 0 &&
+        cudaFuncSetAttribute(call_stream_kernel<SLOTS, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             carveout) != cudaSuccess)
+        (void)cudaGetLastError();
+    if (e == cudaSuccess && ctas_per_sm)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, call_stream_kernel<SLOTS, MODE>,
+                                                          32 * kStreamWarps, smem);
+    return e;
+}
+
+template <int SLOTS, int MODE>
+static cudaError_t launch_stream_one(const CallArgs& a, const StreamQueue& q, int ctas, int carveout,
+                                     cudaStream_t stream) {
+    cudaError_t e = g_launch_attributes ? stream_attr<SLOTS, MODE>(a.L, nullptr, carveout) : cudaSuccess;
+    if (e != cudaSuccess) return e;
+    call_stream_kernel<SLOTS, MODE>
+        <<<ctas, 32 * kStreamWarps, kStreamWarps * stream_warp_smem(SLOTS, a.L, MODE), stream>>>(a, q);
+    return cudaGetLastError();
+}
+
+template <int SLOTS>
+static cudaError_t stream_dispatch(int mode, const CallArgs* a, const StreamQueue* q, int ctas, int carveout,
+                                   cudaStream_t stream, int L, int* ctas_per_sm) {
+    if (!a) {
+        return mode == kStreamStaged     ? stream_attr<SLOTS, kStreamStaged>(L, ctas_per_sm, carveout)
+               : mode == kStreamPrefetch ? stream_attr<SLOTS, kStreamPrefetch>(L, ctas_per_sm, carveout)
+                                         : stream_attr<SLOTS, kStreamPlain>(L, ctas_per_sm, carveout);
+    }
+    return mode == kStreamStaged     ? launch_stream_one<SLOTS, kStreamStaged>(*a, *q, ctas, carveout, stream)
+           : mode == kStreamPrefetch ? launch_stream_one<SLOTS, kStreamPrefetch>(*a, *q, ctas, carveout, stream)
+                                     : launch_stream_one<SLOTS, kStreamPlain>(*a, *q, ctas, carveout, stream);
+}
+
+/* resident CTAs on one SM of the persistent kernel with `slots` record
+ * slots (48 or 64) and read mode `mode` (0 plain, 1 L2 prefetch, 2 staged
+ * in shared memory) */
+int stream_ctas_per_sm(int slots, int L, int mode, int carveout) {
+    int n = 0;
+    const cudaError_t e = slots <= 48 ? stream_dispatch<48>(mode, nullptr, nullptr, 0, carveout, nullptr, L, &n)
+                                      : stream_dispatch<64>(mode, nullptr, nullptr, 0, carveout, nullptr, L, &n);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 1;
+    }
+    return n > 0 ? n : 1;
+}
+
+/* The persistent FP32 kernel over q's tiles with `ctas` CTAs; slots is 48 or
+ * 64.  q.next and q.n_leftover must be zero. */
+cudaError_t launch_stream(const CallArgs& a, const StreamQueue& q, int slots, int mode, int ctas, int carveout,
+                          cudaStream_t stream) {
+    if (q.t_end <= q.t_begin) return cudaSuccess;
+    return slots <= 48 ? stream_dispatch<48>(mode, &a, &q, ctas, carveout, stream, a.L, nullptr)
+                       : stream_dispatch<64>(mode, &a, &q, ctas, carveout, stream, a.L, nullptr);
+}
+
+/* set the bin kernel's shared-memory size and carveout (percent; 0 leaves the
+ * default); with ctas_per_sm, its resident CTAs on one SM */
+template <int SLOTS>
+static cudaError_t fast_attr(int L, int carveout, int* ctas_per_sm) {
+    /* the deep bins run one warp per site (call_deep_kernel) */
+    constexpr bool deep = SLOTS >= kDeepSlots;
+    const int smem = deep ? (int)kDeepSmem : (int)call_smem_bytes(SLOTS, L);
+    const void* fn;
+    if constexpr (deep) fn = reinterpret_cast<const void*>(call_deep_kernel);
+    else fn = reinterpret_cast<const void*>(call_fast_kernel<SLOTS>);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    /* the carveout is a hint: a refusal only costs speed, and its error is
+     * cleared so that it is not taken for the launch's */
+    if (carveout > 0 && cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, carveout) != cudaSuccess)
+        (void)cudaGetLastError();
+    if (ctas_per_sm) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, deep ? kDeepThreads : kTile, smem);
+    return cudaSuccess;
+}
+
+template <int SLOTS>
+static cudaError_t launch_fast(const CallArgs& a, const int32_t* tiles, const BinLaunch& bl, cudaStream_t stream) {
+    cudaError_t e = g_launch_attributes ? fast_attr<SLOTS>(a.L, bl.carveout, nullptr) : cudaSuccess;
+    if (e != cudaSuccess) return e;
+    const unsigned grid = (unsigned)(bl.d_count ? bl.grid : bl.count);
+    if (grid == 0) return cudaSuccess;
+    if constexpr (SLOTS >= kDeepSlots)
+        call_deep_kernel<<<grid, kDeepThreads, kDeepSmem, stream>>>(a, tiles, bl.d_count, bl.d_next);
+    else
+        call_fast_kernel<SLOTS><<<grid, kTile, call_smem_bytes(SLOTS, a.L), stream>>>(a, tiles, bl.d_count,
+                                                                                            bl.d_next);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fast_bin(const CallArgs& a, int bin, const int32_t* tiles, const BinLaunch& bl, cudaStream_t stream) {
+    switch (bin) {
+        case 0: return launch_fast<32>(a, tiles, bl, stream);
+        case 1: return launch_fast<40>(a, tiles, bl, stream);
+        case 2: return launch_fast<48>(a, tiles, bl, stream);
+        case 3: return launch_fast<64>(a, tiles, bl, stream);
+        case 4: return launch_fast<96>(a, tiles, bl, stream);
+        case 5: return launch_fast<128>(a, tiles, bl, stream);
+        default: return launch_fast<256>(a, tiles, bl, stream);
+    }
+}
+
+cudaError_t fast_bin_attr(int bin, int L, int carveout, int* ctas_per_sm) {
+    switch (bin) {
+        case 0: return fast_attr<32>(L, carveout, ctas_per_sm);
+        case 1: return fast_attr<40>(L, carveout, ctas_per_sm);
+        case 2: return fast_attr<48>(L, carveout, ctas_per_sm);
+        case 3: return fast_attr<64>(L, carveout, ctas_per_sm);
+        case 4: return fast_attr<96>(L, carveout, ctas_per_sm);
+        case 5: return fast_attr<128>(L, carveout, ctas_per_sm);
+        default: return fast_attr<256>(L, carveout, ctas_per_sm);
+    }
+}
+
+}  // namespace gsnp

@@ -54,7 +54,7 @@ GSNP_HDI void bitonic_sort(uint32_t* v) {
  * its slot.  A write at slot k = i + (entries left) never reaches a prefix
  * record not yet moved, so no scratch is needed; v is indexed by unrolled
  * constants only, so it stays in registers. */
-template <int T>
+template <int T, int kStride = kTile>
 GSNP_HDI void merge_back(uint32_t* recs, int P, const uint32_t* v, int cnt) {
     int i = P - 1, k = P + cnt - 1;
 #pragma unroll
@@ -62,13 +62,13 @@ GSNP_HDI void merge_back(uint32_t* recs, int P, const uint32_t* v, int cnt) {
         if (j < cnt) {
             const uint32_t x = v[j];
             while (i >= 0) {
-                const uint32_t h = recs[i * kTile];
+                const uint32_t h = recs[i * kStride];
                 if (h <= x) break;
-                recs[k * kTile] = h;
+                recs[k * kStride] = h;
                 --k;
                 --i;
             }
-            recs[k * kTile] = x;
+            recs[k * kStride] = x;
             --k;
         }
     }

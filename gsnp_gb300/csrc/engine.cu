@@ -56,7 +56,6 @@ cudaError_t launch_tile_bounds(const CallArgs& a, int64_t r_begin, int64_t r_end
 cudaError_t launch_empty_calls(const CallArgs& a, SiteCall* calls, uint8_t* valid, cudaStream_t stream);
 int bin_slots(int bin);
 inline int kSlotsOf(int bin) { return bin_slots(bin); }
-int64_t bin_global_words(int kind, int bin, int64_t count);
 
 /* ---- device helpers ---- */
 
@@ -208,9 +207,8 @@ __device__ __forceinline__ uint8_t upper_base(uint8_t b, bool* bad) {
 }
 
 /* The deposited reads in the packed layout of the calling kernels: start,
- * len<<16|hit, len, strand, and the base|quality row with the bases in upper
- * case ('A' past the read's end; a base other than ACGT/acgt sets *error to
- * 2).  Rows [row_begin, row_end); a block holds rows_per_block rows, each
+ * len<<16|hit, len, strand, and the row of elements (make_elem, from the
+ * calling q_min q_call; a base other than ACGT/acgt sets *error to 2).  Rows [row_begin, row_end); a block holds rows_per_block rows, each
  * thread VEC consecutive columns of one row (VEC = 4 when L and the pitch are
  * multiples of 4 and L <= pitch: 32-bit loads, 64-bit stores).  PACKED: seq
  * holds gsnp_pack_reads's bytes (qual is not read), which give the base and
@@ -222,13 +220,18 @@ __device__ __forceinline__ uint32_t unpack_bq(uint32_t byte, int qmin) {
     return base | (q << 8);
 }
 
+/* element of a base and quality char */
+__device__ __forceinline__ uint32_t elem_of(uint32_t base_char, uint32_t qual_char, int q_call) {
+    return make_elem((base_char >> 1) & 3u, (int)(signed char)(uint8_t)qual_char - q_call);
+}
+
 template <int VEC, bool PACKED = false>
 __global__ void __launch_bounds__(256) gather_reads_kernel(
     int64_t row_begin, int64_t row_end, const int64_t* __restrict__ idx, int64_t n_raw, const int32_t* __restrict__ rpos,
     const int32_t* __restrict__ rlen, const int32_t* __restrict__ rhit, const uint8_t* __restrict__ rstrand,
     const uint8_t* __restrict__ seq, const uint8_t* __restrict__ qual, int pitch, int L, int rows_per_block,
     int32_t* __restrict__ pos, int32_t* __restrict__ lenhit, int32_t* __restrict__ len,
-    uint8_t* __restrict__ strand, uint16_t* __restrict__ bq, int* __restrict__ error, int qmin = 0) {
+    uint8_t* __restrict__ strand, uint16_t* __restrict__ bq, int* __restrict__ error, int qmin, int q_call) {
     /* kGatherRows groups of rows per block, one row of each group per thread:
      * the groups' load chains (index, length, bases and qualities) are
      * independent, so they are in flight together */
@@ -279,23 +282,30 @@ __global__ void __launch_bounds__(256) gather_reads_kernel(
             uint32_t lo = 0, hi = 0;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                uint32_t v;
-                if (PACKED) {
-                    v = c0 + k < rl[g] ? unpack_bq((s4[g] >> (8 * k)) & 0xffu, qmin) : (uint32_t)'A';
-                } else {
-                    const uint8_t b = c0 + k < rl[g] ? upper_base((uint8_t)(s4[g] >> (8 * k)), &bad) : (uint8_t)'A';
-                    v = (uint32_t)b | (((q4[g] >> (8 * k)) & 0xffu) << 8);
+                uint32_t v = kElemInvalid;
+                if (c0 + k < rl[g]) {
+                    if (PACKED) {
+                        const uint32_t u = unpack_bq((s4[g] >> (8 * k)) & 0xffu, qmin);
+                        v = elem_of(u & 0xffu, u >> 8, q_call);
+                    } else {
+                        v = elem_of(upper_base((uint8_t)(s4[g] >> (8 * k)), &bad), q4[g] >> (8 * k), q_call);
+                    }
                 }
                 if (k < 2) lo |= v << (16 * k);
                 else hi |= v << (16 * (k - 2));
             }
             *reinterpret_cast<uint2*>(bq + row * L + c0) = make_uint2(lo, hi);
-        } else if (PACKED) {
-            bq[row * L + c0] = (uint16_t)(c0 < pitch && c0 < rl[g] ? unpack_bq(s4[g] & 0xffu, qmin) : (uint32_t)'A');
-        } else {
-            uint8_t b = 'A';
-            if (c0 < pitch && c0 < rl[g]) b = upper_base((uint8_t)s4[g], &bad);
-            bq[row * L + c0] = (uint16_t)b | ((uint16_t)(c0 < pitch ? q4[g] : 0u) << 8);
+        } else if (c0 < L) {
+            uint32_t v = kElemInvalid;
+            if (c0 < pitch && c0 < rl[g]) {
+                if (PACKED) {
+                    const uint32_t u = unpack_bq(s4[g] & 0xffu, qmin);
+                    v = elem_of(u & 0xffu, u >> 8, q_call);
+                } else {
+                    v = elem_of(upper_base((uint8_t)s4[g], &bad), q4[g], q_call);
+                }
+            }
+            bq[row * L + c0] = (uint16_t)v;
         }
     }
     const unsigned any_bad = __ballot_sync(0xffffffffu, bad), any_idx = __ballot_sync(0xffffffffu, bad_idx);
@@ -307,11 +317,11 @@ cudaError_t launch_gather(bool vec4, bool packed, unsigned blocks, cudaStream_t 
                           int64_t row_end, const int64_t* idx, int64_t n_raw, const int32_t* rpos, const int32_t* rlen,
                           const int32_t* rhit, const uint8_t* rstrand, const uint8_t* seq, const uint8_t* qual,
                           int pitch, int L, int rows_per_block, int32_t* pos, int32_t* lenhit, int32_t* len,
-                          uint8_t* strand, uint16_t* bq, int* error, int qmin) {
+                          uint8_t* strand, uint16_t* bq, int* error, int qmin, int q_call) {
 #define GSNP_GATHER(V, P)                                                                                      \
     gather_reads_kernel<V, P><<<blocks, 256, 0, stream>>>(row_begin, row_end, idx, n_raw, rpos, rlen, rhit,    \
                                                           rstrand, seq, qual, pitch, L, rows_per_block, pos,  \
-                                                          lenhit, len, strand, bq, error, qmin)
+                                                          lenhit, len, strand, bq, error, qmin, q_call)
     if (vec4) {
         if (packed) GSNP_GATHER(4, true);
         else GSNP_GATHER(4, false);
@@ -430,6 +440,8 @@ struct gsnp_context {
     /* device tables */
     double* d_lik64 = nullptr;
     float* d_lik32 = nullptr;
+    uint32_t* d_lean_q = nullptr;
+    float* d_lean4 = nullptr;
     uint8_t* d_qadj = nullptr;
     double* d_p_prior = nullptr;
     double* d_log_prior = nullptr;
@@ -488,13 +500,11 @@ struct gsnp_context {
     int64_t dsite_cap = 0, dpool_cap = 0;
     int64_t* d_warp_rng = nullptr;  /* [n_tiles][2] */
     int64_t* d_tile_rng = nullptr;  /* [n_tiles][2] */
-    uint32_t* d_deep = nullptr;     /* record columns of the deep bins' CTAs */
-    int64_t deep_cap = 0;           /* words */
     /* the persistent FP32 kernel: its counters (tiles handed out, leftover
      * count), the leftover tiles, its record slots and grid */
     unsigned long long* d_stream_ctl = nullptr;
     int32_t* d_leftover = nullptr;
-    int stream_slots = 0, stream_ctas = 0, stream_ctas_L = -1, stream_carveout = 0;
+    int stream_slots = 0, stream_ctas = 0, stream_ctas_L = -1, stream_carveout = 72;
     bool stream_path = true;
     int stream_mode = 0;            /* 0 plain loads, 1 L2 bulk prefetch, 2 staged in shared memory */
     /* Device-driven calling: the bins' kernels, the classification of the
@@ -535,7 +545,12 @@ struct gsnp_context {
     int64_t columns_host_windows = 0;
     std::unique_ptr<ColumnsGpuWriter> colw;   /* kept, with its device buffers, from one use to the next */
     int bin_limit[kNumBins] = {32, 40, 48, 64, 96, 128, 256};
-    int bin_carveout[2][kNumBins] = {{0, 0, 0, 0, 0, 0, 0}, {0, 72, 0, 0, 0, 0, 0}};
+    /* preferred shared-memory carveouts: at 72% (164 KB) the FP32 kernels that
+     * use the short form keep about 20 warps an SM and leave 64 KB of L1 for
+     * its tables, whose rows are read at random.  The persistent kernel at c1
+     * (8 Mbp): 1.84 ms at 44%, 1.63 at 58%, 1.54 at 72%, 1.84 at 86% and at
+     * the default (24 warps) */
+    int bin_carveout[2][kNumBins] = {{0, 0, 0, 0, 0, 0, 0}, {0, 72, 72, 0, 0, 0, 0}};
     int bin_grid[2][kNumBins] = {};
     int grid_L = -1, deferred_grid = 0, classify_grid = 0, sms = 0;
     unsigned long long* d_dmax = nullptr;   /* [2] largest deferred request of the call's segments */
@@ -584,6 +599,13 @@ struct gsnp_context {
     uint8_t* d_map = nullptr;
     size_t map_bytes = 0;
     int64_t n_gathered = 0;        /* deposited reads in the packed layout so far */
+    /* the alignments behind the packed layout (d_raw_*) and the q_min its
+     * elements count from: recalled under another q_min, they are gathered
+     * again (regather) */
+    int64_t raw_n = 0;
+    int32_t raw_pitch = 0;
+    bool raw_packed = false;
+    int packed_qmin = 0, gather_qmin = 0;
     /* cns text emission */
     void* d_emit = nullptr;
     size_t emit_bytes = 0;
@@ -730,18 +752,21 @@ cudaError_t from_map(gsnp_context* c, size_t off, void* d_dst, size_t n) {
 }
 
 void free_all(gsnp_context* c) {
-    void* ptrs[] = {c->d_lik64, c->d_lik32, c->d_qadj, c->d_p_prior, c->d_log_prior, c->d_log_prior32,
+    void* ptrs[] = {c->d_lik64, c->d_lik32, c->d_lean_q, c->d_lean4, c->d_qadj, c->d_p_prior, c->d_log_prior, c->d_log_prior32,
                     c->d_p_rank, c->d_codes, c->d_snp, c->d_snp_lp, c->d_snp_lp32, c->d_pos, c->d_lenhit,
                     c->d_len, c->d_strand, c->d_bq, c->d_win_flags, c->d_win_lik_src, c->d_out, c->d_counts,
                     c->d_lik_keep, c->d_error, c->d_stats, c->d_bin_count, c->d_bin_tiles, c->d_dsites,
                     c->d_dpool, c->d_dcount, c->d_warp_rng, c->d_win_host_src, c->d_emit,
                     c->d_text, c->d_chr, c->d_tile_snp, c->d_tile_rng, c->d_empty_calls, c->d_empty_valid,
                     c->d_raw_pos, c->d_raw_len, c->d_raw_hit, c->d_raw_strand, c->d_raw_seq, c->d_raw_qual,
-                    c->d_idx, c->d_dep_off, c->d_gerror, c->d_deep, c->d_stream_ctl, c->d_leftover,
+                    c->d_idx, c->d_dep_off, c->d_gerror, c->d_stream_ctl, c->d_leftover,
                     c->d_dmax, c->d_patch, c->d_bin_hist};
     for (void* p : ptrs)
         if (p) cudaFree(p);
 }
+
+/* the q_min the calling kernels count qualities from: a signed char */
+int call_qmin(const gsnp_context* c) { return (int)(signed char)c->params.q_min; }
 
 CallArgs make_args(gsnp_context* c) {
     CallArgs a;
@@ -763,6 +788,9 @@ CallArgs make_args(gsnp_context* c) {
     a.lik32 = c->d_lik32;
     a.lik32b = c->d_lik32 ? c->d_lik32 + (size_t)c->tables.qa_rows * c->tables.L * 4 * 8 : nullptr;
     a.qa_rows = c->tables.qa_rows;
+    /* the short form's proof is of diploid calls */
+    a.lean_q = c->tables.lean_ok && !c->params.monoploid ? c->d_lean_q : nullptr;
+    a.lean4 = c->d_lean4;
     a.qadj = c->d_qadj;
     a.tmax = c->tables.tmax;
     a.gmax = c->tables.gmax;
@@ -911,12 +939,6 @@ int prepare_calling(gsnp_context* c) {
             c->classify_grid = c->sms * 4;
             c->grid_L = c->params.read_length;
         }
-        /* record columns of the deepest fast bin: one slice per resident CTA */
-        const int64_t words = bin_global_words(kKindFast, kNumBins - 1, c->bin_grid[1][kNumBins - 1]);
-        if (words > c->deep_cap) {
-            CK(dev_alloc(&c->d_deep, (size_t)words), "cudaMalloc deep scratch");
-            c->deep_cap = words;
-        }
     }
     return GSNP_OK;
 }
@@ -962,6 +984,11 @@ int finish_device(gsnp_context* c) {
     c->called = true;
     return GSNP_OK;
 }
+
+/* The persistent kernel calls tiles in the short form (or, with its reads
+ * staged in shared memory, in the general one); without the short form it
+ * would leave every tile. */
+bool stream_takes(const gsnp_context* c, const CallArgs& a) { return a.lean_q != nullptr || c->stream_mode == 2; }
 
 /* device-driven queueing of a calling pass (defined below) */
 int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std::function<int(size_t)>& before,
@@ -1021,29 +1048,13 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
             if (c->h_bin_count[base + b] > 0) order[m++] = b;
         std::sort(order, order + m, [&](int x, int y) { return c->h_bin_count[base + x] > c->h_bin_count[base + y]; });
         if (m == 0) return GSNP_OK;
-        /* the deep bins' record columns: a slice of the scratch per launch */
-        int64_t off[kNumBins] = {}, words = 0;
-        for (int j = 0; j < m; ++j) {
-            off[order[j]] = words;
-            words += bin_global_words(kind, order[j], c->h_bin_count[base + order[j]]);
-        }
-        if (words > c->deep_cap) {
-            CK(cudaStreamSynchronize(c->stream), "deep scratch");
-            CK(dev_alloc(&c->d_deep, (size_t)(words + words / 4)), "cudaMalloc deep scratch");
-            c->deep_cap = words + words / 4;
-        }
-        auto with_scratch = [&](int b) {
-            CallArgs la = args;
-            la.deep_recs = c->d_deep + off[b];
-            return la;
-        };
         if (!side_by_side) {
             for (int j = 0; j < m; ++j) {
                 const int b = order[j];
                 const int nb = c->h_bin_count[base + b];
                 const int k = begin(launch_kind(kind, bin_slots(b)), bin_slots(b), nb);
                 const BinLaunch bl{nb, nullptr, 0, c->bin_carveout[kind == kKindFast][b]};
-                CK(launch_bin(with_scratch(b), kind, b, c->d_bin_tiles + (int64_t)(base + b) * c->tiles_cap, bl, c->stream),
+                CK(launch_bin(args, kind, b, c->d_bin_tiles + (int64_t)(base + b) * c->tiles_cap, bl, c->stream),
                    "calling kernel");
                 end(k);
             }
@@ -1058,7 +1069,7 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
             const int nb = c->h_bin_count[base + b];
             const int k = begin_on(launch_kind(kind, bin_slots(b)), bin_slots(b), nb, st);
             const BinLaunch bl{nb, nullptr, 0, c->bin_carveout[kind == kKindFast][b]};
-            CK(launch_bin(with_scratch(b), kind, b, c->d_bin_tiles + (int64_t)(base + b) * c->tiles_cap, bl, st),
+            CK(launch_bin(args, kind, b, c->d_bin_tiles + (int64_t)(base + b) * c->tiles_cap, bl, st),
                "calling kernel");
             end_on(k, st);
         }
@@ -1079,7 +1090,8 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
         /* In the FP32 form the persistent kernel calls the segment's tiles;
          * the binned kernels take only the tiles it leaves (the FP64 windows'
          * and those with a site deeper than its record slots). */
-        const bool use_stream = c->stream_path && c->params.precision == 1 && segs.size() == 1 && !c->view.on;
+        const bool use_stream =
+            c->stream_path && c->params.precision == 1 && segs.size() == 1 && !c->view.on && stream_takes(c, a);
         int64_t n_left = 0;
         auto run_stream = [&](const CallArgs& as) -> int {
             CK(cudaMemsetAsync(c->d_stream_ctl, 0, 2 * sizeof(unsigned long long), c->stream), "memset");
@@ -1216,7 +1228,7 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
      * (or chunks) ends each segment's launch of it in a tail of its own, and
      * its binned kernels, handing out tiles from counters, were the faster
      * there (c1 e2e in 7 segments: 28.6-29.0 against 29.9 ms) */
-    const bool use_stream = c->stream_path && fast && segs.size() == 1 && !c->view.on;
+    const bool use_stream = c->stream_path && fast && segs.size() == 1 && !c->view.on && stream_takes(c, make_args(c));
     int* d_left = reinterpret_cast<int*>(c->d_stream_ctl + 1);
     /* With several segments the deferred sites of all of them go to one pool
      * and one deferred pass runs after the last segment: the pass takes about
@@ -1230,7 +1242,6 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
     auto deferred_pass = [&]() -> int {
         CallArgs a = make_args(c);
         a.n_reads = c->n_gathered;
-        a.deep_recs = c->d_deep;
         const int kd = begin(kKindDeferred, 0, 0);
         CK(launch_deferred(a, 0, c->stream, c->d_dcount, c->deferred_grid), "deferred calling kernel");
         end(kd);
@@ -1253,16 +1264,16 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
         }
         CallArgs a = make_args(c);
         a.n_reads = c->n_gathered;
-        a.deep_recs = c->d_deep;
         int k = begin(kKindClassify, 0, g.t1 - g.t0);
         CK(launch_tile_bounds(a, g.dlo, g.dhi, g.next_pos, c->stream), "tile bounds kernel");
         if (!defer_to_end) CK(cudaMemsetAsync(c->d_dcount, 0, sizeof(unsigned long long) * 2, c->stream), "memset");
         auto bins = [&](int kind, int pass) -> int {
             const int ki = kind == kKindFast ? 1 : 0;
             for (int b = 0; b < kNumBins; ++b) {
-                /* after the persistent kernel, the fast bins get only tiles
-                 * deeper than its record slots */
-                if (kind == kKindFast && use_stream && kSlotsOf(b) <= c->stream_slots) continue;
+                /* after the persistent kernel in the general form (staged
+                 * reads), the fast bins get only tiles deeper than its record
+                 * slots; the short form leaves shallow tiles too */
+                if (kind == kKindFast && use_stream && c->stream_mode == 2 && kSlotsOf(b) <= c->stream_slots) continue;
                 const BinLaunch bl{0, c->d_bin_count + ki * kNumBins + b, c->bin_grid[ki][b], c->bin_carveout[ki][b],
                                    c->d_bin_count + (2 + ki) * kNumBins + b};
                 const int kb = begin(launch_kind(kind, kSlotsOf(b)), kSlotsOf(b), 0);
@@ -1386,6 +1397,35 @@ std::vector<Segment> plan_segments(const gsnp_context* c, const ReadView& r, int
         if (g.t1 > g.t0 || w1 == P.n_windows) segs.push_back(g);
     }
     return segs;
+}
+
+/* Columns a gather thread takes (VEC of gather_reads_kernel), and the rows of
+ * a block at one group. */
+struct GatherShape {
+    bool vec4;
+    int rows_per_block;
+    GatherShape(int L, int pitch)
+        : vec4(L % 4 == 0 && pitch % 4 == 0 && L <= pitch),
+          rows_per_block(std::max(1, 256 / (vec4 ? L / 4 : L))) {}
+    unsigned blocks(int64_t rows) const {
+        const int64_t per_block = (int64_t)rows_per_block * kGatherRows;
+        return (unsigned)((rows + per_block - 1) / per_block);
+    }
+};
+
+/* The resident reads' elements count qualities from the q_min they were
+ * gathered under; gather them again when the tables have another one. */
+int regather(gsnp_context* c) {
+    if (c->gather_qmin == call_qmin(c) || c->n_dep == 0) return GSNP_OK;
+    const int L = c->params.read_length;
+    const GatherShape gs(L, c->raw_pitch);
+    CK(launch_gather(gs.vec4, c->raw_packed, gs.blocks(c->n_dep), c->stream, 0, c->n_dep, c->d_idx, c->raw_n,
+                     c->d_raw_pos, c->d_raw_len, c->d_raw_hit, c->d_raw_strand, c->d_raw_seq, c->d_raw_qual,
+                     c->raw_pitch, L, gs.rows_per_block, c->d_pos, c->d_lenhit, c->d_len, c->d_strand, c->d_bq,
+                     c->d_gerror, c->packed_qmin, call_qmin(c)),
+       "gather kernel");
+    c->gather_qmin = call_qmin(c);
+    return GSNP_OK;
 }
 
 /* number of segments of a call: one per two million deposited reads, 1 .. 16
@@ -1575,6 +1615,11 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
     }
     c->n_dep = nd;
     c->n_gathered = 0;
+    c->raw_n = n;
+    c->raw_pitch = r->pitch;
+    c->raw_packed = r->packed != nullptr;
+    c->packed_qmin = r->packed_qmin;
+    c->gather_qmin = call_qmin(c);
     c->h2d_bytes = (uint64_t)P.n_windows * 9 + (uint64_t)n * (4 + 4 + 4 + 1) +
                    (r->packed ? 1ULL : 2ULL) * (uint64_t)n * r->pitch;
     c->d2h_bytes = out ? (uint64_t)c->chr_len * sizeof(SiteCall) : 0;
@@ -1606,9 +1651,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
         CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         c->ev_gather.push_back(e);
     }
-    const bool vec4 = L % 4 == 0 && r->pitch % 4 == 0 && L <= r->pitch;
-    const int per_row = vec4 ? L / 4 : L;
-    const int rows_per_block = std::max(1, 256 / per_row);
+    const GatherShape gs(L, r->pitch);
     int64_t gathered_seg = -1, waited_chunk = -1;
     auto gather_through = [&](int64_t target) -> int {
         while (gathered_seg < target) {
@@ -1619,13 +1662,10 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
                  * (the pieces of several copy streams finish in any order) */
                 for (; waited_chunk < chunk; ++waited_chunk)
                     CK(cudaStreamWaitEvent(c->gather_stream, c->ev_chunk[waited_chunk + 1], 0), "wait");
-                const int64_t rows = g.dhi - g.dlo;
-                const int64_t per_block = (int64_t)rows_per_block * kGatherRows;
-                const unsigned blocks = (unsigned)((rows + per_block - 1) / per_block);
-                CK(launch_gather(vec4, r->packed != nullptr, blocks, c->gather_stream, g.dlo, g.dhi, c->d_idx, n,
+                CK(launch_gather(gs.vec4, r->packed != nullptr, gs.blocks(g.dhi - g.dlo), c->gather_stream, g.dlo, g.dhi, c->d_idx, n,
                                  c->d_raw_pos, c->d_raw_len, c->d_raw_hit, c->d_raw_strand, c->d_raw_seq,
-                                 c->d_raw_qual, r->pitch, L, rows_per_block, c->d_pos, c->d_lenhit, c->d_len,
-                                 c->d_strand, c->d_bq, c->d_gerror, c->params.q_min),
+                                 c->d_raw_qual, r->pitch, L, gs.rows_per_block, c->d_pos, c->d_lenhit, c->d_len,
+                                 c->d_strand, c->d_bq, c->d_gerror, c->params.q_min, call_qmin(c)),
                    "gather kernel");
                 CK(cudaGetLastError(), "gather kernel");
             }
@@ -1866,6 +1906,8 @@ int gsnp_load_tables(gsnp_context* c, const gsnp_params* p, const double* p_matr
     const HostTables& t = c->tables;
     CK(dev_alloc(&c->d_lik64, t.lik64.size()), "cudaMalloc");
     CK(dev_alloc(&c->d_lik32, t.lik32.size()), "cudaMalloc");
+    CK(dev_alloc(&c->d_lean_q, t.lean_q.size()), "cudaMalloc");
+    CK(dev_alloc(&c->d_lean4, t.lean4.size()), "cudaMalloc");
     CK(dev_alloc(&c->d_qadj, t.qadj.size()), "cudaMalloc");
     CK(dev_alloc(&c->d_p_prior, 128), "cudaMalloc");
     CK(dev_alloc(&c->d_log_prior, 128), "cudaMalloc");
@@ -1873,6 +1915,8 @@ int gsnp_load_tables(gsnp_context* c, const gsnp_params* p, const double* p_matr
     CK(dev_alloc(&c->d_p_rank, 64UL * 64UL * 2048UL), "cudaMalloc");
     CK(cudaMemcpy(c->d_lik64, t.lik64.data(), t.lik64.size() * 8, cudaMemcpyHostToDevice), "upload");
     CK(cudaMemcpy(c->d_lik32, t.lik32.data(), t.lik32.size() * 4, cudaMemcpyHostToDevice), "upload");
+    CK(cudaMemcpy(c->d_lean_q, t.lean_q.data(), t.lean_q.size() * 4, cudaMemcpyHostToDevice), "upload");
+    CK(cudaMemcpy(c->d_lean4, t.lean4.data(), t.lean4.size() * 4, cudaMemcpyHostToDevice), "upload");
     CK(cudaMemcpy(c->d_qadj, t.qadj.data(), t.qadj.size(), cudaMemcpyHostToDevice), "upload");
     CK(cudaMemcpy(c->d_p_prior, p_prior, 128 * 8, cudaMemcpyHostToDevice), "upload");
     CK(cudaMemcpy(c->d_log_prior, t.log_prior.data(), 128 * 8, cudaMemcpyHostToDevice), "upload");
@@ -2036,7 +2080,7 @@ uint64_t graph_key_of(gsnp_context* c, const Segment& g) {
     mix(c->bin_grid, sizeof c->bin_grid);
     mix(c->bin_carveout, sizeof c->bin_carveout);
     mix(&c->n_gathered, sizeof c->n_gathered);
-    const void* ptrs[] = {c->d_deep, c->d_leftover, c->d_stream_ctl, c->d_dmax, c->d_bin_tiles, c->d_bin_count};
+    const void* ptrs[] = {c->d_leftover, c->d_stream_ctl, c->d_dmax, c->d_bin_tiles, c->d_bin_count};
     mix(ptrs, sizeof ptrs);
     return h;
 }
@@ -2269,6 +2313,10 @@ int gsnp_tune(gsnp_context* c, int sample_windows, char* report, size_t report_c
 int gsnp_recall_resident(gsnp_context* c) {
     if (!c || !c->have_tables || c->plan.n_windows == 0) return fail(c, GSNP_ERR_STATE, "nothing resident");
     cudaSetDevice(c->device);
+    {
+        const int rg = regather(c);
+        if (rg != GSNP_OK) return rg;
+    }
     int rc = c->device_driven && c->use_graphs ? recall_graph(c) : run_calling(c, {whole_segment(c)}, nullptr, nullptr);
     /* the deferred pool was grown to what the pass asked for: run it again */
     if (rc == kRedoDeferred) rc = run_calling(c, {whole_segment(c)}, nullptr, nullptr);
@@ -2798,9 +2846,7 @@ int call_streamed(gsnp_context* c, const gsnp_reads* r, const char* chr_name, gs
     for (auto& s : g->slot) CK(cudaEventRecord(s.free, c->stream), "event");
     if (nk > 0) rc = upload(0);
     uint64_t totals[kNumStats] = {};
-    const bool vec4 = L % 4 == 0 && r->pitch % 4 == 0 && L <= r->pitch;
-    const int per_row = vec4 ? L / 4 : L;
-    const int rows_per_block = std::max(1, 256 / per_row);
+    const GatherShape gs(L, r->pitch);
     for (size_t k = 0; k < nk && rc == GSNP_OK; ++k) {
         if (k + 1 < nk) {
             rc = upload(k + 1);
@@ -2837,11 +2883,9 @@ int call_streamed(gsnp_context* c, const gsnp_reads* r, const char* chr_name, gs
             dep_index_kernel<<<(unsigned)n_chunks, kDepThreads, 0, c->stream>>>(nraw, s.raw_pos, s.raw_len,
                                                                                 c->chr_len, s.dep_off, nd, s.idx);
             CK(cudaGetLastError(), "index kernels");
-            const int64_t per_block = (int64_t)rows_per_block * kGatherRows;
-            const unsigned blocks = (unsigned)((nd + per_block - 1) / per_block);
-            CK(launch_gather(vec4, r->packed != nullptr, blocks, c->stream, 0, nd, s.idx, nraw, s.raw_pos, s.raw_len,
-                             s.raw_hit, s.raw_strand, s.raw_seq, s.raw_qual, r->pitch, L, rows_per_block, s.pos,
-                             s.lenhit, s.len, s.strand, s.bq, c->d_gerror, c->params.q_min),
+            CK(launch_gather(gs.vec4, r->packed != nullptr, gs.blocks(nd), c->stream, 0, nd, s.idx, nraw, s.raw_pos, s.raw_len,
+                             s.raw_hit, s.raw_strand, s.raw_seq, s.raw_qual, r->pitch, L, gs.rows_per_block, s.pos,
+                             s.lenhit, s.len, s.strand, s.bq, c->d_gerror, c->params.q_min, call_qmin(c)),
                "gather kernel");
         }
         if (carry_c[k] >= 0) CK(cudaMemcpyAsync(g->counts, g->carry_counts, sizeof(SiteCounts) * kWin,

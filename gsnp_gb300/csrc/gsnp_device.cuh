@@ -31,11 +31,12 @@ constexpr int kWin = 262144;            /* window size, cpp/common.h:16 */
 constexpr int kMaxRecords = 255;        /* dep_uni cap, kernel/update_kernel.cu:288 */
 constexpr int kMaxQ = 64;               /* MAX_QSCORE */
 
-GSNP_HDI uint32_t make_record(int base_char, int q, uint32_t coord_val,
-                                                         uint32_t strand_val) {
-    const uint32_t prefix = ((uint32_t)((base_char & 0x6) >> 1) << 15) | ((uint32_t)(kMaxQ - q) << 9) |
-                            (coord_val << 1) | strand_val;
+GSNP_HDI uint32_t make_record_of(uint32_t base, int q, uint32_t coord_val, uint32_t strand_val) {
+    const uint32_t prefix = (base << 15) | ((uint32_t)(kMaxQ - q) << 9) | (coord_val << 1) | strand_val;
     return (prefix << 8) | 1u;
+}
+GSNP_HDI uint32_t make_record(int base_char, int q, uint32_t coord_val, uint32_t strand_val) {
+    return make_record_of((uint32_t)((base_char & 0x6) >> 1), q, coord_val, strand_val);
 }
 
 GSNP_HDI int rec_base(uint32_t w) { return (int)((w & 0x01800000u) >> 23); }
@@ -43,6 +44,22 @@ GSNP_HDI int rec_q(uint32_t w) { return kMaxQ - (int)((w & 0x007e0000u) >> 17); 
 GSNP_HDI int rec_coord(uint32_t w) { return (int)((w & 0x0001fe00u) >> 9); }
 GSNP_HDI int rec_strand(uint32_t w) { return (int)((w & 0x00000100u) >> 8); }
 GSNP_HDI int rec_occ(uint32_t w) { return (int)(w & 0xffu); }
+
+/* A base and its quality in a packed read row (16 bits).  q = quality char -
+ * q_min:
+ *   1 <= q <= 63   base << 6 | (64 - q): bits 24:17 of its record word
+ *   other q >= 0   kElemWide | base << 8 | q
+ *   q < 0          kElemInvalid: never part of a pileup (nor are columns past
+ *                  the read's end) */
+constexpr uint32_t kElemInvalid = 0x8000u, kElemWide = 0x4000u;
+
+GSNP_HDI uint32_t make_elem(uint32_t base, int q) {
+    if (q < 0) return kElemInvalid;
+    return q >= 1 && q <= 63 ? base << 6 | (uint32_t)(kMaxQ - q) : kElemWide | base << 8 | (uint32_t)q;
+}
+GSNP_HDI bool elem_valid(uint32_t e) { return (e & kElemInvalid) == 0; }
+GSNP_HDI int elem_base(uint32_t e) { return (int)((e & kElemWide ? e >> 8 : e >> 6) & 3u); }
+GSNP_HDI int elem_q(uint32_t e) { return e & kElemWide ? (int)(e & 0xffu) : kMaxQ - (int)(e & 63u); }
 
 /* genotype code (a1 << 2 | a2) of table column t, a1 <= a2 in ACTG order */
 GSNP_HDI int genotype_of(int t) {

@@ -245,7 +245,7 @@ __device__ __forceinline__ double normal_test(int n1, int n2, double T1, double 
 }
 
 /* Wilcoxon rank-sum p-value of a heterozygous call (kernel/posterior_kernel.cu:506-572) */
-__device__ __noinline__ double rank_test(const double* p_rank, int q_max_min, const uint32_t* recs, int stride,
+static __device__ __noinline__ double rank_test(const double* p_rank, int q_max_min, const uint32_t* recs, int stride,
                                          int num, const int* cu, int bt, bool* normal_path) {
     const int ia = bt & 3, ib = (bt >> 2) & 3;
     if (ia == ib) return 1.0;
@@ -357,6 +357,18 @@ __device__ __forceinline__ void fill_call(SiteCall* out, const SitePileup& p, co
     c.repeat_time = p.repeat;
     c.rank_sum = rs;
     *out = c;
+}
+
+/* A call as the two 16-byte words it is stored in. */
+struct CallWords {
+    uint4 a, b;
+};
+__device__ __forceinline__ CallWords call_words(const SiteCall& c) {
+    const uint64_t rs = (uint64_t)__double_as_longlong(c.rank_sum);
+    return CallWords{{(uint32_t)c.type1 | (uint32_t)c.base1 << 8 | (uint32_t)c.base2 << 16 | (uint32_t)c.q_cns << 24,
+                      (uint32_t)c.avg_q1 | (uint32_t)c.avg_q2 << 8 | (uint32_t)c.flags << 16,
+                      (uint32_t)c.cu1 | (uint32_t)c.ca1 << 16, (uint32_t)c.cu2 | (uint32_t)c.ca2 << 16},
+                     {c.depth, c.repeat_time, (uint32_t)rs, (uint32_t)(rs >> 32)}};
 }
 
 __device__ __forceinline__ bool same_call(const SiteCall& x, const SiteCall& y) {
@@ -472,52 +484,52 @@ __device__ bool site_posterior(const CallArgs& a, uint8_t ori, const SitePileup&
     return true;
 }
 
-/* The FP32 posterior of the fast kernel, for sites whose best genotype is
- * homozygous (the rank-sum value is then 1 and its log10 0).  s holds the FP32
- * likelihood sums by table column, num the record count, and
- * k_units u + num 2^-45 (u = 2^-24) their relative error bound: 6 for the
- * grouping of likelihood_fp32, 9 for the warp form of the deep kernel (per-
- * lane compensated sums, then a tree of 32).  Returns false, writing
- * nothing, when the best genotype is heterozygous or when the FP32 values do
- * not prove the FP64 decisions.
+/* first (i = 0) and second base of table column t */
+GSNP_HDI int col_base(int t, int i) { return i == 0 ? genotype_of(t) >> 2 : genotype_of(t) & 3; }
+
+/* FP32 log10 priors of a site by table column */
+__device__ __forceinline__ void load_log_prior32(const CallArgs& a, int64_t snp_row, uint8_t ori, float* lp) {
+    const float* src = a.log_prior32 + (ori & 7) * 12;
+    if ((ori & 0x8) && a.refine) src = a.snp_lp32 + snp_row * 12;
+    const float4* s4 = reinterpret_cast<const float4*>(src);
+    const float4 x0 = GSNP_LDG(s4), x1 = GSNP_LDG(s4 + 1), x2 = GSNP_LDG(s4 + 2);
+    lp[0] = x0.x; lp[1] = x0.y; lp[2] = x0.z; lp[3] = x0.w;
+    lp[4] = x1.x; lp[5] = x1.y; lp[6] = x1.z; lp[7] = x1.w;
+    lp[8] = x2.x; lp[9] = x2.y;
+}
+
+/* Error bound of tp = s + lp for an FP32 sum s of num records within k_units
+ * u + num 2^-45 (u = 2^-24) of the FP64 one: |s - S64| <= |s| k; the prior's
+ * rounding <= 2^-24 |lp|; the addition's <= 2^-24 |tp| <= 2^-24 (|s| + |lp|);
+ * grown by 2^-20 for the rounding of the bound itself. */
+__device__ __forceinline__ float fast_error_factor(float k_units, int num) {
+    return __fadd_rn(__fadd_rn(k_units * 0x1p-24f, __fmul_rn((float)num, 0x1p-45f)), 0x1p-23f);
+}
+__device__ __forceinline__ float fast_error(float mag, float lp, float kk) {
+    const float grow = 1.0f + 0x1p-20f;
+    return __fmul_rn(__fadd_rn(__fmul_rn(mag, kk), __fmul_rn(fabsf(lp), 0x1p-22f)), grow);
+}
+
+/* The proof of a homozygous call from FP32 values tp[t] (by table column)
+ * within E[t] of the FP64 ones.  Returns false, writing nothing, when the best genotype is
+ * heterozygous or when the values do not prove the FP64 decisions.
  *
- * E_g bounds |tp32[g] - tp64[g]| (the likelihood bound, the FP32 rounding of
- * the prior and of the addition).  With v1 = tp32[type1], v2 the largest
- * other tp32 (genotype g2), d = v1 - v2 and B = max over the others of
- * tp32[g] - v2 + E_g:
+ * With v1 = tp[type1], v2 the largest other tp (genotype g2),
+ * d = v1 - v2 and B = max over all others of tp[g] - v2 + E_g:
  *   tp64[type1] - max(other tp64) lies in [d - E1 - B, d + E1 + E_g2],
  * so type1 is the FP64 best when d > E1 + B, and the truncated, clamped
  * quality is proven when it is the same at both ends of that interval.
  * Every quantity is formed as a difference first, so that each FP32 rounding
  * is relative to these small values; the bounds are then grown to cover
  * those roundings. */
-__device__ __forceinline__ bool fast_posterior(const CallArgs& a, int64_t snp_row, uint8_t ori, const SitePileup& p,
-                                               const float* s, int num, SiteCall* out, float k_units = 6.0f) {
-    const int ori7 = ori & 7;
-    const float* src = a.log_prior32 + ori7 * 12;
-    if ((ori & 0x8) && a.refine) src = a.snp_lp32 + snp_row * 12;
-    float lp[10];
-    {
-        const float4* s4 = reinterpret_cast<const float4*>(src);
-        const float4 x0 = __ldg(s4), x1 = __ldg(s4 + 1), x2 = __ldg(s4 + 2);
-        lp[0] = x0.x; lp[1] = x0.y; lp[2] = x0.z; lp[3] = x0.w;
-        lp[4] = x1.x; lp[5] = x1.y; lp[6] = x1.z; lp[7] = x1.w;
-        lp[8] = x2.x; lp[9] = x2.y;
-    }
-    /* |s - S64| <= |s| k; the prior's rounding <= 2^-24 |lp|; the addition's
-     * <= 2^-24 |tp| <= 2^-24 (|s| + |lp|); grown by 2^-20 for the rounding of
-     * the bound itself */
-    const float kk1 = __fadd_rn(__fadd_rn(k_units * 0x1p-24f, __fmul_rn((float)num, 0x1p-45f)), 0x1p-23f);
+__device__ __forceinline__ bool prove_hom(const CallArgs& a, const SitePileup& p, int ori7, const float* tp, const float* E,
+                                          SiteCall* out) {
     const float grow = 1.0f + 0x1p-20f;
-    float tp[10], E[10];
     int t1 = -1;
     float v1 = 0.f;
 #pragma unroll
     for (int t = 0; t < 10; ++t) {
-        const int g = genotype_of(t);
-        tp[t] = __fadd_rn(s[t], lp[t]);
-        E[t] = __fmul_rn(__fadd_rn(__fmul_rn(fabsf(s[t]), kk1), __fmul_rn(fabsf(lp[t]), 0x1p-22f)), grow);
-        if (a.monoploid && (g >> 2) != (g & 3)) continue;
+        if (a.monoploid && col_base(t, 0) != col_base(t, 1)) continue;
         if (t1 < 0 || tp[t] >= v1) { t1 = t; v1 = tp[t]; }
     }
     const int g1 = genotype_of(t1);
@@ -525,8 +537,7 @@ __device__ __forceinline__ bool fast_posterior(const CallArgs& a, int64_t snp_ro
     float e1 = 0.f, v2 = -INFINITY, e2 = 0.f, emax = 0.f;
 #pragma unroll
     for (int t = 0; t < 10; ++t) {
-        const int g = genotype_of(t);
-        if (a.monoploid && (g >> 2) != (g & 3)) continue;
+        if (a.monoploid && col_base(t, 0) != col_base(t, 1)) continue;
         if (t == t1) {
             e1 = E[t];
             continue;
@@ -537,8 +548,7 @@ __device__ __forceinline__ bool fast_posterior(const CallArgs& a, int64_t snp_ro
     float B = 0.f;
 #pragma unroll
     for (int t = 0; t < 10; ++t) {
-        const int g = genotype_of(t);
-        if ((a.monoploid && (g >> 2) != (g & 3)) || t == t1) continue;
+        if ((a.monoploid && col_base(t, 0) != col_base(t, 1)) || t == t1) continue;
         B = fmaxf(B, __fadd_rn(__fsub_rn(tp[t], v2), E[t]));
     }
     /* |fl(tp - v2 + E) - (tp - v2 + E)| <= 2^-23 (|tp - v2| + E) <= 2^-22 E at
@@ -557,6 +567,26 @@ __device__ __forceinline__ bool fast_posterior(const CallArgs& a, int64_t snp_ro
     if (q != finalize_q(__float2int_rz(__fadd_rn(raw_hi, slack)), true, false, tb, g1)) return false;
     fill_call(out, p, tb, g1, q, false, 1.0);
     return true;
+}
+
+/* The FP32 posterior of the fast kernel, for sites whose best genotype is
+ * homozygous (the rank-sum value is then 1 and its log10 0).  s holds the FP32
+ * likelihood sums by table column, num the record count, and
+ * k_units u + num 2^-45 (u = 2^-24) their relative error bound: 6 for the
+ * grouping of likelihood_fp32, 9 for the warp form of the deep kernel (per-
+ * lane compensated sums, then a tree of 32). */
+__device__ __forceinline__ bool fast_posterior(const CallArgs& a, int64_t snp_row, uint8_t ori, const SitePileup& p,
+                                               const float* s, int num, SiteCall* out, float k_units = 6.0f) {
+    float lp[10];
+    load_log_prior32(a, snp_row, ori, lp);
+    const float kk1 = fast_error_factor(k_units, num);
+    float tp[10], E[10];
+#pragma unroll
+    for (int t = 0; t < 10; ++t) {
+        tp[t] = __fadd_rn(s[t], lp[t]);
+        E[t] = fast_error(fabsf(s[t]), lp[t], kk1);
+    }
+    return prove_hom(a, p, ori & 7, tp, E, out);
 }
 
 }  // namespace gsnp
