@@ -26,14 +26,14 @@
  * Two calling kernels share this structure:
  *   call_tiles_kernel  FP64 sums in the reference's order (the plain form, and
  *                      windows whose likelihood another window reuses);
- *   call_fast_kernel   FP32 compensated sums and an FP32 posterior for
+ *   call_fast_kernel   (calling_fast.cu) FP32 compensated sums and an FP32 posterior for
  *                      homozygous calls that the error bound proves; every
  *                      other site is deferred: its counts and sorted records
  *                      are appended to a small pool.  It runs no FP64
  *                      instruction.
- *   deferred_sites_kernel  one thread per deferred site: the FP32 sums again
- *                      with the double-precision bound checks, the FP64 sums
- *                      where those fail, the rank-sum test.
+ *   deferred_sites_kernel  (deferred.cu) the deferred sites: the FP32 sums
+ *                      again with the double-precision bound checks, the FP64
+ *                      sums where those fail, the rank-sum test.
  * Tiles are binned by their deepest site (kNumBins record-slot capacities) so
  * that shared memory is sized for the tile, not for the worst case.
  */
@@ -249,7 +249,7 @@ __global__ void snp_log_prior_kernel(CallArgs a, double* out, float* out32) {
                 } else {
                     pr = GSNP_DMUL(GSNP_DMUL((a1 == a2 ? 1.0 : GSNP_DMUL(2.0, a.het_val)), e.freq[a1]), e.freq[a2]);
                 }
-                lp[(a1 << 2) | a2] = gsnp_cr_log10(pr);
+                lp[(a1 << 2) | a2] = cr_log10(pr);
             }
     }
     for (int i = 0; i < 16; ++i) out[k * 16 + i] = lp[i];
@@ -328,191 +328,6 @@ __global__ void __launch_bounds__(kTile, kFp64CtasPerSm) call_tiles_kernel(CallA
         return;
     }
     for_each_listed(count, next, [&](int i) { fp64_tile<SLOTS>(a, tiles[i], recs_all, seen_all); });
-}
-
-/* The adjusted-quality table index of every record of a sorted column whose
- * records have occurrence 1 (the deferred pool's), or -1 where q_adj is 1:
- * walk_records' counts with BITS per key, without its table loads, so that
- * the loads can be issued many at a time afterwards. */
-template <int BITS>
-__device__ void walk_qidx(const CallArgs& a, const uint32_t* recs, uint32_t* seen, int num, int* qidx) {
-    constexpr int kPer = 32 / BITS;
-    constexpr uint32_t kMax = (1u << BITS) - 1u;
-    const int L = a.L;
-    const int nw = pcr_words(L, BITS);
-    const bool sat_exact = BITS == 4 && a.tmax <= 16;
-    int gdc = -1, last_o = -1, gstart = 0;
-    for (int i = 0; i < num; ++i) {
-        const uint32_t w = recs[i];
-        const int o = rec_base(w);
-        const int key = rec_strand(w) * L + rec_coord(w);
-        if (o != last_o) {
-            for (int k = 0; k < nw; ++k) seen[k] = 0u;
-            gstart = i;
-            gdc = -1;
-            last_o = o;
-        }
-        uint32_t* cw = seen + key / kPer;
-        const int sh = (key % kPer) * BITS;
-        const uint32_t word = *cw;
-        const uint32_t cnt = (word >> sh) & kMax;
-        int tmp = (int)cnt;
-        if (cnt == kMax && !sat_exact) {
-            tmp = 0;
-            for (int j = gstart; j < i; ++j)
-                if (((recs[j] ^ w) & 0x1ff00u) == 0) tmp += 1;
-        }
-        if (cnt != kMax) *cw = (word & ~(kMax << sh)) | ((cnt + 1u) << sh);
-        if (tmp == 0) gdc += 1;
-        tmp++;
-        qidx[i] = (tmp < a.tmax && gdc < a.gmax) ? (tmp * a.gmax + gdc) * 65 + rec_q(w) : -1;
-    }
-}
-
-/* adjusted quality of record i from walk_qidx's index */
-__device__ __forceinline__ int qa_of(const CallArgs& a, const int* qidx, int i) {
-    return qidx[i] >= 0 ? (int)__ldg(a.qadj + qidx[i]) : 1;
-}
-
-/* likelihood_fp32's sums from walk_qidx's indices: four records' loads at a
- * time, added in the same grouping ((x0 + x1) + (x2 + x3)) and compensation,
- * so the values are those of likelihood_fp32 and of the fast kernels */
-__device__ void deferred_fp32(const CallArgs& a, const uint32_t* recs, const int* qidx, int num, double* tl,
-                              double* eps) {
-    Kahan10 k;
-    k.init();
-    for (int i = 0; i < num; i += 4) {
-        int qa[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) qa[u] = i + u < num ? qa_of(a, qidx, i + u) : 1;
-        float x[10], y[10];
-        lik32_row(a, qa[0], rec_coord(recs[i]), rec_base(recs[i]), x);
-        if (i + 1 < num) {
-            lik32_row(a, qa[1], rec_coord(recs[i + 1]), rec_base(recs[i + 1]), y);
-#pragma unroll
-            for (int v = 0; v < 10; ++v) x[v] = __fadd_rn(x[v], y[v]);
-        }
-        if (i + 2 < num) {
-            float z[10];
-            lik32_row(a, qa[2], rec_coord(recs[i + 2]), rec_base(recs[i + 2]), y);
-            if (i + 3 < num) {
-                lik32_row(a, qa[3], rec_coord(recs[i + 3]), rec_base(recs[i + 3]), z);
-#pragma unroll
-                for (int v = 0; v < 10; ++v) y[v] = __fadd_rn(y[v], z[v]);
-            }
-#pragma unroll
-            for (int v = 0; v < 10; ++v) x[v] = __fadd_rn(x[v], y[v]);
-        }
-        k.add(x);
-    }
-    const double kk = GSNP_FP32_K(num);
-#pragma unroll
-    for (int i = 0; i < 10; ++i) {
-        const int g = genotype_of(i);
-        tl[g] = (double)k.s[i];
-        eps[g] = isinf(tl[g]) ? 0.0 : fabs(tl[g]) * kk;
-    }
-}
-
-/* likelihood_fp64's sums from walk_qidx's indices: four records' rows loaded
- * together, their terms added record by record in the reference's order */
-__device__ void deferred_fp64(const CallArgs& a, const uint32_t* recs, const int* qidx, int num, double* tl) {
-    double s[10];
-#pragma unroll
-    for (int v = 0; v < 10; ++v) s[v] = 0.0;
-    for (int i = 0; i < num; i += 4) {
-        double2 r[4][5];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (i + u < num) {
-                const uint32_t w = recs[i + u];
-                const double2* row = reinterpret_cast<const double2*>(
-                    a.lik64 + ((size_t)(qa_of(a, qidx, i + u) * a.L + rec_coord(w)) * 4 + rec_base(w)) * 10);
-#pragma unroll
-                for (int v = 0; v < 5; ++v) r[u][v] = __ldg(row + v);
-            }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (i + u < num) {
-#pragma unroll
-                for (int v = 0; v < 5; ++v) {
-                    s[2 * v] = GSNP_DADD(s[2 * v], r[u][v].x);
-                    s[2 * v + 1] = GSNP_DADD(s[2 * v + 1], r[u][v].y);
-                }
-            }
-    }
-#pragma unroll
-    for (int i = 0; i < 10; ++i) tl[genotype_of(i)] = s[i];
-}
-
-/* The FP64 pass over the deferred sites, one thread per site: the FP32 sums
- * again (the same pairing, hence the same values) with the double-precision
- * bound checks, then the FP64 sums where those fail.  Sampled sites also get
- * the FP64 sums for the accuracy figure, and when the fast kernel had decided
- * them its call is compared with this one. */
-__device__ __forceinline__ void deferred_site(const CallArgs& a, int64_t i);
-
-/* n sites, or with d_n the count the fast kernels requested (a.dcount[0]),
- * at most the pool's capacity, each thread taking every (grid)-th site */
-__global__ void __launch_bounds__(32) deferred_sites_kernel(CallArgs a, int64_t n, const unsigned long long* d_n) {
-    if (d_n) n = (int64_t)min(*d_n, (unsigned long long)a.dsite_cap);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        deferred_site(a, i);
-}
-
-__device__ __forceinline__ void deferred_site(const CallArgs& a, int64_t i) {
-    const DeferredSite d = a.dsites[i];
-    const int64_t site = d.site;
-    const uint32_t* recs = a.dpool + d.rec_off;
-    uint32_t seen[64];   /* 4-bit pcr counts of 2L <= 510 keys (walk_records) */
-    SitePileup p;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-        p.cu[b] = d.cu[b];
-        p.qs[b] = d.qs[b];
-        p.ca[b] = d.ca[b];
-    }
-    p.depth = d.depth;
-    p.repeat = d.repeat;
-    p.dep_uni = d.dep_uni;
-    p.num = d.num;
-    double tl[16], eps[16];
-#pragma unroll
-    for (int g = 0; g < 16; ++g) { tl[g] = 0.0; eps[g] = 0.0; }
-    /* the walk's table indices once, then the sums with their loads batched */
-    int qidx[256];
-    walk_qidx<4>(a, recs, seen, p.num, qidx);
-    deferred_fp32(a, recs, qidx, p.num, tl, eps);
-    if (d.flags & kCallSampled) {
-        double t64[16];
-#pragma unroll
-        for (int g = 0; g < 16; ++g) t64[g] = 0.0;
-        deferred_fp64(a, recs, qidx, p.num, t64);
-        double m = 0.0;
-#pragma unroll
-        for (int g = 0; g < 16; ++g) m = fmax(m, fabs(t64[g] - tl[g]));
-        atomicMax(a.stats + 3, (unsigned long long)__double_as_longlong(m));
-        atomicAdd(a.stats + 2, 1ull);
-    }
-    const uint8_t ori = __ldg(a.ori + site);
-    double lp[16];
-    load_log_prior(a, d.snp_row, ori, lp);
-    auto nq = [&](int b) { return neighbour_qsum(a, site, b); };
-    SiteCall call;
-    if (!site_posterior<true>(a, ori, p, tl, eps, lp, recs, 1, nq, &call)) {
-        /* FP64 fixup: the FP32 likelihood is too close to a decision boundary */
-        deferred_fp64(a, recs, qidx, p.num, tl);
-        site_posterior<true>(a, ori, p, tl, nullptr, lp, recs, 1, nq, &call);
-        call.flags |= kCallFixup;
-        atomicAdd(a.stats + 1, 1ull);
-    }
-    if (d.flags & kCallPending) {
-        atomicAdd(a.stats + 4, 1ull);
-    } else if (!same_call(a.out[site], call)) {
-        /* a sampled site the fast kernel decided differs from the FP64 call */
-        atomicAdd(a.stats + 5, 1ull);
-    }
-    a.out[site] = call;
 }
 
 /* ------------------------------------------------------------------------ */
@@ -604,19 +419,6 @@ int bin_ctas_per_sm(int kind, int bin, int L, int carveout) {
         return 1;
     }
     return n > 0 ? n : 1;
-}
-
-/* The FP64 pass over n deferred sites, or with d_n over the count the fast
- * kernels requested (read on the device) with a fixed grid of `grid` CTAs. */
-cudaError_t launch_deferred(const CallArgs& a, int64_t n, cudaStream_t stream, const unsigned long long* d_n,
-                            int grid) {
-    if (!d_n && n <= 0) return cudaSuccess;
-    /* one warp per CTA: the deferred sites are few and each is a long serial
-     * computation, so they are spread over as many SMs as possible */
-    const unsigned blocks = d_n ? (unsigned)grid : (unsigned)((n + 31) / 32);
-    if (blocks == 0) return cudaSuccess;
-    deferred_sites_kernel<<<blocks, 32, 0, stream>>>(a, n, d_n);
-    return cudaGetLastError();
 }
 
 int bin_slots(int bin) { return kSlots[bin]; }

@@ -49,6 +49,7 @@ cudaError_t launch_bin(const CallArgs& a, int kind, int bin, const int32_t* tile
 int bin_ctas_per_sm(int kind, int bin, int L, int carveout);
 void set_launch_attributes(bool on);
 cudaError_t launch_snp_log_prior(const CallArgs& a, double* out, float* out32, cudaStream_t stream);
+int deferred_ctas_per_sm();
 cudaError_t launch_deferred(const CallArgs& a, int64_t n, cudaStream_t stream,
                             const unsigned long long* d_n = nullptr, int grid = 0);
 cudaError_t launch_tile_bounds(const CallArgs& a, int64_t r_begin, int64_t r_end, int64_t next_pos,
@@ -437,7 +438,9 @@ struct gsnp_context {
     gsnp_params params{};
     bool have_tables = false;
     HostTables tables;
-    /* device tables */
+    /* device tables: parts of one buffer (d_tables), but for d_p_rank */
+    uint8_t* d_tables = nullptr;
+    size_t tables_bytes = 0;
     double* d_lik64 = nullptr;
     float* d_lik32 = nullptr;
     uint32_t* d_lean_q = nullptr;
@@ -752,8 +755,7 @@ cudaError_t from_map(gsnp_context* c, size_t off, void* d_dst, size_t n) {
 }
 
 void free_all(gsnp_context* c) {
-    void* ptrs[] = {c->d_lik64, c->d_lik32, c->d_lean_q, c->d_lean4, c->d_qadj, c->d_p_prior, c->d_log_prior, c->d_log_prior32,
-                    c->d_p_rank, c->d_codes, c->d_snp, c->d_snp_lp, c->d_snp_lp32, c->d_pos, c->d_lenhit,
+    void* ptrs[] = {c->d_tables, c->d_p_rank, c->d_codes, c->d_snp, c->d_snp_lp, c->d_snp_lp32, c->d_pos, c->d_lenhit,
                     c->d_len, c->d_strand, c->d_bq, c->d_win_flags, c->d_win_lik_src, c->d_out, c->d_counts,
                     c->d_lik_keep, c->d_error, c->d_stats, c->d_bin_count, c->d_bin_tiles, c->d_dsites,
                     c->d_dpool, c->d_dcount, c->d_warp_rng, c->d_win_host_src, c->d_emit,
@@ -935,7 +937,7 @@ int prepare_calling(gsnp_context* c) {
                 for (int b = 0; b < kNumBins; ++b)
                     c->bin_grid[kind][b] = c->sms * bin_ctas_per_sm(kind == 0 ? kKindFP64 : kKindFast, b,
                                                                    c->params.read_length, c->bin_carveout[kind][b]);
-            c->deferred_grid = c->sms * 32;
+            c->deferred_grid = c->sms * deferred_ctas_per_sm();
             c->classify_grid = c->sms * 4;
             c->grid_L = c->params.read_length;
         }
@@ -1156,7 +1158,7 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
                     if (ns > 0) {
                         const int kd = begin(kKindDeferred, 0, (ns + kTile - 1) / kTile);
                         if (kd >= 0) c->launches[kd].sites = ns;
-                        CK(launch_deferred(af, ns, c->stream), "deferred calling kernel");
+                        CK(launch_deferred(af, ns, c->stream, nullptr, 1 << 16), "deferred calling kernel");
                         end(kd);
                     }
                     break;
@@ -1904,23 +1906,37 @@ int gsnp_load_tables(gsnp_context* c, const gsnp_params* p, const double* p_matr
     std::string err;
     if (build_tables(*p, p_matrix, p_prior, &c->tables, &err) != 0) return fail(c, GSNP_ERR_ARG, err);
     const HostTables& t = c->tables;
-    CK(dev_alloc(&c->d_lik64, t.lik64.size()), "cudaMalloc");
-    CK(dev_alloc(&c->d_lik32, t.lik32.size()), "cudaMalloc");
-    CK(dev_alloc(&c->d_lean_q, t.lean_q.size()), "cudaMalloc");
-    CK(dev_alloc(&c->d_lean4, t.lean4.size()), "cudaMalloc");
-    CK(dev_alloc(&c->d_qadj, t.qadj.size()), "cudaMalloc");
-    CK(dev_alloc(&c->d_p_prior, 128), "cudaMalloc");
-    CK(dev_alloc(&c->d_log_prior, 128), "cudaMalloc");
-    CK(dev_alloc(&c->d_log_prior32, 96), "cudaMalloc");
-    CK(dev_alloc(&c->d_p_rank, 64UL * 64UL * 2048UL), "cudaMalloc");
-    CK(cudaMemcpy(c->d_lik64, t.lik64.data(), t.lik64.size() * 8, cudaMemcpyHostToDevice), "upload");
-    CK(cudaMemcpy(c->d_lik32, t.lik32.data(), t.lik32.size() * 4, cudaMemcpyHostToDevice), "upload");
-    CK(cudaMemcpy(c->d_lean_q, t.lean_q.data(), t.lean_q.size() * 4, cudaMemcpyHostToDevice), "upload");
-    CK(cudaMemcpy(c->d_lean4, t.lean4.data(), t.lean4.size() * 4, cudaMemcpyHostToDevice), "upload");
-    CK(cudaMemcpy(c->d_qadj, t.qadj.data(), t.qadj.size(), cudaMemcpyHostToDevice), "upload");
-    CK(cudaMemcpy(c->d_p_prior, p_prior, 128 * 8, cudaMemcpyHostToDevice), "upload");
-    CK(cudaMemcpy(c->d_log_prior, t.log_prior.data(), 128 * 8, cudaMemcpyHostToDevice), "upload");
-    CK(cudaMemcpy(c->d_log_prior32, t.log_prior32.data(), 96 * 4, cudaMemcpyHostToDevice), "upload");
+    /* one device buffer and one copy for all of them: an allocation and a
+     * pageable copy each took longer than building the tables */
+    struct Part {
+        void** dst;
+        const void* src;
+        size_t bytes, at;
+    };
+    Part parts[] = {{(void**)&c->d_lik64, t.lik64.data(), t.lik64.size() * 8, 0},
+                    {(void**)&c->d_lik32, t.lik32.data(), t.lik32.size() * 4, 0},
+                    {(void**)&c->d_lean_q, t.lean_q.data(), t.lean_q.size() * 4, 0},
+                    {(void**)&c->d_lean4, t.lean4.data(), t.lean4.size() * 4, 0},
+                    {(void**)&c->d_qadj, t.qadj.data(), t.qadj.size(), 0},
+                    {(void**)&c->d_p_prior, p_prior, 128 * 8, 0},
+                    {(void**)&c->d_log_prior, t.log_prior.data(), 128 * 8, 0},
+                    {(void**)&c->d_log_prior32, t.log_prior32.data(), 96 * 4, 0}};
+    size_t total = 0;
+    for (Part& q : parts) {
+        q.at = total;
+        total += (q.bytes + 255) & ~(size_t)255;
+    }
+    std::vector<uint8_t> blob(total);
+    for (const Part& q : parts) memcpy(blob.data() + q.at, q.src, q.bytes);
+    if (total > c->tables_bytes) {
+        c->have_tables = false;
+        c->tables_bytes = 0;
+        CK(dev_alloc(&c->d_tables, total), "cudaMalloc tables");
+        c->tables_bytes = total;
+    }
+    for (const Part& q : parts) *q.dst = c->d_tables + q.at;
+    if (!c->d_p_rank) CK(dev_alloc(&c->d_p_rank, 64UL * 64UL * 2048UL), "cudaMalloc");
+    CK(cudaMemcpy(c->d_tables, blob.data(), total, cudaMemcpyHostToDevice), "upload");
     CK(cudaMemcpy(c->d_p_rank, p_rank, 64UL * 64UL * 2048UL * 8, cudaMemcpyHostToDevice), "upload");
     c->have_tables = true;
     c->snp_lp_ready = false;

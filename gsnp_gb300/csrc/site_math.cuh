@@ -43,6 +43,16 @@ static inline T __ldg(const T* p) { return *p; }
 
 namespace gsnp {
 
+/* the correctly rounded functions, out of line on the device: their double-
+ * double code is long and most sites do not reach it */
+#if defined(__CUDACC__)
+static __device__ __noinline__ double cr_log10(double x) { return gsnp_cr_log10(x); }
+static __device__ __noinline__ double cr_exp(double x) { return gsnp_cr_exp(x); }
+#else
+static inline double cr_log10(double x) { return gsnp_cr_log10(x); }
+static inline double cr_exp(double x) { return gsnp_cr_exp(x); }
+#endif
+
 /* SiteCall.flags */
 constexpr uint8_t kCallFixup = 1;    /* the FP32 likelihood was recomputed in FP64 */
 constexpr uint8_t kCallNormal = 2;   /* the rank-sum took the normal approximation */
@@ -226,7 +236,7 @@ __device__ __forceinline__ double normal_value(double z) {
     const double aa = fabs(z);
     const double t = GSNP_DDIV(1.0, GSNP_DADD(1.0, GSNP_DMUL(aa, p)));
     /* z / 2 is computed as z * 0.5: halving is exact, so the value is the same */
-    const double b = GSNP_DMUL(c2, gsnp_cr_exp(GSNP_DMUL(-z, GSNP_DMUL(z, 0.5))));
+    const double b = GSNP_DMUL(c2, cr_exp(GSNP_DMUL(-z, GSNP_DMUL(z, 0.5))));
     double n = GSNP_DADD(GSNP_DMUL(b5, t), b4);
     n = GSNP_DADD(GSNP_DMUL(n, t), b3);
     n = GSNP_DADD(GSNP_DMUL(n, t), b2);
@@ -242,6 +252,14 @@ __device__ __forceinline__ double normal_test(int n1, int n2, double T1, double 
     const double u1 = GSNP_DDIV(GSNP_DSUB(T1, (double)(n1 * (n1 + n2 + 1) / 2)), sd);
     const double u2 = GSNP_DDIV(GSNP_DSUB(T2, (double)(n2 * (n1 + n2 + 1) / 2)), sd);
     return normal_value(fabs(u1) > fabs(u2) ? u1 : u2);
+}
+
+/* p-value of the rank sums Ta, Tb of n1 and n2 records */
+__device__ __forceinline__ double rank_value(const double* p_rank, int n1, int n2, double Ta, double Tb,
+                                             bool* normal_path) {
+    if (n1 + n2 < 64) return table_test(p_rank, n1, n2, Ta, Tb);
+    *normal_path = true;
+    return normal_test(n1, n2, Ta, Tb);
 }
 
 /* Wilcoxon rank-sum p-value of a heterozygous call (kernel/posterior_kernel.cu:506-572) */
@@ -273,10 +291,7 @@ static __device__ __noinline__ double rank_test(const double* p_rank, int q_max_
         Tb = GSNP_DADD(Tb, GSNP_DMUL(ra, (double)cb[q]));
         rank += c;
     }
-    const int n1 = cu[ia], n2 = cu[ib];
-    if (n1 + n2 < 64) return table_test(p_rank, n1, n2, Ta, Tb);
-    *normal_path = true;
-    return normal_test(n1, n2, Ta, Tb);
+    return rank_value(p_rank, cu[ia], cu[ib], Ta, Tb, normal_path);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -399,48 +414,47 @@ __device__ __forceinline__ void load_log_prior(const CallArgs& a, int64_t snp_ro
  * type_likely[g]|; the function then returns false, writing nothing, unless
  * every decision it makes (the genotype order behind type1/type2 and the
  * truncated, clamped consensus quality) is provably the one the FP64 values
- * give.  nq(b) is q_sum[b] of the next site, which the reference reads when
- * base1/base2 name an N reference base. */
-template <bool FAST_LOG = false, class NQ>
-__device__ bool site_posterior(const CallArgs& a, uint8_t ori, const SitePileup& p, const double* tl,
-                               const double* eps, const double* lp, const uint32_t* recs, int stride, NQ&& nq,
-                               SiteCall* out) {
+ * give.  rank(g, &normal) is rank_test's value for genotype g; nq(b) is
+ * q_sum[b] of the next site, which the reference reads when base1/base2 name
+ * an N reference base. */
+template <bool FAST_LOG, class NQ, class RANK>
+__device__ __forceinline__ bool site_posterior_ranked(const CallArgs& a, uint8_t ori, const SitePileup& p,
+                                                      const double* tl, const double* eps, const double* lp,
+                                                      RANK&& rank, NQ&& nq, SiteCall* out) {
     const TopBases tb = top_bases(p, ori & 7);
+    /* rolled loops over the ten genotypes in code order: sites that come here
+     * are few (or their kernel is bound by its FP64 sums), and the short code
+     * is fetched cold */
     double tp[17];
-#pragma unroll
+    GSNP_ROLLED
     for (int i = 0; i < 17; ++i) tp[i] = 0.0;
     int type1 = 16, type2 = 16;
-#pragma unroll
-    for (int a1 = 0; a1 != 4; ++a1)
-#pragma unroll
-        for (int a2 = a1; a2 != 4; ++a2) {
-            const int g = a1 << 2 | a2;
-            if (a.monoploid && a1 != a2) continue;
-            tp[g] = GSNP_DADD(tl[g], lp[g]);
-            if (tp[g] >= tp[type1] || type1 == 16) { type2 = type1; type1 = g; }
-            else if (tp[g] >= tp[type2] || type2 == 16) { type2 = g; }
-        }
+    GSNP_ROLLED
+    for (int g = 0; g < 16; ++g) {
+        const int a1 = g >> 2, a2 = g & 3;
+        if (a1 > a2 || (a.monoploid && a1 != a2)) continue;
+        tp[g] = GSNP_DADD(tl[g], lp[g]);
+        if (tp[g] >= tp[type1] || type1 == 16) { type2 = type1; type1 = g; }
+        else if (tp[g] >= tp[type2] || type2 == 16) { type2 = g; }
+    }
     double ep[16];
     if (eps) {
         /* bound of |tp - tp_FP64|: the likelihood bound plus the rounding of the
          * prior addition; exact (0) where the likelihood is exact */
-#pragma unroll
+        GSNP_ROLLED
         for (int g = 0; g < 16; ++g)
             ep[g] = eps[g] == 0.0 ? 0.0 : eps[g] + 0x1p-51 * (fabs(tl[g]) + fabs(lp[g])) + 0x1p-1000;
-#pragma unroll
-        for (int a1 = 0; a1 != 4; ++a1)
-#pragma unroll
-            for (int a2 = a1; a2 != 4; ++a2) {
-                const int g = a1 << 2 | a2;
-                if ((a.monoploid && a1 != a2) || g == type1) continue;
-                if (ep[g] + ep[type1] > 0.0 && !(tp[type1] - tp[g] > ep[g] + ep[type1])) return false;
-                if (g == type2) continue;
-                if (ep[g] + ep[type2] > 0.0 && !(tp[type2] - tp[g] > ep[g] + ep[type2])) return false;
-            }
+        GSNP_ROLLED
+        for (int g = 0; g < 16; ++g) {
+            const int a1 = g >> 2, a2 = g & 3;
+            if (a1 > a2 || (a.monoploid && a1 != a2) || g == type1) continue;
+            if (ep[g] + ep[type1] > 0.0 && !(tp[type1] - tp[g] > ep[g] + ep[type1])) return false;
+            if (g == type2) continue;
+            if (ep[g] + ep[type2] > 0.0 && !(tp[type2] - tp[g] > ep[g] + ep[type2])) return false;
+        }
     }
     bool normal_path = false;
-    const double rs =
-        a.rank_sum ? rank_test(a.p_rank, a.q_max_min, recs, stride, p.num, p.cu, type1, &normal_path) : 1.0;
+    const double rs = a.rank_sum ? rank(type1, &normal_path) : 1.0;
     const bool hom = (type1 & 3) == ((type1 >> 2) & 3);
     bool het_ok = false;
     if (!hom) {
@@ -463,7 +477,7 @@ __device__ bool site_posterior(const CallArgs& a, uint8_t ori, const SitePileup&
          * error of raw.  The correctly rounded log10 is evaluated only when
          * raw +- dl could change the truncated, clamped quality. */
         const bool approx = FAST_LOG && rs != 1.0;
-        double lg = approx ? log10(rs) : gsnp_cr_log10(rs);
+        double lg = rs == 1.0 ? 0.0 : approx ? log10(rs) : cr_log10(rs);
         double raw = GSNP_DADD(d, GSNP_DMUL(10.0, lg));
         const double dl = approx ? 10.0 * fabs(lg) * 0x1p-40 + 0x1p-48 * (fabs(raw) + 1.0) : 0.0;
         q = finalize_q((int)raw, hom, het_ok, tb, type1);
@@ -475,13 +489,24 @@ __device__ bool site_posterior(const CallArgs& a, uint8_t ori, const SitePileup&
                 return false;
         } else if (approx && finalize_q((int)(raw - dl), hom, het_ok, tb, type1) !=
                                  finalize_q((int)(raw + dl), hom, het_ok, tb, type1)) {
-            lg = gsnp_cr_log10(rs);
+            lg = cr_log10(rs);
             raw = GSNP_DADD(d, GSNP_DMUL(10.0, lg));
             q = finalize_q((int)raw, hom, het_ok, tb, type1);
         }
     }
     fill_call(out, p, tb, type1, q, normal_path, rs);
     return true;
+}
+
+/* the same with the rank-sum test over the site's records */
+template <bool FAST_LOG = false, class NQ>
+__device__ bool site_posterior(const CallArgs& a, uint8_t ori, const SitePileup& p, const double* tl,
+                               const double* eps, const double* lp, const uint32_t* recs, int stride, NQ&& nq,
+                               SiteCall* out) {
+    auto rank = [&](int g, bool* normal) {
+        return rank_test(a.p_rank, a.q_max_min, recs, stride, p.num, p.cu, g, normal);
+    };
+    return site_posterior_ranked<FAST_LOG>(a, ori, p, tl, eps, lp, rank, nq, out);
 }
 
 /* first (i = 0) and second base of table column t */

@@ -150,7 +150,7 @@ __device__ __forceinline__ void store_counts(const CallArgs& a, int64_t site, co
  * called: every deposited read covering site + 1, except that at the last
  * site of a window the next entry is the window's tail, which holds only the
  * reads starting inside the window (kernel/update_kernel.cu:260-325). */
-static __device__ int neighbour_qsum(const CallArgs& a, int64_t site, int b) {
+static __device__ __noinline__ int neighbour_qsum(const CallArgs& a, int64_t site, int b) {
     const int64_t p = site + 1;
     const int64_t win_end = (site / kWin + 1) * (int64_t)kWin;
     const int64_t max_start = (p == win_end) ? win_end - 1 : p;

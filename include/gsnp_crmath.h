@@ -31,8 +31,12 @@
 
 #if defined(__CUDACC__)
 #define GSNP_HD __host__ __device__ __forceinline__
+/* the device evaluates these functions rarely: rolled loops keep their code,
+ * fetched cold, short */
+#define GSNP_ROLLED _Pragma("unroll 1")
 #else
 #define GSNP_HD static inline
+#define GSNP_ROLLED
 #endif
 
 #if defined(__CUDA_ARCH__)
@@ -183,8 +187,9 @@ GSNP_HD double gsnp_cr_exp(double x) {
     r = gsnp_dd_sub(r, gsnp_dd_make(GSNP_DMUL(kd, GSNP_LN2_C), 0.0));
     /* r' = r / 2^10, |r'| < 3.4e-4; expm1(r') by its Taylor series to degree 9 */
     gsnp_dd rp = gsnp_dd_make(GSNP_DMUL(r.hi, 0x1p-10), GSNP_DMUL(r.lo, 0x1p-10));
-    const double inv_n[10][2] = GSNP_INV_N_COEF;
+    static const double inv_n[10][2] = GSNP_INV_N_COEF;
     gsnp_dd s = gsnp_dd_make(1.0, 0.0);
+    GSNP_ROLLED
     for (int n = 9; n >= 2; --n) {
         /* s = 1 + r'/n * s */
         s = gsnp_dd_mul(s, rp);
@@ -193,6 +198,7 @@ GSNP_HD double gsnp_cr_exp(double x) {
     }
     s = gsnp_dd_mul(s, rp); /* expm1(r') */
     /* expm1(2y) = 2 expm1(y) + expm1(y)^2, applied 10 times */
+    GSNP_ROLLED
     for (int i = 0; i < 10; ++i) {
         gsnp_dd sq = gsnp_dd_mul(s, s);
         s = gsnp_dd_add(gsnp_dd_make(GSNP_DMUL(s.hi, 2.0), GSNP_DMUL(s.lo, 2.0)), sq);
@@ -225,8 +231,9 @@ GSNP_HD double gsnp_cr_log10(double x) {
     gsnp_dd den = gsnp_two_sum(m, 1.0);
     gsnp_dd s = gsnp_dd_div(num, den);
     gsnp_dd s2 = gsnp_dd_mul(s, s);
-    const double coef[22][2] = GSNP_ATANH_COEF;
+    static const double coef[22][2] = GSNP_ATANH_COEF;
     gsnp_dd acc = gsnp_dd_make(coef[21][0], coef[21][1]);
+    GSNP_ROLLED
     for (int k = 20; k >= 0; --k) {
         acc = gsnp_dd_mul(acc, s2);
         acc = gsnp_dd_add(acc, gsnp_dd_make(coef[k][0], coef[k][1]));
