@@ -40,6 +40,9 @@
 #include <cuda_runtime.h>
 
 #include "calling.cuh"
+#include "lean.cuh"
+#include "lean_tables.cuh"
+#include "lean_tile.cuh"
 #include "site_math.cuh"
 #include "tile.cuh"
 
@@ -50,6 +53,9 @@ namespace {
 /* resident CTAs per SM the FP64 kernel is compiled for, which caps its
  * registers at 128 */
 constexpr int kFp64CtasPerSm = 16 * 32 / kTile;
+/* warps an SM the persistent FP64 kernel is compiled for (c1, 4 Mbp: 1.49 ms at
+ * 16, 1.37 at 20, 1.35 at 24) */
+constexpr int kStream64Warps = 24;
 
 __device__ __forceinline__ int lower_bound_s(const int32_t* a, int n, int64_t v) {
     int lo = 0, hi = n;
@@ -262,9 +268,118 @@ cudaError_t launch_snp_log_prior(const CallArgs& a, double* out, float* out32, c
     return cudaGetLastError();
 }
 
+/* the short form's tables, once per table load */
+__global__ void lean_tables_kernel(const double* lik64, const uint8_t* qadj, int tmax, int gmax, int qa_rows, int L,
+                                   const int8_t* gap, uint32_t* lean_q, float4* lean4, double2* lean2d) {
+    const int64_t step = (int64_t)gridDim.x * blockDim.x, first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t i = first; i < kLeanQ; i += step) lean_q[i] = lean_q_entry(qadj, tmax, gmax, L, gap, i);
+    for (int64_t i = first; i < lean4_rows(qa_rows, L); i += step) {
+        float v[4];
+        lean4_row(lik64, qa_rows, L, i, v);
+        lean4[i] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+    for (int64_t i = first; i < lean2d_rows(qa_rows, L); i += step) {
+        double v[2];
+        lean2d_row(lik64, qa_rows, L, i, v);
+        lean2d[i] = make_double2(v[0], v[1]);
+    }
+}
+
+cudaError_t launch_lean_tables(const double* lik64, const uint8_t* qadj, int tmax, int gmax, int qa_rows, int L,
+                               const int8_t* gap, uint32_t* lean_q, float* lean4, double* lean2d, cudaStream_t stream) {
+    lean_tables_kernel<<<256, 256, 0, stream>>>(lik64, qadj, tmax, gmax, qa_rows, L, gap, lean_q,
+                                                reinterpret_cast<float4*>(lean4), reinterpret_cast<double2*>(lean2d));
+    return cudaGetLastError();
+}
+
 /* ------------------------------------------------------------------------ */
 /* the FP64 calling kernel                                                   */
 /* ------------------------------------------------------------------------ */
+
+/* A site of a tile in the short form that needs all ten genotypes (its best is
+ * not (maj, maj), or the bounds do not name the second): the sums in the
+ * reference's order over its walked column, then the general posterior.  Out of
+ * line: about one site in a thousand comes here.  The column becomes record
+ * words, which the rank-sum test reads. */
+static __device__ __noinline__ void lean_general64(const CallArgs& a, int64_t site, uint8_t ori, int32_t snp_row,
+                                                   LeanPile pile, uint32_t cu4, uint64_t qs4, uint32_t* recs) {
+    LeanSums z;
+    z.cu4 = cu4;
+    z.qs4 = qs4;
+    const SitePileup p = lean_counts(pile, z);
+    double s[10];
+#pragma unroll
+    for (int v = 0; v < 10; ++v) s[v] = 0.0;
+    for (int i = 0; i < pile.num; ++i) {
+        const uint32_t w = recs[i * kTile];
+        const double2* row = reinterpret_cast<const double2*>(
+            a.lik64 + ((size_t)lean_qa(w) * a.L + ((w >> 16) & 0xffu)) * 40 + (w >> 30) * 10);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+            const double2 x = __ldg(row + v);
+            s[2 * v] = GSNP_DADD(s[2 * v], x.x);
+            s[2 * v + 1] = GSNP_DADD(s[2 * v + 1], x.y);
+        }
+        recs[i * kTile] = lean_to_record(w);
+    }
+    double tl[16], lp[16];
+#pragma unroll
+    for (int g = 0; g < 16; ++g) tl[g] = 0.0;
+#pragma unroll
+    for (int v = 0; v < 10; ++v) tl[genotype_of(v)] = s[v];
+    load_log_prior(a, snp_row, ori, lp);
+    auto nq = [&](int b) { return neighbour_qsum(a, site, b); };
+    SiteCall call;
+    site_posterior<true>(a, ori, p, tl, nullptr, lp, recs, kTile, nq, &call);
+    a.out[site] = call;
+}
+
+/* A tile in the short form (lean.cuh) with FP64 sums; every lane of the warp
+ * calls it.  False (for the warp, nothing written) when lean_pileup leaves it.
+ *
+ * The FP64 pipe bounds the FP64 form (an FP64 instruction of a warp takes 16
+ * cycles of the SM's pipe): the short form adds two terms a record instead of
+ * ten, those of the best genotype and of the second, which FP32 sums with
+ * their bounds name beforehand on the idle FP32 pipes.  c1, 4 Mbp: 3.2 ms in
+ * the general form, 1.73 with four FP64 sums (73% of the FP64 pipe), 1.35 with
+ * two (44%). */
+template <int SLOTS>
+__device__ __forceinline__ bool lean_tile64(const CallArgs& a, int64_t tile, int64_t r_lo, int64_t r_hi, uint8_t wflags,
+                                            uint32_t* recs_all, uint32_t* scratch) {
+    const int t = threadIdx.x & 31;
+    const int64_t s0 = tile * kTile, site = s0 + t;
+    const bool active = site < a.chr_len;
+    uint32_t* recs = recs_all + t;
+    LeanPile pile;
+    if (!lean_columns<SLOTS>(a, s0, r_lo, r_hi, recs_all, scratch, &pile)) return false;
+    const uint8_t ori = active ? __ldg(a.ori + site) : 0;
+    const int32_t snp_row = tile_snp_row(a, tile, (ori & 8) != 0);
+    LeanSums z;
+    lean_walk<kTile, true>(a, recs, pile.num, ori & 3, &z);
+    if (active) {
+        if (wflags & kWinKeepCounts) store_counts(a, site, lean_counts(pile, z));
+        CallWords call;
+        bool decided = true;
+        if (pile.num == 0 && pile.extra4 == 0 && a.empty_valid[ori]) {
+            /* no record and no count: the call depends on the site code only */
+            const uint4* src = reinterpret_cast<const uint4*>(a.empty_calls + ori);
+            call.a = __ldg(src);
+            call.b = __ldg(src + 1);
+            call.b.x = pile.depth;
+            call.b.y = pile.repeat;
+        } else {
+            decided = lean_posterior64<kTile>(a, snp_row, ori, pile, z, recs, &call);
+        }
+        if (decided) {
+            uint4* dst = reinterpret_cast<uint4*>(a.out + site);
+            dst[0] = call.a;
+            dst[1] = call.b;
+        } else {
+            lean_general64(a, site, ori, snp_row, pile, z.cu4, z.qs4, recs);
+        }
+    }
+    return true;
+}
 
 /* One tile of the FP64 kernel; every lane of the warp calls it. */
 template <int SLOTS>
@@ -275,6 +390,12 @@ __device__ __forceinline__ void fp64_tile(const CallArgs& a, int64_t tile, uint3
     const uint8_t wflags = a.win_flags[win];
     const int64_t r_lo = a.warp_rng[tile * 2];
     const int64_t r_hi = a.warp_rng[tile * 2 + 1];
+    if constexpr (SLOTS <= kLeanG) {
+        if (a.lean_q && !(wflags & (kWinKeepLik | kWinExternalLik)) &&
+            lean_tile64<lean_slots(SLOTS)>(a, tile, r_lo, r_hi, wflags, recs_all, recs_all + lean_slots(SLOTS) * kTile))
+            return;
+        __syncwarp();
+    }
     const int64_t site = s0 + t;
     const bool active = site < a.chr_len;
     const uint8_t ori = active ? __ldg(a.ori + site) : 0;
@@ -309,7 +430,7 @@ __device__ __forceinline__ void fp64_tile(const CallArgs& a, int64_t tile, uint3
     load_log_prior(a, snp_row, ori, lp);
     auto nq = [&](int b) { return neighbour_qsum(a, site, b); };
     SiteCall call;
-    site_posterior(a, ori, p, tl, nullptr, lp, recs, kTile, nq, &call);
+    site_posterior<true>(a, ori, p, tl, nullptr, lp, recs, kTile, nq, &call);
     a.out[site] = call;
 }
 
@@ -318,8 +439,9 @@ __device__ __forceinline__ void fp64_tile(const CallArgs& a, int64_t tile, uint3
  * for_each_listed (a grid sized to the resident CTAs, whatever the count the
  * device holds). */
 template <int SLOTS>
-__global__ void __launch_bounds__(kTile, kFp64CtasPerSm) call_tiles_kernel(CallArgs a, const int32_t* __restrict__ tiles,
-                                                                           const int* __restrict__ count, int* next) {
+__global__ void __launch_bounds__(kTile, kFp64CtasPerSm)
+    call_tiles_kernel(const __grid_constant__ CallArgs a, const int32_t* __restrict__ tiles,
+                      const int* __restrict__ count, int* next) {
     extern __shared__ __align__(16) uint8_t smem[];
     uint32_t* recs_all = reinterpret_cast<uint32_t*>(smem);                   /* [SLOTS][kTile] */
     uint32_t* seen_all = reinterpret_cast<uint32_t*>(smem) + SLOTS * kTile;    /* [nw][kTile] */
@@ -330,6 +452,36 @@ __global__ void __launch_bounds__(kTile, kFp64CtasPerSm) call_tiles_kernel(CallA
     for_each_listed(count, next, [&](int i) { fp64_tile<SLOTS>(a, tiles[i], recs_all, seen_all); });
 }
 
+/* The persistent kernel of the FP64 form: call_stream_kernel's hand-out of
+ * tiles in genome order, each in the short form; the tiles it cannot take go to
+ * the leftover list for the binned kernels. */
+template <int SLOTS>
+__global__ void __launch_bounds__(32 * kStreamWarps, kStream64Warps / kStreamWarps)
+    call_stream64_kernel(const __grid_constant__ CallArgs a, StreamQueue q) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const size_t warp_bytes = (lean_smem_bytes(SLOTS, a.L) + 15) & ~(size_t)15;
+    uint32_t* recs_all = reinterpret_cast<uint32_t*>(smem + (threadIdx.x >> 5) * warp_bytes);
+    const int t = threadIdx.x & 31;
+    const int64_t n = q.t_end - q.t_begin;
+    for (;;) {
+        unsigned long long first = 0;
+        if (t == 0) first = atomicAdd(q.next, (unsigned long long)kStreamChunk);
+        first = __shfl_sync(kFull, first, 0);
+        if ((int64_t)first >= n) return;
+        const int64_t end = min((int64_t)first + (int64_t)kStreamChunk, n);
+        for (int64_t i = (int64_t)first; i < end; ++i) {
+            const int64_t tile = q.t_begin + i;
+            const uint8_t wflags = a.win_flags[(int)(tile * kTile / kWin)];
+            const bool called =
+                !(wflags & (kWinKeepLik | kWinExternalLik)) &&
+                lean_tile64<SLOTS>(a, tile, a.tile_rng[tile * 2], a.tile_rng[tile * 2 + 1], wflags, recs_all,
+                                   recs_all + SLOTS * kTile);
+            if (!called && t == 0) q.leftover[atomicAdd(q.n_leftover, 1)] = (int32_t)tile;
+            __syncwarp();
+        }
+    }
+}
+
 /* ------------------------------------------------------------------------ */
 /* launchers                                                                 */
 /* ------------------------------------------------------------------------ */
@@ -338,8 +490,11 @@ thread_local bool g_launch_attributes = true;
 void set_launch_attributes(bool on) { g_launch_attributes = on; }
 
 static size_t fp64_smem_bytes(int slots, int L) {
-    /* records [slots][kTile], then the pcr state */
-    return ((size_t)slots * kTile + (size_t)pcr_smem_words(slots, L, false)) * 4;
+    /* records [slots][kTile], then the pcr state; the bins that try the short
+     * form first: its records and scratch in the same place */
+    const size_t general = ((size_t)slots * kTile + (size_t)pcr_smem_words(slots, L, false)) * 4;
+    const size_t lean = slots <= kLeanG ? lean_smem_bytes(slots, L) : 0;
+    return general > lean ? general : lean;
 }
 
 /* Classify tiles [t_begin, t_end) (with a list, list[t_begin, t_end); with
@@ -356,6 +511,50 @@ cudaError_t launch_classify(const CallArgs& a, int pass, int64_t t_begin, int64_
     classify_tiles_kernel<<<blocks, kClassifyThreads, 0, stream>>>(a, pass, t_begin, t_end, d_bin_count, d_bin_tiles,
                                                                    list, d_count);
     return cudaGetLastError();
+}
+
+template <int SLOTS>
+static cudaError_t stream64_attr(int L, int carveout, int* ctas_per_sm) {
+    const int smem = (int)(kStreamWarps * ((lean_smem_bytes(SLOTS, L) + 15) & ~(size_t)15));
+    cudaError_t e = cudaFuncSetAttribute(call_stream64_kernel<SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess && carveout > 0 &&
+        cudaFuncSetAttribute(call_stream64_kernel<SLOTS>, cudaFuncAttributePreferredSharedMemoryCarveout, carveout) !=
+            cudaSuccess)
+        (void)cudaGetLastError();
+    if (e == cudaSuccess && ctas_per_sm)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, call_stream64_kernel<SLOTS>, 32 * kStreamWarps, smem);
+    return e;
+}
+
+/* resident CTAs on one SM of the persistent FP64 kernel with 48 or 64 record
+ * slots */
+int stream64_ctas_per_sm(int slots, int L, int carveout) {
+    int n = 0;
+    const cudaError_t e = slots <= 48 ? stream64_attr<48>(L, carveout, &n) : stream64_attr<64>(L, carveout, &n);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 1;
+    }
+    return n > 0 ? n : 1;
+}
+
+template <int SLOTS>
+static cudaError_t launch_stream64_one(const CallArgs& a, const StreamQueue& q, int ctas, int carveout,
+                                       cudaStream_t stream) {
+    cudaError_t e = g_launch_attributes ? stream64_attr<SLOTS>(a.L, carveout, nullptr) : cudaSuccess;
+    if (e != cudaSuccess) return e;
+    const size_t smem = kStreamWarps * ((lean_smem_bytes(SLOTS, a.L) + 15) & ~(size_t)15);
+    call_stream64_kernel<SLOTS><<<ctas, 32 * kStreamWarps, smem, stream>>>(a, q);
+    return cudaGetLastError();
+}
+
+/* The persistent FP64 kernel over q's tiles (as launch_stream); a.lean_q must
+ * be set. */
+cudaError_t launch_stream64(const CallArgs& a, const StreamQueue& q, int slots, int ctas, int carveout,
+                            cudaStream_t stream) {
+    if (q.t_end <= q.t_begin) return cudaSuccess;
+    return slots <= 48 ? launch_stream64_one<48>(a, q, ctas, carveout, stream)
+                       : launch_stream64_one<64>(a, q, ctas, carveout, stream);
 }
 
 /* set the FP64 bin kernel's shared-memory size and carveout (percent; 0

@@ -120,6 +120,7 @@ struct CallArgs {
     int qa_rows;
     const uint32_t* lean_q;      /* [16][kLeanG][64] the short form's q_adj table (lean.cuh), or null: no short form */
     const float* lean4;          /* [4][1 + qa_rows * L][4] its terms: base o's records, genotypes (o, 0..3) */
+    const double* lean2d;        /* [4][4][qa_rows * L][2] base o's records, (o, o) and (o, x) in FP64 by [o][x] */
     const uint8_t* qadj;         /* [tmax][gmax][65] adjusted quality */
     int tmax, gmax;
     const double* p_prior;       /* [8][16] */

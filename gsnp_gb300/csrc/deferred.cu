@@ -212,7 +212,7 @@ __device__ __noinline__ bool deferred_posterior(const CallArgs& a, const Deferre
  * at most the pool's capacity.  Sampled sites also get the FP64 sums for the
  * accuracy figure, and when the fast kernel had decided them its call is
  * compared with this one. */
-__global__ void __launch_bounds__(32 * kDefWarps) deferred_sites_kernel(CallArgs a, int64_t n,
+__global__ void __launch_bounds__(32 * kDefWarps) deferred_sites_kernel(const __grid_constant__ CallArgs a, int64_t n,
                                                                         const unsigned long long* d_n) {
     __shared__ __align__(16) DefWarp warps[kDefWarps];
     DefWarp& sm = warps[threadIdx.x >> 5];

@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "calling.cuh"
+#include "lean_tables.cuh"
 #include "columns.h"
 #include "columns_gpu.h"
 #include "emit.h"
@@ -44,10 +45,15 @@ cudaError_t launch_classify(const CallArgs& a, int pass, int64_t t_begin, int64_
 cudaError_t launch_stream(const CallArgs& a, const StreamQueue& q, int slots, int mode, int ctas, int carveout,
                           cudaStream_t stream);
 int stream_ctas_per_sm(int slots, int L, int mode, int carveout);
+cudaError_t launch_stream64(const CallArgs& a, const StreamQueue& q, int slots, int ctas, int carveout,
+                            cudaStream_t stream);
+int stream64_ctas_per_sm(int slots, int L, int carveout);
 cudaError_t launch_bin(const CallArgs& a, int kind, int bin, const int32_t* tiles, const BinLaunch& bl,
                        cudaStream_t stream);
 int bin_ctas_per_sm(int kind, int bin, int L, int carveout);
 void set_launch_attributes(bool on);
+cudaError_t launch_lean_tables(const double* lik64, const uint8_t* qadj, int tmax, int gmax, int qa_rows, int L,
+                               const int8_t* gap, uint32_t* lean_q, float* lean4, double* lean2d, cudaStream_t stream);
 cudaError_t launch_snp_log_prior(const CallArgs& a, double* out, float* out32, cudaStream_t stream);
 int deferred_ctas_per_sm();
 cudaError_t launch_deferred(const CallArgs& a, int64_t n, cudaStream_t stream,
@@ -445,6 +451,7 @@ struct gsnp_context {
     float* d_lik32 = nullptr;
     uint32_t* d_lean_q = nullptr;
     float* d_lean4 = nullptr;
+    double* d_lean2d = nullptr;
     uint8_t* d_qadj = nullptr;
     double* d_p_prior = nullptr;
     double* d_log_prior = nullptr;
@@ -507,7 +514,7 @@ struct gsnp_context {
      * count), the leftover tiles, its record slots and grid */
     unsigned long long* d_stream_ctl = nullptr;
     int32_t* d_leftover = nullptr;
-    int stream_slots = 0, stream_ctas = 0, stream_ctas_L = -1, stream_carveout = 72;
+    int stream_slots = 0, stream_ctas = 0, stream64_ctas = 0, stream_ctas_L = -1, stream_carveout = 72;
     bool stream_path = true;
     int stream_mode = 0;            /* 0 plain loads, 1 L2 bulk prefetch, 2 staged in shared memory */
     /* Device-driven calling: the bins' kernels, the classification of the
@@ -793,6 +800,7 @@ CallArgs make_args(gsnp_context* c) {
     /* the short form's proof is of diploid calls */
     a.lean_q = c->tables.lean_ok && !c->params.monoploid ? c->d_lean_q : nullptr;
     a.lean4 = c->d_lean4;
+    a.lean2d = c->d_lean2d;
     a.qadj = c->d_qadj;
     a.tmax = c->tables.tmax;
     a.gmax = c->tables.gmax;
@@ -906,6 +914,7 @@ int prepare_calling(gsnp_context* c) {
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device), "device attribute");
         c->stream_ctas =
             sms * stream_ctas_per_sm(c->stream_slots, c->params.read_length, c->stream_mode, c->stream_carveout);
+        c->stream64_ctas = sms * stream64_ctas_per_sm(c->stream_slots, c->params.read_length, c->stream_carveout);
         c->stream_ctas_L = c->params.read_length;
     }
     if (c->dsite_cap == 0) {
@@ -987,10 +996,19 @@ int finish_device(gsnp_context* c) {
     return GSNP_OK;
 }
 
-/* The persistent kernel calls tiles in the short form (or, with its reads
- * staged in shared memory, in the general one); without the short form it
- * would leave every tile. */
-bool stream_takes(const gsnp_context* c, const CallArgs& a) { return a.lean_q != nullptr || c->stream_mode == 2; }
+/* The persistent kernels call tiles in the short form (or, in the FP32 form
+ * with its reads staged in shared memory, in the general one); without the
+ * short form they would leave every tile. */
+bool stream_takes(const gsnp_context* c, const CallArgs& a) {
+    return a.lean_q != nullptr || (a.precision == 1 && c->stream_mode == 2);
+}
+
+/* the persistent kernel of the call's form over q's tiles */
+cudaError_t launch_stream_form(const gsnp_context* c, const CallArgs& a, const StreamQueue& q) {
+    return a.precision == 1 ? launch_stream(a, q, c->stream_slots, c->stream_mode, c->stream_ctas, c->stream_carveout,
+                                            c->stream)
+                            : launch_stream64(a, q, c->stream_slots, c->stream64_ctas, c->stream_carveout, c->stream);
+}
 
 /* device-driven queueing of a calling pass (defined below) */
 int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std::function<int(size_t)>& before,
@@ -1092,15 +1110,13 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
         /* In the FP32 form the persistent kernel calls the segment's tiles;
          * the binned kernels take only the tiles it leaves (the FP64 windows'
          * and those with a site deeper than its record slots). */
-        const bool use_stream =
-            c->stream_path && c->params.precision == 1 && segs.size() == 1 && !c->view.on && stream_takes(c, a);
+        const bool use_stream = c->stream_path && segs.size() == 1 && !c->view.on && stream_takes(c, a);
         int64_t n_left = 0;
         auto run_stream = [&](const CallArgs& as) -> int {
             CK(cudaMemsetAsync(c->d_stream_ctl, 0, 2 * sizeof(unsigned long long), c->stream), "memset");
             const StreamQueue q{g.t0, g.t1, c->d_stream_ctl, c->d_leftover, reinterpret_cast<int*>(c->d_stream_ctl + 1)};
             const int ks = begin(kKindStream, c->stream_slots, g.t1 - g.t0);
-            CK(launch_stream(as, q, c->stream_slots, c->stream_mode, c->stream_ctas, c->stream_carveout, c->stream),
-               "persistent calling kernel");
+            CK(launch_stream_form(c, as, q), "persistent calling kernel");
             end(ks);
             return GSNP_OK;
         };
@@ -1230,7 +1246,7 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
      * (or chunks) ends each segment's launch of it in a tail of its own, and
      * its binned kernels, handing out tiles from counters, were the faster
      * there (c1 e2e in 7 segments: 28.6-29.0 against 29.9 ms) */
-    const bool use_stream = c->stream_path && fast && segs.size() == 1 && !c->view.on && stream_takes(c, make_args(c));
+    const bool use_stream = c->stream_path && segs.size() == 1 && !c->view.on && stream_takes(c, make_args(c));
     int* d_left = reinterpret_cast<int*>(c->d_stream_ctl + 1);
     /* With several segments the deferred sites of all of them go to one pool
      * and one deferred pass runs after the last segment: the pass takes about
@@ -1292,8 +1308,7 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
             end(k);
             const StreamQueue q{g.t0, g.t1, c->d_stream_ctl, c->d_leftover, d_left};
             const int ks = begin(kKindStream, c->stream_slots, g.t1 - g.t0);
-            CK(launch_stream(a, q, c->stream_slots, c->stream_mode, c->stream_ctas, c->stream_carveout, c->stream),
-               "persistent calling kernel");
+            CK(launch_stream_form(c, a, q), "persistent calling kernel");
             end(ks);
             k = begin(kKindClassify, 0, 0);
             CK(launch_classify(a, 0, 0, 0, c->d_bin_count, c->d_bin_tiles, c->stream, c->d_leftover, d_left,
@@ -1913,21 +1928,27 @@ int gsnp_load_tables(gsnp_context* c, const gsnp_params* p, const double* p_matr
         const void* src;
         size_t bytes, at;
     };
+    int8_t* d_gap = nullptr;
     Part parts[] = {{(void**)&c->d_lik64, t.lik64.data(), t.lik64.size() * 8, 0},
                     {(void**)&c->d_lik32, t.lik32.data(), t.lik32.size() * 4, 0},
-                    {(void**)&c->d_lean_q, t.lean_q.data(), t.lean_q.size() * 4, 0},
-                    {(void**)&c->d_lean4, t.lean4.data(), t.lean4.size() * 4, 0},
                     {(void**)&c->d_qadj, t.qadj.data(), t.qadj.size(), 0},
                     {(void**)&c->d_p_prior, p_prior, 128 * 8, 0},
                     {(void**)&c->d_log_prior, t.log_prior.data(), 128 * 8, 0},
-                    {(void**)&c->d_log_prior32, t.log_prior32.data(), 96 * 4, 0}};
-    size_t total = 0;
+                    {(void**)&c->d_log_prior32, t.log_prior32.data(), 96 * 4, 0},
+                    {(void**)&d_gap, t.lean_gap.data(), t.lean_gap.size(), 0},
+                    /* made on the device from the ones before */
+                    {(void**)&c->d_lean_q, nullptr, (size_t)kLeanQ * 4, 0},
+                    {(void**)&c->d_lean4, nullptr, (size_t)lean4_rows(t.qa_rows, t.L) * 16, 0},
+                    {(void**)&c->d_lean2d, nullptr, (size_t)lean2d_rows(t.qa_rows, t.L) * 16, 0}};
+    size_t total = 0, uploaded = 0;
     for (Part& q : parts) {
         q.at = total;
         total += (q.bytes + 255) & ~(size_t)255;
+        if (q.src) uploaded = total;
     }
-    std::vector<uint8_t> blob(total);
-    for (const Part& q : parts) memcpy(blob.data() + q.at, q.src, q.bytes);
+    std::vector<uint8_t> blob(uploaded);
+    for (const Part& q : parts)
+        if (q.src) memcpy(blob.data() + q.at, q.src, q.bytes);
     if (total > c->tables_bytes) {
         c->have_tables = false;
         c->tables_bytes = 0;
@@ -1936,7 +1957,11 @@ int gsnp_load_tables(gsnp_context* c, const gsnp_params* p, const double* p_matr
     }
     for (const Part& q : parts) *q.dst = c->d_tables + q.at;
     if (!c->d_p_rank) CK(dev_alloc(&c->d_p_rank, 64UL * 64UL * 2048UL), "cudaMalloc");
-    CK(cudaMemcpy(c->d_tables, blob.data(), total, cudaMemcpyHostToDevice), "upload");
+    CK(cudaMemcpy(c->d_tables, blob.data(), uploaded, cudaMemcpyHostToDevice), "upload");
+    CK(launch_lean_tables(c->d_lik64, c->d_qadj, t.tmax, t.gmax, t.qa_rows, t.L, d_gap, c->d_lean_q, c->d_lean4,
+                          c->d_lean2d, c->stream),
+       "table kernel");
+    CK(cudaStreamSynchronize(c->stream), "table kernel");   /* the next call may run on another stream */
     CK(cudaMemcpy(c->d_p_rank, p_rank, 64UL * 64UL * 2048UL * 8, cudaMemcpyHostToDevice), "upload");
     c->have_tables = true;
     c->snp_lp_ready = false;
@@ -2090,7 +2115,7 @@ uint64_t graph_key_of(gsnp_context* c, const Segment& g) {
     const CallArgs a = make_args(c);
     mix(&a, sizeof a);
     mix(&g, sizeof g);
-    const int cfg[] = {c->stream_path, c->stream_slots, c->stream_mode, c->stream_carveout, c->stream_ctas,
+    const int cfg[] = {c->stream_path, c->stream_slots, c->stream_mode, c->stream_carveout, c->stream_ctas, c->stream64_ctas,
                        c->deferred_grid, c->classify_grid};
     mix(cfg, sizeof cfg);
     mix(c->bin_grid, sizeof c->bin_grid);

@@ -162,13 +162,19 @@ GSNP_HDI uint32_t add_top(uint32_t x, uint32_t acc) {
 #endif
 }
 
+/* a lean record with the q_adj of its lean_q entry in bits 13:6 (for a second
+ * walk over the column) */
+GSNP_HDI uint32_t lean_with_qa(uint32_t w, uint32_t e) { return (w & ~0x3fc0u) | ((e >> 10) & 0x3fc0u); }
+GSNP_HDI int lean_qa(uint32_t w) { return (int)((w >> 6) & 0xffu); }
+
 /* The walk over a sorted lean column of num records (kStride words apart, at
  * most kLeanG of them; up to three words past the last one are read and not
- * used).  none is the maj of a site without records.  lean_q's entries hold
+ * used).  none is the maj of a site without records; KEEP_QA leaves each
+ * record's q_adj in it.  lean_q's entries hold
  * q_adj * L in bits 15:0, q_adj in bits 23:16 and the gap (signed) in bits
  * 31:24. */
-template <int kStride>
-__device__ __forceinline__ void lean_walk(const CallArgs& a, const uint32_t* recs, int num, int none, LeanSums* o) {
+template <int kStride, bool KEEP_QA = false>
+__device__ __forceinline__ void lean_walk(const CallArgs& a, uint32_t* recs, int num, int none, LeanSums* o) {
     const int maj = num > 0 ? (int)(recs[(num >> 1) * kStride] >> 30) : none;
     /* maj's records are [gb, ge) */
     int gb = 0, ge = num;
@@ -186,7 +192,7 @@ __device__ __forceinline__ void lean_walk(const CallArgs& a, const uint32_t* rec
          * this one's rows are on their way */
         LeanCounts k;
         const uint32_t* lq = a.lean_q - maj * 64;
-        const uint32_t* p = recs + gb * kStride;
+        uint32_t* p = recs + gb * kStride;
         const float4* rows = reinterpret_cast<const float4*>(a.lean4) + (size_t)(maj * (a.qa_rows * a.L + 1));
         uint32_t w[4], e[4];
         auto entries = [&](int i) {
@@ -212,6 +218,7 @@ __device__ __forceinline__ void lean_walk(const CallArgs& a, const uint32_t* rec
                 gap = add_top_signed(e[u], gap);
                 const uint32_t row = (e[u] & 0xffffu) + ((w[u] >> 16) & 0xffu) + 1u;
                 x[u] = GSNP_LDG(rows + (i + u < m ? row : 0u));   /* row 0 is all zero */
+                if (KEEP_QA && i + u < m) recs[(gb + i + u) * kStride] = lean_with_qa(w[u], e[u]);
             }
             if (i + 4 < m) entries(i + 4);
             const float v[4] = {__fadd_rn(__fadd_rn(x[0].x, x[1].x), __fadd_rn(x[2].x, x[3].x)),
@@ -253,9 +260,59 @@ __device__ __forceinline__ void lean_walk(const CallArgs& a, const uint32_t* rec
         for (int t = 0; t < 10; ++t) o->mn[t] = __fadd_rn(o->mn[t], x[t]);
         o->cu4 += 1u << (8 * ob);
         o->qs4 += (uint64_t)(kMaxQ - ((w >> 24) & 63u)) << (16 * ob);
+        if (KEEP_QA) recs[i * kStride] = lean_with_qa(w, e);
         ++i;
         if (i == gb) i = ge;
     }
+}
+
+/* The FP64 sums of the genotypes (maj, maj) and (maj, win) over a column that
+ * lean_walk<KEEP_QA> has walked, every record in the reference's order: bit
+ * for bit likelihood_fp64's.  maj's records take both terms in one 16-byte
+ * load (lean2d), the others one each from the general table. */
+template <int kStride>
+__device__ __forceinline__ void lean_sums64(const CallArgs& a, const uint32_t* recs, int num, const LeanSums& z, int win,
+                                            double* best, double* second) {
+    const int maj = z.maj, lo = maj < win ? maj : win, hi = maj < win ? win : maj;
+    const double* t0 = a.lik64 + col_of(maj, maj);
+    const double* t1 = a.lik64 + col_of(lo, hi);
+    const double2* rows = reinterpret_cast<const double2*>(a.lean2d) + (size_t)((maj * 4 + win) * a.qa_rows) * a.L;
+    double s0 = 0.0, s1 = 0.0;
+    const int m = (int)((z.cu4 >> (8 * maj)) & 0xffu);
+    /* the other bases' records before maj's, maj's, and those after: one loop
+     * each, so that the lanes of a warp run maj's together */
+    auto other = [&](int i) {
+        const uint32_t w = recs[i * kStride];
+        const size_t row = ((size_t)(lean_qa(w) * a.L) + ((w >> 16) & 0xffu)) * 40 + (w >> 30) * 10;
+        s0 = GSNP_DADD(s0, GSNP_LDG(t0 + row));
+        s1 = GSNP_DADD(s1, GSNP_LDG(t1 + row));
+    };
+    int gb = 0;
+#pragma unroll 1
+    for (; gb < num && (int)(recs[gb * kStride] >> 30) != maj; ++gb) other(gb);
+    const uint32_t* p = recs + gb * kStride;
+#pragma unroll 1
+    for (int i = 0; i < m; i += 4, p += 4 * kStride) {
+        double2 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            x[u] = double2{0.0, 0.0};   /* adding it changes nothing: the sums are not -0 */
+            if (i + u < m) {
+                const uint32_t v = p[u * kStride];
+                x[u] = GSNP_LDG(rows + lean_qa(v) * a.L + (int)((v >> 16) & 0xffu));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (u == 0 || i + u < m) {
+                s0 = GSNP_DADD(s0, x[u].x);
+                s1 = GSNP_DADD(s1, x[u].y);
+            }
+    }
+#pragma unroll 1
+    for (int i = gb + m; i < num; ++i) other(i);
+    *best = s0;
+    *second = s1;
 }
 
 __device__ __forceinline__ SitePileup lean_counts(const LeanPile& pile, const LeanSums& z) {
@@ -299,8 +356,8 @@ __device__ __forceinline__ void lean_fill(CallWords* out, const LeanPile& pile, 
     out->b.w = 0x3ff00000u;
 }
 
-/* fast_posterior's proof (prove_hom) over the walk's sums, for diploid calls.
- * With tp_j the value of (maj, j) and v2 the largest for j != maj:
+/* The values and bounds behind a lean call, for diploid calls.  With tp_j the
+ * value of (maj, j) and v2 the largest for j != maj (j = win):
  *
  *   |tp_j - tp64_j| <= E_j: maj's sum carries 6 u and the record count's term
  *   (likelihood_fp32's grouping), the minor sum n_minor u, and the three
@@ -308,13 +365,18 @@ __device__ __forceinline__ void lean_fill(CallWords* out, const LeanPile& pile, 
  *
  *   Any of the other six is at most M = max_j(s4_j) - gap + max(minor sum +
  *   prior over the six), within E_M, j over the three others.
- *
- * tp64[maj maj] - max(other tp64) then lies in [d - E1 - B, d + E1 + E2] with
- * d = tp_maj - v2, B = max(tp_j - v2 + E_j, M - v2 + E_M). */
-__device__ __forceinline__ bool lean_posterior(const CallArgs& a, int64_t snp_row, uint8_t ori, const LeanPile& pile,
-                                               const LeanSums& z, CallWords* out) {
-    const int num = pile.num;
-    const float inf = INFINITY, u = 0x1p-24f, grow = 1.0f + 0x1p-18f;
+ */
+struct LeanBounds {
+    float v1, e1, v2, e2;   /* (maj, maj), and the best of the other three */
+    float rest;             /* the largest of tp_j + E_j - v2 over the two after it, and M + E_M - v2 */
+    float ball;             /* the same over all three and M */
+    float slack;            /* of E_j and E_M: covers the roundings of such differences */
+    int win;
+};
+
+__device__ __forceinline__ LeanBounds lean_bounds(const CallArgs& a, int64_t snp_row, uint8_t ori, const LeanSums& z,
+                                                  int num) {
+    const float inf = INFINITY, u = 0x1p-24f;
     float t[10];
     load_log_prior32(a, snp_row, ori, t);
     float lp_mag = 0.f, mn_mag = 0.f;
@@ -341,17 +403,21 @@ __device__ __forceinline__ bool lean_posterior(const CallArgs& a, int64_t snp_ro
     /* what every bound shares: the minor sum's error and every rounding after it */
     const float rest = __fadd_rn(__fmul_rn(mn_mag, (float)(z.n_minor + 8) * u), __fmul_rn(lp_mag, 8.f * u));
     const float kk = __fadd_rn(9.f * u, __fmul_rn((float)num, 0x1p-45f));
-    float v1 = 0.f, e1 = 0.f, v2 = -inf, e2 = 0.f, top = -inf, e_top = 0.f, tp[4], E[4];
+    LeanBounds b;
+    b.v1 = b.e1 = b.e2 = 0.f;
+    b.v2 = -inf;
+    b.win = 0;
+    float top = -inf, e_top = 0.f, tp[4], E[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         tp[j] = __fadd_rn(z.s4[j], t4[j]);
         E[j] = __fadd_rn(__fmul_rn(fabsf(z.s4[j]), kk), rest);
         if (z.maj == j) {
-            v1 = tp[j];
-            e1 = E[j];
+            b.v1 = tp[j];
+            b.e1 = E[j];
             tp[j] = -inf;
         } else {
-            if (tp[j] >= v2) { v2 = tp[j]; e2 = E[j]; }
+            if (tp[j] >= b.v2) { b.v2 = tp[j]; b.e2 = E[j]; b.win = j; }
             top = fmaxf(top, z.s4[j]);
             e_top = fmaxf(e_top, E[j]);
         }
@@ -359,16 +425,31 @@ __device__ __forceinline__ bool lean_posterior(const CallArgs& a, int64_t snp_ro
     /* M and its bound: three more additions of at most these magnitudes */
     const float M = __fadd_rn(__fsub_rn(top, gap), six);
     const float e_m = __fadd_rn(e_top, __fmul_rn(__fadd_rn(__fadd_rn(fabsf(top), fabsf(gap)), fabsf(six)), 4.f * u));
-    float B = __fadd_rn(__fsub_rn(M, v2), e_m);
+    b.rest = __fadd_rn(__fsub_rn(M, b.v2), e_m);
+    b.ball = b.rest;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) B = fmaxf(B, __fadd_rn(__fsub_rn(tp[j], v2), E[j]));
-    /* the roundings of the differences here: 2^-23 of quantities of E's size
-     * where B is small, and of B itself where a bound lies above v2 */
-    B = __fmul_rn(__fadd_rn(fmaxf(B, 0.f), __fmul_rn(__fadd_rn(e_top, e_m), 0x1p-20f)), grow);
-    if (!(isfinite(v1) && isfinite(v2) && isfinite(B))) return false;
-    const float d = __fsub_rn(v1, v2);
-    const float below = __fmul_rn(__fadd_rn(e1, B), grow);
-    const float above = __fmul_rn(__fadd_rn(e1, e2), grow);
+    for (int j = 0; j < 4; ++j) {
+        const float x = __fadd_rn(__fsub_rn(tp[j], b.v2), E[j]);
+        b.ball = fmaxf(b.ball, x);
+        if (j != b.win) b.rest = fmaxf(b.rest, x);
+    }
+    b.slack = __fadd_rn(e_top, e_m);
+    return b;
+}
+
+/* fast_posterior's proof (prove_hom) over the walk's sums: with d = v1 - v2 and
+ * B = ball, tp64[maj maj] - max(other tp64) lies in [d - E1 - B, d + E1 + E2]. */
+__device__ __forceinline__ bool lean_posterior(const CallArgs& a, int64_t snp_row, uint8_t ori, const LeanPile& pile,
+                                               const LeanSums& z, CallWords* out) {
+    const float grow = 1.0f + 0x1p-18f;
+    const LeanBounds b = lean_bounds(a, snp_row, ori, z, pile.num);
+    /* the roundings of the differences: 2^-23 of quantities of E's size where
+     * B is small, and of B itself where a bound lies above v2 */
+    const float B = __fmul_rn(__fadd_rn(fmaxf(b.ball, 0.f), __fmul_rn(b.slack, 0x1p-20f)), grow);
+    if (!(isfinite(b.v1) && isfinite(b.v2) && isfinite(B))) return false;
+    const float d = __fsub_rn(b.v1, b.v2);
+    const float below = __fmul_rn(__fadd_rn(b.e1, B), grow);
+    const float above = __fmul_rn(__fadd_rn(b.e1, b.e2), grow);
     if (!(__fsub_rn(__fmul_rn(d, 1.0f - 0x1p-22f), below) > 0.f)) return false;
     const TopBases tb = top_bases(lean_counts(pile, z), ori & 7);
     const float raw_lo = __fmul_rn(10.f, __fsub_rn(d, below));
@@ -378,6 +459,32 @@ __device__ __forceinline__ bool lean_posterior(const CallArgs& a, int64_t snp_ro
     const int q = finalize_q(__float2int_rz(__fsub_rn(raw_lo, slack)), true, false, tb, g1);
     if (q != finalize_q(__float2int_rz(__fadd_rn(raw_hi, slack)), true, false, tb, g1)) return false;
     lean_fill(out, pile, z, tb, g1, q);
+    return true;
+}
+
+/* The FP64 form's call from the FP64 sums of two genotypes, for diploid calls.
+ * The FP32 sums only say which two: (maj, win) is the best of the genotypes
+ * other than (maj, maj) when every other one's bound lies below its own.  Its
+ * FP64 value is then the second best, and the best one's too if that is
+ * larger.  False, writing nothing, when they do not say it, or when the best
+ * genotype is not (maj, maj): the site then takes all ten in FP64. */
+template <int kStride>
+__device__ __forceinline__ bool lean_posterior64(const CallArgs& a, int64_t snp_row, uint8_t ori, const LeanPile& pile,
+                                                 const LeanSums& z, const uint32_t* recs, CallWords* out) {
+    const float grow = 1.0f + 0x1p-18f;
+    const LeanBounds b = lean_bounds(a, snp_row, ori, z, pile.num);
+    const float rest = __fadd_rn(b.rest, __fmul_rn(__fadd_rn(b.slack, fabsf(b.rest)), 0x1p-18f));
+    if (!(isfinite(b.v2) && __fadd_rn(rest, __fmul_rn(b.e2, grow)) < 0.f && b.v1 > b.v2)) return false;
+    const double* prior = (ori & 0x8) && a.refine ? a.snp_lp + snp_row * 16 : a.log_prior + ((ori & 7) << 4);
+    double s0, s1;
+    lean_sums64<kStride>(a, recs, pile.num, z, b.win, &s0, &s1);
+    const int g1 = z.maj << 2 | z.maj, g2 = z.maj <= b.win ? z.maj << 2 | b.win : b.win << 2 | z.maj;
+    const double best = GSNP_DADD(s0, GSNP_LDG(prior + g1)), second = GSNP_DADD(s1, GSNP_LDG(prior + g2));
+    if (!(best > second)) return false;
+    /* the rank-sum value of a homozygous call is 1 and its log10 0 */
+    const TopBases tb = top_bases(lean_counts(pile, z), ori & 7);
+    const double raw = GSNP_DMUL(10.0, GSNP_DSUB(best, second));
+    lean_fill(out, pile, z, tb, g1, finalize_q((int)raw, true, false, tb, g1));
     return true;
 }
 

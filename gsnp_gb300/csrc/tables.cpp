@@ -29,57 +29,43 @@ int q_adjust(int q, int tmp, int gdc, double pcr, double glob, const double* log
     return qa;
 }
 
-/* The short form's tables (lean.cuh).  gap(q_adj) is the least of
+/* The gaps of the short form (lean.cuh).  gap(q_adj) is the least of
  * min(term[o x], term[o y]) - term[xy] over the cycles, the observed bases o
  * and the pairs xy without o, in units of kLeanGapUnit rounded down; -128 ..
  * 127 units hold every table whose terms lie within 4 of each other. */
-void build_lean_tables(HostTables* t) {
+void build_lean_gaps(HostTables* t) {
     const int L = t->L, rows = t->qa_rows;
-    /* columns of the pairs of bases, and for each base the six pairs without it */
-    int col[4][4], pairs[4][6][2];
+    /* columns of the pairs of bases, and for each base the six pairs without
+     * it: the columns of (o, x), (o, y) and (x, y) */
+    int col[4][4], six[4][6][3];
     for (int x = 0, k = 0; x < 4; ++x)
         for (int y = x; y < 4; ++y) col[x][y] = col[y][x] = k++;
     for (int o = 0; o < 4; ++o)
         for (int x = 0, i = 0; x < 4; ++x)
             for (int y = x; y < 4; ++y)
                 if (x != o && y != o) {
-                    pairs[o][i][0] = x;
-                    pairs[o][i++][1] = y;
+                    six[o][i][0] = col[o][x];
+                    six[o][i][1] = col[o][y];
+                    six[o][i++][2] = col[x][y];
                 }
-    std::vector<int> gap((size_t)rows, 0);
-    t->lean_ok = true;
-    t->lean4.assign((size_t)4 * ((size_t)rows * L + 1) * 4, 0.0f);
+    t->lean_gap.assign((size_t)rows, 0);
+    t->lean_ok = (size_t)rows * L <= 65535 && rows <= 256;
     for (int q = 0; q < rows; ++q) {
         double least = 127.0 * kLeanGapUnit;
         bool nan = false;
         for (int c = 0; c < L; ++c)
             for (int o = 0; o < 4; ++o) {
                 const double* r = &t->lik64[(((size_t)q * L + c) * 4 + o) * 10];
-                float* out = &t->lean4[((size_t)o * ((size_t)rows * L + 1) + 1 + (size_t)q * L + c) * 4];
-                for (int j = 0; j < 4; ++j) out[j] = (float)r[col[o][j]];
-                for (int i = 0; i < 6; ++i) {
-                    const int x = pairs[o][i][0], y = pairs[o][i][1];
-                    const double d = std::min(r[col[o][x]], r[col[o][y]]) - r[col[x][y]];
+                for (const int* p : six[o]) {
+                    const double d = std::min(r[p[0]], r[p[1]]) - r[p[2]];
                     nan |= d != d;   /* both terms -inf */
                     least = std::min(least, d);
                 }
             }
         const double units = std::floor(least / kLeanGapUnit - 1e-3);
         if (nan || !(units >= -128.0)) t->lean_ok = false;
-        else gap[(size_t)q] = (int)units;
+        else t->lean_gap[(size_t)q] = (int8_t)units;
     }
-    if ((size_t)rows * L > 65535 || rows > 256) t->lean_ok = false;
-    t->lean_q.assign((size_t)16 * kLeanG * 64, 0);
-    for (int tmp = 0; tmp < 16; ++tmp)
-        for (int g = 0; g < kLeanG; ++g)
-            for (int f = 0; f < 64; ++f) {
-                const int q = 64 - f;
-                const int qa = tmp + 1 < t->tmax && g < t->gmax
-                                   ? t->qadj[((size_t)(tmp + 1) * t->gmax + g) * 65 + q]
-                                   : 1;
-                t->lean_q[((size_t)tmp * kLeanG + g) * 64 + f] =
-                    (uint32_t)(qa * L) | (uint32_t)qa << 16 | (uint32_t)(uint8_t)(int8_t)gap[(size_t)qa] << 24;
-            }
 }
 
 }  // namespace
@@ -155,7 +141,7 @@ int build_tables(const gsnp_params& p, const double* pm, const double* p_prior, 
         for (int k = 8; k < 10; ++k) t->lik32[rows * 8 + r * 2 + (k - 8)] = (float)t->lik64[r * 10 + k];
     }
 
-    build_lean_tables(t);
+    build_lean_gaps(t);
 
     t->log_prior.resize(128);
     for (int i = 0; i < 128; ++i) t->log_prior[i] = gsnp_cr_log10(p_prior[i]);

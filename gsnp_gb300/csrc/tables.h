@@ -21,12 +21,11 @@ struct HostTables {
     std::vector<float> lik32;       /* FP32: [qa_rows][L][4][8] columns 0-7 of each row, then
                                        [qa_rows][L][4][2] columns 8-9 */
     std::vector<uint8_t> qadj;      /* [tmax][gmax][65] */
-    /* the short form (lean.cuh): q_adj * L | q_adj << 16 | gap << 24 by
-     * [tmp][distinct keys][64 - q], and per base o a row of zeros, then by
-     * [qa_rows][L] the FP32 terms of the genotypes (o, 0..3) for a record of o */
-    std::vector<uint32_t> lean_q;   /* [16][kLeanG][64] */
-    std::vector<float> lean4;       /* [4][1 + qa_rows * L][4] */
-    bool lean_ok = false;           /* every gap fits its field */
+    /* the short form (lean.cuh): the gap of each q_adj, in kLeanGapUnit, and
+     * whether every one fits its field; its tables are made from these and
+     * the ones above on the device (lean_tables.cuh) */
+    std::vector<int8_t> lean_gap;   /* [qa_rows] */
+    bool lean_ok = false;
     std::vector<double> log_prior;  /* [128] correctly rounded log10 of p_prior */
     std::vector<float> log_prior32; /* [8][12] log_prior in FP32 by table column */
     bool all_nonpositive = true;    /* every lik64 entry <= 0, none of them an FP32 subnormal */

@@ -203,6 +203,10 @@ __device__ __forceinline__ void for_each_listed(const int* __restrict__ count, i
     }
 }
 
+/* warps of a CTA of the persistent kernels: each works by itself; several share
+ * the CTA's reserved shared memory */
+constexpr int kStreamWarps = 4;
+
 /* record-slot capacity of each depth bin */
 constexpr int kSlots[kNumBins] = {32, 40, 48, 64, 96, 128, 256};
 

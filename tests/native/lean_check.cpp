@@ -14,8 +14,9 @@
  * Sites as posterior_check.cpp's, at depths 0 to 64 (kLeanG) with qualities 1
  * to 63, under calibrations from plain to noisy (rows in which another base is
  * likelier than the read's own, so that gaps are negative).
- * Prints "sites <n> decided <d> of <h> homozygous adversarial <a>" and exits
- * 0, or names the first failing site and exits 1.
+ * The FP64 form's two sums are checked beside it bit for bit, and its calls.
+ * Prints "sites <n> decided <d> of <h> homozygous adversarial <a> decided64
+ * <e>" and exits 0, or names the first failing site and exits 1.
  * Usage: lean_check <sites> <seed> <read length>
  */
 #include <stdio.h>
@@ -28,6 +29,7 @@
 #include <vector>
 
 #include "lean.cuh"
+#include "lean_tables.cuh"
 #include "tables.h"
 
 using namespace gsnp;
@@ -59,7 +61,7 @@ int main(int argc, char** argv) {
     prior_table(p, p.transition_dominant, p.het_novel, p.althom_novel, prior.data());
     rank_table(rank.data());
     std::vector<uint32_t> seen(64);
-    long decided = 0, hom = 0, adversarial = 0;
+    long decided = 0, hom = 0, adversarial = 0, decided64 = 0;
     constexpr int kCalibrations = 4;
     for (int cal = 0; cal < kCalibrations; ++cal) {
         /* error 10^(-q/10) over the three other bases, varying with the cycle
@@ -86,8 +88,17 @@ int main(int argc, char** argv) {
         a.lik64 = t.lik64.data();
         a.lik32 = t.lik32.data();
         a.lik32b = t.lik32.data() + (size_t)t.qa_rows * t.L * 4 * 8;
-        a.lean_q = t.lean_q.data();
-        a.lean4 = t.lean4.data();
+        std::vector<uint32_t> lean_q((size_t)kLeanQ);
+        std::vector<float> lean4((size_t)lean4_rows(t.qa_rows, t.L) * 4);
+        std::vector<double> lean2d((size_t)lean2d_rows(t.qa_rows, t.L) * 2);
+        for (size_t i = 0; i < lean_q.size(); ++i)
+            lean_q[i] = lean_q_entry(t.qadj.data(), t.tmax, t.gmax, t.L, t.lean_gap.data(), (int64_t)i);
+        for (size_t i = 0; i < lean4.size() / 4; ++i) lean4_row(t.lik64.data(), t.qa_rows, t.L, (int64_t)i, &lean4[i * 4]);
+        for (size_t i = 0; i < lean2d.size() / 2; ++i)
+            lean2d_row(t.lik64.data(), t.qa_rows, t.L, (int64_t)i, &lean2d[i * 2]);
+        a.lean_q = lean_q.data();
+        a.lean4 = lean4.data();
+        a.lean2d = lean2d.data();
         a.qa_rows = t.qa_rows;
         a.qadj = t.qadj.data();
         a.tmax = t.tmax;
@@ -201,6 +212,35 @@ int main(int argc, char** argv) {
             SiteCall want, got;
             site_posterior<false>(a, ori, sp, tl64, nullptr, lp, recs.data(), 1, nq, &want);
             hom += (want.type1 >> 2) == (want.type1 & 3);
+            /* the FP64 form: its two sums bit for bit, and its calls */
+            {
+                std::vector<uint32_t> kept = lean;
+                LeanSums y;
+                lean_walk<1, true>(a, kept.data(), sp.num, ori & 3, &y);
+                for (int x = 0; x < 4; ++x) {
+                    double s0, s1;
+                    lean_sums64<1>(a, kept.data(), sp.num, y, x, &s0, &s1);
+                    if (s0 != tl64[genotype_of(pair_col(y.maj, y.maj))] || s1 != tl64[genotype_of(pair_col(y.maj, x))]) {
+                        printf("site %ld: FP64 sums of (%d, %d) differ\n", site, y.maj, x);
+                        return 1;
+                    }
+                }
+                CallWords words;
+                if (lean_posterior64<1>(a, -1, ori, pile, y, kept.data(), &words)) {
+                    ++decided64;
+                    memcpy(&got, &words, sizeof got);
+                    if (!same_call(got, want)) {
+                        printf("site %ld: the FP64 short form gives type %d q %d, FP64 type %d q %d (num %d, ori %d)\n",
+                               site, got.type1, got.q_cns, want.type1, want.q_cns, sp.num, ori);
+                        return 1;
+                    }
+                }
+                for (int i = 0; i < sp.num; ++i)
+                    if (lean_to_record(kept[(size_t)i]) != recs[(size_t)i]) {
+                        printf("site %ld: record %d changed\n", site, i);
+                        return 1;
+                    }
+            }
             CallWords words;
             if (!lean_posterior(a, -1, ori, pile, z, &words)) continue;
             memcpy(&got, &words, sizeof got);
@@ -235,6 +275,7 @@ int main(int argc, char** argv) {
             }
         }
     }
-    printf("sites %ld decided %ld of %ld homozygous adversarial %ld\n", n_sites, decided, hom, adversarial);
+    printf("sites %ld decided %ld of %ld homozygous adversarial %ld decided64 %ld\n", n_sites, decided, hom,
+           adversarial, decided64);
     return 0;
 }

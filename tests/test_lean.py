@@ -41,7 +41,8 @@ def test_lean_decisions_equal_fp64(sites, seed, length, lean_check):
     assert r.returncode == 0, r.stdout + r.stderr
     words = r.stdout.split()
     decided, hom = int(words[words.index("decided") + 1]), int(words[words.index("of") + 1])
-    assert decided > hom * 9 // 10, r.stdout   # not vacuous
+    decided64 = int(words[words.index("decided64") + 1])
+    assert decided > hom * 9 // 10 and decided64 > hom * 9 // 10, r.stdout   # not vacuous
 
 
 def edge_workload(kind: str) -> synth.Workload:
