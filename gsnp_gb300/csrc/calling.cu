@@ -160,7 +160,7 @@ constexpr int kClassifyTiles = kClassifyThreads / kTile;
 constexpr int kClassifyStage = 256;   /* read starts staged in shared memory per tile */
 static_assert(kClassifyThreads % kTile == 0, "a classify CTA holds whole tiles");
 
-__global__ void __launch_bounds__(kClassifyThreads) classify_tiles_kernel(CallArgs a, int pass, int64_t t_begin,
+__global__ void __launch_bounds__(kClassifyThreads) classify_tiles_kernel(CallArgs a, int pass, int min_bin, int64_t t_begin,
                                                                           int64_t t_end, int* bin_count,
                                                                           int32_t* bin_tiles,
                                                                           const int32_t* __restrict__ list,
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kClassifyThreads) classify_tiles_kernel(CallAr
     if (part && tt == 0) {
         const int m = smax[lt];
         const bool fast = a.precision == 1 && !(wflags & (kWinKeepLik | kWinExternalLik));
-        int bin = 0;
+        int bin = min_bin;
         while (bin < kNumBins - 1 && m > a.bin_limit[bin]) ++bin;
         my_bin = bin + (fast ? kNumBins : 0);
         my_rank = atomicAdd(&sbin_count[my_bin], 1);
@@ -499,17 +499,16 @@ static size_t fp64_smem_bytes(int slots, int L) {
 
 /* Classify tiles [t_begin, t_end) (with a list, list[t_begin, t_end); with
  * d_count, list[0, *d_count) read on the device, by a fixed grid of `grid`
- * CTAs) into the depth bins. */
-cudaError_t launch_classify(const CallArgs& a, int pass, int64_t t_begin, int64_t t_end, int* d_bin_count,
+ * CTAs) into the depth bins from min_bin on; d_bin_count's kBinCountInts ints
+ * are zero. */
+cudaError_t launch_classify(const CallArgs& a, int pass, int min_bin, int64_t t_begin, int64_t t_end, int* d_bin_count,
                             int32_t* d_bin_tiles, cudaStream_t stream, const int32_t* list, const int* d_count,
                             int grid) {
-    cudaError_t e = cudaMemsetAsync(d_bin_count, 0, sizeof(int) * kBinCountInts, stream);
-    if (e != cudaSuccess) return e;
     const unsigned blocks =
         d_count ? (unsigned)grid : (unsigned)((t_end - t_begin + kClassifyTiles - 1) / kClassifyTiles);
     if (blocks == 0) return cudaSuccess;
-    classify_tiles_kernel<<<blocks, kClassifyThreads, 0, stream>>>(a, pass, t_begin, t_end, d_bin_count, d_bin_tiles,
-                                                                   list, d_count);
+    classify_tiles_kernel<<<blocks, kClassifyThreads, 0, stream>>>(a, pass, min_bin, t_begin, t_end, d_bin_count,
+                                                                   d_bin_tiles, list, d_count);
     return cudaGetLastError();
 }
 

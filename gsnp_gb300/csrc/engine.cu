@@ -39,7 +39,7 @@
 
 namespace gsnp {
 
-cudaError_t launch_classify(const CallArgs& a, int pass, int64_t t_begin, int64_t t_end, int* d_bin_count,
+cudaError_t launch_classify(const CallArgs& a, int pass, int min_bin, int64_t t_begin, int64_t t_end, int* d_bin_count,
                             int32_t* d_bin_tiles, cudaStream_t stream, const int32_t* list = nullptr,
                             const int* d_count = nullptr, int grid = 0);
 cudaError_t launch_stream(const CallArgs& a, const StreamQueue& q, int slots, int mode, int ctas, int carveout,
@@ -96,9 +96,15 @@ __global__ void deferred_calls_kernel(const DeferredSite* __restrict__ ds, const
     }
 }
 
-/* dmax[i] = max(dmax[i], v[i]) for i < 2 (one thread each) */
-__global__ void track_max_kernel(const unsigned long long* __restrict__ v, unsigned long long* __restrict__ dmax) {
-    if (threadIdx.x < 2) dmax[threadIdx.x] = max(dmax[threadIdx.x], v[threadIdx.x]);
+/* out[site] = call of deferred site i, i < n; out is mapped host memory */
+__global__ void deferred_out_kernel(const DeferredSite* __restrict__ ds, const SiteCall* __restrict__ calls, int64_t n,
+                                    SiteCall* __restrict__ out) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint4* src = reinterpret_cast<const uint4*>(calls + ds[i].site);
+        uint4* dst = reinterpret_cast<uint4*>(out + ds[i].site);
+        dst[0] = src[0];
+        dst[1] = src[1];
+    }
 }
 
 /* bytes between device memory and mapped host memory (small control data) */
@@ -436,6 +442,22 @@ __global__ void __launch_bounds__(512) calib_count_smem_kernel(
 
 using namespace gsnp;
 
+/* What a calling pass counts on the device, cleared before it (gerror, which
+ * the gathers set, before the call) and copied to the host after it. */
+struct PassCtl {                         /* of one segment */
+    unsigned long long next;             /* the persistent kernel's tiles handed out, */
+    int n_leftover, pad;                 /* and left */
+    int bins[2][kBinCountInts];          /* by pass: tiles of the FP64 bins, of the fast bins, then hand-out counters */
+};
+struct Control {
+    int gerror;                          /* 2: a base other than ACGT/acgt, 3: index list mismatch */
+    int pad0[15];
+    int error, pad1[15];
+    unsigned long long stats[kNumStats];
+    unsigned long long dcount[2], pad2[6];
+};
+static_assert(sizeof(Control) == 256 && offsetof(Control, error) == 64, "control block layout");
+
 struct gsnp_context {
     int device = 0;
     std::string error;
@@ -489,6 +511,7 @@ struct gsnp_context {
     uint16_t* d_bq = nullptr;
     /* window plan */
     WindowPlan plan;
+    uint8_t* d_win = nullptr;       /* one buffer of the three tables */
     uint8_t* d_win_flags = nullptr;
     int32_t* d_win_lik_src = nullptr;
     int32_t* d_win_host_src = nullptr;
@@ -500,19 +523,22 @@ struct gsnp_context {
     int64_t out_sites = 0;
     bool have_counts = false, have_lik_keep = false;
     /* scratch */
+    /* The control block of the passes (Control, then one PassCtl per segment):
+     * one clear before a pass and one copy to the host after it. */
+    uint8_t* d_ctl = nullptr;
+    int ctl_segs = 0;               /* segments it has room for */
+    int* d_gerror = nullptr;        /* its parts */
     int* d_error = nullptr;
     unsigned long long* d_stats = nullptr;
-    int* d_bin_count = nullptr;     /* [kBinCountInts]: counts of the FP64 bins, then fast bins, then counters */
+    unsigned long long* d_dcount = nullptr;  /* [2] requested sites, record words */
     int32_t* d_bin_tiles = nullptr; /* [2 * kNumBins][n_tiles] */
     DeferredSite* d_dsites = nullptr;        /* sites the fast kernel deferred */
     uint32_t* d_dpool = nullptr;             /* their sorted records */
-    unsigned long long* d_dcount = nullptr;  /* [2] requested sites, record words */
     int64_t dsite_cap = 0, dpool_cap = 0;
     int64_t* d_warp_rng = nullptr;  /* [n_tiles][2] */
     int64_t* d_tile_rng = nullptr;  /* [n_tiles][2] */
-    /* the persistent FP32 kernel: its counters (tiles handed out, leftover
-     * count), the leftover tiles, its record slots and grid */
-    unsigned long long* d_stream_ctl = nullptr;
+    /* the persistent kernels: the leftover tiles (two lists, one a segment in
+     * turn), their record slots and grids */
     int32_t* d_leftover = nullptr;
     int stream_slots = 0, stream_ctas = 0, stream64_ctas = 0, stream_ctas_L = -1, stream_carveout = 72;
     bool stream_path = true;
@@ -563,8 +589,6 @@ struct gsnp_context {
     int bin_carveout[2][kNumBins] = {{0, 0, 0, 0, 0, 0, 0}, {0, 72, 72, 0, 0, 0, 0}};
     int bin_grid[2][kNumBins] = {};
     int grid_L = -1, deferred_grid = 0, classify_grid = 0, sms = 0;
-    unsigned long long* d_dmax = nullptr;   /* [2] largest deferred request of the call's segments */
-    int* d_bin_hist = nullptr;              /* [2][2 * kNumBins] bin counts of each pass (launch records) */
     cudaGraphExec_t graph_exec = nullptr;
     cudaStream_t capture_stream = nullptr;
     uint64_t graph_key = 0;
@@ -580,11 +604,11 @@ struct gsnp_context {
     static const int kMaxLaunches = 128;
     cudaEvent_t ev[2 * kMaxLaunches] = {};
     gsnp_launch_info launches[kMaxLaunches];
-    int launch_ref[kMaxLaunches] = {};   /* a device-driven bin launch: its count in d_bin_hist, else -1 */
+    int launch_ref[kMaxLaunches] = {};   /* a device-driven bin launch: its count's byte in the control block, else -1 */
     int n_launches = 0;
     uint64_t h2d_bytes = 0, d2h_bytes = 0;
     /* the call's copy streams: uploads in chunks, downloads per segment */
-    static const int kUploadChunks = 16;
+    static const int kUploadChunks = 32;   /* at most; of 4 MB at least */
     static const int kMaxUpStreams = 4;
     cudaStream_t up_stream = nullptr, down_stream = nullptr, gather_stream = nullptr;
     /* the upload's pieces go round-robin over n_up copy streams (up_stream is
@@ -598,9 +622,8 @@ struct gsnp_context {
      * wave overlaps the next bin's first */
     static const int kBinStreams = 3;
     cudaStream_t bin_stream[kBinStreams] = {};
-    cudaEvent_t ev_fork = nullptr, ev_join[kBinStreams] = {};
+    cudaEvent_t ev_fork = nullptr, ev_join[kBinStreams] = {}, ev_side[2] = {};
     cudaEvent_t ev_small = nullptr, ev_seg = nullptr, ev_chunk[kUploadChunks] = {};
-    int* d_gerror = nullptr;       /* gather: 2 a base other than ACGT/acgt, 3 index list mismatch */
     /* Pinned host memory mapped into the device: the small values the host
      * reads back between launches (bin counts, deferred counts, error flags,
      * statistics) and the window tables it sends.  A kernel moves them, so
@@ -616,6 +639,7 @@ struct gsnp_context {
     int32_t raw_pitch = 0;
     bool raw_packed = false;
     int packed_qmin = 0, gather_qmin = 0;
+    int gather_error = 0;          /* the control block's gerror as last fetched */
     /* cns text emission */
     void* d_emit = nullptr;
     size_t emit_bytes = 0;
@@ -725,16 +749,31 @@ int host_threads() {
     return n;
 }
 
-/* layout of the mapped control area */
-constexpr size_t kMapBins = 0;       /* int[2 * kNumBins] */
-constexpr size_t kMapDcount = 64;    /* unsigned long long[2] */
-constexpr size_t kMapError = 96;     /* int */
-constexpr size_t kMapGerror = 100;   /* int */
-constexpr size_t kMapLeftover = 104; /* int */
-constexpr size_t kMapStats = 128;    /* unsigned long long[kNumStats] */
-constexpr size_t kMapBinHist = 256;  /* int[2][2 * kNumBins]: each pass's bin counts */
-constexpr size_t kMapWindows = 512;  /* the call's window tables */
-static_assert(sizeof(int) * 2 * kNumBins <= kMapDcount, "bin counts overlap the deferred counts");
+size_t ctl_bytes(int segs) { return sizeof(Control) + (size_t)segs * sizeof(PassCtl); }
+
+/* the control block with room for segs segments */
+cudaError_t ensure_ctl(gsnp_context* c, int segs) {
+    if (segs <= c->ctl_segs) return cudaSuccess;
+    segs = std::max(segs, 17);
+    if (c->d_ctl) cudaFree(c->d_ctl);
+    c->d_ctl = nullptr;
+    c->ctl_segs = 0;
+    cudaError_t e = cudaMalloc((void**)&c->d_ctl, ctl_bytes(segs));
+    if (e == cudaSuccess) e = cudaMemset(c->d_ctl, 0, ctl_bytes(segs));
+    if (e != cudaSuccess) return e;
+    c->ctl_segs = segs;
+    c->d_gerror = reinterpret_cast<int*>(c->d_ctl + offsetof(Control, gerror));
+    c->d_error = reinterpret_cast<int*>(c->d_ctl + offsetof(Control, error));
+    c->d_stats = reinterpret_cast<unsigned long long*>(c->d_ctl + offsetof(Control, stats));
+    c->d_dcount = reinterpret_cast<unsigned long long*>(c->d_ctl + offsetof(Control, dcount));
+    return cudaSuccess;
+}
+PassCtl* pass_ctl(const gsnp_context* c, size_t seg) {
+    return reinterpret_cast<PassCtl*>(c->d_ctl + sizeof(Control)) + seg;
+}
+
+/* the mapped control area: a copy of the control block, then the window tables */
+size_t map_windows(const gsnp_context* c) { return (ctl_bytes(c->ctl_segs) + 255) & ~(size_t)255; }
 
 int ensure_map(gsnp_context* c, size_t bytes) {
     if (bytes <= c->map_bytes) return GSNP_OK;
@@ -751,8 +790,18 @@ int ensure_map(gsnp_context* c, size_t bytes) {
 
 /* device bytes to the mapped area at off, and back, on the context's stream */
 cudaError_t to_map(gsnp_context* c, const void* d_src, size_t off, size_t n) {
-    copy_bytes_kernel<<<1, 128, 0, c->stream>>>((const uint8_t*)d_src, c->d_map + off, n);
+    copy_bytes_kernel<<<(unsigned)std::max<size_t>(1, std::min<size_t>(8, n / 1024)), 256, 0, c->stream>>>(
+        (const uint8_t*)d_src, c->d_map + off, n);
     return cudaGetLastError();
+}
+
+/* the control block of a pass of segs segments to the host, once the stream's
+ * work is done */
+cudaError_t fetch_ctl(gsnp_context* c, size_t segs, Control* ctl) {
+    cudaError_t e = to_map(c, c->d_ctl, 0, ctl_bytes((int)segs));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) memcpy(ctl, c->h_map, sizeof *ctl);
+    return e;
 }
 
 cudaError_t from_map(gsnp_context* c, size_t off, void* d_dst, size_t n) {
@@ -763,13 +812,12 @@ cudaError_t from_map(gsnp_context* c, size_t off, void* d_dst, size_t n) {
 
 void free_all(gsnp_context* c) {
     void* ptrs[] = {c->d_tables, c->d_p_rank, c->d_codes, c->d_snp, c->d_snp_lp, c->d_snp_lp32, c->d_pos, c->d_lenhit,
-                    c->d_len, c->d_strand, c->d_bq, c->d_win_flags, c->d_win_lik_src, c->d_out, c->d_counts,
-                    c->d_lik_keep, c->d_error, c->d_stats, c->d_bin_count, c->d_bin_tiles, c->d_dsites,
-                    c->d_dpool, c->d_dcount, c->d_warp_rng, c->d_win_host_src, c->d_emit,
+                    c->d_len, c->d_strand, c->d_bq, c->d_win, c->d_out, c->d_counts,
+                    c->d_lik_keep, c->d_ctl, c->d_bin_tiles, c->d_dsites,
+                    c->d_dpool, c->d_warp_rng, c->d_emit,
                     c->d_text, c->d_chr, c->d_tile_snp, c->d_tile_rng, c->d_empty_calls, c->d_empty_valid,
                     c->d_raw_pos, c->d_raw_len, c->d_raw_hit, c->d_raw_strand, c->d_raw_seq, c->d_raw_qual,
-                    c->d_idx, c->d_dep_off, c->d_gerror, c->d_stream_ctl, c->d_leftover,
-                    c->d_dmax, c->d_patch, c->d_bin_hist};
+                    c->d_idx, c->d_dep_off, c->d_leftover, c->d_patch};
     for (void* p : ptrs)
         if (p) cudaFree(p);
 }
@@ -880,11 +928,12 @@ struct Segment {
  * on the device), after(s) once its calls are queued. */
 /* Allocations and one-time work of a calling pass, done before any of its
  * work is queued (and outside a graph capture). */
-int prepare_calling(gsnp_context* c) {
+int prepare_calling(gsnp_context* c, size_t segs) {
     /* the tile arrays hold the chromosome's tiles, or a streamed chunk's */
     const int64_t n_tiles = c->view.on ? c->view.tiles_need : (c->chr_len + kTile - 1) / kTile;
     {
-        const int rc = ensure_map(c, kMapWindows);
+        CK(ensure_ctl(c, (int)segs), "cudaMalloc control block");
+        const int rc = ensure_map(c, map_windows(c));
         if (rc != GSNP_OK) return rc;
     }
     if (!c->snp_lp_ready) {
@@ -903,10 +952,9 @@ int prepare_calling(gsnp_context* c) {
         CK(dev_alloc(&c->d_bin_tiles, (size_t)n_tiles * 2 * kNumBins), "cudaMalloc bins");
         CK(dev_alloc(&c->d_warp_rng, (size_t)n_tiles * 2), "cudaMalloc ranges");
         CK(dev_alloc(&c->d_tile_rng, (size_t)n_tiles * 2), "cudaMalloc ranges");
-        CK(dev_alloc(&c->d_leftover, (size_t)n_tiles), "cudaMalloc leftover tiles");
+        CK(dev_alloc(&c->d_leftover, (size_t)n_tiles * 2), "cudaMalloc leftover tiles");
         c->tiles_cap = n_tiles;
     }
-    if (!c->d_stream_ctl) CK(dev_alloc(&c->d_stream_ctl, 2), "cudaMalloc stream counters");
     if (c->stream_ctas_L != c->params.read_length || c->stream_slots == 0) {
         /* the persistent kernel's grid: every resident CTA of the GPU */
         if (c->stream_slots == 0) c->stream_slots = 48;
@@ -928,17 +976,13 @@ int prepare_calling(gsnp_context* c) {
         for (int i = 0; i < 2 * gsnp_context::kMaxLaunches; ++i) CK(cudaEventCreate(&c->ev[i]), "cudaEventCreate");
     if (!c->ev_fork) {
         CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming), "cudaEventCreate");
+        for (cudaEvent_t& e : c->ev_side) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         for (int i = 0; i < gsnp_context::kBinStreams; ++i) {
             CK(cudaStreamCreateWithFlags(&c->bin_stream[i], cudaStreamNonBlocking), "cudaStreamCreate");
             CK(cudaEventCreateWithFlags(&c->ev_join[i], cudaEventDisableTiming), "cudaEventCreate");
         }
     }
     if (c->device_driven) {
-        if (!c->d_dmax) CK(dev_alloc(&c->d_dmax, 2), "cudaMalloc");
-        if (!c->d_bin_hist) {
-            CK(dev_alloc(&c->d_bin_hist, 4 * kNumBins), "cudaMalloc");
-            CK(cudaMemset(c->d_bin_hist, 0, sizeof(int) * 4 * kNumBins), "memset");
-        }
         if (c->grid_L != c->params.read_length) {
             /* grids of the device-driven launches: the resident CTAs */
             CK(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device), "device attribute");
@@ -959,26 +1003,21 @@ int prepare_calling(gsnp_context* c) {
  * the mapped control area. */
 constexpr int kRedoDeferred = -100;   /* the deferred pool was too small: it was grown, call again */
 
-int finish_device(gsnp_context* c) {
-    CK(to_map(c, c->d_error, kMapError, sizeof(int)), "error flag");
-    CK(to_map(c, c->d_stats, kMapStats, sizeof(c->stats)), "stats");
-    CK(to_map(c, c->d_dmax, kMapDcount, sizeof(c->h_dcount)), "deferred counts");
-    if (c->d_bin_hist) CK(to_map(c, c->d_bin_hist, kMapBinHist, sizeof(int) * 4 * kNumBins), "bin counts");
-    CK(cudaStreamSynchronize(c->stream), "calling");
-    if (c->d_bin_hist) {
-        /* the tiles each recorded bin launch took, now that they are known */
-        int hist[4 * kNumBins];
-        memcpy(hist, c->h_map + kMapBinHist, sizeof hist);
-        for (int k = 0; k < c->n_launches; ++k)
-            if (c->launch_ref[k] >= 0) {
-                c->launches[k].tiles = hist[c->launch_ref[k]];
-                c->launches[k].sites = std::min<int64_t>((int64_t)hist[c->launch_ref[k]] * kTile, c->chr_len);
-            }
-    }
-    int err = 0;
-    memcpy(&err, c->h_map + kMapError, sizeof(int));
-    memcpy(c->stats, c->h_map + kMapStats, sizeof(c->stats));
-    memcpy(c->h_dcount, c->h_map + kMapDcount, sizeof(c->h_dcount));
+int finish_device(gsnp_context* c, size_t segs) {
+    Control ctl;
+    CK(fetch_ctl(c, segs, &ctl), "calling");
+    /* the tiles each recorded bin launch took, now that they are known */
+    for (int k = 0; k < c->n_launches; ++k)
+        if (c->launch_ref[k] >= 0) {
+            int tiles = 0;
+            memcpy(&tiles, c->h_map + c->launch_ref[k], sizeof tiles);
+            c->launches[k].tiles = tiles;
+            c->launches[k].sites = std::min<int64_t>((int64_t)tiles * kTile, c->chr_len);
+        }
+    const int err = ctl.error;
+    c->gather_error = ctl.gerror;
+    memcpy(c->stats, ctl.stats, sizeof(c->stats));
+    memcpy(c->h_dcount, ctl.dcount, sizeof(c->h_dcount));
     for (int k = 0; k < c->n_launches; ++k) cudaEventElapsedTime(&c->launches[k].ms, c->ev[2 * k], c->ev[2 * k + 1]);
     if (err == 1) return fail(c, GSNP_ERR_CAPACITY, "a site is covered by more than 65535 alignments");
     if (err == 5) return fail(c, GSNP_ERR_STATE, "a staging bulk copy of the calling kernel did not complete");
@@ -1012,23 +1051,31 @@ cudaError_t launch_stream_form(const gsnp_context* c, const CallArgs& a, const S
 
 /* device-driven queueing of a calling pass (defined below) */
 int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std::function<int(size_t)>& before,
-                   const std::function<int(size_t)>& after, bool record);
+                   const std::function<int(size_t, cudaStream_t)>& after, bool record);
 
 int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::function<int(size_t)>& before,
-                const std::function<int(size_t)>& after) {
-    const int64_t n_tiles = (c->chr_len + kTile - 1) / kTile;
+                const std::function<int(size_t, cudaStream_t)>& after) {
     c->deferred_at_end = false;
     {
-        const int rc = prepare_calling(c);
+        const int rc = prepare_calling(c, segs.size());
         if (rc != GSNP_OK) return rc;
     }
     if (c->device_driven) {
         const int rc = enqueue_device(c, segs, before, after, true);
         if (rc != GSNP_OK) return rc;
-        return finish_device(c);
+        return finish_device(c, segs.size());
     }
-    CK(cudaMemsetAsync(c->d_error, 0, sizeof(int), c->stream), "memset");
-    CK(cudaMemsetAsync(c->d_stats, 0, sizeof(unsigned long long) * kNumStats, c->stream), "memset");
+    CK(cudaMemsetAsync(c->d_error, 0, ctl_bytes(1) - offsetof(Control, error), c->stream), "memset");
+    PassCtl* const pc = pass_ctl(c, 0);
+    int* const d_bins = pc->bins[0];
+    Control ctl;
+    auto fetch = [&]() { return fetch_ctl(c, 1, &ctl); };
+    PassCtl host_pc;
+    auto fetch_pass = [&]() {
+        const cudaError_t e = fetch();
+        memcpy(&host_pc, c->h_map + sizeof(Control), sizeof host_pc);
+        return e;
+    };
     const CallArgs a = make_args(c);
     bool any_external = false;
     for (int64_t w = 0; w < c->plan.n_windows; ++w) any_external |= (c->plan.flags[w] & kWinExternalLik) != 0;
@@ -1110,11 +1157,11 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
         /* In the FP32 form the persistent kernel calls the segment's tiles;
          * the binned kernels take only the tiles it leaves (the FP64 windows'
          * and those with a site deeper than its record slots). */
-        const bool use_stream = c->stream_path && segs.size() == 1 && !c->view.on && stream_takes(c, a);
+        const bool use_stream = c->stream_path && stream_takes(c, a);
         int64_t n_left = 0;
         auto run_stream = [&](const CallArgs& as) -> int {
-            CK(cudaMemsetAsync(c->d_stream_ctl, 0, 2 * sizeof(unsigned long long), c->stream), "memset");
-            const StreamQueue q{g.t0, g.t1, c->d_stream_ctl, c->d_leftover, reinterpret_cast<int*>(c->d_stream_ctl + 1)};
+            CK(cudaMemsetAsync(pc, 0, 16, c->stream), "memset");
+            const StreamQueue q{g.t0, g.t1, &pc->next, c->d_leftover, &pc->n_leftover};
             const int ks = begin(kKindStream, c->stream_slots, g.t1 - g.t0);
             CK(launch_stream_form(c, as, q), "persistent calling kernel");
             end(ks);
@@ -1127,22 +1174,19 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
                 CK(cudaMemsetAsync(c->d_dcount, 0, sizeof(unsigned long long) * 2, c->stream), "memset");
                 const int rc = run_stream(a);
                 if (rc != GSNP_OK) return rc;
-                CK(to_map(c, c->d_stream_ctl + 1, kMapLeftover, sizeof(int)), "leftover count");
-                CK(cudaStreamSynchronize(c->stream), "persistent calling kernel");
-                int nl = 0;
-                memcpy(&nl, c->h_map + kMapLeftover, sizeof(int));
-                n_left = nl;
+                CK(fetch_pass(), "persistent calling kernel");
+                n_left = host_pc.n_leftover;
             }
             const int k = begin(kKindClassify, 0, use_stream ? n_left : g.t1 - g.t0);
+            CK(cudaMemsetAsync(d_bins, 0, sizeof(int) * kBinCountInts, c->stream), "memset");
             if (use_stream)
-                CK(launch_classify(a, pass, 0, n_left, c->d_bin_count, c->d_bin_tiles, c->stream, c->d_leftover),
+                CK(launch_classify(a, pass, 0, 0, n_left, d_bins, c->d_bin_tiles, c->stream, c->d_leftover),
                    "classify kernel");
             else
-                CK(launch_classify(a, pass, g.t0, g.t1, c->d_bin_count, c->d_bin_tiles, c->stream), "classify kernel");
+                CK(launch_classify(a, pass, 0, g.t0, g.t1, d_bins, c->d_bin_tiles, c->stream), "classify kernel");
             end(k);
-            CK(to_map(c, c->d_bin_count, kMapBins, sizeof(c->h_bin_count)), "bin counts");
-            CK(cudaStreamSynchronize(c->stream), "classify");
-            memcpy(c->h_bin_count, c->h_map + kMapBins, sizeof(c->h_bin_count));
+            CK(fetch_pass(), "classify");
+            memcpy(c->h_bin_count, host_pc.bins[0], sizeof(c->h_bin_count));
             bool any_fast = stream_pass;
             for (int b = 0; b < kNumBins; ++b) any_fast |= c->h_bin_count[kNumBins + b] > 0;
             {
@@ -1166,9 +1210,8 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
                     const int rc = launch_bins(af, kKindFast, kNumBins);
                     if (rc != GSNP_OK) return rc;
                 }
-                CK(to_map(c, c->d_dcount, kMapDcount, sizeof(c->h_dcount)), "deferred counts");
-                CK(cudaStreamSynchronize(c->stream), "fast calling");
-                memcpy(c->h_dcount, c->h_map + kMapDcount, sizeof(c->h_dcount));
+                CK(fetch(), "fast calling");
+                memcpy(c->h_dcount, ctl.dcount, sizeof(c->h_dcount));
                 const int64_t ns = (int64_t)c->h_dcount[0], nw = (int64_t)c->h_dcount[1];
                 if (ns <= c->dsite_cap && nw <= c->dpool_cap) {
                     if (ns > 0) {
@@ -1191,16 +1234,14 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
             }
         }
         if (after) {
-            const int rc = after(si);
+            const int rc = after(si, c->stream);
             if (rc != GSNP_OK) return rc;
         }
     }
-    int err = 0;
-    CK(to_map(c, c->d_error, kMapError, sizeof(int)), "error flag");
-    CK(to_map(c, c->d_stats, kMapStats, sizeof(c->stats)), "stats");
-    CK(cudaStreamSynchronize(c->stream), "calling");
-    memcpy(&err, c->h_map + kMapError, sizeof(int));
-    memcpy(c->stats, c->h_map + kMapStats, sizeof(c->stats));
+    CK(fetch(), "calling");
+    const int err = ctl.error;
+    c->gather_error = ctl.gerror;
+    memcpy(c->stats, ctl.stats, sizeof(c->stats));
     for (int k = 0; k < c->n_launches; ++k) cudaEventElapsedTime(&c->launches[k].ms, c->ev[2 * k], c->ev[2 * k + 1]);
     if (err == 1) return fail(c, GSNP_ERR_CAPACITY, "a site is covered by more than 65535 alignments");
     if (err == 5) return fail(c, GSNP_ERR_STATE, "a staging bulk copy of the calling kernel did not complete");
@@ -1212,21 +1253,23 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
 
 
 /* One pass queued with its launch sizes read on the device (see the
- * device_driven field of the context): per segment the tile ranges, in the
- * FP32 form the persistent kernel and the classification of the tiles it
- * leaves, the depth bins' kernels (each a grid of its resident CTAs taking the
- * bin's tiles in turn), the deferred pass, and, when the segment has windows
- * that take their likelihood from another window, the second pass of those.
- * Nothing here waits on the host.  record: launch records with events
- * (false while a graph is captured). */
+ * device_driven field of the context): per segment the tile ranges, the
+ * persistent kernel of the call's form and the classification of the tiles it
+ * leaves, their depth bins' kernels (each a grid of its resident CTAs taking
+ * the bin's tiles in turn), and, when the segment has windows that take their
+ * likelihood from another window, the second pass of those; then the deferred
+ * pass.  Nothing here waits on the host.  record: launch records with events
+ * (false while a graph is captured).
+ *
+ * With several segments the leftover tiles of one (a few, each of a whole
+ * tile's latency) run on a stream of their own beside the next segment's
+ * persistent kernel; after(s, stream) gets the stream that segment s's calls
+ * are final on. */
 int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std::function<int(size_t)>& before,
-                   const std::function<int(size_t)>& after, bool record) {
-    const int64_t n_tiles = (c->chr_len + kTile - 1) / kTile;
-    CK(cudaMemsetAsync(c->d_error, 0, sizeof(int), c->stream), "memset");
-    CK(cudaMemsetAsync(c->d_stats, 0, sizeof(unsigned long long) * kNumStats, c->stream), "memset");
-    CK(cudaMemsetAsync(c->d_dmax, 0, 2 * sizeof(unsigned long long), c->stream), "memset");
+                   const std::function<int(size_t, cudaStream_t)>& after, bool record) {
+    CK(cudaMemsetAsync(c->d_error, 0, ctl_bytes((int)segs.size()) - offsetof(Control, error), c->stream), "memset");
     c->n_launches = 0;
-    auto begin = [&](int kind, int sl, int64_t tiles) -> int {
+    auto begin = [&](int kind, int sl, int64_t tiles, cudaStream_t st) -> int {
         if (!record || c->n_launches >= gsnp_context::kMaxLaunches) return -1;
         const int k = c->n_launches++;
         c->launches[k].kind = kind;
@@ -1235,38 +1278,27 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
         c->launches[k].sites = std::min<int64_t>(tiles * kTile, c->chr_len);
         c->launches[k].ms = 0.f;
         c->launch_ref[k] = -1;
-        cudaEventRecord(c->ev[2 * k], c->stream);
+        cudaEventRecord(c->ev[2 * k], st);
         return k;
     };
-    auto end = [&](int k) {
-        if (k >= 0) cudaEventRecord(c->ev[2 * k + 1], c->stream);
+    auto end = [&](int k, cudaStream_t st) {
+        if (k >= 0) cudaEventRecord(c->ev[2 * k + 1], st);
     };
-    const bool fast = make_args(c).precision == 1;
-    /* the persistent kernel for a whole-chromosome pass: a call in segments
-     * (or chunks) ends each segment's launch of it in a tail of its own, and
-     * its binned kernels, handing out tiles from counters, were the faster
-     * there (c1 e2e in 7 segments: 28.6-29.0 against 29.9 ms) */
-    const bool use_stream = c->stream_path && segs.size() == 1 && !c->view.on && stream_takes(c, make_args(c));
-    int* d_left = reinterpret_cast<int*>(c->d_stream_ctl + 1);
+    const CallArgs a0 = make_args(c);
+    const bool fast = a0.precision == 1;
+    const bool use_stream = c->stream_path && stream_takes(c, a0);
+    const bool several = segs.size() > 1;
+    cudaStream_t const side = several && use_stream ? c->bin_stream[0] : c->stream;
+    /* after the persistent kernel in the general form (staged reads), the fast
+     * bins get only tiles deeper than its record slots; the short form leaves
+     * shallow tiles too, so few that the 64-slot bin takes them all */
+    int min_bin = 0;
+    if (use_stream && !(fast && c->stream_mode == 2))
+        while (kSlotsOf(min_bin) < kLeanG) ++min_bin;
     /* With several segments the deferred sites of all of them go to one pool
-     * and one deferred pass runs after the last segment: the pass takes about
-     * the time of its slowest site (one thread per site, serial FP64 work),
-     * whatever their number, so a pass per segment would cost that time per
-     * segment.  The segments' downloads then hold those sites pending, and
-     * call_chromosome patches them in (patch_deferred_calls). */
-    const bool defer_to_end = fast && segs.size() > 1;
-    c->deferred_at_end = defer_to_end;
-    if (defer_to_end) CK(cudaMemsetAsync(c->d_dcount, 0, sizeof(unsigned long long) * 2, c->stream), "memset");
-    auto deferred_pass = [&]() -> int {
-        CallArgs a = make_args(c);
-        a.n_reads = c->n_gathered;
-        const int kd = begin(kKindDeferred, 0, 0);
-        CK(launch_deferred(a, 0, c->stream, c->d_dcount, c->deferred_grid), "deferred calling kernel");
-        end(kd);
-        track_max_kernel<<<1, 2, 0, c->stream>>>(c->d_dcount, c->d_dmax);
-        CK(cudaGetLastError(), "deferred counts");
-        return GSNP_OK;
-    };
+     * and one deferred pass runs after the last segment, whose calls then are
+     * put into the host copy (patch_deferred_calls). */
+    c->deferred_at_end = fast && several;
     for (size_t si = 0; si < segs.size(); ++si) {
         const Segment& g = segs[si];
         if (before) {
@@ -1282,45 +1314,45 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
         }
         CallArgs a = make_args(c);
         a.n_reads = c->n_gathered;
-        int k = begin(kKindClassify, 0, g.t1 - g.t0);
+        PassCtl* const pc = pass_ctl(c, si);
+        int32_t* const left = c->d_leftover + (si & 1) * c->tiles_cap;
+        int k = begin(kKindClassify, 0, g.t1 - g.t0, c->stream);
         CK(launch_tile_bounds(a, g.dlo, g.dhi, g.next_pos, c->stream), "tile bounds kernel");
-        if (!defer_to_end) CK(cudaMemsetAsync(c->d_dcount, 0, sizeof(unsigned long long) * 2, c->stream), "memset");
         auto bins = [&](int kind, int pass) -> int {
             const int ki = kind == kKindFast ? 1 : 0;
-            for (int b = 0; b < kNumBins; ++b) {
-                /* after the persistent kernel in the general form (staged
-                 * reads), the fast bins get only tiles deeper than its record
-                 * slots; the short form leaves shallow tiles too */
-                if (kind == kKindFast && use_stream && c->stream_mode == 2 && kSlotsOf(b) <= c->stream_slots) continue;
-                const BinLaunch bl{0, c->d_bin_count + ki * kNumBins + b, c->bin_grid[ki][b], c->bin_carveout[ki][b],
-                                   c->d_bin_count + (2 + ki) * kNumBins + b};
-                const int kb = begin(launch_kind(kind, kSlotsOf(b)), kSlotsOf(b), 0);
-                if (kb >= 0) c->launch_ref[kb] = pass * 2 * kNumBins + ki * kNumBins + b;
-                CK(launch_bin(a, kind, b, c->d_bin_tiles + (int64_t)(ki * kNumBins + b) * c->tiles_cap, bl, c->stream),
+            for (int b = pass == 0 ? min_bin : 0; b < kNumBins; ++b) {
+                if (kind == kKindFast && use_stream && min_bin == 0 && kSlotsOf(b) <= c->stream_slots) continue;
+                int* const cnt = pc->bins[pass] + ki * kNumBins + b;
+                const BinLaunch bl{0, cnt, c->bin_grid[ki][b], c->bin_carveout[ki][b], cnt + 2 * kNumBins};
+                const int kb = begin(launch_kind(kind, kSlotsOf(b)), kSlotsOf(b), 0, side);
+                if (kb >= 0) c->launch_ref[kb] = (int)(reinterpret_cast<uint8_t*>(cnt) - c->d_ctl);
+                CK(launch_bin(a, kind, b, c->d_bin_tiles + (int64_t)(ki * kNumBins + b) * c->tiles_cap, bl, side),
                    "calling kernel");
-                end(kb);
+                end(kb, side);
             }
             return GSNP_OK;
         };
         /* pass 0 */
         if (use_stream) {
-            CK(cudaMemsetAsync(c->d_stream_ctl, 0, 2 * sizeof(unsigned long long), c->stream), "memset");
-            end(k);
-            const StreamQueue q{g.t0, g.t1, c->d_stream_ctl, c->d_leftover, d_left};
-            const int ks = begin(kKindStream, c->stream_slots, g.t1 - g.t0);
+            end(k, c->stream);
+            /* the leftover list of the segment before last is done with */
+            if (side != c->stream && si >= 2) CK(cudaStreamWaitEvent(c->stream, c->ev_side[si & 1], 0), "wait");
+            const StreamQueue q{g.t0, g.t1, &pc->next, left, &pc->n_leftover};
+            const int ks = begin(kKindStream, c->stream_slots, g.t1 - g.t0, c->stream);
             CK(launch_stream_form(c, a, q), "persistent calling kernel");
-            end(ks);
-            k = begin(kKindClassify, 0, 0);
-            CK(launch_classify(a, 0, 0, 0, c->d_bin_count, c->d_bin_tiles, c->stream, c->d_leftover, d_left,
+            end(ks, c->stream);
+            if (side != c->stream) {
+                CK(cudaEventRecord(c->ev_fork, c->stream), "event");
+                CK(cudaStreamWaitEvent(side, c->ev_fork, 0), "wait");
+            }
+            k = begin(kKindClassify, 0, 0, side);
+            CK(launch_classify(a, 0, min_bin, 0, 0, pc->bins[0], c->d_bin_tiles, side, left, &pc->n_leftover,
                                c->classify_grid),
                "classify kernel");
         } else {
-            CK(launch_classify(a, 0, g.t0, g.t1, c->d_bin_count, c->d_bin_tiles, c->stream), "classify kernel");
+            CK(launch_classify(a, 0, 0, g.t0, g.t1, pc->bins[0], c->d_bin_tiles, side), "classify kernel");
         }
-        end(k);
-        CK(cudaMemcpyAsync(c->d_bin_hist, c->d_bin_count, sizeof(int) * 2 * kNumBins, cudaMemcpyDeviceToDevice,
-                           c->stream),
-           "bin counts");
+        end(k, side);
         if (!fast || keep_lik) {
             const int rc = bins(kKindFP64, 0);
             if (rc != GSNP_OK) return rc;
@@ -1328,47 +1360,63 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
         if (fast) {
             const int rc = bins(kKindFast, 0);
             if (rc != GSNP_OK) return rc;
-            if (!defer_to_end) {
-                const int rd = deferred_pass();
-                if (rd != GSNP_OK) return rd;
-            }
         }
         /* pass 1: the windows whose likelihood another window kept */
         if (external) {
-            const int kc = begin(kKindClassify, 0, 0);
+            const int kc = begin(kKindClassify, 0, 0, side);
             if (use_stream)
-                CK(launch_classify(a, 1, 0, 0, c->d_bin_count, c->d_bin_tiles, c->stream, c->d_leftover, d_left,
+                CK(launch_classify(a, 1, 0, 0, 0, pc->bins[1], c->d_bin_tiles, side, left, &pc->n_leftover,
                                    c->classify_grid),
                    "classify kernel");
             else
-                CK(launch_classify(a, 1, g.t0, g.t1, c->d_bin_count, c->d_bin_tiles, c->stream), "classify kernel");
-            end(kc);
-            CK(cudaMemcpyAsync(c->d_bin_hist + 2 * kNumBins, c->d_bin_count, sizeof(int) * 2 * kNumBins,
-                               cudaMemcpyDeviceToDevice, c->stream),
-               "bin counts");
+                CK(launch_classify(a, 1, 0, g.t0, g.t1, pc->bins[1], c->d_bin_tiles, side), "classify kernel");
+            end(kc, side);
             const int rc = bins(kKindFP64, 1);
             if (rc != GSNP_OK) return rc;
         }
-        if (after) {
-            const int rc = after(si);
+        if (side != c->stream) CK(cudaEventRecord(c->ev_side[si & 1], side), "event");
+        if (after && (several || !fast)) {
+            const int rc = after(si, side);
             if (rc != GSNP_OK) return rc;
         }
     }
-    if (defer_to_end) return deferred_pass();
+    if (side != c->stream) CK(cudaStreamWaitEvent(c->stream, c->ev_side[(segs.size() - 1) & 1], 0), "wait");
+    if (fast) {
+        CallArgs a = make_args(c);
+        a.n_reads = c->n_gathered;
+        const int kd = begin(kKindDeferred, 0, 0, c->stream);
+        CK(launch_deferred(a, 0, c->stream, c->d_dcount, c->deferred_grid), "deferred calling kernel");
+        end(kd, c->stream);
+        if (after && !several) return after(0, c->stream);
+    }
     return GSNP_OK;
 }
 
 /* After a pass whose deferred sites ran once after its last segment: their
  * final calls into the host copy `out`, whose segments were downloaded with
- * those sites still pending.  The streams that wrote `out` are idle. */
+ * those sites still pending.  The streams that wrote `out` are idle.  Page-
+ * locked memory the kernel writes directly; other memory gets a list. */
 int patch_deferred_calls(gsnp_context* c, gsnp_site_call* out) {
     const int64_t n = std::min<int64_t>((int64_t)c->h_dcount[0], c->dsite_cap);
     if (n <= 0) return GSNP_OK;
+    c->d2h_bytes += (uint64_t)n * sizeof(DeferredCall);
+    const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, 1024);
+    cudaPointerAttributes first{}, last{};
+    if (cudaPointerGetAttributes(&first, out) == cudaSuccess && first.type == cudaMemoryTypeHost &&
+        first.devicePointer && cudaPointerGetAttributes(&last, out + c->chr_len - 1) == cudaSuccess &&
+        last.type == cudaMemoryTypeHost && last.devicePointer &&
+        (SiteCall*)last.devicePointer - (SiteCall*)first.devicePointer == c->chr_len - 1 &&
+        ((uintptr_t)first.devicePointer & 15) == 0) {
+        deferred_out_kernel<<<blocks, 256, 0, c->stream>>>(c->d_dsites, c->d_out, n, (SiteCall*)first.devicePointer);
+        CK(cudaGetLastError(), "deferred calls");
+        CK(cudaStreamSynchronize(c->stream), "deferred calls");
+        return GSNP_OK;
+    }
+    (void)cudaGetLastError();
     if (n > c->patch_cap) {
         CK(dev_alloc(&c->d_patch, (size_t)n), "cudaMalloc deferred calls");
         c->patch_cap = n;
     }
-    const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, 1024);
     deferred_calls_kernel<<<blocks, 256, 0, c->stream>>>(c->d_dsites, c->d_out, n, c->d_patch);
     CK(cudaGetLastError(), "deferred calls");
     std::vector<DeferredCall> h((size_t)n);
@@ -1377,7 +1425,6 @@ int patch_deferred_calls(gsnp_context* c, gsnp_site_call* out) {
     CK(cudaStreamSynchronize(c->stream), "download");
     SiteCall* o = reinterpret_cast<SiteCall*>(out);
     for (const DeferredCall& d : h) o[d.site] = d.call;
-    c->d2h_bytes += (uint64_t)n * sizeof(DeferredCall);
     return GSNP_OK;
 }
 
@@ -1445,10 +1492,14 @@ int regather(gsnp_context* c) {
     return GSNP_OK;
 }
 
-/* number of segments of a call: one per two million deposited reads, 1 .. 16
- * (GSNP_SEGMENTS overrides) */
-int segment_count(int64_t n_dep, int64_t n_windows) {
-    int n = (int)std::min<int64_t>(16, std::max<int64_t>(1, n_dep / 2000000));
+/* Number of segments of a call that moves `bytes` over the host link
+ * (GSNP_SEGMENTS overrides).  With S segments the first one's upload and the
+ * last one's download are not overlapped, bytes / (S x 200 GB/s) in all, and
+ * each segment adds about 50 us (the last tiles of its persistent kernel, its
+ * launches); the sum is least at S = sqrt(bytes / 10 MB).  c1 (16 Mbp, packed,
+ * 1.05 GB): 8.2 ms in the 2 segments of one per two million reads, 5.9 in 10. */
+int segment_count(uint64_t bytes, int64_t n_windows) {
+    int n = (int)std::min(16.0, std::max(1.0, std::floor(std::sqrt((double)bytes / 10e6) + 0.5)));
     if (const char* e = getenv("GSNP_SEGMENTS")) n = std::max(1, atoi(e));
     return (int)std::max<int64_t>(1, std::min<int64_t>(n, n_windows));
 }
@@ -1475,7 +1526,6 @@ int ensure_call_streams(gsnp_context* c) {
     CK(cudaEventCreateWithFlags(&c->ev_seg, cudaEventDisableTiming), "cudaEventCreate");
     for (int i = 0; i < gsnp_context::kUploadChunks; ++i)
         CK(cudaEventCreateWithFlags(&c->ev_chunk[i], cudaEventDisableTiming), "cudaEventCreate");
-    CK(dev_alloc(&c->d_gerror, 1), "cudaMalloc");
     return GSNP_OK;
 }
 
@@ -1524,7 +1574,9 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
         c->raw_cap = cap;
         c->raw_bytes = std::max<size_t>(raw, 1);
     }
-    const int64_t chunk_rows = std::max<int64_t>(1, (n + gsnp_context::kUploadChunks - 1) / gsnp_context::kUploadChunks);
+    const int pieces = (int)std::max<int64_t>(
+        1, std::min<int64_t>(gsnp_context::kUploadChunks, (int64_t)((r->packed ? 1 : 2) * raw >> 22)));
+    const int64_t chunk_rows = std::max<int64_t>(1, (n + pieces - 1) / pieces);
     GpuTimeline tl(timer.on);
     tl.rec("start", c->up_stream);
     if (n > 0) {
@@ -1538,7 +1590,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
         /* the other copy streams start after the small arrays' copies */
         for (int i = 0; i + 1 < c->n_up; ++i) CK(cudaStreamWaitEvent(c->up_extra[i], c->ev_small, 0), "wait");
     }
-    for (int k = 0; k < gsnp_context::kUploadChunks; ++k) {
+    for (int k = 0; k < pieces; ++k) {
         const int64_t b = std::min(n, k * chunk_rows), e = std::min(n, (k + 1) * chunk_rows);
         cudaStream_t us = c->up(k);
         if (e > b) {
@@ -1553,7 +1605,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
             }
         }
         CK(cudaEventRecord(c->ev_chunk[k], us), "event");
-        if (k == 0 || k == gsnp_context::kUploadChunks / 2 - 1 || k == gsnp_context::kUploadChunks - 1)
+        if (k == 0 || k == pieces / 2 - 1 || k == pieces - 1)
             tl.rec("uploaded piece " + std::to_string(k), us);
     }
     timer.mark("uploads issued");
@@ -1582,30 +1634,41 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
     timer.mark("window replay");
     const WindowPlan& P = c->plan;
     const int64_t nd = P.n_deposited;
-
-    /* window tables */
-    if (P.n_windows > c->n_win_alloc) {
-        CK(dev_alloc(&c->d_win_flags, (size_t)P.n_windows), "cudaMalloc");
-        CK(dev_alloc(&c->d_win_lik_src, (size_t)P.n_windows), "cudaMalloc");
-        CK(dev_alloc(&c->d_win_host_src, (size_t)P.n_windows), "cudaMalloc");
-        c->n_win_alloc = P.n_windows;
-    }
+    const std::vector<Segment> segs = plan_segments(
+        c, v, segment_count((uint64_t)n * (13 + (r->packed ? 1 : 2) * (uint64_t)r->pitch) +
+                                (out ? (uint64_t)c->chr_len * sizeof(SiteCall) : 0),
+                            P.n_windows));
     {
-        /* through the mapped area: a copy on the copy engine would wait for
-         * the alignment uploads queued before it */
-        const size_t nw = (size_t)P.n_windows, off_f = kMapWindows, off_l = off_f + ((nw + 15) & ~(size_t)15),
-                     off_h = off_l + nw * 4;
-        const int rcm = ensure_map(c, off_h + nw * 4);
+        /* before the window tables take their place after it */
+        const cudaError_t e = ensure_ctl(c, (int)segs.size());
+        if (e != cudaSuccess) {
+            drain();
+            return cuda_fail(c, e, "cudaMalloc control block");
+        }
+    }
+
+    /* window tables, through the mapped area: a copy on the copy engine would
+     * wait for the alignment uploads queued before it */
+    {
+        const size_t nw = (size_t)P.n_windows, off_l = (nw + 15) & ~(size_t)15, off_h = off_l + nw * 4;
+        if (P.n_windows > c->n_win_alloc) {
+            c->n_win_alloc = 0;
+            CK(dev_alloc(&c->d_win, nw * 9 + 16), "cudaMalloc");
+            c->n_win_alloc = P.n_windows;
+        }
+        c->d_win_flags = c->d_win;
+        c->d_win_lik_src = reinterpret_cast<int32_t*>(c->d_win + off_l);
+        c->d_win_host_src = reinterpret_cast<int32_t*>(c->d_win + off_h);
+        const size_t at = map_windows(c);
+        const int rcm = ensure_map(c, at + off_h + nw * 4);
         if (rcm != GSNP_OK) {
             drain();
             return rcm;
         }
-        memcpy(c->h_map + off_f, P.flags.data(), nw);
-        memcpy(c->h_map + off_l, P.lik_src.data(), nw * 4);
-        memcpy(c->h_map + off_h, P.host_src.data(), nw * 4);
-        CK(from_map(c, off_f, c->d_win_flags, nw), "window tables");
-        CK(from_map(c, off_l, c->d_win_lik_src, nw * 4), "window tables");
-        CK(from_map(c, off_h, c->d_win_host_src, nw * 4), "window tables");
+        memcpy(c->h_map + at, P.flags.data(), nw);
+        memcpy(c->h_map + at + off_l, P.lik_src.data(), nw * 4);
+        memcpy(c->h_map + at + off_h, P.host_src.data(), nw * 4);
+        CK(from_map(c, at, c->d_win, off_h + nw * 4), "window tables");
     }
     bool need_counts = false, need_lik = false;
     for (int64_t w = 0; w < P.n_windows; ++w) {
@@ -1662,7 +1725,6 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
      *    is called once it is gathered), calls, downloads */
     CK(cudaEventRecord(c->ev_index, c->stream), "event");
     CK(cudaStreamWaitEvent(c->gather_stream, c->ev_index, 0), "wait");
-    const std::vector<Segment> segs = plan_segments(c, v, segment_count(nd, P.n_windows));
     while (c->ev_gather.size() < segs.size()) {
         cudaEvent_t e;
         CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
@@ -1674,7 +1736,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
         while (gathered_seg < target) {
             const Segment& g = segs[(size_t)++gathered_seg];
             if (g.dhi > g.dlo) {
-                const int64_t chunk = std::min<int64_t>((g.raw_hi - 1) / chunk_rows, gsnp_context::kUploadChunks - 1);
+                const int64_t chunk = std::min<int64_t>((g.raw_hi - 1) / chunk_rows, pieces - 1);
                 /* every piece up to the one holding the segment's last row
                  * (the pieces of several copy streams finish in any order) */
                 for (; waited_chunk < chunk; ++waited_chunk)
@@ -1705,12 +1767,12 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
         tl.rec("calling " + std::to_string(si), c->stream);
         return GSNP_OK;
     };
-    auto after = [&](size_t si) -> int {
-        tl.rec("called " + std::to_string(si), c->stream);
+    auto after = [&](size_t si, cudaStream_t st) -> int {
+        tl.rec("called " + std::to_string(si), st);
         if (!out) return GSNP_OK;
         const int64_t s0 = segs[si].t0 * kTile, s1 = std::min(segs[si].t1 * kTile, c->chr_len);
         if (s1 <= s0) return GSNP_OK;
-        CK(cudaEventRecord(c->ev_seg, c->stream), "event");
+        CK(cudaEventRecord(c->ev_seg, st), "event");
         CK(cudaStreamWaitEvent(c->down_stream, c->ev_seg, 0), "wait");
         CK(cudaMemcpyAsync(out + s0, c->d_out + s0, (size_t)(s1 - s0) * sizeof(SiteCall), cudaMemcpyDeviceToHost,
                            c->down_stream),
@@ -1748,10 +1810,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
     CK(e_up, "upload");
     CK(e_down, "download");
     CK(e_gather, "gather");
-    int gerr = 0;
-    CK(to_map(c, c->d_gerror, kMapGerror, sizeof(int)), "error flag");
-    CK(cudaStreamSynchronize(c->stream), "error flag");
-    memcpy(&gerr, c->h_map + kMapGerror, sizeof(int));
+    const int gerr = c->gather_error;   /* fetched after the last segment's pass, which waits for its gather */
     if (gerr == 3) return fail(c, GSNP_ERR_STATE, "deposited alignment list does not match the window replay");
     if (gerr) return fail(c, GSNP_ERR_INPUT, "unknown base when encoding (only ACGT/acgt are accepted)");
     if (out && c->deferred_at_end) return patch_deferred_calls(c, out);
@@ -1805,10 +1864,7 @@ int gsnp_context_create(int device, gsnp_context** out) {
     c->device = device;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_error, sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_stats, sizeof(unsigned long long) * kNumStats);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_bin_count, sizeof(int) * kBinCountInts);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_dcount, sizeof(unsigned long long) * 2);
+    if (e == cudaSuccess) e = ensure_ctl(c, 1);
     if (e != cudaSuccess) {
         free_all(c);
         delete c;
@@ -1878,6 +1934,8 @@ void gsnp_context_destroy(gsnp_context* c) {
         }
     }
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+    for (cudaEvent_t e : c->ev_side)
+        if (e) cudaEventDestroy(e);
     if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
     if (c->capture_stream) cudaStreamDestroy(c->capture_stream);
     for (cudaEvent_t e : c->ev_gather) cudaEventDestroy(e);
@@ -2121,7 +2179,7 @@ uint64_t graph_key_of(gsnp_context* c, const Segment& g) {
     mix(c->bin_grid, sizeof c->bin_grid);
     mix(c->bin_carveout, sizeof c->bin_carveout);
     mix(&c->n_gathered, sizeof c->n_gathered);
-    const void* ptrs[] = {c->d_leftover, c->d_stream_ctl, c->d_dmax, c->d_bin_tiles, c->d_bin_count};
+    const void* ptrs[] = {c->d_leftover, c->d_ctl, c->d_bin_tiles};
     mix(ptrs, sizeof ptrs);
     return h;
 }
@@ -2131,7 +2189,7 @@ uint64_t graph_key_of(gsnp_context* c, const Segment& g) {
  * changes. */
 int recall_graph(gsnp_context* c) {
     {
-        const int rc = prepare_calling(c);
+        const int rc = prepare_calling(c, 1);
         if (rc != GSNP_OK) return rc;
     }
     const std::vector<Segment> segs{whole_segment(c)};
@@ -2180,7 +2238,7 @@ int recall_graph(gsnp_context* c) {
     cudaEventRecord(c->ev[0], c->stream);
     CK(cudaGraphLaunch(c->graph_exec, c->stream), "graph launch");
     cudaEventRecord(c->ev[1], c->stream);
-    return finish_device(c);
+    return finish_device(c, 1);
 }
 
 }  // namespace gsnp
@@ -2216,6 +2274,10 @@ int gsnp_tune(gsnp_context* c, int sample_windows, char* report, size_t report_c
     if (!c->called || !c->have_tables || c->n_gathered < c->n_dep)
         return fail(c, GSNP_ERR_STATE, "tuning samples the resident reads of a finished call");
     cudaSetDevice(c->device);
+    {
+        const int rg = regather(c);
+        if (rg != GSNP_OK) return rg;
+    }
     const WindowPlan& P = c->plan;
     const int64_t n_tiles = (c->chr_len + kTile - 1) / kTile;
     const int64_t w0 = P.n_windows / 3, w1 = std::min<int64_t>(P.n_windows, w0 + std::max(1, sample_windows));
@@ -3001,10 +3063,7 @@ int call_streamed(gsnp_context* c, const gsnp_reads* r, const char* chr_name, gs
     close_outputs();
     timer.mark("chunks");
     if (rc != GSNP_OK) return rc;
-    int gerr = 0;
-    CK(to_map(c, c->d_gerror, kMapGerror, sizeof(int)), "error flag");
-    CK(cudaStreamSynchronize(c->stream), "error flag");
-    memcpy(&gerr, c->h_map + kMapGerror, sizeof(int));
+    const int gerr = nk > 0 ? c->gather_error : 0;   /* fetched with each chunk's pass */
     if (gerr == 3) return fail(c, GSNP_ERR_STATE, "deposited alignment list does not match the window replay");
     if (gerr) return fail(c, GSNP_ERR_INPUT, "unknown base when encoding (only ACGT/acgt are accepted)");
     totals[0] = (uint64_t)c->chr_len;
