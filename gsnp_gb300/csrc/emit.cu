@@ -9,11 +9,22 @@
  * come from make_row (rows.h), which reproduces the reference's stale host
  * count arrays in gap windows.
  *
- * The text of a range of sites is built in three steps: every thread formats
- * its row once to learn its length, an exclusive scan turns the lengths into
- * byte offsets, and every thread formats its row again into place.
+ * The text of a range of sites is built in three steps over blocks of kRows
+ * rows.  A first kernel measures the rows and leaves each block's byte count;
+ * one CTA scans those into byte offsets (8 bytes per 128 rows instead of 12
+ * bytes per row); the write kernel measures again - its rows' values stay in
+ * registers - scans the 128 lengths in the CTA, puts the characters into
+ * shared memory and stores them as aligned 16-byte words.  A row's call is
+ * read twice (64 bytes) against 66 bytes of text written; the link that takes
+ * the text to the host is what bounds a program that wants it.
+ * 4 M rows of the 10x shape, 264 MB, size and text wanted: 20.1 -> 1.78 ms,
+ * 1.37 of it the copy to the host (before: a row per thread formatted in local
+ * memory and stored byte by byte, 1.7 ms in the write kernel alone, and a
+ * host thread's memcpy out of a pinned buffer).
  */
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "emit.h"
 #include "fmt_g6.h"
@@ -26,113 +37,185 @@ namespace {
 __constant__ char c_abbv[17] = {'A', 'M', 'W', 'R', 'M', 'C', 'Y', 'S', 'W', 'Y', 'T', 'K', 'R', 'S', 'K', 'G', 'N'};
 __constant__ char c_actgn[8] = {'A', 'C', 'T', 'G', 'N', 'N', 'N', 'N'};
 
-constexpr int kRowMax = 384;          /* chromosome name (<= 255) + fields */
+constexpr int kRows = kEmitRows;      /* rows of a CTA, one per thread */
+constexpr int kRowFields = 128;       /* most characters of a row after the name (the fields add up to 111) */
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
-constexpr int kScanBlock = kScanThreads * kScanItems;
+__constant__ char c_nlit[] = "\tN\tN\t0\tN\t0\t0\t0\tN\t0\t0\t0\t0\t1.000\t255.000\t0\n";
+constexpr int kNLen = (int)sizeof(c_nlit) - 1;
 
-struct Out {
-    char* p;
-    int n;
-    __device__ void c(char x) { p[n++] = x; }
-    __device__ void s(const char* x, int len) {
-        for (int i = 0; i < len; ++i) p[n++] = x[i];
+__device__ __forceinline__ int digits(uint32_t v) {
+    int n = 1;
+    if (v >= 10000) {
+        n = 5;
+        v /= 10000;
+        if (v >= 10000) return 9 + (v >= 100000);
     }
-    __device__ void u(uint64_t v) {
-        char d[20];
-        int k = 0;
-        do {
-            d[k++] = (char)('0' + v % 10);
-            v /= 10;
-        } while (v);
-        while (k) p[n++] = d[--k];
+    return n + (v >= 10) + (v >= 100) + (v >= 1000);
+}
+
+__device__ __forceinline__ int digits_i(int v) { return v < 0 ? 1 + digits(0u - (uint32_t)v) : digits((uint32_t)v); }
+
+/* v's digits at p, from the back; returns the end */
+__device__ __forceinline__ char* put_u(char* p, uint32_t v, int n) {
+    for (int i = n - 1; i >= 0; --i) {
+        const uint32_t q = v / 10;
+        p[i] = (char)('0' + (v - q * 10));
+        v = q;
     }
-    __device__ void i(int v) {
-        if (v < 0) {
-            c('-');
-            u((uint64_t)(-(int64_t)v));
-        } else {
-            u((uint64_t)v);
-        }
+    return p + n;
+}
+
+__device__ __forceinline__ char* put_i(char* p, int v) {
+    if (v < 0) {
+        *p++ = '-';
+        v = (int)(0u - (uint32_t)v);
     }
-    __device__ bool g(double v) {
-        const int k = fmt_g6(v, p + n);
-        n += k;
-        return k > 0;
-    }
+    return put_u(p, (uint32_t)v, digits((uint32_t)v));
+}
+
+/* One row: its values and the length of its text, 0 when a double is outside
+ * the exact formatter's range. */
+struct Row {
+    CnsRow r;
+    G6 rank, ratio;
+    uint32_t pos;       /* 1-based */
+    int len;
+    bool ok;
 };
 
-/* Format the row of site `site`; returns its length, or -1 when a double is
- * outside the exact formatter's range. */
-__device__ int format_row(const EmitArgs& e, int64_t site, char* buf) {
+__device__ __forceinline__ Row measure_row(const EmitArgs& e, int64_t site) {
+    Row o;
     const int64_t w = site / kWin, j = site - w * kWin;
-    const CnsRow r = make_row(e.host_src[w], w, j, e.codes, e.calls, e.counts);
-    Out o{buf, 0};
-    o.s(e.chr, e.chr_n);
-    o.c('\t');
-    o.u((uint64_t)(site + 1));
+    o.r = make_row(e.host_src[w], w, j, e.codes, e.calls, e.counts);
+    o.pos = (uint32_t)(site + 1);
+    o.ok = true;
+    o.len = e.chr_n + 1 + digits(o.pos);
+    const CnsRow& r = o.r;
     if (!r.called()) {
-        const char lit[] = "\tN\tN\t0\tN\t0\t0\t0\tN\t0\t0\t0\t0\t1.000\t255.000\t0\n";
-        o.s(lit, (int)sizeof(lit) - 1);
-        return o.n;
+        o.len += kNLen;
+        return o;
     }
-    o.c('\t');
-    o.c(c_actgn[r.ori & 7]);
-    o.c('\t');
-    o.c(c_abbv[r.type1]);
-    o.c('\t');
-    o.i(r.q_cns);
-    o.c('\t');
-    o.c(c_actgn[r.base1]);
-    o.c('\t');
-    o.i(r.avg1);
-    o.c('\t');
-    o.i(r.cu1);
-    o.c('\t');
-    o.i(r.ca1);
-    o.c('\t');
-    if (r.base2 < 4) {
-        o.c(c_actgn[r.base2]);
-        o.c('\t');
-        o.i(r.avg2);
-        o.c('\t');
-        o.i(r.cu2);
-        o.c('\t');
-        o.i(r.ca2);
-    } else {
-        o.s("N\t0\t0\t0", 7);
+    o.rank = fmt_g6_parse(r.rank_sum);
+    o.ratio = fmt_g6_parse(r.depth == 0 ? 255.0 : (double)r.repeat / r.depth);
+    /* 15 tabs after the position; ref, type, base1, dbsnp, end of line */
+    o.len += 15 + 5 + digits_i(r.q_cns) + digits_i(r.avg1) + digits_i(r.cu1) + digits_i(r.ca1);
+    o.len += r.base2 < 4 ? 1 + digits_i(r.avg2) + digits_i(r.cu2) + digits_i(r.ca2) : 4;
+    o.len += digits(r.depth) + o.rank.len + o.ratio.len;
+    if (o.rank.len == 0 || o.ratio.len == 0) {
+        o.ok = false;
+        o.len = 0;
     }
-    o.c('\t');
-    o.u(r.depth);
-    o.c('\t');
-    bool ok = o.g(r.rank_sum);
-    o.c('\t');
-    ok = ok && o.g(r.depth == 0 ? 255.0 : (double)r.repeat / r.depth);
-    o.c('\t');
-    o.c((r.ori & 8) ? '1' : '0');
-    o.c('\n');
-    return ok ? o.n : -1;
+    return o;
 }
 
-__global__ void row_len_kernel(EmitArgs e) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= e.n) return;
-    char buf[kRowMax];
-    const int len = format_row(e, e.site0 + i, buf);
-    if (len < 0) atomicExch(e.error, 1);
-    e.len[i] = len < 0 ? 0u : (uint32_t)len;
+__device__ __forceinline__ void put_row(const EmitArgs& e, const Row& o, const char* name, char* p) {
+    const CnsRow& r = o.r;
+    for (int i = 0; i < e.chr_n; ++i) *p++ = name[i];
+    *p++ = '\t';
+    p = put_u(p, o.pos, digits(o.pos));
+    if (!r.called()) {
+        for (int i = 0; i < kNLen; ++i) p[i] = c_nlit[i];
+        return;
+    }
+    *p++ = '\t';
+    *p++ = c_actgn[r.ori & 7];
+    *p++ = '\t';
+    *p++ = c_abbv[r.type1];
+    *p++ = '\t';
+    p = put_i(p, r.q_cns);
+    /* base, avgQ, unique and all counts of the best and the second base */
+    for (int k = 0; k < 2; ++k) {
+        const bool any = k == 0 || r.base2 < 4;
+        *p++ = '\t';
+        *p++ = any ? c_actgn[k == 0 ? r.base1 : r.base2] : 'N';
+        *p++ = '\t';
+        p = put_i(p, any ? (k == 0 ? r.avg1 : r.avg2) : 0);
+        *p++ = '\t';
+        p = put_i(p, any ? (k == 0 ? r.cu1 : r.cu2) : 0);
+        *p++ = '\t';
+        p = put_i(p, any ? (k == 0 ? r.ca1 : r.ca2) : 0);
+    }
+    *p++ = '\t';
+    p = put_u(p, r.depth, digits(r.depth));
+    /* the rank sum's p-value, the copy ratio */
+    for (int k = 0; k < 2; ++k) {
+        const G6 g = k == 0 ? o.rank : o.ratio;
+        *p++ = '\t';
+        fmt_g6_put(g, p);
+        p += g.len;
+    }
+    *p++ = '\t';
+    *p++ = (r.ori & 8) ? '1' : '0';
+    *p++ = '\n';
 }
 
-__global__ void row_write_kernel(EmitArgs e) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= e.n) return;
-    char buf[kRowMax];
-    const int len = format_row(e, e.site0 + i, buf);
-    char* dst = e.text + e.off[i];
-    for (int k = 0; k < len; ++k) dst[k] = buf[k];
+/* the bytes of each CTA's rows */
+__global__ void __launch_bounds__(kRows) row_len_kernel(EmitArgs e) {
+    const int64_t i = (int64_t)blockIdx.x * kRows + threadIdx.x;
+    __shared__ uint32_t s_sum[kRows / 32];
+    uint32_t len = 0;
+    if (i < e.n) {
+        const Row o = measure_row(e, e.site0 + i);
+        if (!o.ok) atomicExch(e.error, 1);
+        len = (uint32_t)o.len;
+    }
+    len = __reduce_add_sync(0xffffffffu, len);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = len;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t t = 0;
+        for (int k = 0; k < kRows / 32; ++k) t += s_sum[k];
+        e.off[blockIdx.x] = t;
+    }
 }
 
-/* exclusive scan of e.len into e.off, 64-bit */
+/* The text of blocks [block0, block0 + gridDim.x) at e.text, which receives
+ * block0's first byte.  The characters go to shared memory at the place they
+ * have within their 16-byte word of the output, so that whole words can be
+ * stored. */
+__global__ void __launch_bounds__(kRows) row_write_kernel(EmitArgs e, int64_t block0) {
+    extern __shared__ uint4 s_words[];
+    __shared__ uint32_t s_sum[kRows / 32];
+    __shared__ char s_name[256];
+    char* s_text = (char*)s_words;
+    const int64_t b = block0 + blockIdx.x, i = b * kRows + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int k = threadIdx.x; k < e.chr_n; k += kRows) s_name[k] = e.chr[k];
+    char* dst = e.text + (e.off[b] - e.off[block0]);
+    const uint32_t head = (uint32_t)((uintptr_t)dst & 15);
+    Row o;
+    o.len = 0;
+    if (i < e.n) o = measure_row(e, e.site0 + i);
+    uint32_t x = (uint32_t)o.len;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    if (lane == 31) s_sum[warp] = x;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    for (int k = 0; k < kRows / 32; ++k) {
+        if (k < warp) before += s_sum[k];
+        total += s_sum[k];
+    }
+    if (o.len) put_row(e, o, s_name, s_text + head + before + x - (uint32_t)o.len);
+    __syncthreads();
+    char* word0 = dst - head;
+    const uint32_t end = head + total;
+    const uint32_t first = head ? 16 : 0, last = end & ~15u;
+    for (uint32_t k = first + threadIdx.x * 16; k < last; k += kRows * 16) *(uint4*)(word0 + k) = s_words[k / 16];
+    /* the bytes of the words shared with the neighbouring blocks */
+    if (threadIdx.x < 16) {
+        const uint32_t k = threadIdx.x;
+        if (head && k >= head && k < end) word0[k] = s_text[k];
+    } else if (threadIdx.x < 32) {
+        const uint32_t k = last + threadIdx.x - 16;
+        if (k >= first && k < end) word0[k] = s_text[k];
+    }
+}
+
+/* exclusive prefix of v over the CTA */
 __device__ uint64_t block_exclusive(uint64_t v, uint64_t* total) {
     __shared__ uint64_t warp_sums[kScanThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -158,82 +241,57 @@ __device__ uint64_t block_exclusive(uint64_t v, uint64_t* total) {
     return before;
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(const uint32_t* len, int64_t n, uint64_t* bsum) {
-    const int64_t base = (int64_t)blockIdx.x * kScanBlock + (int64_t)threadIdx.x * kScanItems;
-    uint64_t v = 0;
-    for (int k = 0; k < kScanItems; ++k)
-        if (base + k < n) v += len[base + k];
-    uint64_t total;
-    block_exclusive(v, &total);
-    if (threadIdx.x == 0) bsum[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kScanThreads) scan_blocks_kernel(uint64_t* bsum, int64_t nb, uint64_t* grand) {
+/* off[0, nb): byte counts to offsets, in place; off[nb, padded): the total */
+__global__ void __launch_bounds__(kScanThreads) scan_blocks_kernel(uint64_t* off, int64_t nb, int64_t padded) {
     uint64_t carry = 0;
-    for (int64_t b0 = 0; b0 < nb; b0 += kScanThreads) {
-        const int64_t b = b0 + threadIdx.x;
-        const uint64_t v = b < nb ? bsum[b] : 0;
+    for (int64_t b0 = 0; b0 < nb; b0 += kScanThreads * kScanItems) {
+        const int64_t b = b0 + (int64_t)threadIdx.x * kScanItems;
+        uint64_t v[kScanItems], t = 0;
+        for (int k = 0; k < kScanItems; ++k) {
+            v[k] = b + k < nb ? off[b + k] : 0;
+            t += v[k];
+        }
         uint64_t total;
-        const uint64_t ex = block_exclusive(v, &total);
-        if (b < nb) bsum[b] = carry + ex;
+        uint64_t run = carry + block_exclusive(t, &total);
+        for (int k = 0; k < kScanItems; ++k)
+            if (b + k < nb) {
+                off[b + k] = run;
+                run += v[k];
+            }
         carry += total;
     }
-    if (threadIdx.x == 0) *grand = carry;
+    for (int64_t b = nb + threadIdx.x; b < padded; b += kScanThreads) off[b] = carry;
 }
-
-__global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t* len, int64_t n, const uint64_t* bsum,
-                                                                uint64_t* off) {
-    const int64_t base = (int64_t)blockIdx.x * kScanBlock + (int64_t)threadIdx.x * kScanItems;
-    uint64_t v[kScanItems], t = 0;
-    for (int k = 0; k < kScanItems; ++k) {
-        v[k] = base + k < n ? len[base + k] : 0;
-        t += v[k];
-    }
-    uint64_t total;
-    uint64_t run = bsum[blockIdx.x] + block_exclusive(t, &total);
-    for (int k = 0; k < kScanItems; ++k)
-        if (base + k < n) {
-            off[base + k] = run;
-            run += v[k];
-        }
-}
-
-unsigned grid(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
 
-size_t emit_scratch_bytes(int64_t n) {
-    const int64_t nb = (n + kScanBlock - 1) / kScanBlock;
-    return (size_t)n * 4 + (size_t)n * 8 + (size_t)(nb + 1) * 8 + 16;
+int64_t emit_pieces(int64_t n) { return (n + kEmitPiece - 1) / kEmitPiece; }
+
+size_t emit_scratch_bytes(int64_t n) { return (size_t)(emit_pieces(n) * kPieceBlocks + 1) * 8; }
+
+cudaError_t emit_lengths(EmitArgs& e, void* scratch, cudaStream_t stream) {
+    e.off = (uint64_t*)scratch;
+    const int64_t nb = (e.n + kRows - 1) / kRows;
+    if (nb) row_len_kernel<<<(unsigned)nb, kRows, 0, stream>>>(e);
+    scan_blocks_kernel<<<1, kScanThreads, 0, stream>>>(e.off, nb, emit_pieces(e.n) * kPieceBlocks + 1);
+    return cudaGetLastError();
 }
 
-cudaError_t emit_lengths(EmitArgs& e, void* scratch, cudaStream_t stream, uint64_t* h_total) {
-    uint8_t* p = (uint8_t*)scratch;
-    e.len = (uint32_t*)p;
-    p += ((size_t)e.n * 4 + 15) & ~(size_t)15;
-    e.off = (uint64_t*)p;
-    p += (size_t)e.n * 8;
-    uint64_t* bsum = (uint64_t*)p;
-    const int64_t nb = (e.n + kScanBlock - 1) / kScanBlock;
-    uint64_t* grand = bsum + nb;
-    if (e.n == 0) {
-        *h_total = 0;
-        return cudaSuccess;
+cudaError_t emit_offsets(const EmitArgs& e, uint64_t* h_off, cudaStream_t stream) {
+    return cudaMemcpy2DAsync(h_off, 8, e.off, kPieceBlocks * 8, 8, (size_t)emit_pieces(e.n) + 1,
+                             cudaMemcpyDeviceToHost, stream);
+}
+
+cudaError_t emit_text(const EmitArgs& e, int64_t piece, cudaStream_t stream) {
+    const int64_t b0 = piece * kPieceBlocks, b1 = std::min((e.n + kRows - 1) / kRows, b0 + kPieceBlocks);
+    if (b1 <= b0) return cudaSuccess;
+    const size_t smem = 16 + (size_t)kRows * (size_t)(kRowFields + e.chr_n);
+    if (smem > 47 * 1024) {   /* names near 255 bytes; the kernel's static 0.3 KB count too */
+        const cudaError_t err =
+            cudaFuncSetAttribute(row_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (err != cudaSuccess) return err;
     }
-    row_len_kernel<<<grid(e.n, 128), 128, 0, stream>>>(e);
-    scan_sums_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(e.len, e.n, bsum);
-    scan_blocks_kernel<<<1, kScanThreads, 0, stream>>>(bsum, nb, grand);
-    scan_apply_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(e.len, e.n, bsum, e.off);
-    cudaError_t err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-    err = cudaMemcpyAsync(h_total, grand, 8, cudaMemcpyDeviceToHost, stream);
-    if (err != cudaSuccess) return err;
-    return cudaStreamSynchronize(stream);
-}
-
-cudaError_t emit_text(const EmitArgs& e, cudaStream_t stream) {
-    if (e.n == 0) return cudaSuccess;
-    row_write_kernel<<<grid(e.n, 128), 128, 0, stream>>>(e);
+    row_write_kernel<<<(unsigned)(b1 - b0), kRows, smem, stream>>>(e, b0);
     return cudaGetLastError();
 }
 

@@ -19,21 +19,31 @@ struct EmitArgs {
     const char* chr;            /* chromosome name (device) */
     int chr_n;
     int64_t site0, n;           /* rows of sites [site0, site0 + n) */
-    uint32_t* len;              /* scratch: row lengths */
-    uint64_t* off;              /* scratch: byte offsets */
-    char* text;                 /* output of emit_text */
+    uint64_t* off;              /* scratch: byte offset of every kEmitRows-th row */
+    char* text;                 /* output of emit_text: one piece's text */
     int* error;                 /* set when a value is outside the formatter's range */
 };
+
+constexpr int kEmitRows = 128;                              /* rows of a CTA */
+constexpr int64_t kEmitPiece = kWin;                        /* rows of a piece, about 17 MB of text */
+constexpr int64_t kPieceBlocks = kEmitPiece / kEmitRows;
+static_assert(kEmitPiece % kEmitRows == 0, "a piece is whole blocks");
+
+/* pieces of n rows */
+int64_t emit_pieces(int64_t n);
 
 /* device scratch of emit_lengths for n rows */
 size_t emit_scratch_bytes(int64_t n);
 
-/* Row lengths and offsets of e's rows in scratch (sets e.len, e.off);
- * *h_total receives the byte count of the rows' text.  Synchronises. */
-cudaError_t emit_lengths(EmitArgs& e, void* scratch, cudaStream_t stream, uint64_t* h_total);
+/* Measure e's rows: byte offsets in scratch (sets e.off). */
+cudaError_t emit_lengths(EmitArgs& e, void* scratch, cudaStream_t stream);
 
-/* Write the rows' text to e.text (after emit_lengths). */
-cudaError_t emit_text(const EmitArgs& e, cudaStream_t stream);
+/* Copy the first byte of every piece and, last, the total to
+ * h_off[0, emit_pieces(e.n)] (after emit_lengths). */
+cudaError_t emit_offsets(const EmitArgs& e, uint64_t* h_off, cudaStream_t stream);
+
+/* Write one piece's text to e.text (after emit_lengths). */
+cudaError_t emit_text(const EmitArgs& e, int64_t piece, cudaStream_t stream);
 
 }  // namespace gsnp
 
