@@ -594,7 +594,7 @@ cudaError_t launch_bin(const CallArgs& a, int kind, int bin, const int32_t* tile
         case 3: return launch_one<64>(a, tiles, bl, stream);
         case 4: return launch_one<96>(a, tiles, bl, stream);
         case 5: return launch_one<128>(a, tiles, bl, stream);
-        default: return launch_one<256>(a, tiles, bl, stream);
+        default: return launch_deep64(a, tiles, bl, stream);
     }
 }
 
@@ -610,7 +610,7 @@ int bin_ctas_per_sm(int kind, int bin, int L, int carveout) {
         case 3: e = bin_attr<64>(L, carveout, &n); break;
         case 4: e = bin_attr<96>(L, carveout, &n); break;
         case 5: e = bin_attr<128>(L, carveout, &n); break;
-        default: e = bin_attr<256>(L, carveout, &n); break;
+        default: e = deep64_attr(&n); break;
     }
     if (e != cudaSuccess) {
         (void)cudaGetLastError();

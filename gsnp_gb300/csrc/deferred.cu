@@ -22,6 +22,7 @@
 #include <algorithm>
 
 #include "calling.cuh"
+#include "deep.cuh"
 #include "site_math.cuh"
 #include "tile.cuh"
 
@@ -31,11 +32,10 @@ namespace {
 
 constexpr int kDefWarps = 4;     /* warps of a CTA, each by itself */
 constexpr int kDefBatch = 16;    /* most sites a warp holds at a time */
-constexpr int kDefKeys = 4 * 2 * 256;
 
 /* a warp's shared memory */
 struct DefWarp {
-    uint8_t cnt[kDefKeys];             /* occurrences by (base, strand, cycle) key */
+    uint8_t cnt[kDeepKeys];             /* occurrences by (base, strand, cycle) key */
     int32_t hist[2][66];               /* records by quality of the candidate's two alleles */
     float tl32[kDefBatch][10];         /* FP32 sums by table column */
     double tl64[kDefBatch][10];        /* FP64 sums, where they are wanted */
@@ -43,18 +43,15 @@ struct DefWarp {
     int32_t cand[kDefBatch];           /* best genotype of the FP32 values, -1: no rank sums */
 };
 
-/* The dependency walk and the sums of a sorted column by a warp, 32 records a
- * step (record c0 + lane on that lane), as deep_walk_sums counts them; lane v
- * < 10 then adds column v of the step's records in order.  T = float: groups of
- * four added pairwise and compensated, the values of likelihood_fp32; T =
- * double: the reference's order.  Returns column `lane`'s sum on lanes 0-9. */
+/* The dependency walk and the sums of a sorted column by a warp: the walk's 32
+ * records a step, of which lane v < 10 adds column v in order.  T = float:
+ * groups of four added pairwise and compensated, the values of
+ * likelihood_fp32; T = double: the reference's order.  Returns column `lane`'s
+ * sum on lanes 0-9. */
 template <class T>
 __device__ __forceinline__ T deferred_sum(const CallArgs& a, const uint32_t* recs, int num, uint8_t* cnt) {
     constexpr bool kSingle = sizeof(T) == 4;
     const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u, le = (lt << 1) | 1u;
-    for (int i = lane; i < kDefKeys / 16; i += 32) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0u, 0u, 0u, 0u);
-    __syncwarp();
     /* where column `lane` of a row lies */
     const int col = lane < 10 ? lane : 0;
     const T* base;
@@ -67,33 +64,8 @@ __device__ __forceinline__ T deferred_sum(const CallArgs& a, const uint32_t* rec
         stride = 10;
     }
     T s = 0, c = 0;
-    int carry_firsts = 0, carry_base = -1;
-    for (int c0 = 0; c0 < num; c0 += 32) {
-        const bool valid = c0 + lane < num;
-        const uint32_t w = valid ? recs[c0 + lane] : 0u;
-        const int o = rec_base(w), coord = rec_coord(w);
-        const int key = valid ? (o << 9) | (rec_strand(w) << 8) | coord : kDefKeys + lane;
-        const unsigned peers = __match_any_sync(kFull, key);
-        const int seen = valid ? (int)cnt[key] : 0;
-        __syncwarp();
-        const int tmp = seen + __popc(peers & lt);
-        if (valid && (peers >> lane) == 1u) cnt[key] = (uint8_t)(seen + __popc(peers));
-        __syncwarp();
-        const int prev_o = __shfl_up_sync(kFull, o, 1);
-        const bool brk = valid && o != (lane == 0 ? carry_base : prev_o);
-        const unsigned bm = __ballot_sync(kFull, brk) & le;
-        const unsigned fm = __ballot_sync(kFull, valid && tmp == 0) & le;
-        const int firsts = bm ? __popc(fm & ~((1u << (31 - __clz(bm))) - 1u)) : carry_firsts + __popc(fm);
-        carry_firsts = __shfl_sync(kFull, firsts, 31);
-        carry_base = __shfl_sync(kFull, o, 31);
-        int row = 0;
-        if (valid) {
-            const int gdc = firsts - 1, t1 = tmp + 1;
-            const int qa = (t1 < a.tmax && gdc < a.gmax)
-                               ? (int)__ldg(a.qadj + ((size_t)t1 * a.gmax + gdc) * 65 + rec_q(w))
-                               : 1;
-            row = (qa * a.L + coord) * 4 + o;
-        }
+    deep_walk(a, recs, cnt, num, [&](int c0, bool valid, int qa, int coord, int o) {
+        const int row = valid ? (qa * a.L + coord) * 4 + o : 0;
         const int n = num - c0 < 32 ? num - c0 : 32;
         for (int j = 0; j < n; j += 8) {
             T x[8];
@@ -118,53 +90,9 @@ __device__ __forceinline__ T deferred_sum(const CallArgs& a, const uint32_t* rec
                     if (j + u < n) s = GSNP_DADD(s, x[u]);
             }
         }
-    }
+    });
     __syncwarp();
     return s;
-}
-
-/* Twice the rank sums of genotype g's two alleles over the site's records
- * (rank_test's Ta and Tb are half-integers far below 2^52, so its FP64 sums are
- * exact and any order gives them): a histogram by quality, and the rank of a
- * quality from the counts below it. */
-__device__ __forceinline__ void deferred_ranks(const CallArgs& a, const uint32_t* recs, int num, int g, int32_t (*hist)[66],
-                                               int32_t* rank2) {
-    const int lane = threadIdx.x & 31;
-    const int ia = g & 3, ib = (g >> 2) & 3;
-    for (int i = lane; i < 132; i += 32) hist[0][i] = 0;
-    __syncwarp();
-    for (int i = lane; i < num; i += 32) {
-        const uint32_t w = recs[i];
-        const int o = rec_base(w);
-        if (o == ia) atomicAdd(&hist[0][rec_q(w)], 1);
-        else if (o == ib) atomicAdd(&hist[1][rec_q(w)], 1);
-    }
-    __syncwarp();
-    /* qualities above q_max - q_min + 1 keep rank 0 as in the reference */
-    const int top = a.q_max_min + 1 < 64 ? a.q_max_min + 1 : 64;
-    int below = 0, ta = 0, tb = 0;
-    for (int q0 = 0; q0 <= 64; q0 += 32) {
-        const int q = q0 + lane;
-        const int ca = q <= top ? hist[0][q] : 0, cb = q <= top ? hist[1][q] : 0;
-        int before = ca + cb;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int y = __shfl_up_sync(kFull, before, d);
-            if (lane >= d) before += y;
-        }
-        const int total = __shfl_sync(kFull, before, 31);
-        const int ra = 2 * (below + before - ca - cb) + 1 + ca + cb;   /* twice the average rank */
-        ta += ra * ca;
-        tb += ra * cb;
-        below += total;
-    }
-    ta = __reduce_add_sync(kFull, ta);
-    tb = __reduce_add_sync(kFull, tb);
-    if (lane == 0) {
-        rank2[0] = ta;
-        rank2[1] = tb;
-    }
-    __syncwarp();
 }
 
 /* The posterior of deferred site d by one lane: from its FP32 sums with their
@@ -244,7 +172,7 @@ __global__ void __launch_bounds__(32 * kDefWarps) deferred_sites_kernel(const __
             best = __shfl_sync(kFull, best, 0);
             if (lane < 10) sm.tl32[j][lane] = s;
             if (lane == 0) sm.cand[j] = best;
-            if (a.rank_sum && (best >> 2) != (best & 3)) deferred_ranks(a, recs, num, best, sm.hist, sm.rank2[j]);
+            if (a.rank_sum && (best >> 2) != (best & 3)) warp_ranks(a, recs, num, best, sm.hist, sm.rank2[j]);
         }
         __syncwarp();
         DeferredSite d;

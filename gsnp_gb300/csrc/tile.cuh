@@ -222,6 +222,10 @@ extern thread_local bool g_launch_attributes;
 
 /* launchers of the FP32 kernels (calling_fast.cu) behind launch_bin */
 cudaError_t fast_bin_attr(int bin, int L, int carveout, int* ctas_per_sm);
+
+/* the FP64 kernel of the deep bin (calling_deep64.cu) */
+cudaError_t launch_deep64(const CallArgs& a, const int32_t* tiles, const BinLaunch& bl, cudaStream_t stream);
+cudaError_t deep64_attr(int* ctas_per_sm);
 cudaError_t launch_fast_bin(const CallArgs& a, int bin, const int32_t* tiles, const BinLaunch& bl, cudaStream_t stream);
 
 }  // namespace gsnp
