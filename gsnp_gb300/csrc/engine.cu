@@ -1324,16 +1324,29 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
         CK(launch_tile_bounds(a, g.dlo, g.dhi, g.next_pos, c->stream), "tile bounds kernel");
         auto bins = [&](int kind, int pass) -> int {
             const int ki = kind == kKindFast ? 1 : 0;
+            /* a segment's bins side by side: few tiles each, of a whole tile's latency */
+            const bool fork = side != c->stream;
+            if (fork) {
+                CK(cudaEventRecord(c->ev_join[0], side), "event");
+                for (int i = 1; i < gsnp_context::kBinStreams; ++i)
+                    CK(cudaStreamWaitEvent(c->bin_stream[i], c->ev_join[0], 0), "wait");
+            }
             for (int b = pass == 0 ? min_bin : 0; b < kNumBins; ++b) {
                 if (kind == kKindFast && use_stream && min_bin == 0 && kSlotsOf(b) <= c->stream_slots) continue;
                 int* const cnt = pc->bins[pass] + ki * kNumBins + b;
                 const BinLaunch bl{0, cnt, c->bin_grid[ki][b], c->bin_carveout[ki][b], cnt + 2 * kNumBins};
-                const int kb = begin(launch_kind(kind, kSlotsOf(b)), kSlotsOf(b), 0, side);
+                cudaStream_t const st = fork ? c->bin_stream[(kNumBins - 1 - b) % gsnp_context::kBinStreams] : side;
+                const int kb = begin(launch_kind(kind, kSlotsOf(b)), kSlotsOf(b), 0, st);
                 if (kb >= 0) c->launch_ref[kb] = (int)(reinterpret_cast<uint8_t*>(cnt) - c->d_ctl);
-                CK(launch_bin(a, kind, b, c->d_bin_tiles + (int64_t)(ki * kNumBins + b) * c->tiles_cap, bl, side),
+                CK(launch_bin(a, kind, b, c->d_bin_tiles + (int64_t)(ki * kNumBins + b) * c->tiles_cap, bl, st),
                    "calling kernel");
-                end(kb, side);
+                end(kb, st);
             }
+            if (fork)
+                for (int i = 1; i < gsnp_context::kBinStreams; ++i) {
+                    CK(cudaEventRecord(c->ev_join[i], c->bin_stream[i]), "event");
+                    CK(cudaStreamWaitEvent(side, c->ev_join[i], 0), "wait");
+                }
             return GSNP_OK;
         };
         /* pass 0 */
