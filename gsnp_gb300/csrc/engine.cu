@@ -461,6 +461,15 @@ struct Control {
 };
 static_assert(sizeof(Control) == 256 && offsetof(Control, error) == 64, "control block layout");
 
+/* the calibration pass's pieces: bytes of rows, and how many are on the device.
+ * Each piece's four small copies leave the link idle for some 30 us and its
+ * histogram, 65 us at 16 MB, waits for the whole piece (c1, 8 Mbp, 480 MB:
+ * 4.20 ms in pieces of 8 MB, 3.74 of 16, 3.32 of 32, 3.23 of 64, 3.34 of 128,
+ * 2.4 of them the copies; 6.1 with everything copied first into buffers of the
+ * call's own). */
+constexpr size_t kCalibPiece = 32u << 20;
+constexpr int kCalibSlots = 2;
+
 struct gsnp_context {
     int device = 0;
     std::string error;
@@ -652,6 +661,10 @@ struct gsnp_context {
     char* h_text = nullptr;      /* pinned staging of two pieces on the way to a file */
     size_t h_text_bytes = 0;
     cudaEvent_t ev_text[2] = {}, ev_copied[2] = {};
+    /* calibration: the counts, then kCalibSlots pieces of alignments */
+    uint8_t* d_calib = nullptr;
+    size_t calib_bytes = 0;
+    cudaEvent_t ev_cal_up[kCalibSlots] = {}, ev_cal_done[kCalibSlots] = {};
 };
 
 namespace {
@@ -1935,6 +1948,10 @@ void gsnp_context_destroy(gsnp_context* c) {
     c->ring = nullptr;
     c->colw.reset();
     if (c->h_text) cudaFreeHost(c->h_text);
+    if (c->d_calib) cudaFree(c->d_calib);
+    for (cudaEvent_t* e : {c->ev_cal_up, c->ev_cal_done})
+        for (int i = 0; i < kCalibSlots; ++i)
+            if (e[i]) cudaEventDestroy(e[i]);
     for (int i = 0; i < 2; ++i) {
         if (c->ev_text[i]) cudaEventDestroy(c->ev_text[i]);
         if (c->ev_copied[i]) cudaEventDestroy(c->ev_copied[i]);
@@ -2106,65 +2123,126 @@ int gsnp_calibrate(gsnp_context* c, const gsnp_params* p, const gsnp_reads* r, d
     const int L = p->read_length;
     const int nq = p->q_max - p->q_min + 1;
     const size_t nbins = (size_t)nq * L * 16;
-    for (int64_t i = 0; i < r->n; ++i)
-        if (r->len[i] < 0 || r->len[i] > L || r->len[i] > r->pitch)
-            return fail(c, GSNP_ERR_INPUT, "alignment " + std::to_string(i) + " is longer than -L");
-    unsigned long long* d_counts = nullptr;
-    int32_t *d_pos = nullptr, *d_len = nullptr, *d_hit = nullptr;
-    uint8_t *d_strand = nullptr, *d_seq = nullptr, *d_qual = nullptr;
-    const size_t raw = (size_t)r->n * r->pitch;
-    CallTemps tmp;
-    CK(tmp.alloc(&d_counts, nbins * 8), "cudaMalloc");
-    CK(tmp.alloc(&d_pos, std::max<int64_t>(r->n, 1) * 4), "cudaMalloc");
-    CK(tmp.alloc(&d_len, std::max<int64_t>(r->n, 1) * 4), "cudaMalloc");
-    CK(tmp.alloc(&d_hit, std::max<int64_t>(r->n, 1) * 4), "cudaMalloc");
-    CK(tmp.alloc(&d_strand, std::max<int64_t>(r->n, 1)), "cudaMalloc");
-    CK(tmp.alloc(&d_seq, std::max<size_t>(raw, 1)), "cudaMalloc");
-    CK(tmp.alloc(&d_qual, std::max<size_t>(raw, 1)), "cudaMalloc");
-    CK(cudaMemsetAsync(d_counts, 0, nbins * 8, c->stream), "memset");
-    CK(cudaMemcpyAsync(d_pos, r->pos, r->n * 4, cudaMemcpyHostToDevice, c->stream), "upload");
-    CK(cudaMemcpyAsync(d_len, r->len, r->n * 4, cudaMemcpyHostToDevice, c->stream), "upload");
-    CK(cudaMemcpyAsync(d_hit, r->hit, r->n * 4, cudaMemcpyHostToDevice, c->stream), "upload");
-    CK(cudaMemcpyAsync(d_strand, r->strand, r->n, cudaMemcpyHostToDevice, c->stream), "upload");
-    if (r->packed) {
-        CK(cudaMemcpyAsync(d_seq, r->packed, raw, cudaMemcpyHostToDevice, c->stream), "upload");
+    /* Pieces of about kCalibPiece bytes of rows go through kCalibSlots buffers:
+     * a piece's copies wait for the histogram of the piece that had the buffer
+     * before, and its histogram runs beside the next piece's copies.  The host
+     * checks the lengths while the first pieces are copied and writes the
+     * matrix's constant part while the last ones are. */
+    const size_t nb = sizeof(unsigned long long) * nbins;
+    const int64_t pitch = std::max<int64_t>(r->pitch, 1);
+    const int64_t rows = std::min<int64_t>(std::max<int64_t>(r->n, 1),
+                                           std::max<int64_t>(1, (int64_t)(kCalibPiece / (size_t)pitch)));
+    auto pad = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t col = pad((size_t)rows * 4), row_bytes = pad((size_t)rows * pitch);
+    const size_t slot_bytes = 4 * col + 2 * row_bytes;
+    const size_t need = pad(nb) + kCalibSlots * slot_bytes;
+    {
+        const int rc = ensure_call_streams(c);
+        if (rc != GSNP_OK) return rc;
+    }
+    for (cudaEvent_t* e : {c->ev_cal_up, c->ev_cal_done})
+        for (int i = 0; i < kCalibSlots; ++i)
+            if (!e[i]) CK(cudaEventCreateWithFlags(&e[i], cudaEventDisableTiming), "cudaEventCreate");
+    if (need > c->calib_bytes) {
+        if (c->d_calib) cudaFree(c->d_calib);
+        c->d_calib = nullptr;
+        c->calib_bytes = 0;
+        CK(cudaMalloc((void**)&c->d_calib, need), "cudaMalloc");
+        c->calib_bytes = need;
+    }
+    /* the copies read the caller's arrays, the download writes counts */
+    std::vector<unsigned long long> counts(nbins);
+    struct Drain {
+        cudaStream_t a, b;
+        ~Drain() {
+            cudaStreamSynchronize(a);
+            cudaStreamSynchronize(b);
+        }
+    } drain{c->up_stream, c->stream};
+    unsigned long long* const d_counts = reinterpret_cast<unsigned long long*>(c->d_calib);
+    CK(cudaMemsetAsync(d_counts, 0, nb, c->stream), "memset");
+    /* the matching bins in shared memory when they fit (41 qualities x 4
+     * bases x 100 cycles: 64 KB), else every bin in global memory */
+    const size_t smem = (size_t)nq * 4 * L * 4;
+    int dev_smem = 0, n_sm = 0;
+    cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, c->device);
+    const bool in_smem = smem <= 160 * 1024 && smem <= (size_t)dev_smem;
+    if (in_smem)
+        CK(cudaFuncSetAttribute(calib_count_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+           "calibration kernel attribute");
+    struct Slot {
+        int32_t *pos, *len, *hit;
+        uint8_t *strand, *seq, *qual;
+    };
+    auto slot_of = [&](int64_t k) {
+        uint8_t* at = c->d_calib + pad(nb) + (size_t)(k % kCalibSlots) * slot_bytes;
+        return Slot{(int32_t*)at, (int32_t*)(at + col), (int32_t*)(at + 2 * col), at + 3 * col, at + 4 * col,
+                    at + 4 * col + row_bytes};
+    };
+    const int64_t pieces = (r->n + rows - 1) / rows;
+    auto upload = [&](int64_t k) -> int {
+        const int64_t i0 = k * rows, n = std::min(rows, r->n - i0);
+        const size_t raw = (size_t)n * r->pitch, off = (size_t)i0 * r->pitch;
+        const Slot s = slot_of(k);
+        cudaStream_t us = c->up_stream;
+        if (k >= kCalibSlots) CK(cudaStreamWaitEvent(us, c->ev_cal_done[k % kCalibSlots], 0), "wait");
+        CK(cudaMemcpyAsync(s.pos, r->pos + i0, n * 4, cudaMemcpyHostToDevice, us), "upload");
+        CK(cudaMemcpyAsync(s.len, r->len + i0, n * 4, cudaMemcpyHostToDevice, us), "upload");
+        CK(cudaMemcpyAsync(s.hit, r->hit + i0, n * 4, cudaMemcpyHostToDevice, us), "upload");
+        CK(cudaMemcpyAsync(s.strand, r->strand + i0, n, cudaMemcpyHostToDevice, us), "upload");
         if (raw > 0) {
+            CK(cudaMemcpyAsync(s.seq, (r->packed ? r->packed : r->seq) + off, raw, cudaMemcpyHostToDevice, us), "upload");
+            if (!r->packed) CK(cudaMemcpyAsync(s.qual, r->qual + off, raw, cudaMemcpyHostToDevice, us), "upload");
+        }
+        CK(cudaEventRecord(c->ev_cal_up[k % kCalibSlots], us), "event");
+        return GSNP_OK;
+    };
+    auto count = [&](int64_t k) -> int {
+        const int64_t n = std::min(rows, r->n - k * rows);
+        const size_t raw = (size_t)n * r->pitch;
+        const Slot s = slot_of(k);
+        CK(cudaStreamWaitEvent(c->stream, c->ev_cal_up[k % kCalibSlots], 0), "wait");
+        if (r->packed && raw > 0) {
             unpack_reads_kernel<<<(unsigned)std::min<size_t>((raw + 255) / 256, 1u << 16), 256, 0, c->stream>>>(
-                d_seq, raw, (int)(signed char)p->q_min, d_seq, d_qual);
+                s.seq, raw, (int)(signed char)p->q_min, s.seq, s.qual);
             CK(cudaGetLastError(), "unpack kernel");
         }
-    } else {
-        CK(cudaMemcpyAsync(d_seq, r->seq, raw, cudaMemcpyHostToDevice, c->stream), "upload");
-        CK(cudaMemcpyAsync(d_qual, r->qual, raw, cudaMemcpyHostToDevice, c->stream), "upload");
-    }
-    if (r->n > 0) {
-        /* the matching bins in shared memory when they fit (41 qualities x
-         * 4 bases x 100 cycles: 64 KB), else every bin in global memory */
-        const size_t smem = (size_t)nq * 4 * L * 4;
-        int dev_smem = 0, n_sm = 0;
-        cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, c->device);
-        if (smem <= 160 * 1024 && smem <= (size_t)dev_smem) {
-            CK(cudaFuncSetAttribute(calib_count_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-               "calibration kernel attribute");
+        if (in_smem) {
             const int per_sm = std::max(1, (int)(200 * 1024 / std::max<size_t>(smem, 1)));
-            const int64_t want = (r->n + 15) / 16;
-            const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)n_sm * per_sm, want));
+            const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)n_sm * per_sm, (n + 15) / 16));
             calib_count_smem_kernel<<<blocks, 512, smem, c->stream>>>(
-                r->n, d_pos, d_len, d_hit, d_strand, d_seq, d_qual, r->pitch, c->d_codes, c->chr_len,
+                n, s.pos, s.len, s.hit, s.strand, s.seq, s.qual, r->pitch, c->d_codes, c->chr_len,
                 (int)(signed char)p->q_min, (int)(signed char)p->q_max, L, d_counts);
         } else {
-            const int64_t threads = r->n * 32;
-            calib_count_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, c->stream>>>(
-                r->n, d_pos, d_len, d_hit, d_strand, d_seq, d_qual, r->pitch, c->d_codes, c->chr_len,
+            calib_count_kernel<<<(unsigned)((n * 32 + 255) / 256), 256, 0, c->stream>>>(
+                n, s.pos, s.len, s.hit, s.strand, s.seq, s.qual, r->pitch, c->d_codes, c->chr_len,
                 (int)(signed char)p->q_min, (int)(signed char)p->q_max, L, d_counts);
         }
         CK(cudaGetLastError(), "calibration kernel");
+        CK(cudaEventRecord(c->ev_cal_done[k % kCalibSlots], c->stream), "event");
+        return GSNP_OK;
+    };
+    for (int64_t k = 0; k < std::min<int64_t>(pieces, kCalibSlots); ++k) {
+        const int rc = upload(k);
+        if (rc != GSNP_OK) return rc;
     }
-    std::vector<unsigned long long> counts(nbins);
-    CK(cudaMemcpyAsync(counts.data(), d_counts, nbins * 8, cudaMemcpyDeviceToHost, c->stream), "download");
-    CK(cudaStreamSynchronize(c->stream), "calibration");
+    /* no kernel sees a length before it is checked */
+    const int most = std::min(L, r->pitch);
+    int64_t bad = 0;
+    for (int64_t i = 0; i < r->n; ++i) bad += r->len[i] < 0 || r->len[i] > most;
+    if (bad)
+        for (int64_t i = 0; i < r->n; ++i)
+            if (r->len[i] < 0 || r->len[i] > most)
+                return fail(c, GSNP_ERR_INPUT, "alignment " + std::to_string(i) + " is longer than -L");
+    for (int64_t k = 0; k < pieces; ++k) {
+        int rc = count(k);
+        if (rc == GSNP_OK && k + kCalibSlots < pieces) rc = upload(k + kCalibSlots);
+        if (rc != GSNP_OK) return rc;
+    }
+    CK(cudaMemcpyAsync(counts.data(), d_counts, nb, cudaMemcpyDeviceToHost, c->stream), "download");
     for (size_t i = 0; i < 256UL * 256UL * 16UL; ++i) pm[i] = 1.0;
+    CK(cudaStreamSynchronize(c->stream), "calibration");
     calibration_fill(*p, counts.data(), pm);
     return GSNP_OK;
 }
