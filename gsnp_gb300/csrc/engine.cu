@@ -468,7 +468,7 @@ static_assert(sizeof(Control) == 256 && offsetof(Control, error) == 64, "control
  * 2.4 of them the copies; 6.1 with everything copied first into buffers of the
  * call's own). */
 constexpr size_t kCalibPiece = 32u << 20;
-constexpr int kCalibSlots = 2;
+constexpr int kCalibSlots = 3;
 
 struct gsnp_context {
     int device = 0;
