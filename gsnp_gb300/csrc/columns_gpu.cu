@@ -3,11 +3,12 @@
  *
  * The five binary files of the -C output (cpp/compress.h:86-1312; the byte
  * layouts are those of columns.cpp, which is pinned to the reference's files)
- * are encoded window by window from the calls resident on the device: one CTA
- * of 1024 threads per window, each thread owning 256 consecutive rows.  A
- * window's rows are those the host writer builds (rows.h make_row: the site's
- * call with the count columns of the window the reference's host arrays held),
- * and each file's block is written in place into a per-window slice of a
+ * are encoded window by window from the calls resident on the device: a CTA
+ * of 1024 threads per file of a window, or per column of the run-length file,
+ * each warp walking 8,192 rows in order.  A window's rows are those the host
+ * writer builds (rows.h make_row: the site's call with the count columns of
+ * the window the reference's host arrays held), and each block is written in
+ * place into a per-window slice of a
  * batch buffer:
  *   .3_4_6            2-bit reference bases, N ids, genotype and best-base
  *                     differences (ids by block-wide scans, in row order);
@@ -27,7 +28,8 @@
  *
  * A window whose block would not fit its slice, or whose double column has
  * more distinct values than the hash set holds, is flagged; the host encodes
- * that window itself.  The host then writes the blocks in window order.
+ * that window itself.  A batch's blocks are then packed file by file into one
+ * buffer, which comes down in one copy and is written in window order.
  */
 #include <cuda_runtime.h>
 
@@ -62,9 +64,28 @@ constexpr unsigned long long kEmptyKey = ~0ull;       /* a NaN pattern, never a 
 /* per-window slice of each file's batch buffer: the worst case of every file
  * but the run-length one (15, 4.25, 40 and 16 bytes per row at most), whose
  * worst case a window of a few thousand runs is far from */
-constexpr size_t kCapHost[5] = {4u << 20, 12u << 20, 1300u << 10, 11u << 20, 5u << 20};
+constexpr int kRleCols = 6;
+constexpr size_t kRleColCap = 3u << 20;   /* of each run-length column */
+constexpr size_t kCapHost[5] = {4u << 20, kRleCols * kRleColCap, 1300u << 10, 11u << 20, 5u << 20};
 
 enum : int { kF346 = 0, kFRle = 1, kF10 = 2, kF111213 = 3, kF1517 = 4 };
+
+/* What a CTA encodes of a window: one of the run-length file's six columns
+ * (tasks 0-5), or another file, the longer ones first.  A file's block is its
+ * tasks' blocks in order. */
+constexpr int kTasks = kRleCols + 4;
+__host__ __device__ constexpr int task_file(int t) {
+    return t < kRleCols ? kFRle : t == kRleCols ? kF111213 : t == kRleCols + 1 ? kF346 : t == kRleCols + 2 ? kF10 : kF1517;
+}
+__host__ __device__ constexpr int file_task(int f) {
+    return f == kFRle ? 0 : f == kF111213 ? kRleCols : f == kF346 ? kRleCols + 1 : f == kF10 ? kRleCols + 2 : kRleCols + 3;
+}
+__host__ __device__ constexpr int file_tasks(int f) { return f == kFRle ? kRleCols : 1; }
+__host__ __device__ constexpr size_t task_at(int t) { return t < kRleCols ? (size_t)t * kRleColCap : 0; }
+/* windows of a batch: kTasks CTAs each, and kPackThreads tasks at most */
+constexpr int kPackThreads = 1024;
+constexpr int64_t kMostWindows = 64;
+static_assert(kMostWindows * kTasks <= kPackThreads, "one thread per block of a batch");
 
 __constant__ char c_abbv[17] = {'A', 'M', 'W', 'R', 'M', 'C', 'Y', 'S', 'W', 'Y', 'T', 'K', 'R', 'S', 'K', 'G', 'N'};
 __constant__ char c_actgn[8] = {'A', 'C', 'T', 'G', 'N', 'N', 'N', 'N'};
@@ -79,13 +100,13 @@ struct EncArgs {
     const uint8_t* bits;             /* bits per dictionary index of a dictionary of d values */
     uint8_t* out[5];                 /* [batch][cap[f]] */
     uint64_t cap[5];
-    uint64_t* len;                   /* [batch][5] bytes used */
-    int* fallback;                   /* [batch][5]: the file's block did not fit */
-    /* scratch, [batch][2][kWin] each: one slot for the run-length file, one
-     * for .11_12_13 */
-    uint64_t* s_val;                 /* run values (integer or double bits), sparse values */
-    uint32_t* s_aux;                 /* run starts, then run lengths */
-    uint64_t* s_dict;                /* dictionary values */
+    uint64_t* len;                   /* [batch][kTasks] bytes used */
+    int* fallback;                   /* [batch][kTasks]: the block did not fit */
+    uint32_t* s_runs;                /* [batch][kRleCols][kWin] run starts of the run-length columns */
+    /* the sparse values of .11_12_13, [batch][kWin] each */
+    uint64_t* s_val;
+    uint32_t* s_aux;
+    uint64_t* s_dict;
     /* per row, from rows_prep_kernel: the six run-length columns' values
      * (columns 5 7 8 9 14 as [5][batch][kWin] integers, 16 as [batch][kWin]
      * double bits), and per window whether any row is not an N row */
@@ -102,6 +123,8 @@ __device__ __forceinline__ void put32(uint8_t* p, uint32_t v) {
     p[2] = (uint8_t)(v >> 16);
     p[3] = (uint8_t)(v >> 24);
 }
+/* at a multiple of four bytes */
+__device__ __forceinline__ void put32a(uint8_t* p, uint32_t v) { *reinterpret_cast<uint32_t*>(p) = v; }
 __device__ __forceinline__ void put64(uint8_t* p, uint64_t v) {
     put32(p, (uint32_t)v);
     put32(p + 4, (uint32_t)(v >> 32));
@@ -157,19 +180,18 @@ struct Enc {
     int n;            /* rows */
     int hs;
     bool bad;         /* CTA-uniform: the window falls back to the host */
-    int slot;         /* the file's scratch slot (two files use scratch) */
+    int task;
+    uint64_t used;    /* bytes of the block */
 
     __device__ CnsRow row(int j) const { return make_row(hs, w, j, e.codes, e.calls, e.counts); }
     __device__ uint8_t* out(int f) const { return e.out[f] + (size_t)b * e.cap[f]; }
-    __device__ uint64_t* sval() const { return e.s_val + ((size_t)b * 2 + slot) * kWin; }
-    __device__ uint32_t* saux() const { return e.s_aux + ((size_t)b * 2 + slot) * kWin; }
-    __device__ uint64_t* sdict() const { return e.s_dict + ((size_t)b * 2 + slot) * kWin; }
-    /* value of run-length column k of row j */
-    __device__ uint64_t rle(int k, int64_t j) const {
-        return k < 5 ? (uint64_t)e.rle32[((size_t)k * e.stride + b) * kWin + j] : e.rle64[(size_t)b * kWin + j];
-    }
+    __device__ uint64_t* sval() const { return e.s_val + (size_t)b * kWin; }
+    __device__ uint32_t* saux() const { return e.s_aux + (size_t)b * kWin; }
+    __device__ uint64_t* sdict() const { return e.s_dict + (size_t)b * kWin; }
+    __device__ const uint32_t* rle32(int k) const { return e.rle32 + ((size_t)k * e.stride + b) * kWin; }
+    __device__ const uint64_t* rle64() const { return e.rle64 + (size_t)b * kWin; }
     __device__ bool fits(int f, uint64_t bytes) {
-        if (bytes > e.cap[f]) bad = true;
+        if (bytes > (f == kFRle ? kRleColCap : e.cap[f])) bad = true;
         return !bad;
     }
 };
@@ -228,8 +250,8 @@ struct IntDict {
     int d;
 
     template <class V>
-    __device__ int build(const V* vals, int m) {
-        int64_t mn = INT64_MAX, mx = INT64_MIN;
+    __device__ int build(const V& vals, int m) {
+        int64_t mn = INT64_MAX, mx = -1;   /* a thread without a value leaves the bounds as they are */
         for (int i = threadIdx.x; i < m; i += kEncThreads) {
             mn = min(mn, (int64_t)vals[i]);
             mx = max(mx, (int64_t)vals[i]);
@@ -279,7 +301,7 @@ struct IntDict {
             while (bits && r < (uint32_t)d) {
                 const int i = __ffs(bits) - 1;
                 bits &= bits - 1;
-                put32(dst + 4 * (size_t)r++, (uint32_t)(lo + (int64_t)k * 32 + i));
+                put32a(dst + 4 * (size_t)r++, (uint32_t)(lo + (int64_t)k * 32 + i));
             }
         }
     }
@@ -298,7 +320,8 @@ struct DblDict {
     int* negzero;              /* shared */
     int d;
 
-    __device__ int build(const uint64_t* vals, int m) {
+    template <class V>
+    __device__ int build(const V& vals, int m) {
         for (int i = threadIdx.x; i < kHashCap; i += kEncThreads) tab[i] = kEmptyKey;
         if (threadIdx.x == 0) {
             *counter = 0;
@@ -370,6 +393,13 @@ struct DblDict {
         }
         return (uint32_t)lo;
     }
+    __device__ void put_values(uint8_t* dst) const {
+        for (int i = threadIdx.x; i < d; i += kEncThreads) {
+            const uint64_t v = value(i);
+            put32a(dst + 8 * (size_t)i, (uint32_t)v);
+            put32a(dst + 8 * (size_t)i + 4, (uint32_t)(v >> 32));
+        }
+    }
     /* value bits of entry i, the zero entry -0.0 when any input was -0.0 */
     __device__ uint64_t value(int i) const {
         const double v = __longlong_as_double((long long)tab[i]);
@@ -379,9 +409,9 @@ struct DblDict {
 };
 
 /* the m indices of vals packed MSB-first, floor(32 / bits) per word, into
- * dst (4 bytes per word) when write; returns the word count */
+ * dst (4 bytes per word, aligned) when write; returns the word count */
 template <class D, class V>
-__device__ uint64_t pack(const D& dict, const uint8_t* bits_tab, const V* vals, int m, uint8_t* dst, bool write) {
+__device__ uint64_t pack(const D& dict, const uint8_t* bits_tab, const V& vals, int m, uint8_t* dst, bool write) {
     if (m == 0) return 0;
     const int bits = bits_tab[dict.d];
     const int per = 32 / bits;
@@ -391,7 +421,7 @@ __device__ uint64_t pack(const D& dict, const uint8_t* bits_tab, const V* vals, 
             const int first = (int)(k * per), last = min(m, first + per);
             uint32_t word = 0;
             for (int i = first; i < last; ++i) word = (word << bits) | dict.index(vals[i]);
-            put32(dst + 4 * k, word);
+            put32a(dst + 4 * k, word);
         }
     return (uint64_t)nw;
 }
@@ -409,7 +439,7 @@ __device__ void file_346(Enc& x, bool all_n) {
         if (threadIdx.x == 0) {
             const uint64_t param[7] = {1, 0, n, 0, 0, 0, 0};
             for (int i = 0; i < 7; ++i) put64(o + 8 * i, param[i]);
-            x.e.len[x.b * 5 + kF346] = 56;
+            x.used = 56;
         }
         return;
     }
@@ -465,7 +495,7 @@ __device__ void file_346(Enc& x, bool all_n) {
         const uint64_t param[7] = {0, (uint64_t)(5 * N4 + 5 * N6 + 4 * NN) + 4 * nw, n, nw, (uint64_t)NN,
                                    (uint64_t)N4, (uint64_t)N6};
         for (int i = 0; i < 7; ++i) put64(o + 8 * i, param[i]);
-        x.e.len[x.b * 5 + kF346] = total;
+        x.used = total;
     }
 }
 
@@ -486,111 +516,102 @@ __device__ __forceinline__ uint64_t rle_value(const CnsRow& r, int k) {
     }
 }
 
-__device__ void file_rle(Enc& x, bool all_n, IntDict& idict, DblDict& ddict) {
-    uint8_t* o = x.out(kFRle);
-    __shared__ uint64_t pos;
-    if (threadIdx.x == 0) {
-        put32(o, all_n ? 1u : 0u);
-        pos = 4;
-    }
-    __syncthreads();
-    if (all_n) {
-        if (threadIdx.x == 0) x.e.len[x.b * 5 + kFRle] = 4;
-        return;
-    }
-    uint64_t* rv = x.sval();    /* run values */
-    uint32_t* rs = x.saux();    /* run starts */
-    uint64_t* rl = x.sdict();   /* run lengths */
+/* the runs of a column whose run starts are rs[0, R): their lengths and values */
+struct RunLengths {
+    const uint32_t* rs;
+    int64_t n;
+    int R;
+    __device__ int64_t operator[](int64_t r) const { return (r + 1 < R ? (int64_t)rs[r + 1] : n) - (int64_t)rs[r]; }
+};
+template <class T>
+struct RunValues {
+    const uint32_t* rs;
+    const T* col;
+    __device__ T operator[](int64_t r) const { return col[rs[r]]; }
+};
+
+/* Column k of the run-length file: its block, the first one's after the
+ * file's header.  ints and lens: dictionaries of the values and the run
+ * lengths, in separate shared memory (a double column's values are in dbls). */
+template <class T, class D>
+__device__ void rle_column(Enc& x, int k, const T* col, D& vals, IntDict& lens) {
+    constexpr uint64_t kBytes = sizeof(T);
+    uint8_t* o = x.out(kFRle) + task_at(k);
+    const uint64_t p0 = k == 0 ? 4 : 0;
+    uint32_t* rs = x.e.s_runs + ((size_t)x.b * kRleCols + k) * kWin;
     const int lane = threadIdx.x & 31;
     const int64_t wb = warp_base();
-    for (int k = 0; k < 6; ++k) {
-        /* run starts: a row whose value differs from the row before (the row
-         * before a lane's is the lane below's, or for lane 0 the last row of
-         * the warp's previous 32, or the row before the warp's range) */
-        auto starts = [&](auto&& take) {
-            uint64_t carry = wb > 0 && wb < x.n ? x.rle(k, wb - 1) : 0;
-            for (int64_t j0 = wb; j0 < wb + kWarpRows && j0 < x.n; j0 += 32) {
-                const int64_t j = j0 + lane;
-                const bool in = j < x.n;
-                const uint64_t v = in ? x.rle(k, j) : 0;
-                const uint64_t up = __shfl_up_sync(kEncFull, v, 1);
-                const uint64_t prev = lane == 0 ? carry : up;
-                carry = __shfl_sync(kEncFull, v, 31);
-                take(in && (j == 0 || v != prev), j, v);
+    /* run starts: a row whose value differs from the row before (the row
+     * before a lane's is the lane below's, or for lane 0 the last row of
+     * the warp's previous 32, or the row before the warp's range) */
+    auto starts = [&](auto&& take) {
+        T carry = wb > 0 && wb < x.n ? col[wb - 1] : 0;
+        for (int64_t j0 = wb; j0 < wb + kWarpRows && j0 < x.n; j0 += 128) {
+            T v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int64_t j = j0 + 32 * u + lane;
+                v[u] = j < x.n ? col[j] : 0;
             }
-        };
-        int cs = 0;
-        starts([&](bool p, int64_t, uint64_t) { cs += __popc(__ballot_sync(kEncFull, p)); });
-        int64_t R;
-        int64_t orun = warp_prefix(cs, &R);
-        starts([&](bool p, int64_t j, uint64_t v) {
-            const int64_t slot = list_slot(p, &orun);
-            if (p) {
-                rv[slot] = v;
-                rs[slot] = (uint32_t)j;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int64_t j = j0 + 32 * u + lane;
+                const T up = __shfl_up_sync(kEncFull, v[u], 1);
+                const T prev = lane == 0 ? carry : up;
+                carry = __shfl_sync(kEncFull, v[u], 31);
+                take(j < x.n && (j == 0 || v[u] != prev), j);
             }
-        });
-        __syncthreads();
-        for (int64_t r = threadIdx.x; r < R; r += kEncThreads)
-            rl[r] = (uint64_t)((r + 1 < R ? (int64_t)rs[r + 1] : (int64_t)x.n) - (int64_t)rs[r]);
-        __syncthreads();
-        const int m = (int)R;
-        const bool dbl = k == 5;
-        const uint64_t val_bytes = dbl ? 8 : 4;
-        /* sizes: the lengths' dictionary, then the values' */
-        if (idict.build(rl, m) < 0) {
-            x.bad = true;
-            return;
         }
-        const uint64_t ndl = (uint64_t)idict.d, nwl = pack(idict, x.e.bits, rl, m, (uint8_t*)nullptr, false);
-        uint64_t ndv, nwv;
-        if (dbl) {
-            if (ddict.build(rv, m) < 0) {
-                x.bad = true;
-                return;
-            }
-            ndv = (uint64_t)ddict.d;
-            nwv = pack(ddict, x.e.bits, rv, m, (uint8_t*)nullptr, false);
-        } else {
-            if (idict.build(rv, m) < 0) {
-                x.bad = true;
-                return;
-            }
-            ndv = (uint64_t)idict.d;
-            nwv = pack(idict, x.e.bits, rv, m, (uint8_t*)nullptr, false);
-        }
-        const uint64_t p0 = pos;
-        const uint64_t b_cval = p0 + 48, b_clen = b_cval + 4 * nwv, b_dval = b_clen + 4 * nwl,
-                       b_dlen = b_dval + val_bytes * ndv, end = b_dlen + 4 * ndl;
-        if (!x.fits(kFRle, end)) return;
-        /* the values' words and dictionary (the dictionary built last) */
-        if (dbl) {
-            pack(ddict, x.e.bits, rv, m, o + b_cval, true);
-            for (int i = threadIdx.x; i < ddict.d; i += kEncThreads) put64(o + b_dval + 8 * (size_t)i, ddict.value(i));
-        } else {
-            pack(idict, x.e.bits, rv, m, o + b_cval, true);
-            idict.put_values(o + b_dval);
-        }
-        __syncthreads();
-        /* the lengths' dictionary again, for its words and values */
-        idict.build(rl, m);
-        pack(idict, x.e.bits, rl, m, o + b_clen, true);
-        idict.put_values(o + b_dlen);
-        if (threadIdx.x == 0) {
-            const uint64_t param[6] = {(uint64_t)R, nwv, nwl, ndv, ndl, 4 * nwv + 4 * nwl + val_bytes * ndv + 4 * ndl};
-            for (int i = 0; i < 6; ++i) put64(o + p0 + 8 * i, param[i]);
-            pos = end;
-        }
-        __syncthreads();
+    };
+    int cs = 0;
+    starts([&](bool p, int64_t) { cs += __popc(__ballot_sync(kEncFull, p)); });
+    int64_t R;
+    int64_t orun = warp_prefix(cs, &R);
+    starts([&](bool p, int64_t j) {
+        const int64_t slot = list_slot(p, &orun);
+        if (p) rs[slot] = (uint32_t)j;
+    });
+    __syncthreads();
+    const int m = (int)R;
+    const RunLengths rl{rs, x.n, m};
+    const RunValues<T> rv{rs, col};
+    if (lens.build(rl, m) < 0 || vals.build(rv, m) < 0) {
+        x.bad = true;
+        return;
     }
-    if (threadIdx.x == 0) x.e.len[x.b * 5 + kFRle] = pos;
+    const uint64_t ndl = (uint64_t)lens.d, nwl = pack(lens, x.e.bits, rl, m, (uint8_t*)nullptr, false);
+    const uint64_t ndv = (uint64_t)vals.d, nwv = pack(vals, x.e.bits, rv, m, (uint8_t*)nullptr, false);
+    const uint64_t b_cval = p0 + 48, b_clen = b_cval + 4 * nwv, b_dval = b_clen + 4 * nwl, b_dlen = b_dval + kBytes * ndv,
+                   end = b_dlen + 4 * ndl;
+    if (!x.fits(kFRle, end)) return;
+    pack(vals, x.e.bits, rv, m, o + b_cval, true);
+    vals.put_values(o + b_dval);
+    pack(lens, x.e.bits, rl, m, o + b_clen, true);
+    lens.put_values(o + b_dlen);
+    if (threadIdx.x == 0) {
+        if (k == 0) put32a(o, 0u);
+        const uint64_t param[6] = {(uint64_t)R, nwv, nwl, ndv, ndl, 4 * nwv + 4 * nwl + kBytes * ndv + 4 * ndl};
+        for (int i = 0; i < 6; ++i) put64(o + p0 + 8 * i, param[i]);
+    }
+    x.used = end;
+}
+
+__device__ void file_rle(Enc& x, int k, bool all_n, IntDict& idict, IntDict& vdict, DblDict& ddict) {
+    if (all_n) {
+        if (k == 0 && threadIdx.x == 0) put32a(x.out(kFRle), 1u);
+        x.used = k == 0 ? 4 : 0;
+    } else if (k < kRleCols - 1) {
+        rle_column(x, k, x.rle32(k), vdict, idict);
+    } else {
+        rle_column(x, k, x.rle64(), ddict, idict);
+    }
 }
 
 __device__ void file_10(Enc& x, bool all_n) {
     uint8_t* o = x.out(kF10);
     if (threadIdx.x == 0) put32(o, all_n ? 1u : 0u);
     if (all_n) {
-        if (threadIdx.x == 0) x.e.len[x.b * 5 + kF10] = 4;
+        x.used = 4;
         return;
     }
     auto letter = [&](int j) {
@@ -623,7 +644,7 @@ __device__ void file_10(Enc& x, bool all_n) {
         put64(o + 4, (uint64_t)NN);
         put64(o + 12, nw);
         put64(o + 20, n);
-        x.e.len[x.b * 5 + kF10] = total;
+        x.used = total;
     }
 }
 
@@ -631,7 +652,7 @@ __device__ void file_111213(Enc& x, bool all_n, IntDict& idict) {
     uint8_t* o = x.out(kF111213);
     if (threadIdx.x == 0) put32(o, all_n ? 1u : 0u);
     if (all_n) {
-        if (threadIdx.x == 0) x.e.len[x.b * 5 + kF111213] = 4;
+        x.used = 4;
         return;
     }
     /* 0: common, 1: extra column 12, 2: extra column 13, -1: none */
@@ -716,7 +737,7 @@ __device__ void file_111213(Enc& x, bool all_n, IntDict& idict) {
         put64(o + 12, (uint64_t)NC);
         put64(o + 20, (uint64_t)N12);
         put64(o + 28, (uint64_t)N13);
-        x.e.len[x.b * 5 + kF111213] = p;
+        x.used = p;
     }
 }
 
@@ -724,7 +745,7 @@ __device__ void file_1517(Enc& x, bool all_n) {
     uint8_t* o = x.out(kF1517);
     if (threadIdx.x == 0) put32(o, all_n ? 1u : 0u);
     if (all_n) {
-        if (threadIdx.x == 0) x.e.len[x.b * 5 + kF1517] = 4;
+        x.used = 4;
         return;
     }
     const int lane = threadIdx.x & 31;
@@ -765,7 +786,7 @@ __device__ void file_1517(Enc& x, bool all_n) {
     if (threadIdx.x == 0) {
         put32(o + 4, (uint32_t)NR);
         put32(o + b_cnt2, (uint32_t)NS);
-        x.e.len[x.b * 5 + kF1517] = total;
+        x.used = total;
     }
 }
 
@@ -804,23 +825,74 @@ __global__ void __launch_bounds__(kEncThreads) encode_windows_kernel(EncArgs e) 
     ddict.negzero = &hash_negzero;
     ddict.d = 0;
 
-    /* one CTA per (window, file): the five files of a window are
-     * independent, so a small batch of windows still fills the GPU */
-    const int f = (int)blockIdx.y;
-    Enc x{e, (int)blockIdx.x, e.w0 + blockIdx.x, 0, 0, false, f == kF111213 ? 1 : 0};
+    IntDict vdict = idict;   /* in the hash set's place */
+    vdict.bm = reinterpret_cast<uint32_t*>(ddict.tab);
+    vdict.pre = vdict.bm + kBitmapWords;
+
+    /* One CTA per (window, task): the files of a window, and the columns of
+     * the run-length file, are independent, so that a small batch of windows
+     * still fills the GPU.  A chunk of 16 windows with the run-length file's
+     * six columns in one CTA, which then had most of the work: 4.1 ms; a CTA
+     * each: 0.75 ms. */
+    const int t = (int)blockIdx.y;
+    Enc x{e, (int)blockIdx.x, e.w0 + blockIdx.x, 0, 0, false, t, 0};
     x.n = (int)e.call_len[x.w];
     x.hs = e.host_src[x.w];
     const bool all_n = e.not_n[x.b] == 0;
-    switch (f) {
+    switch (task_file(t)) {
         case kF346: file_346(x, all_n); break;
-        case kFRle: file_rle(x, all_n, idict, ddict); break;
+        case kFRle: file_rle(x, t, all_n, idict, vdict, ddict); break;
         case kF10: file_10(x, all_n); break;
         case kF111213: file_111213(x, all_n, idict); break;
         default: file_1517(x, all_n); break;
     }
-    if (threadIdx.x == 0) e.fallback[x.b * 5 + f] = x.bad ? 1 : 0;
+    if (threadIdx.x == 0) {
+        e.fallback[x.b * kTasks + t] = x.bad ? 1 : 0;
+        e.len[x.b * kTasks + t] = x.bad ? 0 : x.used;
+    }
 }
 
+/* A batch's blocks one after another in dst - the files in order, each file's
+ * windows in order, without the windows left to the host - so that they come
+ * down in one copy.  Grid: (parts, windows, tasks); every CTA finds its
+ * block's place from the lengths, a thread per block. */
+__global__ void __launch_bounds__(kPackThreads) pack_blocks_kernel(EncArgs e, int nb, uint8_t* dst) {
+    __shared__ int64_t s_at;
+    const int b = (int)blockIdx.y, t = (int)blockIdx.z;
+    /* thread i: block i in file, window, task order */
+    int i = threadIdx.x, f = 0, tb = 0, tt = 0;
+    int64_t len = 0;
+    if (i < nb * kTasks) {
+        while (i >= nb * file_tasks(f)) i -= nb * file_tasks(f++);
+        tb = i / file_tasks(f);
+        tt = file_task(f) + i % file_tasks(f);
+        bool bad = false;
+        for (int k = 0; k < kTasks; ++k) bad |= e.fallback[tb * kTasks + k] != 0;
+        len = bad ? 0 : (int64_t)e.len[tb * kTasks + tt];
+    }
+    int64_t total;
+    const int64_t at = block_scan(len, &total);
+    __shared__ int64_t s_len;
+    if ((int)threadIdx.x < nb * kTasks && tb == b && tt == t) {
+        s_at = at;
+        s_len = len;
+    }
+    __syncthreads();
+    const uint8_t* src = e.out[task_file(t)] + (size_t)b * e.cap[task_file(t)] + task_at(t);
+    uint8_t* d = dst + s_at;
+    const int64_t n = s_len, step = (int64_t)gridDim.x * kPackThreads;
+    const int64_t first = (int64_t)blockIdx.x * kPackThreads + threadIdx.x;
+    if ((s_at & 3) == 0) {
+        const int64_t n4 = n / 4;
+        for (int64_t k = first; k < n4; k += step)
+            reinterpret_cast<uint32_t*>(d)[k] = reinterpret_cast<const uint32_t*>(src)[k];
+        if (first < (n & 3)) d[n4 * 4 + first] = src[n4 * 4 + first];
+    } else {
+        for (int64_t k = first; k < n; k += step) d[k] = src[k];
+    }
+}
+
+static_assert(2 * kBitmapWords * 4 <= kHashCap * 8, "a second integer dictionary in the hash set's place");
 constexpr size_t kEncSmem = 2 * kBitmapWords * 4 + kHashCap * 8;
 static_assert(kEncSmem <= 220 * 1024, "the encoder's shared memory fits one CTA per SM");
 
@@ -841,9 +913,8 @@ ColumnsGpuWriter::~ColumnsGpuWriter() {
         close(&e);
     }
     release();
-    for (int set = 0; set < 2; ++set)
-        for (int f = 0; f < 5; ++f)
-            if (hbuf_[set][f]) cudaFreeHost(hbuf_[set][f]);
+    for (char* h : hbuf_)
+        if (h) cudaFreeHost(h);
 }
 
 void ColumnsGpuWriter::release() {
@@ -855,6 +926,11 @@ void ColumnsGpuWriter::release() {
     cudaFree(d_len_tab_);
     cudaFree(d_len_);
     cudaFree(d_fb_);
+    cudaFree(d_runs_);
+    cudaFree(d_pack_);
+    d_runs_ = nullptr;
+    d_pack_ = nullptr;
+    pack_cap_ = 0;
     cudaFree(d_sval_);
     cudaFree(d_sdict_);
     cudaFree(d_saux_);
@@ -900,17 +976,18 @@ int ColumnsGpuWriter::open(const WindowPlan& plan, const char* chr_name, const s
         fprintf(f12_, "%s\t%lu\t%lu\n", chr_name, (unsigned long)(w * (int64_t)kWin + 1),
                 (unsigned long)plan.call_len[w]);
     /* device buffers of one batch of windows, kept from one use to the next */
-    batch = std::max<int64_t>(1, batch);
+    batch = std::max<int64_t>(1, std::min<int64_t>(batch, kMostWindows));
     cudaError_t ce = cudaSuccess;
     if (batch > batch_cap_) {
         release();
         for (int f = 0; f < 5 && ce == cudaSuccess; ++f) ce = cudaMalloc((void**)&d_out_[f], kCapHost[f] * (size_t)batch);
         if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_bits_, kWin + 2);
-        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_len_, sizeof(uint64_t) * 5 * batch);
-        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_fb_, sizeof(int) * 5 * batch);
-        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_sval_, sizeof(uint64_t) * kWin * 2 * batch);
-        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_sdict_, sizeof(uint64_t) * kWin * 2 * batch);
-        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_saux_, sizeof(uint32_t) * kWin * 2 * batch);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_len_, sizeof(uint64_t) * kTasks * batch);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_fb_, sizeof(int) * kTasks * batch);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_runs_, sizeof(uint32_t) * kWin * kRleCols * batch);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_sval_, sizeof(uint64_t) * kWin * batch);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_sdict_, sizeof(uint64_t) * kWin * batch);
+        if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_saux_, sizeof(uint32_t) * kWin * batch);
         if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_rle32_, sizeof(uint32_t) * kWin * 5 * batch);
         if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_rle64_, sizeof(uint64_t) * kWin * batch);
         if (ce == cudaSuccess) ce = cudaMalloc((void**)&d_not_n_, sizeof(int) * batch);
@@ -963,8 +1040,14 @@ int ColumnsGpuWriter::write(int64_t w0, int64_t w1, const uint8_t* d_codes, cons
     const WindowPlan& plan = *plan_;
     int rc = 0;
     cudaError_t ce = cudaSuccess;
-    std::vector<uint64_t> h_len((size_t)(5 * batch_cap_));
-    std::vector<int> h_fb5((size_t)(5 * batch_cap_)), h_fb((size_t)batch_cap_);
+    std::vector<uint64_t> h_len((size_t)(kTasks * batch_cap_));
+    std::vector<int> h_fb5((size_t)(kTasks * batch_cap_)), h_fb((size_t)batch_cap_);
+    /* bytes of window b's block of file f */
+    auto file_len = [&](int64_t b, int f) {
+        size_t n = 0;
+        for (int t = file_task(f); t < file_task(f) + file_tasks(f); ++t) n += (size_t)h_len[(size_t)(kTasks * b + t)];
+        return n;
+    };
     for (int64_t b0 = w0; b0 < w1 && rc == 0; b0 += batch_cap_) {
         const int64_t nb = std::min(batch_cap_, w1 - b0);
         EncArgs e;
@@ -981,6 +1064,7 @@ int ColumnsGpuWriter::write(int64_t w0, int64_t w1, const uint8_t* d_codes, cons
         }
         e.len = d_len_;
         e.fallback = d_fb_;
+        e.s_runs = d_runs_;
         e.s_val = d_sval_;
         e.s_aux = d_saux_;
         e.s_dict = d_sdict_;
@@ -994,16 +1078,16 @@ int ColumnsGpuWriter::write(int64_t w0, int64_t w1, const uint8_t* d_codes, cons
             ce = cudaGetLastError();
         }
         if (ce == cudaSuccess) {
-            encode_windows_kernel<<<dim3((unsigned)nb, 5), kEncThreads, kEncSmem, stream>>>(e);
+            encode_windows_kernel<<<dim3((unsigned)nb, kTasks), kEncThreads, kEncSmem, stream>>>(e);
             ce = cudaGetLastError();
         }
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(h_len.data(), d_len_, sizeof(uint64_t) * 5 * nb, cudaMemcpyDeviceToHost, stream);
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(h_fb5.data(), d_fb_, sizeof(int) * 5 * nb, cudaMemcpyDeviceToHost, stream);
+        if (ce == cudaSuccess) ce = cudaMemcpyAsync(h_len.data(), d_len_, sizeof(uint64_t) * kTasks * nb, cudaMemcpyDeviceToHost, stream);
+        if (ce == cudaSuccess) ce = cudaMemcpyAsync(h_fb5.data(), d_fb_, sizeof(int) * kTasks * nb, cudaMemcpyDeviceToHost, stream);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream);
         /* a window goes to the host encoder when any of its files did not fit */
         for (int64_t b = 0; b < nb; ++b) {
             int any = 0;
-            for (int f = 0; f < 5; ++f) any |= h_fb5[(size_t)(5 * b + f)];
+            for (int t = 0; t < kTasks; ++t) any |= h_fb5[(size_t)(kTasks * b + t)];
             h_fb[(size_t)b] = any;
         }
         if (ce != cudaSuccess) {
@@ -1011,9 +1095,9 @@ int ColumnsGpuWriter::write(int64_t w0, int64_t w1, const uint8_t* d_codes, cons
             rc = 1;
             break;
         }
-        /* the batch's blocks, window by window, into one pinned host buffer
-         * per file, of the set the batch before last used (its writes are
-         * waited for first) */
+        /* the batch's blocks, file by file, into one pinned host buffer, of
+         * the set the batch before last used (its writes are waited for
+         * first) */
         const int set = set_;
         set_ ^= 1;
         if (!wait_set(set)) {
@@ -1021,29 +1105,31 @@ int ColumnsGpuWriter::write(int64_t w0, int64_t w1, const uint8_t* d_codes, cons
             rc = 1;
             break;
         }
-        size_t tot[5] = {};
-        for (int64_t b = 0; b < nb; ++b)
-            if (!h_fb[(size_t)b])
-                for (int f = 0; f < 5; ++f) tot[f] += h_len[(size_t)(5 * b + f)];
-        for (int f = 0; f < 5 && ce == cudaSuccess; ++f)
-            if (hcap_[set][f] < tot[f]) {
-                /* pinned, so that the blocks come down at the link's speed */
-                if (hbuf_[set][f]) cudaFreeHost(hbuf_[set][f]);
-                hbuf_[set][f] = nullptr;
-                hcap_[set][f] = 0;
-                ce = cudaMallocHost((void**)&hbuf_[set][f], tot[f] + tot[f] / 4);
-                if (ce == cudaSuccess) hcap_[set][f] = tot[f] + tot[f] / 4;
-            }
-        size_t off[5] = {};
-        for (int64_t b = 0; b < nb && ce == cudaSuccess; ++b) {
-            if (h_fb[(size_t)b]) continue;
-            for (int f = 0; f < 5 && ce == cudaSuccess; ++f) {
-                const size_t bytes = (size_t)h_len[(size_t)(5 * b + f)];
-                if (bytes)
-                    ce = cudaMemcpyAsync(hbuf_[set][f] + off[f], d_out_[f] + (size_t)b * kCapHost[f], bytes,
-                                         cudaMemcpyDeviceToHost, stream);
-                off[f] += bytes;
-            }
+        size_t total = 0, at[5] = {};
+        for (int f = 0; f < 5; ++f) {
+            at[f] = total;
+            for (int64_t b = 0; b < nb; ++b)
+                if (!h_fb[(size_t)b]) total += file_len(b, f);
+        }
+        if (pack_cap_ < total) {
+            cudaFree(d_pack_);
+            d_pack_ = nullptr;
+            pack_cap_ = 0;
+            ce = cudaMalloc((void**)&d_pack_, total + total / 4);
+            if (ce == cudaSuccess) pack_cap_ = total + total / 4;
+        }
+        if (ce == cudaSuccess && hcap_[set] < total) {
+            /* pinned, so that the blocks come down at the link's speed */
+            if (hbuf_[set]) cudaFreeHost(hbuf_[set]);
+            hbuf_[set] = nullptr;
+            hcap_[set] = 0;
+            ce = cudaMallocHost((void**)&hbuf_[set], total + total / 4);
+            if (ce == cudaSuccess) hcap_[set] = total + total / 4;
+        }
+        if (ce == cudaSuccess && total > 0) {
+            pack_blocks_kernel<<<dim3(4, (unsigned)nb, kTasks), kPackThreads, 0, stream>>>(e, (int)nb, d_pack_);
+            ce = cudaGetLastError();
+            if (ce == cudaSuccess) ce = cudaMemcpyAsync(hbuf_[set], d_pack_, total, cudaMemcpyDeviceToHost, stream);
         }
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream);
         if (ce != cudaSuccess) {
@@ -1096,13 +1182,17 @@ int ColumnsGpuWriter::write(int64_t w0, int64_t w1, const uint8_t* d_codes, cons
         /* each file's pieces in window order: the encoder's blocks, and the
          * host-encoded windows in their places */
         std::vector<Piece> pieces[5];
-        size_t wo[5] = {};
         for (int64_t b = 0; b < nb; ++b) {
             if (!h_fb[(size_t)b]) {
                 for (int f = 0; f < 5; ++f) {
-                    const size_t bytes = (size_t)h_len[(size_t)(5 * b + f)];
-                    if (bytes) pieces[f].push_back(Piece{hbuf_[set][f] + wo[f], bytes, nullptr});
-                    wo[f] += bytes;
+                    const size_t bytes = file_len(b, f);
+                    const char* src = hbuf_[set] + at[f];
+                    at[f] += bytes;
+                    if (!bytes) continue;
+                    if (!pieces[f].empty() && !pieces[f].back().own && pieces[f].back().p + pieces[f].back().n == src)
+                        pieces[f].back().n += bytes;
+                    else
+                        pieces[f].push_back(Piece{src, bytes, nullptr});
                 }
                 continue;
             }
@@ -1142,7 +1232,8 @@ int ColumnsGpuWriter::write(int64_t w0, int64_t w1, const uint8_t* d_codes, cons
 size_t ColumnsGpuWriter::device_bytes() const {
     size_t n = 0;
     for (int f = 0; f < 5; ++f) n += kCapHost[f] * (size_t)batch_cap_;
-    return n + (size_t)batch_cap_ * (kWin * (40 + 28) + 64) + (kWin + 2) + (size_t)len_tab_windows_ * 8;
+    return n + (size_t)batch_cap_ * (kWin * (4 * kRleCols + 20 + 28) + kTasks * 12 + 4) + pack_cap_ + (kWin + 2) +
+           (size_t)len_tab_windows_ * 8;
 }
 
 bool ColumnsGpuWriter::wait_set(int set) {

@@ -64,10 +64,13 @@ private:
     int* d_fb_ = nullptr;
     uint64_t *d_sval_ = nullptr, *d_sdict_ = nullptr;
     uint32_t* d_saux_ = nullptr;
+    uint32_t* d_runs_ = nullptr;
+    uint8_t* d_pack_ = nullptr;
+    size_t pack_cap_ = 0;
     uint32_t* d_rle32_ = nullptr;
     uint64_t* d_rle64_ = nullptr;
     int* d_not_n_ = nullptr;
-    /* two sets of pinned buffers, a batch's blocks of each file, used in
+    /* two pinned buffers, a batch's blocks file by file, used in
      * turn; the file writes of a batch run on their own threads, one per
      * file, each after the same file's previous batch */
     struct Piece {
@@ -76,8 +79,8 @@ private:
         std::shared_ptr<std::string> own;   /* a host-encoded block */
     };
     bool wait_set(int set);
-    char* hbuf_[2][5] = {};
-    size_t hcap_[2][5] = {};
+    char* hbuf_[2] = {};
+    size_t hcap_[2] = {};
     int set_ = 0;
     std::shared_future<bool> last_[5];
     std::shared_future<bool> pend_[2][5];
