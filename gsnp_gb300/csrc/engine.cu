@@ -1525,11 +1525,14 @@ int regather(gsnp_context* c) {
 /* Number of segments of a call that moves `bytes` over the host link
  * (GSNP_SEGMENTS overrides).  With S segments the first one's upload and the
  * last one's download are not overlapped, bytes / (S x 200 GB/s) in all, and
- * each segment adds about 50 us (the last tiles of its persistent kernel, its
- * launches); the sum is least at S = sqrt(bytes / 10 MB).  c1 (16 Mbp, packed,
- * 1.05 GB): 8.2 ms in the 2 segments of one per two million reads, 5.9 in 10. */
+ * each segment adds about 100 us (the last tiles of its persistent kernel, its
+ * leftover tiles waiting for room, its launches); the sum is least at
+ * S = sqrt(bytes / 20 MB).  Measured, in ms: c1, 16 Mbp (FP32): 9.9 in 1, 6.8
+ * in 4, 6.3 in 8, 6.4 in 12; c3, 5 Mbp: 4.4 in 1, 2.8 in 4, 2.8 in 6, 3.1 in
+ * 10; c2, 10 Mbp: 11.2 in 1, 7.9 in 5, 8.3 in 10; c1, 6 Mbp (FP64): 5.9 in 1,
+ * 3.9 in 5, 4.1 in 10; c0, 1 Mbp: 0.78 in 1, 0.77 in 2, 0.84 in 4. */
 int segment_count(uint64_t bytes, int64_t n_windows) {
-    int n = (int)std::min(16.0, std::max(1.0, std::floor(std::sqrt((double)bytes / 10e6) + 0.5)));
+    int n = (int)std::min(16.0, std::max(1.0, std::floor(std::sqrt((double)bytes / 20e6) + 0.5)));
     if (const char* e = getenv("GSNP_SEGMENTS")) n = std::max(1, atoi(e));
     return (int)std::max<int64_t>(1, std::min<int64_t>(n, n_windows));
 }
