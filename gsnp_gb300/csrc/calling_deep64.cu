@@ -13,8 +13,10 @@
  * takes the posterior of all of them at once, a site per lane.  Heterozygous
  * candidates, about one site in a thousand, have their column piled up again
  * for the rank sums, which saves holding the qualities of every site.
- * c2, 3 Mbp, 14,470 tiles of the bin: 7.2 -> 4.1 ms.  What bounds it now is the
- * pileup: every site scans the starts of all reads over its tile.
+ * c2, 3 Mbp, 14,470 tiles of the bin: 7.2 -> 4.1 ms.  While its SMs are busy
+ * half of their issue slots and of their FP64 pipe's are taken; the rest is the
+ * latency of a site's shuffles and table rows (loading the next eight terms
+ * ahead of the additions changed nothing).
  */
 #include <cuda_runtime.h>
 
@@ -30,8 +32,7 @@ namespace gsnp {
 
 namespace {
 
-constexpr int kBatch = 8;                     /* sites a warp holds; a tile is four batches */
-constexpr int kBatches = kTile / kBatch;
+constexpr int kBatch = kDeepBatch;            /* sites a warp holds */
 constexpr int kAtOnce = 3;                    /* sites summed together, ten lanes each */
 constexpr int kDeep64Warps = 24;
 
@@ -47,6 +48,8 @@ struct DeepWarp {
             int32_t hist[2][66];
         } s;
     } u;
+    uint32_t span[2 * (kBatch + 1)];
+    uint32_t pad[2];
     int32_t rank2[kBatch][2];                 /* twice the rank sums of the candidate's alleles */
     uint16_t num[kBatch], base_end[kBatch][3];   /* records; the end of bases 0, 1 and 2 among them */
 };
@@ -73,13 +76,13 @@ __device__ __noinline__ void deep_posterior(const CallArgs& a, int64_t site, uin
     a.out[site] = call;
 }
 
-/* Sites [first, first + kBatch) of a tile by one warp. */
-__device__ __forceinline__ void deep_batch(const CallArgs& a, int64_t tile, int first, DeepWarp& sm) {
+/* Sites [first, first + sites) of a tile, sites <= kBatch, by one warp. */
+__device__ __forceinline__ void deep_batch(const CallArgs& a, int64_t tile, int first, int sites, DeepWarp& sm) {
     const int lane = threadIdx.x & 31;
     const int64_t s0 = tile * kTile;
     const uint8_t ori_t = s0 + lane < a.chr_len ? __ldg(a.ori + s0 + lane) : 0;
     const int32_t snp_t = tile_snp_row(a, tile, (ori_t & 8) != 0);
-    const int n = (int)min((int64_t)kBatch, a.chr_len - (s0 + first));
+    const int n = (int)min((int64_t)sites, a.chr_len - (s0 + first));
     if (n <= 0) return;
     /* lane j < n owns site s0 + first + j */
     const int64_t site = s0 + first + lane;
@@ -89,10 +92,16 @@ __device__ __forceinline__ void deep_batch(const CallArgs& a, int64_t tile, int 
     const uint8_t wflags = a.win_flags[win];
     const int64_t r_lo = a.warp_rng[tile * 2], r_hi = a.warp_rng[tile * 2 + 1];
     const bool external = (wflags & kWinExternalLik) != 0;
+    const DeepSpan span = deep_spans(a, r_lo, r_hi, s0 + first, sm.span);
+    auto pileup = [&](int j) {
+        const SitePileup p = deep_pileup(a, r_lo + __shfl_sync(kFull, span.skip, j), r_hi, s0 + first + j,
+                                         __shfl_sync(kFull, span.depth, j), __shfl_sync(kFull, span.repeat, j), sm.recs);
+        __syncwarp();
+        return p;
+    };
     SitePileup mine = {};
     for (int j = 0; j < n; ++j) {
-        const SitePileup p = deep_pileup(a, r_lo, r_hi, s0 + first + j, sm.recs);
-        __syncwarp();
+        const SitePileup p = pileup(j);
         if (lane == j) mine = p;
         if (lane == 0) {
             sm.num[j] = (uint16_t)p.num;
@@ -171,16 +180,15 @@ __device__ __forceinline__ void deep_batch(const CallArgs& a, int64_t tile, int 
     for (unsigned m = __ballot_sync(kFull, het); m; m &= m - 1) {
         const int j = __ffs(m) - 1;
         const int g = __shfl_sync(kFull, best, j);
-        const SitePileup p = deep_pileup(a, r_lo, r_hi, s0 + first + j, sm.recs);
-        __syncwarp();
+        const SitePileup p = pileup(j);
         warp_ranks(a, sm.recs, p.num, g, sm.u.s.hist, sm.rank2[j]);
     }
     if (lane < n) deep_posterior(a, site, ori, snp_row, mine, sm.u.s.sum[lane], lp, sm.rank2[lane]);
     __syncwarp();
 }
 
-/* The first n tiles of the list, or with count the first *count, a batch of
- * kBatch sites at a time; from *next (zero before the launch), or in strides
+/* The first n tiles of the list, or with count the first *count, some
+ * sites (deep_sites) at a time to each warp; from *next (zero before the launch), or in strides
  * of the grid. */
 __global__ void __launch_bounds__(32 * kDeep64Warps, 1)
     call_deep64_kernel(const __grid_constant__ CallArgs a, const int32_t* __restrict__ tiles, int n,
@@ -188,11 +196,13 @@ __global__ void __launch_bounds__(32 * kDeep64Warps, 1)
     extern __shared__ __align__(16) uint8_t smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     DeepWarp& sm = reinterpret_cast<DeepWarp*>(smem)[w];
-    const unsigned items = (unsigned)(count ? *count : n) * kBatches;
+    if (count) n = *count;
     const unsigned step = gridDim.x * kDeep64Warps;
+    const int sites = deep_sites(n, (int)step);
+    const unsigned per = (unsigned)(kTile / sites), items = (unsigned)n * per;
     unsigned item = blockIdx.x * kDeep64Warps + w;
     while (item < items) {
-        deep_batch(a, tiles[item / kBatches], (int)(item % kBatches) * kBatch, sm);
+        deep_batch(a, tiles[item / per], (int)(item % per) * sites, sites, sm);
         unsigned nx = item + step;
         if (next) {
             if (lane == 0) nx = (unsigned)atomicAdd(next, 1) + step;
@@ -220,7 +230,7 @@ cudaError_t launch_deep64(const CallArgs& a, const int32_t* tiles, const BinLaun
     const cudaError_t e = g_launch_attributes ? deep64_attr(nullptr) : cudaSuccess;
     if (e != cudaSuccess) return e;
     const unsigned grid = bl.d_count ? (unsigned)bl.grid
-                                     : (unsigned)(((int64_t)bl.count * kBatches + kDeep64Warps - 1) / kDeep64Warps);
+                                     : (unsigned)(((int64_t)bl.count * kDeepBatches + kDeep64Warps - 1) / kDeep64Warps);
     if (grid == 0) return cudaSuccess;
     call_deep64_kernel<<<grid, 32 * kDeep64Warps, kDeep64Smem, stream>>>(a, tiles, bl.count, bl.d_count,
                                                                        bl.d_count ? bl.d_next : nullptr);

@@ -248,13 +248,27 @@ __global__ void __launch_bounds__(kTile, kFastCtasPerSm) call_fast_kernel(const 
 /* the deep bins of the FP32 form: one warp per site                          */
 /* ------------------------------------------------------------------------ */
 
-/* Tiles with a site of more than 64 records (hotspots of hundreds of reads)
- * are called by a CTA of 32 warps, warp w calling site w of the tile, so that
- * a site's hundreds of records are spread over 32 lanes instead of walked by
- * one.  Per warp, in shared memory: the site's record column (at most 255
- * records) and a byte counter per (base, strand, cycle) key. */
+/* Tiles with a site of more than 128 records (hotspots of hundreds of reads)
+ * are called by warps of kDeepBatch neighbouring sites each: a site's hundreds
+ * of records are spread over 32 lanes instead of walked by one, one site
+ * after another, and the posteriors of the batch are taken together, a site
+ * per lane.  What bounds the kernel is instruction issue; c2, 4 Mbp, some
+ * 9,000 tiles: 2.26 ms with a warp per site that scanned all the tile's reads
+ * for its depth, 1.87 in batches that count the depth of their sites in one
+ * pass and end each site's own scan at its 255th record. */
 constexpr int kDeepThreads = 32 * kTile;
-constexpr size_t kDeepSmem = (size_t)kTile * (kDeepCap * 4 + kDeepKeys);
+
+/* a warp's shared memory */
+struct DeepWarp32 {
+    uint32_t recs[kDeepCap];
+    uint8_t cnt[kDeepKeys];
+    float sum[kDeepBatch][12];
+    SitePileup pile[kDeepBatch];
+    uint32_t span[2 * (kDeepBatch + 1)];
+    uint32_t pad[2];
+};
+static_assert(sizeof(DeepWarp32) % 16 == 0, "16-byte aligned per warp");
+constexpr size_t kDeepSmem = (size_t)kTile * sizeof(DeepWarp32);
 
 /* The FP32 sums of a sorted column by its warp: each lane sums its records'
  * rows with compensation; the 32 sums are then added in a tree (the bound of
@@ -278,26 +292,45 @@ __device__ __forceinline__ void deep_walk_sums(const CallArgs& a, const uint32_t
     }
 }
 
-/* Site w of a deep tile, called by one warp (as fast_site: counts kept for
- * later gap windows, the FP32 posterior, or the site deferred with its
- * records). */
-__device__ __forceinline__ void deep_tile(const CallArgs& a, int64_t tile, int w, uint32_t* recs, uint8_t* cnt) {
+/* Sites [first, first + sites) of a deep tile, called by one warp (as
+ * fast_site: counts kept for later gap windows, the FP32 posterior, or the
+ * site deferred with its records, which are piled up and sorted once more for
+ * that: one site in some hundreds). */
+__device__ __forceinline__ void deep_batch(const CallArgs& a, int64_t tile, int first, int sites, DeepWarp32& sm) {
     const int lane = threadIdx.x & 31;
-    const int64_t s0 = tile * kTile, site = s0 + w;
-    const int64_t sl = s0 + lane;
-    const uint8_t ori_l = sl < a.chr_len ? __ldg(a.ori + sl) : 0;
-    const unsigned flagged = __ballot_sync(kFull, (ori_l & 8) != 0);
-    if (site >= a.chr_len) return;
-    const uint8_t ori = (uint8_t)__shfl_sync(kFull, ori_l, w);
-    const int32_t snp_row = (ori & 8) ? a.tile_snp[tile] + __popc(flagged & ((1u << w) - 1u)) : -1;
+    const int64_t s0 = tile * kTile, b0 = s0 + first;
+    const uint8_t ori_t = s0 + lane < a.chr_len ? __ldg(a.ori + s0 + lane) : 0;
+    const int32_t snp_t = tile_snp_row(a, tile, (ori_t & 8) != 0);
+    const int n = (int)min((int64_t)sites, a.chr_len - b0);
+    if (n <= 0) return;
     const uint8_t wflags = a.win_flags[s0 / kWin];
-    const SitePileup p = deep_pileup(a, a.warp_rng[tile * 2], a.warp_rng[tile * 2 + 1], site, recs);
-    __syncwarp();
-    deep_sort(recs, p.num);
-    float s[10];
-    deep_walk_sums(a, recs, cnt, p.num, s);
+    const int64_t r_lo = a.warp_rng[tile * 2], r_hi = a.warp_rng[tile * 2 + 1];
+    const DeepSpan span = deep_spans(a, r_lo, r_hi, b0, sm.span);
+    auto pileup = [&](int j) {
+        const SitePileup p = deep_pileup(a, r_lo + __shfl_sync(kFull, span.skip, j), r_hi, b0 + j,
+                                         __shfl_sync(kFull, span.depth, j), __shfl_sync(kFull, span.repeat, j), sm.recs);
+        __syncwarp();
+        deep_sort(sm.recs, p.num);
+        return p;
+    };
+    for (int j = 0; j < n; ++j) {
+        const SitePileup p = pileup(j);
+        if (lane == 0) sm.pile[j] = p;
+        float s[10];
+        deep_walk_sums(a, sm.recs, sm.cnt, p.num, s);
+        if (lane == 0) {
+#pragma unroll
+            for (int v = 0; v < 10; ++v) sm.sum[j][v] = s[v];
+        }
+        __syncwarp();
+    }
+    /* lane j < n: site b0 + j */
+    const int64_t site = b0 + lane;
+    const uint8_t ori = (uint8_t)__shfl_sync(kFull, ori_t, (first + lane) & 31);
+    const int32_t snp_row = __shfl_sync(kFull, snp_t, (first + lane) & 31);
     uint8_t dflags = 0;
-    if (lane == 0) {
+    if (lane < n) {
+        const SitePileup p = sm.pile[lane];
         if (p.depth > 0xffff) atomicExch(a.error, 1);
         if (wflags & kWinKeepCounts) store_counts(a, site, p);
         SiteCall call;
@@ -308,70 +341,81 @@ __device__ __forceinline__ void deep_tile(const CallArgs& a, int64_t tile, int w
             call.depth = p.depth;
             call.repeat_time = p.repeat;
             call.flags |= dflags;
-        } else if (fast_posterior(a, snp_row, ori, p, s, p.num, &call, 9.0f)) {
-            call.flags |= dflags;
         } else {
-            call = SiteCall{};
-            dflags |= kCallPending;
-            call.flags = dflags;
+            float s[10];
+#pragma unroll
+            for (int v = 0; v < 10; ++v) s[v] = sm.sum[lane][v];
+            if (fast_posterior(a, snp_row, ori, p, s, p.num, &call, 9.0f)) {
+                call.flags |= dflags;
+            } else {
+                call = SiteCall{};
+                dflags |= kCallPending;
+                call.flags = dflags;
+            }
         }
         a.out[site] = call;
     }
-    dflags = (uint8_t)__shfl_sync(kFull, dflags, 0);
-    if (!dflags) return;
-    /* the site and its sorted records to the deferred pool */
-    unsigned long long slot = 0, off = 0;
-    if (lane == 0) {
-        slot = atomicAdd(a.dcount, 1ull);
-        off = atomicAdd(a.dcount + 1, (unsigned long long)p.num);
-    }
-    slot = __shfl_sync(kFull, slot, 0);
-    off = __shfl_sync(kFull, off, 0);
-    if ((int64_t)slot >= a.dsite_cap || (int64_t)(off + p.num) > a.dpool_cap) return;
-    for (int i = lane; i < p.num; i += 32) a.dpool[off + i] = recs[i];
-    if (lane == 0) {
-        DeferredSite d;
-        d.site = site;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            d.cu[b] = (uint16_t)p.cu[b];
-            d.qs[b] = (uint16_t)p.qs[b];
-            d.ca[b] = p.ca[b];
+    /* the deferred sites and their sorted records to the pool */
+    for (unsigned m = __ballot_sync(kFull, dflags != 0); m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const SitePileup p = pileup(j);
+        const uint8_t fl = (uint8_t)__shfl_sync(kFull, dflags, j);
+        const int32_t row = __shfl_sync(kFull, snp_row, j);
+        unsigned long long slot = 0, off = 0;
+        if (lane == 0) {
+            slot = atomicAdd(a.dcount, 1ull);
+            off = atomicAdd(a.dcount + 1, (unsigned long long)p.num);
         }
-        d.depth = p.depth;
-        d.repeat = p.repeat;
-        d.rec_off = (uint32_t)off;
-        d.num = (uint16_t)p.num;
-        d.dep_uni = (uint16_t)p.dep_uni;
-        d.snp_row = snp_row;
-        d.flags = dflags;
+        slot = __shfl_sync(kFull, slot, 0);
+        off = __shfl_sync(kFull, off, 0);
+        if ((int64_t)slot >= a.dsite_cap || (int64_t)(off + p.num) > a.dpool_cap) continue;
+        for (int i = lane; i < p.num; i += 32) a.dpool[off + i] = sm.recs[i];
+        if (lane == 0) {
+            DeferredSite d;
+            d.site = b0 + j;
 #pragma unroll
-        for (int b = 0; b < 3; ++b) d.pad[b] = 0;
-        a.dsites[slot] = d;
+            for (int b = 0; b < 4; ++b) {
+                d.cu[b] = (uint16_t)p.cu[b];
+                d.qs[b] = (uint16_t)p.qs[b];
+                d.ca[b] = p.ca[b];
+            }
+            d.depth = p.depth;
+            d.repeat = p.repeat;
+            d.rec_off = (uint32_t)off;
+            d.num = (uint16_t)p.num;
+            d.dep_uni = (uint16_t)p.dep_uni;
+            d.snp_row = row;
+            d.flags = fl;
+#pragma unroll
+            for (int b = 0; b < 3; ++b) d.pad[b] = 0;
+            a.dsites[slot] = d;
+        }
+        __syncwarp();
     }
+    __syncwarp();
 }
 
-/* The tiles of a deep FP32 bin: tiles[blockIdx.x] with count == nullptr, warp
- * w calling its site w; else the sites of the first *count tiles of the list,
- * handed out one at a time to each warp from *next (zero before the launch),
- * so that no warp waits for the deepest site of a tile. */
+/* The first n tiles of the list, or with count the first *count, some
+ * sites (deep_sites) at a time to each warp: from *next (zero before the launch), or in
+ * strides of the grid. */
 __global__ void __launch_bounds__(kDeepThreads, 1) call_deep_kernel(const __grid_constant__ CallArgs a, const int32_t* __restrict__ tiles,
-                                                                    const int* __restrict__ count, int* next) {
+                                                                    int n, const int* __restrict__ count, int* next) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t* recs = reinterpret_cast<uint32_t*>(smem) + (size_t)w * kDeepCap;
-    uint8_t* cnt = smem + (size_t)kTile * kDeepCap * 4 + (size_t)w * kDeepKeys;
-    if (!count) {
-        deep_tile(a, tiles[blockIdx.x], w, recs, cnt);
-        return;
-    }
-    const unsigned items = (unsigned)*count * kTile;   /* tile-list index * kTile + site */
-    unsigned item = blockIdx.x * kTile + w;
+    DeepWarp32& sm = reinterpret_cast<DeepWarp32*>(smem)[w];
+    if (count) n = *count;
+    const unsigned step = gridDim.x * (kDeepThreads / 32);
+    const int sites = deep_sites(n, (int)step);
+    const unsigned per = (unsigned)(kTile / sites), items = (unsigned)n * per;
+    unsigned item = blockIdx.x * (kDeepThreads / 32) + w;
     while (item < items) {
-        deep_tile(a, tiles[item / kTile], (int)(item % kTile), recs, cnt);
-        unsigned nx = 0;
-        if (lane == 0) nx = (unsigned)atomicAdd(next, 1) + gridDim.x * kTile;
-        item = __shfl_sync(kFull, nx, 0);
+        deep_batch(a, tiles[item / per], (int)(item % per) * sites, sites, sm);
+        unsigned nx = item + step;
+        if (next) {
+            if (lane == 0) nx = (unsigned)atomicAdd(next, 1) + step;
+            nx = __shfl_sync(kFull, nx, 0);
+        }
+        item = nx;
     }
 }
 
@@ -681,10 +725,14 @@ template <int SLOTS>
 static cudaError_t launch_fast(const CallArgs& a, const int32_t* tiles, const BinLaunch& bl, cudaStream_t stream) {
     cudaError_t e = g_launch_attributes ? fast_attr<SLOTS>(a.L, bl.carveout, nullptr) : cudaSuccess;
     if (e != cudaSuccess) return e;
-    const unsigned grid = (unsigned)(bl.d_count ? bl.grid : bl.count);
+    constexpr int64_t kWarps = kDeepThreads / 32;
+    const unsigned grid = (unsigned)(bl.d_count                ? bl.grid
+                                     : SLOTS >= kDeepSlots ? ((int64_t)bl.count * kDeepBatches + kWarps - 1) / kWarps
+                                                           : bl.count);
     if (grid == 0) return cudaSuccess;
     if constexpr (SLOTS >= kDeepSlots)
-        call_deep_kernel<<<grid, kDeepThreads, kDeepSmem, stream>>>(a, tiles, bl.d_count, bl.d_next);
+        call_deep_kernel<<<grid, kDeepThreads, kDeepSmem, stream>>>(a, tiles, bl.count, bl.d_count,
+                                                                    bl.d_count ? bl.d_next : nullptr);
     else
         call_fast_kernel<SLOTS><<<grid, kTile, call_smem_bytes(SLOTS, a.L), stream>>>(a, tiles, bl.d_count,
                                                                                             bl.d_next);

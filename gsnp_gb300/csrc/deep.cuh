@@ -16,45 +16,112 @@ namespace gsnp {
 constexpr int kDeepCap = 256;              /* records of a column (at most 255), a power of two */
 constexpr int kDeepKeys = 4 * 2 * 256;     /* (base, strand, cycle) keys */
 
-/* The pileup of one site by its warp (kernel/update_kernel.cu:260-325, as
- * PileupAcc::take): the reads [r_lo, r_hi) 32 at a time, in order.  A
- * covering read counts in depth and repeat; one that is not N and reaches
- * q_min is taken while the site has fewer than 255 unique records, and a
- * unique one (hit 1) adds a record.  Whether the cap still admits a read
- * depends only on the unique valid reads before it, which a ballot gives, so
- * the 32 reads of a step are decided together with the reference's result.
- * Once the cap is reached a read can only add to depth and repeat, which
- * need no base or quality; the scan ends at the first step whose reads all
- * start past the site.
- *
- * The scan is bound by load latency (each step's base and quality load
- * depends on the read's start), so its loads run ahead of the decisions: an
- * iteration loads the starts and lengths of its kDeepAhead steps' reads in
- * the iteration before, and their bases, qualities and strands all at its
- * start (for every covering read, when the site was below the cap as the
- * iteration began; a step that finds the site capped leaves its loads
- * unused).  The steps are then decided in order, as above. */
+/* neighbouring sites of a tile that a warp takes together */
+constexpr int kDeepBatch = 8;
+constexpr int kDeepBatches = kTile / kDeepBatch;
 constexpr int kDeepAhead = 2;
 
+/* Sites a warp takes at a time of n tiles over `warps` warps: a power of two,
+ * halved from kDeepBatch while there are not two rounds of work - a segment
+ * with a few hundred deep tiles would otherwise take eight sites' latency. */
+__device__ __forceinline__ int deep_sites(int n, int warps) {
+    int sites = kDeepBatch;
+    while (sites > 1 && (int64_t)n * (kTile / sites) < 2 * (int64_t)warps) sites >>= 1;
+    return sites;
+}
+
+/* What the reads [r_lo, r_hi) are to the kDeepBatch sites from s0 on, lane j < kDeepBatch
+ * site s0 + j: how many cover it, their hits' sum, and how many of the first
+ * ones end before it whatever their length (they start at site - L or before).
+ * One pass over the reads' starts and lengths for all the sites: a read that
+ * covers them all is counted by ballot; the others add where they begin and
+ * take away where they end, in shared memory.  scratch: 2 (kDeepBatch + 1)
+ * words. */
+struct DeepSpan {
+    uint32_t depth, repeat;
+    int skip;
+};
+__device__ __forceinline__ DeepSpan deep_spans(const CallArgs& a, int64_t r_lo, int64_t r_hi, int64_t s0,
+                                               uint32_t* scratch) {
+    const int lane = threadIdx.x & 31;
+    uint32_t* const dep = scratch;
+    uint32_t* const rep = scratch + kDeepBatch + 1;
+    if (lane < 2 * (kDeepBatch + 1)) scratch[lane] = 0u;
+    __syncwarp();
+    uint32_t whole_n = 0, whole_rep = 0;
+    DeepSpan out = {0u, 0u, 0};
+    for (int64_t rb = r_lo; rb < r_hi; rb += 32 * kDeepAhead) {
+        int32_t st[kDeepAhead];
+        uint32_t lh[kDeepAhead];
+#pragma unroll
+        for (int u = 0; u < kDeepAhead; ++u) {
+            const int64_t r = rb + 32 * u + lane;
+            st[u] = r < r_hi ? __ldg(a.pos + r) : 0;
+            lh[u] = r < r_hi ? (uint32_t)__ldg(a.lenhit + r) : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < kDeepAhead; ++u) {
+            const bool in = rb + 32 * u + lane < r_hi;
+            const int t = (int)(st[u] - s0);
+            const int from = max(t, 0), to = min(t + (int)(lh[u] >> 16), kDeepBatch);
+            const uint32_t hit = lh[u] & 0xffffu;
+            const bool some = in && from < to, whole = some && to - from == kDeepBatch;
+            whole_n += (uint32_t)__popc(__ballot_sync(kFull, whole));
+            whole_rep += whole ? hit : 0u;
+            if (some && !whole) {
+                atomicAdd(dep + from, 1u);
+                atomicAdd(rep + from, hit);
+                atomicSub(dep + to, 1u);
+                atomicSub(rep + to, hit);
+            }
+            const int past = in ? t + a.L : kDeepBatch;   /* the first site out of reach */
+            if (__any_sync(kFull, past < kDeepBatch))
+#pragma unroll
+                for (int j = 0; j < kDeepBatch; ++j) {
+                    const int n = __popc(__ballot_sync(kFull, past <= j));
+                    if (lane == j) out.skip += n;
+                }
+        }
+    }
+    whole_rep = __reduce_add_sync(kFull, whole_rep);
+    __syncwarp();
+    out.depth = whole_n;
+    out.repeat = whole_rep;
+#pragma unroll
+    for (int j = 0; j < kDeepBatch; ++j) {
+        if (j > lane) continue;
+        out.depth += dep[j];
+        out.repeat += rep[j];
+    }
+    return out;
+}
+
+/* The pileup of one site by its warp (kernel/update_kernel.cu:260-325, as
+ * PileupAcc::take): the reads [r_lo, r_hi) 32 at a time, in order, whose
+ * depth and repeat the caller has (deep_spans).  A covering read that is not
+ * N and reaches q_min is taken while the site has fewer than 255 unique
+ * records, and a unique one (hit 1) adds a record.  Whether the cap still
+ * admits a read depends only on the unique valid reads before it, which a
+ * ballot gives, so the 32 reads of a step are decided together with the
+ * reference's result.  The scan ends once the cap is reached, or at the first
+ * step whose reads all start past the site.
+ *
+ * Its loads run ahead of the decisions (each step's base and quality load
+ * depends on the read's start): an iteration loads the starts and lengths of
+ * its kDeepAhead steps' reads in the iteration before, and their bases,
+ * qualities and strands all at its start.  The steps are then decided in
+ * order, as above. */
 __device__ __forceinline__ SitePileup deep_pileup(const CallArgs& a, int64_t r_lo, int64_t r_hi, int64_t site,
-                                                  uint32_t* recs) {
+                                                  uint32_t depth, uint32_t repeat, uint32_t* recs) {
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int L = a.L;
-    SitePileup p;
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-        p.cu[b] = 0;
-        p.qs[b] = 0;
-        p.ca[b] = 0;
-    }
-    p.depth = 0;
-    p.repeat = 0;
-    p.dep_uni = 0;
-    p.num = 0;
-    /* repeat and the quality sums per lane, added over the warp after the
-     * scan (the same sums, modulo 2^32 as before) */
-    uint32_t rep_l = 0, qs_l[4] = {0u, 0u, 0u, 0u};
+    int num = 0;   /* records so far */
+    /* Counts by base per lane, added over the warp after the scan: records in
+     * bytes (their total is at most 255), accepted reads and quality sums (at
+     * most 255 x 255) in half words.  Counting each step's by ballots takes a
+     * popc a base, which the SM issues at a quarter of the rate. */
+    uint32_t cu_l = 0, ca_l[2] = {0u, 0u}, qs_l[2] = {0u, 0u};
     int32_t nst[kDeepAhead];
     uint32_t nlh[kDeepAhead];
 #pragma unroll
@@ -63,11 +130,10 @@ __device__ __forceinline__ SitePileup deep_pileup(const CallArgs& a, int64_t r_l
         nst[u] = r < r_hi ? __ldg(a.pos + r) : 0;
         nlh[u] = r < r_hi ? (uint32_t)__ldg(a.lenhit + r) : 0u;
     }
-    for (int64_t rb = r_lo; rb < r_hi; rb += 32 * kDeepAhead) {
+    for (int64_t rb = r_lo; rb < r_hi && num < 0xFF; rb += 32 * kDeepAhead) {
         int coord[kDeepAhead];
         uint32_t lh[kDeepAhead], bq[kDeepAhead];
         bool cov[kDeepAhead], minus[kDeepAhead];
-        const bool capped_at_start = p.dep_uni >= 0xFF;
 #pragma unroll
         for (int u = 0; u < kDeepAhead; ++u) {
             const int64_t r = rb + 32 * u + lane;
@@ -77,7 +143,7 @@ __device__ __forceinline__ SitePileup deep_pileup(const CallArgs& a, int64_t r_l
             cov[u] = in && coord[u] >= 0 && coord[u] < (int)(lh[u] >> 16);
             bq[u] = 0;
             minus[u] = false;
-            if (cov[u] && !capped_at_start) {
+            if (cov[u]) {
                 bq[u] = __ldg(a.bq + r * L + coord[u]);
                 minus[u] = __ldg(a.strand + r) != '+';
             }
@@ -92,38 +158,45 @@ __device__ __forceinline__ SitePileup deep_pileup(const CallArgs& a, int64_t r_l
                 past = true;
                 break;
             }
-            const unsigned mc = __ballot_sync(kFull, cov[u]);
-            if (mc == 0) continue;
-            const uint32_t hit = lh[u] & 0xffffu;
-            p.depth += (uint32_t)__popc(mc);
-            rep_l += cov[u] ? hit : 0u;
-            if (p.dep_uni >= 0xFF) continue;
+            if (num >= 0xFF) break;
             const bool valid = cov[u] && elem_valid(bq[u]);
             const int bi = elem_base(bq[u]), q = elem_q(bq[u]);
-            const bool uni = valid && hit == 1;
-            const int uni_before = p.dep_uni + __popc(__ballot_sync(kFull, uni) & lt);
+            const bool uni = valid && (lh[u] & 0xffffu) == 1;
+            const unsigned mu = __ballot_sync(kFull, uni);
+            const int uni_before = num + __popc(mu & lt);
             const bool acc = valid && uni_before < 0xFF;
             const bool rec = acc && uni;
-            const unsigned mr = __ballot_sync(kFull, rec);
             if (rec) {
                 const uint32_t cv =
                     minus[u] ? (uint32_t)((int)(lh[u] >> 16) - 1 - coord[u]) : (uint32_t)coord[u];
-                recs[p.num + __popc(mr & lt)] = make_record_of((uint32_t)bi, q, cv, (uint32_t)minus[u]);
+                recs[uni_before] = make_record_of((uint32_t)bi, q, cv, (uint32_t)minus[u]);
             }
-            p.num += __popc(mr);
-            p.dep_uni += __popc(mr);
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                p.cu[b] += __popc(__ballot_sync(kFull, rec && bi == b));
-                qs_l[b] += (rec && bi == b) ? (uint32_t)q : 0u;
-                p.ca[b] += (uint32_t)__popc(__ballot_sync(kFull, acc && bi == b));
-            }
+            num = min(0xFF, num + __popc(mu));   /* the unique valid ones below the cap */
+            const uint32_t half = 16u * (bi & 1);
+            cu_l += rec ? 1u << (8 * bi) : 0u;
+            ca_l[0] += acc && bi < 2 ? 1u << half : 0u;
+            ca_l[1] += acc && bi >= 2 ? 1u << half : 0u;
+            qs_l[0] += rec && bi < 2 ? (uint32_t)q << half : 0u;
+            qs_l[1] += rec && bi >= 2 ? (uint32_t)q << half : 0u;
         }
         if (past) break;
     }
-    p.repeat = __reduce_add_sync(kFull, rep_l);
+    SitePileup p;
+    p.depth = depth;
+    p.repeat = repeat;
+    p.dep_uni = num;
+    p.num = num;
+    cu_l = __reduce_add_sync(kFull, cu_l);
 #pragma unroll
-    for (int b = 0; b < 4; ++b) p.qs[b] = (int)__reduce_add_sync(kFull, qs_l[b]);
+    for (int b = 0; b < 4; ++b) p.cu[b] = (int)((cu_l >> (8 * b)) & 0xffu);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t ca = __reduce_add_sync(kFull, ca_l[h]), qs = __reduce_add_sync(kFull, qs_l[h]);
+        p.ca[2 * h] = ca & 0xffffu;
+        p.ca[2 * h + 1] = ca >> 16;
+        p.qs[2 * h] = (int)(qs & 0xffffu);
+        p.qs[2 * h + 1] = (int)(qs >> 16);
+    }
     return p;
 }
 
