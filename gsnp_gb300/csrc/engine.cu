@@ -279,6 +279,9 @@ __global__ void __launch_bounds__(256) gather_reads_kernel(
         if (VEC == 4) {
             s4[g] = *reinterpret_cast<const uint32_t*>(seq + src[g] * pitch + c0);
             if (!PACKED) q4[g] = *reinterpret_cast<const uint32_t*>(qual + src[g] * pitch + c0);
+        } else if (VEC == 2) {
+            s4[g] = *reinterpret_cast<const uint16_t*>(seq + src[g] * pitch + c0);
+            if (!PACKED) q4[g] = *reinterpret_cast<const uint16_t*>(qual + src[g] * pitch + c0);
         } else if (c0 < pitch) {
             s4[g] = seq[src[g] * pitch + c0];
             if (!PACKED) q4[g] = qual[src[g] * pitch + c0];
@@ -294,10 +297,10 @@ __global__ void __launch_bounds__(256) gather_reads_kernel(
             lenhit[row] = (int32_t)(((uint32_t)(rl[g] & 0xffff) << 16) | ((uint32_t)rhit[src[g]] & 0xffffu));
             strand[row] = rstrand[src[g]];
         }
-        if (VEC == 4) {
+        if (VEC > 1) {
             uint32_t lo = 0, hi = 0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
+            for (int k = 0; k < VEC; ++k) {
                 uint32_t v = kElemInvalid;
                 if (c0 + k < rl[g]) {
                     if (PACKED) {
@@ -310,7 +313,8 @@ __global__ void __launch_bounds__(256) gather_reads_kernel(
                 if (k < 2) lo |= v << (16 * k);
                 else hi |= v << (16 * (k - 2));
             }
-            *reinterpret_cast<uint2*>(bq + row * L + c0) = make_uint2(lo, hi);
+            if (VEC == 4) *reinterpret_cast<uint2*>(bq + row * L + c0) = make_uint2(lo, hi);
+            else *reinterpret_cast<uint32_t*>(bq + row * L + c0) = lo;
         } else if (c0 < L) {
             uint32_t v = kElemInvalid;
             if (c0 < pitch && c0 < rl[g]) {
@@ -329,7 +333,7 @@ __global__ void __launch_bounds__(256) gather_reads_kernel(
 }
 
 /* gather_reads_kernel in the form the pitch and the read layout allow */
-cudaError_t launch_gather(bool vec4, bool packed, unsigned blocks, cudaStream_t stream, int64_t row_begin,
+cudaError_t launch_gather(int vec, bool packed, unsigned blocks, cudaStream_t stream, int64_t row_begin,
                           int64_t row_end, const int64_t* idx, int64_t n_raw, const int32_t* rpos, const int32_t* rlen,
                           const int32_t* rhit, const uint8_t* rstrand, const uint8_t* seq, const uint8_t* qual,
                           int pitch, int L, int rows_per_block, int32_t* pos, int32_t* lenhit, int32_t* len,
@@ -338,9 +342,12 @@ cudaError_t launch_gather(bool vec4, bool packed, unsigned blocks, cudaStream_t 
     gather_reads_kernel<V, P><<<blocks, 256, 0, stream>>>(row_begin, row_end, idx, n_raw, rpos, rlen, rhit,    \
                                                           rstrand, seq, qual, pitch, L, rows_per_block, pos,  \
                                                           lenhit, len, strand, bq, error, qmin, q_call)
-    if (vec4) {
+    if (vec == 4) {
         if (packed) GSNP_GATHER(4, true);
         else GSNP_GATHER(4, false);
+    } else if (vec == 2) {
+        if (packed) GSNP_GATHER(2, true);
+        else GSNP_GATHER(2, false);
     } else {
         if (packed) GSNP_GATHER(1, true);
         else GSNP_GATHER(1, false);
@@ -1494,13 +1501,16 @@ std::vector<Segment> plan_segments(const gsnp_context* c, const ReadView& r, int
 }
 
 /* Columns a gather thread takes (VEC of gather_reads_kernel), and the rows of
- * a block at one group. */
+ * a block at one group: as many columns as divide the rows of both arrays, so
+ * that every row's words are aligned.  The kernel is bound by its loads and
+ * stores in flight: 250 bp rows (c5, 3 Mbp) 608 us a column at a time, 245
+ * two; 50 bp rows (c0, 1 Mbp) 61 and 31. */
 struct GatherShape {
-    bool vec4;
+    int vec;
     int rows_per_block;
     GatherShape(int L, int pitch)
-        : vec4(L % 4 == 0 && pitch % 4 == 0 && L <= pitch),
-          rows_per_block(std::max(1, 256 / (vec4 ? L / 4 : L))) {}
+        : vec(L > pitch ? 1 : (L | pitch) % 4 == 0 ? 4 : (L | pitch) % 2 == 0 ? 2 : 1),
+          rows_per_block(std::max(1, 256 / (L / vec))) {}
     unsigned blocks(int64_t rows) const {
         const int64_t per_block = (int64_t)rows_per_block * kGatherRows;
         return (unsigned)((rows + per_block - 1) / per_block);
@@ -1513,7 +1523,7 @@ int regather(gsnp_context* c) {
     if (c->gather_qmin == call_qmin(c) || c->n_dep == 0) return GSNP_OK;
     const int L = c->params.read_length;
     const GatherShape gs(L, c->raw_pitch);
-    CK(launch_gather(gs.vec4, c->raw_packed, gs.blocks(c->n_dep), c->stream, 0, c->n_dep, c->d_idx, c->raw_n,
+    CK(launch_gather(gs.vec, c->raw_packed, gs.blocks(c->n_dep), c->stream, 0, c->n_dep, c->d_idx, c->raw_n,
                      c->d_raw_pos, c->d_raw_len, c->d_raw_hit, c->d_raw_strand, c->d_raw_seq, c->d_raw_qual,
                      c->raw_pitch, L, gs.rows_per_block, c->d_pos, c->d_lenhit, c->d_len, c->d_strand, c->d_bq,
                      c->d_gerror, c->packed_qmin, call_qmin(c)),
@@ -1774,7 +1784,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
                  * (the pieces of several copy streams finish in any order) */
                 for (; waited_chunk < chunk; ++waited_chunk)
                     CK(cudaStreamWaitEvent(c->gather_stream, c->ev_chunk[waited_chunk + 1], 0), "wait");
-                CK(launch_gather(gs.vec4, r->packed != nullptr, gs.blocks(g.dhi - g.dlo), c->gather_stream, g.dlo, g.dhi, c->d_idx, n,
+                CK(launch_gather(gs.vec, r->packed != nullptr, gs.blocks(g.dhi - g.dlo), c->gather_stream, g.dlo, g.dhi, c->d_idx, n,
                                  c->d_raw_pos, c->d_raw_len, c->d_raw_hit, c->d_raw_strand, c->d_raw_seq,
                                  c->d_raw_qual, r->pitch, L, gs.rows_per_block, c->d_pos, c->d_lenhit, c->d_len,
                                  c->d_strand, c->d_bq, c->d_gerror, c->params.q_min, call_qmin(c)),
@@ -3172,7 +3182,7 @@ int call_streamed(gsnp_context* c, const gsnp_reads* r, const char* chr_name, gs
             dep_index_kernel<<<(unsigned)n_chunks, kDepThreads, 0, c->stream>>>(nraw, s.raw_pos, s.raw_len,
                                                                                 c->chr_len, s.dep_off, nd, s.idx);
             CK(cudaGetLastError(), "index kernels");
-            CK(launch_gather(gs.vec4, r->packed != nullptr, gs.blocks(nd), c->stream, 0, nd, s.idx, nraw, s.raw_pos, s.raw_len,
+            CK(launch_gather(gs.vec, r->packed != nullptr, gs.blocks(nd), c->stream, 0, nd, s.idx, nraw, s.raw_pos, s.raw_len,
                              s.raw_hit, s.raw_strand, s.raw_seq, s.raw_qual, r->pitch, L, gs.rows_per_block, s.pos,
                              s.lenhit, s.len, s.strand, s.bq, c->d_gerror, c->params.q_min, call_qmin(c)),
                "gather kernel");
