@@ -2464,18 +2464,19 @@ int gsnp_tune(gsnp_context* c, int sample_windows, char* report, size_t report_c
     c->bin_limit[0] = rc == GSNP_OK ? kLimits[best_lim][0] : saved0;
     c->bin_limit[1] = rc == GSNP_OK ? kLimits[best_lim][1] : saved1;
 
-    /* 3. the persistent kernel (FP32 form): slots, carveout, read mode */
+    /* 3. the persistent kernel: slots, carveout, read mode (FP32 form) */
     float best_pers = 1e30f;
-    int best_slots = 48, best_cv = 0, best_mode = 0;
-    if (fast) {
+    int best_slots = 48, best_cv = 0, best_mode = c->stream_mode;
+    {
         c->stream_path = true;
         for (int slots : {48, 64})
             for (int cv : {0, 72, 86})
                 for (int mode : {0, 1}) {
                     if (rc != GSNP_OK) break;
+                    if (!fast && mode != 0) continue;
                     c->stream_slots = slots;
                     c->stream_carveout = cv;
-                    c->stream_mode = mode;
+                    if (fast) c->stream_mode = mode;
                     c->stream_ctas_L = -1;
                     const float ms = time_pass(c, g, 2, &rc);
                     snprintf(line, sizeof line, "persistent slots %d carveout %d mode %d: %.3f ms\n", slots, cv, mode,
@@ -2485,7 +2486,7 @@ int gsnp_tune(gsnp_context* c, int sample_windows, char* report, size_t report_c
                         best_pers = ms;
                         best_slots = slots;
                         best_cv = cv;
-                        best_mode = mode;
+                        best_mode = c->stream_mode;
                     }
                 }
         c->stream_slots = best_slots;
@@ -2493,7 +2494,7 @@ int gsnp_tune(gsnp_context* c, int sample_windows, char* report, size_t report_c
         c->stream_mode = best_mode;
         c->stream_ctas_L = -1;
     }
-    c->stream_path = fast && best_pers < best_binned;
+    c->stream_path = best_pers < best_binned;
     c->use_graphs = saved_graphs;
     if (rc != GSNP_OK) return rc;
 

@@ -193,11 +193,11 @@ int gsnp_recall_resident(gsnp_context* ctx);
 /* No counterpart in the reference (its launch configuration is fixed at
  * build time).  Set a launch option of the context; the next calling pass
  * uses it.  Names and values:
- *   persistent            FP32 form: 1 the persistent region-ordered kernel
+ *   persistent            1 the persistent region-ordered kernel of the form
  *                         with the binned kernels for the tiles it leaves,
  *                         0 the depth-binned kernels only
  *   persistent_slots      48 or 64 record slots of the persistent kernel
- *   persistent_mode       0 read loads, 1 after a bulk L2 prefetch of the
+ *   persistent_mode       (FP32) 0 read loads, 1 after a bulk L2 prefetch of the
  *                         next tile's rows, 2 rows staged in shared memory by
  *                         bulk copies
  *   persistent_carveout   preferred shared-memory carveout, percent (0: the
@@ -224,9 +224,9 @@ int gsnp_set_option(gsnp_context* ctx, const char* name, int64_t value);
  * with candidate launch settings, and keeps the fastest:
  *   - each binned kernel's shared-memory carveout (0, 58, 72, 86%), per bin;
  *   - the column-depth limits of the two shallowest bins;
- *   - for the FP32 form, the persistent kernel's record slots (48, 64),
- *     carveout (0, 72, 86%) and read mode (loads, L2 prefetch), and whether
- *     it or the binned kernels alone call the FP32 windows.
+ *   - the persistent kernel's record slots (48, 64), carveout (0, 72, 86%)
+ *     and, in the FP32 form, read mode (loads, L2 prefetch), and whether it or
+ *     the binned kernels alone call the windows.
  * The chosen settings are written to `report` as "name value" lines (the
  * gsnp_set_option names), followed by the measurements as "#"-led and plain
  * lines; when GSNP_TUNE_FILE is set the option lines are written to that file,
@@ -272,9 +272,9 @@ int gsnp_check_columns(const char* cns_path, const char* base, char* report, int
  * context's stream. */
 typedef struct gsnp_launch_info {
     int kind;          /* 0: tile classification; calling kernel of one depth bin: 1 FP64,
-                          2 FP32 fast form, 6 FP32 fast form with one warp per site (the deep
-                          bins); 3 FP64 pass over the fast form's deferred sites; 4 the
-                          persistent FP32 kernel; 5 a whole pass replayed as a CUDA graph */
+                          2 FP32 fast form, 6 FP32 fast form with a warp's lanes on one site (the
+                          deep bin); 3 FP64 pass over the fast form's deferred sites; 4 the
+                          persistent kernel of the form; 5 a whole pass replayed as a CUDA graph */
     int slots;         /* record slots per site of the bin (calling kernels) */
     int64_t tiles;     /* 32-site tiles processed (0 when the count is read on the device) */
     int64_t sites;
