@@ -187,7 +187,7 @@ RAM_DIR = "/dev/shm" if os.path.isdir("/dev/shm") and os.access("/dev/shm", os.W
 
 NCU_BYTES_PER_SITE = {
     ("c1", 2, 40): 150.6,   # call_fast_kernel<40>: 324.6 MB (dram__bytes.sum) over 2,154,656 sites
-    ("c1", 4, 48): 95.0,    # call_stream_kernel<48>: 325.2 MB read + 150.1 MB written over 5,000,000 sites
+    ("c1", 4, 48): 85.3,    # call_stream_kernel<48>: 119.9 MB read + 36.7 MB written over 1,835,008 sites
 }
 
 

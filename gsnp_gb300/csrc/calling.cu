@@ -13,8 +13,7 @@
  * site's column ([slot][site] layout, so a warp's accesses fall in 32 distinct
  * banks whatever slot each lane is at), the column is sorted in place
  * (column.cuh), the likelihood walks it in that order, and only the 32-byte
- * SiteCall leaves the SM.  (The FP32 kernel's 256-slot bin keeps its columns
- * in a global scratch slice per CTA, read through L1.)
+ * SiteCall leaves the SM.
  *
  * The pileup of a site is every deposited read that covers it, in (start, file)
  * order.  That equals the reference's window-resident pileup: its carried-over
@@ -23,14 +22,22 @@
  * walks the reads that can cover any of its 32 sites once, in that order; each
  * read's row is read with one coalesced load per lane band.
  *
- * Two calling kernels share this structure:
- *   call_tiles_kernel  FP64 sums in the reference's order (the plain form, and
- *                      windows whose likelihood another window reuses);
- *   call_fast_kernel   (calling_fast.cu) FP32 compensated sums and an FP32 posterior for
- *                      homozygous calls that the error bound proves; every
- *                      other site is deferred: its counts and sorted records
+ * Most tiles are called in the short form (lean.cuh, lean_tile.cuh), which sums
+ * only the genotypes that can decide a call; the rest in the general form of
+ * tile.cuh.  The kernels:
+ *   call_stream64_kernel, call_stream_kernel (calling_fast.cu)  persistent, one
+ *                      launch per segment, tiles in genome order: FP64 sums,
+ *                      or FP32 sums and an FP32 posterior for homozygous calls
+ *                      that the error bound proves; tiles they cannot take go
+ *                      to the binned kernels;
+ *   call_tiles_kernel  FP64 sums in the reference's order, the tiles of a depth
+ *                      bin (and windows whose likelihood another window reuses);
+ *   call_fast_kernel   (calling_fast.cu) the FP32 form of a depth bin; a site it
+ *                      cannot prove is deferred: its counts and sorted records
  *                      are appended to a small pool.  It runs no FP64
- *                      instruction.
+ *                      instruction;
+ *   call_deep64_kernel, call_deep_kernel  (calling_deep64.cu, calling_fast.cu)
+ *                      the deepest bin;
  *   deferred_sites_kernel  (deferred.cu) the deferred sites: the FP32 sums
  *                      again with the double-precision bound checks, the FP64
  *                      sums where those fail, the rank-sum test.

@@ -28,9 +28,9 @@ enum CallKind : int {
     kKindFP64 = 1,      /* FP64 likelihood, every site of the tile */
     kKindFast = 2,      /* FP32 likelihood and posterior, hard sites deferred */
     kKindDeferred = 3,  /* FP64 pass over the sites the fast kernel deferred */
-    kKindStream = 4,    /* the persistent FP32 kernel over a segment's tiles */
+    kKindStream = 4,    /* the persistent kernel of the call's form over a segment's tiles */
     kKindGraph = 5,     /* a whole pass replayed as a CUDA graph */
-    kKindDeep = 6,      /* FP32, one warp per site: the deep bins' tiles */
+    kKindDeep = 6,      /* FP32, a warp's lanes on one site's records: the deep bin's tiles */
 };
 
 /* A site the fast kernel left to the FP64 pass: its pileup counts and the
@@ -56,12 +56,12 @@ enum WindowFlags : uint8_t {
     kWinExternalLik = 4,  /* likelihood comes from another window (or zeros) */
 };
 
-/* FP32 bins of at least this many record slots are called one warp per
- * site (call_deep_kernel).  At c2 (hotspots of 300-1000x) the warp form took
- * the 256-slot bin from 26.9 to 17.9 ms, but the 96- and 128-slot bins from
- * 2.8 and 4.7 to 12.0 and 13.4 ms: below 255 records the lanes of a warp
- * sharing one scan of the tile's reads (one site each) beat a warp re-scanning
- * them per site. */
+/* Bins of at least this many record slots are called by warps whose lanes
+ * share one site's records (call_deep_kernel, calling_deep64.cu).  At c2
+ * (hotspots of 300-1000x) that form took the FP32 256-slot bin from 26.9 to
+ * 17.9 ms when it was new, but the 96- and 128-slot bins from 2.8 and 4.7 to
+ * 12.0 and 13.4 ms: below 255 records the lanes of a warp sharing one scan of
+ * the tile's reads (one site each) beat a warp scanning them per site. */
 constexpr int kDeepSlots = 256;
 
 /* the short FP32 form (lean.cuh): record groups per adjusted-quality table row
@@ -70,7 +70,7 @@ constexpr int kDeepSlots = 256;
 constexpr int kLeanG = 64;
 constexpr float kLeanGapUnit = 0x1p-5f;
 
-/* tiles a warp of the persistent FP32 kernel takes per counter increment */
+/* tiles a warp of a persistent kernel takes per counter increment */
 constexpr int kStreamChunk = 2;
 
 /* One launch of a depth bin's kernel: `count` tiles, one CTA each; or, with
@@ -88,7 +88,7 @@ struct BinLaunch {
  * each fast bin, then the same bins' hand-out counters (classify zeroes all) */
 constexpr int kBinCountInts = 4 * kNumBins;
 
-/* work queue of one launch of the persistent FP32 kernel (call_stream_kernel) */
+/* work queue of one launch of a persistent kernel (call_stream_kernel, call_stream64_kernel) */
 struct StreamQueue {
     int64_t t_begin, t_end;       /* the segment's tiles */
     unsigned long long* next;     /* tiles handed out so far (zero before the launch) */

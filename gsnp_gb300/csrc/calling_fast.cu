@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kTile, kFastCtasPerSm) call_fast_kernel(const 
 }
 
 /* ------------------------------------------------------------------------ */
-/* the deep bins of the FP32 form: one warp per site                          */
+/* the deep bin of the FP32 form: a warp's lanes on one site's records         */
 /* ------------------------------------------------------------------------ */
 
 /* Tiles with a site of more than 128 records (hotspots of hundreds of reads)
@@ -705,7 +705,7 @@ cudaError_t launch_stream(const CallArgs& a, const StreamQueue& q, int slots, in
  * default); with ctas_per_sm, its resident CTAs on one SM */
 template <int SLOTS>
 static cudaError_t fast_attr(int L, int carveout, int* ctas_per_sm) {
-    /* the deep bins run one warp per site (call_deep_kernel) */
+    /* the deep bin has its own kernel (call_deep_kernel) */
     constexpr bool deep = SLOTS >= kDeepSlots;
     const int smem = deep ? (int)kDeepSmem : (int)call_smem_bytes(SLOTS, L);
     const void* fn;
