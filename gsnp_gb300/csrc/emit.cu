@@ -288,7 +288,8 @@ cudaError_t emit_text(const EmitArgs& e, int64_t piece, cudaStream_t stream) {
     const size_t smem = 16 + (size_t)kRows * (size_t)(kRowFields + e.chr_n);
     if (smem > 47 * 1024) {   /* names near 255 bytes; the kernel's static 0.3 KB count too */
         const cudaError_t err =
-            cudaFuncSetAttribute(row_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaFuncSetAttribute(row_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 16 + kRows * (kRowFields + 255));   /* the same for every name: threads share it */
         if (err != cudaSuccess) return err;
     }
     row_write_kernel<<<(unsigned)(b1 - b0), kRows, smem, stream>>>(e, b0);
