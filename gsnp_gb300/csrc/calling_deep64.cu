@@ -7,7 +7,8 @@
  * tile over the whole chip.  Here a warp takes kBatch neighbouring sites of a
  * tile.  One after another it piles up, sorts and walks each of them, a record
  * per lane (deep.cuh), and keeps of each record the table row its walk led to,
- * 16 bits in shared memory.  Then it adds the FP64 terms in the reference's
+ * 16 bits in shared memory, and the base of its word in two bit planes (the
+ * word's, not the read's: a quality of 0 or above 64 spills into it).  Then it adds the FP64 terms in the reference's
  * order, a genotype per lane and three sites at a time - an FP64 instruction
  * costs a warp 16 cycles of the SM's pipe however many lanes have work - and
  * takes the posterior of all of them at once, a site per lane.  Heterozygous
@@ -40,6 +41,7 @@ constexpr int kDeep64Warps = 24;
  * histogram are used one after another */
 struct DeepWarp {
     uint16_t row[kBatch][kDeepCap];           /* adjusted quality * L + cycle of each record */
+    uint2 base[kBatch][kDeepCap / 32];        /* bits 0 and 1 of 32 records' bases */
     uint32_t recs[kDeepCap];
     union {
         uint8_t cnt[kDeepKeys];
@@ -51,7 +53,7 @@ struct DeepWarp {
     uint32_t span[2 * (kBatch + 1)];
     uint32_t pad[2];
     int32_t rank2[kBatch][2];                 /* twice the rank sums of the candidate's alleles */
-    uint16_t num[kBatch], base_end[kBatch][3];   /* records; the end of bases 0, 1 and 2 among them */
+    uint16_t num[kBatch];                     /* records */
 };
 static_assert(sizeof(DeepWarp) % 16 == 0, "16-byte aligned per warp");
 
@@ -103,16 +105,13 @@ __device__ __forceinline__ void deep_batch(const CallArgs& a, int64_t tile, int 
     for (int j = 0; j < n; ++j) {
         const SitePileup p = pileup(j);
         if (lane == j) mine = p;
-        if (lane == 0) {
-            sm.num[j] = (uint16_t)p.num;
-            sm.base_end[j][0] = (uint16_t)p.cu[0];
-            sm.base_end[j][1] = (uint16_t)(p.cu[0] + p.cu[1]);
-            sm.base_end[j][2] = (uint16_t)(p.cu[0] + p.cu[1] + p.cu[2]);
-        }
+        if (lane == 0) sm.num[j] = (uint16_t)p.num;
         if (external) continue;
         deep_sort(sm.recs, p.num);
-        deep_walk(a, sm.recs, sm.u.cnt, p.num, [&](int c0, bool valid, int qa, int coord, int) {
+        deep_walk(a, sm.recs, sm.u.cnt, p.num, [&](int c0, bool valid, int qa, int coord, int o) {
             if (valid) sm.row[j][c0 + lane] = (uint16_t)(qa * a.L + coord);
+            const uint2 planes = make_uint2(__ballot_sync(kFull, o & 1), __ballot_sync(kFull, o & 2));
+            if (lane == 0) sm.base[j][c0 / 32] = planes;
         });
         __syncwarp();
     }
@@ -133,17 +132,19 @@ __device__ __forceinline__ void deep_batch(const CallArgs& a, int64_t tile, int 
         } else {
             const int jj = has ? j : 0;
             const int num = has ? sm.num[jj] : 0;
-            const int b0 = sm.base_end[jj][0], b1 = sm.base_end[jj][1], b2 = sm.base_end[jj][2];
             const int most = (int)__reduce_max_sync(kFull, (unsigned)num);
             const uint16_t* rows = sm.row[jj];
             const double* col = a.lik64 + v;
             for (int i0 = 0; i0 < most; i0 += 8) {
                 double x[8];
+                const uint2 planes = sm.base[jj][i0 / 32];
+                const uint32_t p0 = planes.x >> (i0 & 31), p1 = planes.y >> (i0 & 31);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const int i = i0 + k;
                     x[k] = 0.0;
-                    if (i < num) x[k] = __ldg(col + ((int)rows[i] * 4 + (i >= b0) + (i >= b1) + (i >= b2)) * 10);
+                    if (i < num)
+                        x[k] = __ldg(col + ((int)rows[i] * 4 + (int)((p0 >> k & 1u) | (p1 >> k & 1u) << 1)) * 10);
                 }
 #pragma unroll
                 for (int k = 0; k < 8; ++k)

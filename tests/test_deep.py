@@ -70,3 +70,34 @@ def test_deep_columns_match_oracle(kind, tmp_path, oracle_bin, native_lib):
         if got != ref["cns"]:
             i, x, y = first_diff(got, ref["cns"])
             pytest.fail(f"{kind}, precision {prec}: first differing row {i}:\n gpu   : {x!r}\n oracle: {y!r}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["plain", "gap"])
+def test_deep_columns_with_spilling_qualities(kind, tmp_path, oracle_bin, native_lib):
+    """Qualities whose record lies under another base than the read's: a score
+    of 0 or above 64 spills into the record word's base, as in the reference.
+    A deep site's terms, and the likelihood a later window takes from it, go by
+    the record's base; its counts go by the read's."""
+    w = deep_workload(kind)
+    rng = np.random.default_rng(17)
+    odd = rng.random(w.qual.shape)
+    q = w.qual.astype(np.int64) - 64
+    q = np.where(odd < 0.02, 0, np.where(odd < 0.05, rng.integers(63, 67, w.qual.shape), q))
+    w.qual = np.where(w.qual > 0, 33 + q, 0).astype(np.uint8)
+    w.config = dataclasses.replace(w.config, flags=w.config.flags + ["-z", "!", "-Q", "d"])
+    paths = synth.write_inputs(w, str(tmp_path))
+    flags = flags_for(w, paths)
+    ref = oracle_outputs(oracle_bin, w, flags, str(tmp_path))
+    assert ref["rc"] == 0, ref["stderr"]
+    for prec in (api.PRECISION_FP64, api.PRECISION_FP32_FIXUP):
+        c, _, _ = api.run_workload(w, flags, precision=prec)
+        try:
+            got = c.format_cns(w.chr_name)
+            slots = [launch["slots"] for launch in c.last_launches() if launch["tiles"]]
+        finally:
+            c.close()
+        assert 256 in slots
+        if got != ref["cns"]:
+            i, x, y = first_diff(got, ref["cns"])
+            pytest.fail(f"{kind}, precision {prec}: first differing row {i}:\n gpu   : {x!r}\n oracle: {y!r}")
