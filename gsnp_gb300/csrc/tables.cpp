@@ -29,7 +29,8 @@ int q_adjust(int q, int tmp, int gdc, double pcr, double glob, const double* log
     return qa;
 }
 
-/* The gaps of the short form (lean.cuh).  gap(q_adj) is the least of
+/* The gaps of the short form (lean.cuh), whose bounds are relative and so, like
+ * the FP32 form's, want every term zero or less (all_nonpositive).  gap(q_adj) is the least of
  * min(term[o x], term[o y]) - term[xy] over the cycles, the observed bases o
  * and the pairs xy without o, in units of kLeanGapUnit rounded down; -128 ..
  * 127 units hold every table whose terms lie within 4 of each other. */
@@ -49,7 +50,7 @@ void build_lean_gaps(HostTables* t) {
                     six[o][i++][2] = col[x][y];
                 }
     t->lean_gap.assign((size_t)rows, 0);
-    t->lean_ok = (size_t)rows * L <= 65535 && rows <= 256;
+    t->lean_ok = t->all_nonpositive && (size_t)rows * L <= 65535 && rows <= 256;
     for (int q = 0; q < rows; ++q) {
         double least = 127.0 * kLeanGapUnit;
         bool nan = false;

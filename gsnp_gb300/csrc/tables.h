@@ -22,7 +22,7 @@ struct HostTables {
                                        [qa_rows][L][4][2] columns 8-9 */
     std::vector<uint8_t> qadj;      /* [tmax][gmax][65] */
     /* the short form (lean.cuh): the gap of each q_adj, in kLeanGapUnit, and
-     * whether every one fits its field; its tables are made from these and
+     * whether every one fits its field and all_nonpositive holds; its tables are made from these and
      * the ones above on the device (lean_tables.cuh) */
     std::vector<int8_t> lean_gap;   /* [qa_rows] */
     bool lean_ok = false;

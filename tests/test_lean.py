@@ -139,3 +139,42 @@ def test_recall_under_another_qmin(native_lib):
         finally:
             c.close()
     assert got[True].tobytes() == got[False].tobytes()
+
+
+def test_short_form_needs_terms_of_zero_or_less(tmp_path):
+    """A matrix entry above 1 gives a positive term, for which the FP32 bounds
+    that choose the second genotype do not hold."""
+    from gsnp_gb300 import build
+    exe = str(tmp_path / "lean_rules_check")
+    csrc = os.path.join(ROOT, "gsnp_gb300", "csrc")
+    r = subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-fno-fast-math", "-I" + csrc,
+                        "-I" + os.path.join(ROOT, "include"), "-I" + build._cuda_include(),
+                        os.path.join(ROOT, "tests", "native", "lean_rules_check.cpp"),
+                        os.path.join(csrc, "tables.cpp"), "-o", exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
+    assert r.stdout.split("\n")[:3] == ["plain lean 1", "above lean 0", "unreached lean 1"], r.stdout
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [api.PRECISION_FP64, api.PRECISION_FP32_FIXUP])
+def test_matrix_entry_above_one_takes_the_general_form(precision, native_lib):
+    """Either form then runs the binned FP64 kernels, whatever "persistent" says."""
+    w = edge_workload("plain")
+    c, reads, pm = api.run_workload(w, list(w.config.flags), precision=precision)
+    try:
+        assert 4 in [launch["kind"] for launch in c.last_launches()]
+        p = api.params_from_flags(w.config.flags, precision)
+        pm = pm.copy()
+        pm[30 << 12 | 50 << 4 | 5] = 1.2
+        c.load_tables(p, pm, c.prior_table(p), c.rank_table())
+        got = {}
+        for persistent in (1, 0):
+            c.set_option("persistent", persistent)
+            c.call(reads)
+            got[persistent] = c.fetch().tobytes()
+            assert {launch["kind"] for launch in c.last_launches() if launch["tiles"]} <= {0, 1}
+        assert got[0] == got[1]
+    finally:
+        c.close()
