@@ -136,8 +136,10 @@ __device__ __noinline__ bool deferred_posterior(const CallArgs& a, const Deferre
 
 }  // namespace
 
-/* n sites, or with d_n the count the fast kernels requested (a.dcount[0]),
- * at most the pool's capacity.  Sampled sites also get the FP64 sums for the
+/* n sites, or with d_n = a.dcount the sites the fast kernels requested.  A pool
+ * that did not hold all of them has slots nobody wrote (a site whose records
+ * found no room keeps its slot); the host reads the counts after the pass,
+ * grows the pool and runs the whole pass again, so nothing is done here.  Sampled sites also get the FP64 sums for the
  * accuracy figure, and when the fast kernel had decided them its call is
  * compared with this one. */
 __global__ void __launch_bounds__(32 * kDefWarps) deferred_sites_kernel(const __grid_constant__ CallArgs a, int64_t n,
@@ -145,7 +147,10 @@ __global__ void __launch_bounds__(32 * kDefWarps) deferred_sites_kernel(const __
     __shared__ __align__(16) DefWarp warps[kDefWarps];
     DefWarp& sm = warps[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    if (d_n) n = (int64_t)min(*d_n, (unsigned long long)a.dsite_cap);
+    if (d_n) {
+        n = (int64_t)d_n[0];
+        if (n > a.dsite_cap || (int64_t)d_n[1] > a.dpool_cap) return;
+    }
     const int64_t n_warps = (int64_t)gridDim.x * kDefWarps;
     const int64_t warp = (int64_t)blockIdx.x * kDefWarps + (threadIdx.x >> 5);
     const int batch = (int)min((int64_t)kDefBatch, max((int64_t)1, (n + n_warps - 1) / n_warps));
@@ -216,8 +221,8 @@ __global__ void __launch_bounds__(32 * kDefWarps) deferred_sites_kernel(const __
     }
 }
 
-/* The FP64 pass over n deferred sites, or with d_n over the count the fast
- * kernels requested (read on the device) with a grid of the resident CTAs. */
+/* The FP64 pass over n deferred sites, or with d_n (a.dcount) over those the
+ * fast kernels requested (read on the device) with a grid of the resident CTAs. */
 cudaError_t launch_deferred(const CallArgs& a, int64_t n, cudaStream_t stream, const unsigned long long* d_n,
                             int grid) {
     if (!d_n && n <= 0) return cudaSuccess;
