@@ -522,7 +522,7 @@ struct gsnp_context {
     size_t raw_bytes = 0;
     /* resident reads (deposited, packed) */
     int64_t n_dep = 0;
-    int64_t cap_dep = 0;
+    int64_t cap_dep = 0, cap_bq = 0;   /* reads, and elements of their rows */
     int32_t* d_pos = nullptr;
     int32_t* d_lenhit = nullptr;
     int32_t* d_len = nullptr;
@@ -1731,10 +1731,13 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
         CK(dev_alloc(&c->d_lenhit, (size_t)nd), "cudaMalloc reads");
         CK(dev_alloc(&c->d_len, (size_t)nd), "cudaMalloc reads");
         CK(dev_alloc(&c->d_strand, (size_t)nd), "cudaMalloc reads");
-        /* 64 elements of slack: the staging bulk copies of the persistent
-         * kernel round a row window up to 16 bytes past the last row */
-        CK(dev_alloc(&c->d_bq, (size_t)nd * L + 64), "cudaMalloc reads");
         c->cap_dep = nd;
+    }
+    /* 64 elements of slack: the staging bulk copies of the persistent kernel
+     * round a row window up to 16 bytes past the last row */
+    if (nd * L + 64 > c->cap_bq) {
+        CK(dev_alloc(&c->d_bq, (size_t)nd * L + 64), "cudaMalloc reads");
+        c->cap_bq = nd * L + 64;
     }
     c->n_dep = nd;
     c->n_gathered = 0;
