@@ -540,7 +540,8 @@ struct gsnp_context {
     SiteCounts* d_counts = nullptr;
     double* d_lik_keep = nullptr;
     int64_t out_sites = 0;
-    bool have_counts = false, have_lik_keep = false;
+    int64_t counts_sites = 0, lik_sites = 0;   /* sites d_counts and d_lik_keep have room for */
+    bool have_counts = false;                  /* the resident calls' windows show kept counts */
     /* scratch */
     /* The control block of the passes (Control, then one PassCtl per segment):
      * one clear before a pass and one copy to the host after it. */
@@ -1718,13 +1719,14 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
         need_counts |= (P.flags[w] & kWinKeepCounts) != 0;
         need_lik |= (P.flags[w] & kWinKeepLik) != 0;
     }
-    if (need_counts && !c->have_counts) {
+    c->have_counts = need_counts;
+    if (need_counts && c->counts_sites < c->chr_len) {
         CK(dev_alloc(&c->d_counts, (size_t)c->chr_len), "cudaMalloc counts");
-        c->have_counts = true;
+        c->counts_sites = c->chr_len;
     }
-    if (need_lik && !c->have_lik_keep) {
+    if (need_lik && c->lik_sites < c->chr_len) {
         CK(dev_alloc(&c->d_lik_keep, (size_t)c->chr_len * 10), "cudaMalloc likelihood");
-        c->have_lik_keep = true;
+        c->lik_sites = c->chr_len;
     }
     if (nd > c->cap_dep) {
         CK(dev_alloc(&c->d_pos, (size_t)nd), "cudaMalloc reads");

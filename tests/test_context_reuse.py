@@ -1,6 +1,8 @@
 """One context used for one chromosome after another, and with other tables in
 between: what it keeps on the device has to fit each call, and the calls are
 those of a context of their own."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -37,3 +39,37 @@ def test_longer_reads_after_more_reads(native_lib):
         for w in (short, long, short):
             c.call(load(c, w))
             assert c.fetch().tobytes() == own_context(w)
+
+
+def gap_workload(windows: int):
+    """The reads of a small workload in the first window and again in the last,
+    and in a window between them as reads of several hits, which leave no
+    record: that one takes another's likelihood, and the empty ones show
+    another's counts."""
+    w = edge_workload("plain")
+    n, G = w.config.genome_len, windows * 262144 + w.config.genome_len
+    at = [0, windows // 2 * 262144 + 500, G - n]
+    ref = np.frombuffer(b"ACTG", dtype=np.uint8)[np.random.default_rng(windows).integers(0, 4, G)]
+    for x in at:
+        ref[x:x + n] = w.ref
+    thrice = lambda x: np.concatenate([x, x, x])
+    return dataclasses.replace(w, ref=ref, config=dataclasses.replace(w.config, genome_len=G),
+                               pos=np.concatenate([w.pos + x for x in at]).astype(np.int32), length=thrice(w.length),
+                               hit=np.concatenate([w.hit, np.full_like(w.hit, 2), w.hit]), strand=thrice(w.strand),
+                               seq=thrice(w.seq), qual=thrice(w.qual), mismatch=thrice(w.mismatch))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [api.PRECISION_FP64, api.PRECISION_FP32_FIXUP])
+def test_longer_chromosome_with_gap_windows(precision, native_lib):
+    """Kept counts and likelihoods of a longer chromosome than those they were
+    made for."""
+    first, longer, plain = gap_workload(2), gap_workload(6), edge_workload("plain")
+    with api.Caller() as c:
+        for w in (plain, first, longer, plain, first):
+            c.call(load(c, w, precision))
+            got, text = c.fetch().tobytes(), c.format_cns("chr1")
+            with api.Caller() as own:
+                own.call(load(own, w, precision))
+                assert got == own.fetch().tobytes()
+                assert text == own.format_cns("chr1")
