@@ -652,6 +652,10 @@ struct gsnp_context {
     uint8_t* d_map = nullptr;
     size_t map_bytes = 0;
     int64_t n_gathered = 0;        /* deposited reads in the packed layout so far */
+    /* the read length the resident rows were gathered for, 0 while the rows,
+     * the window plan and d_out are not those of one finished call on the
+     * loaded reference */
+    int resident_L = 0;
     /* the alignments behind the packed layout (d_raw_*) and the q_min its
      * elements count from: recalled under another q_min, they are gathered
      * again (regather) */
@@ -1518,6 +1522,15 @@ struct GatherShape {
     }
 };
 
+/* Whether the kernels may run over the resident reads: a call of the loaded
+ * reference left them, and the tables have the rows' read length. */
+int check_resident(gsnp_context* c) {
+    if (!c || !c->have_tables || c->resident_L == 0) return fail(c, GSNP_ERR_STATE, "nothing resident");
+    if (c->n_dep > 0 && c->resident_L != c->params.read_length)
+        return fail(c, GSNP_ERR_STATE, "the resident reads are laid out for another read length");
+    return GSNP_OK;
+}
+
 /* The resident reads' elements count qualities from the q_min they were
  * gathered under; gather them again when the tables have another one. */
 int regather(gsnp_context* c) {
@@ -1589,6 +1602,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
         if (rc != GSNP_OK) return rc;
     }
     c->streamed = false;
+    c->resident_L = 0;
     if (!c->d_out || c->out_sites < c->chr_len) {
         /* the resident calls of the chromosome (a streamed call keeps none) */
         CK(dev_alloc(&c->d_out, (size_t)c->chr_len), "cudaMalloc calls");
@@ -1860,6 +1874,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
     CK(e_gather, "gather");
     const int gerr = c->gather_error;   /* fetched after the last segment's pass, which waits for its gather */
     if (gerr == 3) return fail(c, GSNP_ERR_STATE, "deposited alignment list does not match the window replay");
+    c->resident_L = L;
     if (gerr) return fail(c, GSNP_ERR_INPUT, "unknown base when encoding (only ACGT/acgt are accepted)");
     if (out && c->deferred_at_end) return patch_deferred_calls(c, out);
     return GSNP_OK;
@@ -2115,6 +2130,7 @@ int gsnp_load_reference(gsnp_context* c, const uint8_t* codes, int64_t length, c
     if (c->d_out) cudaFree(c->d_out);
     c->d_out = nullptr;
     c->out_sites = 0;
+    c->resident_L = 0;
     c->snp_lp_ready = false;
     c->called = false;
     return GSNP_OK;
@@ -2390,6 +2406,10 @@ int gsnp_tune(gsnp_context* c, int sample_windows, char* report, size_t report_c
     if (!c) return GSNP_ERR_ARG;
     if (!c->called || !c->have_tables || c->n_gathered < c->n_dep)
         return fail(c, GSNP_ERR_STATE, "tuning samples the resident reads of a finished call");
+    {
+        const int rs = check_resident(c);
+        if (rs != GSNP_OK) return rs;
+    }
     cudaSetDevice(c->device);
     {
         const int rg = regather(c);
@@ -2532,7 +2552,10 @@ int gsnp_tune(gsnp_context* c, int sample_windows, char* report, size_t report_c
 }
 
 int gsnp_recall_resident(gsnp_context* c) {
-    if (!c || !c->have_tables || c->plan.n_windows == 0) return fail(c, GSNP_ERR_STATE, "nothing resident");
+    {
+        const int rs = check_resident(c);
+        if (rs != GSNP_OK) return rs;
+    }
     cudaSetDevice(c->device);
     {
         const int rg = regather(c);
@@ -3348,14 +3371,20 @@ extern "C" int gsnp_write_columns(gsnp_context* c, const char* chr_name, const c
 extern "C" int gsnp_call_streamed(gsnp_context* c, const gsnp_reads* r, const char* chr_name, gsnp_site_call* out,
                                   const char* cns_path, const char* columns_base) {
     if (!c) return GSNP_ERR_ARG;
-    /* the chunk view stays off whatever way the call ends */
-    struct ViewOff {
+    /* Whatever way the call ends, the chunk view is off and the resident
+     * reads have their window plan back (the device's window tables and rows
+     * are still theirs), but no call stays resident. */
+    struct Resident {
         gsnp_context* c;
-        ~ViewOff() {
+        WindowPlan plan;
+        int64_t n_gathered;
+        ~Resident() {
             c->view.on = false;
-            c->called = false;   /* no call stays resident */
+            c->called = false;
+            c->plan = std::move(plan);
+            c->n_gathered = n_gathered;
         }
-    } off{c};
+    } resident{c, std::move(c->plan), c->n_gathered};
     c->columns_host_windows = 0;
     return gsnp::call_streamed(c, r, chr_name, out, cns_path, columns_base);
 }

@@ -187,7 +187,9 @@ int gsnp_call_streamed(gsnp_context* ctx, const gsnp_reads* reads, const char* c
 int gsnp_stream_footprint(gsnp_context* ctx, uint64_t* ring_bytes, uint64_t* writer_bytes);
 
 /* Re-run the calling kernels on the alignments already resident on the device
- * (no host transfer); used to time the kernels alone. */
+ * (no host transfer); used to time the kernels alone.  GSNP_ERR_STATE unless a
+ * resident call of the loaded reference left its alignments there, and when
+ * the tables have since got another read_length. */
 int gsnp_recall_resident(gsnp_context* ctx);
 
 /* No counterpart in the reference (its launch configuration is fixed at

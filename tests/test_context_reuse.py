@@ -73,3 +73,40 @@ def test_longer_chromosome_with_gap_windows(precision, native_lib):
                 own.call(load(own, w, precision))
                 assert got == own.fetch().tobytes()
                 assert text == own.format_cns("chr1")
+
+
+@pytest.mark.gpu
+def test_recall_needs_a_resident_call_of_this_reference(native_lib):
+    """Refused: before any call, after another reference, after only a streamed
+    call, under another read length.  A streamed call in between leaves the
+    resident alignments as they were."""
+    w, other, long = edge_workload("plain"), gap_workload(2), edge_workload("lengths")
+    refused = pytest.raises(RuntimeError, match=r"\(3\)")
+    with api.Caller() as c:
+        reads = load(c, w)
+        with refused:
+            c.recall_resident()
+        c.call_streamed(reads)
+        with refused:
+            c.recall_resident()
+        c.call(reads)
+        want = c.fetch().tobytes()
+        c.call_streamed(api.Caller.reads_struct(*[x[:300] for x in arrays(w)]))
+        c.recall_resident()
+        assert c.fetch().tobytes() == want
+        # longer rows in the tables than on the device
+        p = api.params_from_flags(long.config.flags, api.PRECISION_FP32_FIXUP)
+        pm = c.calibrate(p, reads)
+        c.load_tables(p, pm, c.prior_table(p), c.rank_table())
+        with refused:
+            c.recall_resident()
+        with refused:
+            c.tune(1)
+        assert c.fetch().tobytes() == want
+        reads = load(c, other)
+        with refused:
+            c.recall_resident()
+        c.call(reads)
+        want = c.fetch().tobytes()
+        c.recall_resident()
+        assert c.fetch().tobytes() == want
