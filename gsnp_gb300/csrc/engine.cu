@@ -611,7 +611,7 @@ struct gsnp_context {
     int grid_L = -1, deferred_grid = 0, classify_grid = 0, sms = 0;
     cudaGraphExec_t graph_exec = nullptr;
     cudaStream_t capture_stream = nullptr;
-    uint64_t graph_key = 0;
+    std::string graph_key;
     bool graph_failed = false;      /* a capture failed: graphs were turned off */
     SiteCall* d_empty_calls = nullptr;  /* [16] */
     uint8_t* d_empty_valid = nullptr;   /* [16] */
@@ -1281,6 +1281,21 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
 }
 
 
+/* Which passes a segment's windows need, by the host replay: their likelihood
+ * kept for another window, or taken from one. */
+struct WindowModes {
+    bool keep_lik = false, external = false;
+};
+WindowModes window_modes(const gsnp_context* c, const Segment& g) {
+    WindowModes m;
+    const int64_t w0 = g.t0 * kTile / kWin, w1 = std::min<int64_t>(c->plan.n_windows, (g.t1 * kTile + kWin - 1) / kWin);
+    for (int64_t w = w0; w < w1; ++w) {
+        m.keep_lik |= (c->plan.flags[w] & kWinKeepLik) != 0;
+        m.external |= (c->plan.flags[w] & kWinExternalLik) != 0;
+    }
+    return m;
+}
+
 /* One pass queued with its launch sizes read on the device (see the
  * device_driven field of the context): per segment the tile ranges, the
  * persistent kernel of the call's form and the classification of the tiles it
@@ -1334,13 +1349,7 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
             const int rc = before(si);
             if (rc != GSNP_OK) return rc;
         }
-        /* which passes the segment's windows need (the host replay knows) */
-        bool keep_lik = false, external = false;
-        const int64_t w0 = g.t0 * kTile / kWin, w1 = std::min<int64_t>(c->plan.n_windows, (g.t1 * kTile + kWin - 1) / kWin);
-        for (int64_t w = w0; w < w1; ++w) {
-            keep_lik |= (c->plan.flags[w] & kWinKeepLik) != 0;
-            external |= (c->plan.flags[w] & kWinExternalLik) != 0;
-        }
+        const WindowModes modes = window_modes(c, g);
         CallArgs a = make_args(c);
         a.n_reads = c->n_gathered;
         PassCtl* const pc = pass_ctl(c, si);
@@ -1395,7 +1404,7 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
             CK(launch_classify(a, 0, 0, g.t0, g.t1, pc->bins[0], c->d_bin_tiles, side), "classify kernel");
         }
         end(k, side);
-        if (!fast || keep_lik) {
+        if (!fast || modes.keep_lik) {
             const int rc = bins(kKindFP64, 0);
             if (rc != GSNP_OK) return rc;
         }
@@ -1404,7 +1413,7 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
             if (rc != GSNP_OK) return rc;
         }
         /* pass 1: the windows whose likelihood another window kept */
-        if (external) {
+        if (modes.external) {
             const int kc = begin(kKindClassify, 0, 0, side);
             if (use_stream)
                 CK(launch_classify(a, 1, 0, 0, 0, pc->bins[1], c->d_bin_tiles, side, left, &pc->n_leftover,
@@ -2296,25 +2305,24 @@ int gsnp_rank_table(double* out) {
 namespace gsnp {
 
 /* everything a captured pass depends on: its arguments (pointers, sizes,
- * parameters), the segment and the launch configuration */
-uint64_t graph_key_of(gsnp_context* c, const Segment& g) {
-    uint64_t h = 1469598103934665603ull;
-    auto mix = [&](const void* p, size_t n) {
-        const uint8_t* b = static_cast<const uint8_t*>(p);
-        for (size_t i = 0; i < n; ++i) h = (h ^ b[i]) * 1099511628211ull;
-    };
+ * parameters), the segment, the passes its windows need and the launch
+ * configuration, byte for byte */
+std::string graph_key_of(gsnp_context* c, const Segment& g) {
+    std::string key;
+    auto add = [&](const void* p, size_t n) { key.append(static_cast<const char*>(p), n); };
     const CallArgs a = make_args(c);
-    mix(&a, sizeof a);
-    mix(&g, sizeof g);
-    const int cfg[] = {c->stream_path, c->stream_slots, c->stream_mode, c->stream_carveout, c->stream_ctas, c->stream64_ctas,
-                       c->deferred_grid, c->classify_grid};
-    mix(cfg, sizeof cfg);
-    mix(c->bin_grid, sizeof c->bin_grid);
-    mix(c->bin_carveout, sizeof c->bin_carveout);
-    mix(&c->n_gathered, sizeof c->n_gathered);
+    add(&a, sizeof a);
+    add(&g, sizeof g);
+    const WindowModes m = window_modes(c, g);
+    const int cfg[] = {m.keep_lik, m.external, c->stream_path, c->stream_slots, c->stream_mode, c->stream_carveout,
+                       c->stream_ctas, c->stream64_ctas, c->deferred_grid, c->classify_grid};
+    add(cfg, sizeof cfg);
+    add(c->bin_grid, sizeof c->bin_grid);
+    add(c->bin_carveout, sizeof c->bin_carveout);
+    add(&c->n_gathered, sizeof c->n_gathered);
     const void* ptrs[] = {c->d_leftover, c->d_ctl, c->d_bin_tiles};
-    mix(ptrs, sizeof ptrs);
-    return h;
+    add(ptrs, sizeof ptrs);
+    return key;
 }
 
 /* The resident recall as a CUDA graph: the device-driven pass over the whole
@@ -2326,7 +2334,7 @@ int recall_graph(gsnp_context* c) {
         if (rc != GSNP_OK) return rc;
     }
     const std::vector<Segment> segs{whole_segment(c)};
-    const uint64_t key = graph_key_of(c, segs[0]);
+    const std::string key = graph_key_of(c, segs[0]);
     if (!c->graph_exec || key != c->graph_key) {
         if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
         c->graph_exec = nullptr;

@@ -110,3 +110,26 @@ def test_recall_needs_a_resident_call_of_this_reference(native_lib):
         want = c.fetch().tobytes()
         c.recall_resident()
         assert c.fetch().tobytes() == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [api.PRECISION_FP64, api.PRECISION_FP32_FIXUP])
+def test_recall_after_a_call_with_other_gap_windows(precision, native_lib):
+    """A recall's graph holds the passes that the call's windows need: captured
+    for alignments without gap windows, it is not replayed for as many with one."""
+    gap = gap_workload(2)
+    full = dataclasses.replace(gap, hit=np.ones_like(gap.hit))
+    reads = {w: api.Caller.reads_struct(*a) for w, a in (("gap", arrays(gap)), ("full", arrays(full)))}
+    with api.Caller() as c:
+        load(c, gap, precision)
+        for w in ("gap", "full"):
+            c.call(reads[w])
+        c.recall_resident()
+        c.call(reads["gap"])
+        p = api.params_from_flags(gap.config.flags + ["-e", "0.2"], precision)
+        c.load_tables(p, c.calibrate(p, reads["gap"]), c.prior_table(p), c.rank_table())
+        before = c.fetch().tobytes()
+        c.recall_resident()
+        got = c.fetch().tobytes()
+        c.call(reads["gap"])
+        assert got == c.fetch().tobytes() != before
