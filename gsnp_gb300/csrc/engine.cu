@@ -452,8 +452,10 @@ __global__ void __launch_bounds__(512) calib_count_smem_kernel(
 
 using namespace gsnp;
 
-/* What a calling pass counts on the device, cleared before it (gerror, which
- * the gathers set, before the call) and copied to the host after it. */
+/* What a calling pass counts on the device, cleared before it (from error on;
+ * gerror, which the gathers set, before the call) and copied to the host after
+ * it.  text_error is the cns text's (emit_prepare clears it): the passes of a
+ * streamed call run between its rows. */
 struct PassCtl {                         /* of one segment */
     unsigned long long next;             /* the persistent kernel's tiles handed out, */
     int n_leftover, pad;                 /* and left */
@@ -461,7 +463,8 @@ struct PassCtl {                         /* of one segment */
 };
 struct Control {
     int gerror;                          /* 2: a base other than ACGT/acgt, 3: index list mismatch */
-    int pad0[15];
+    int text_error;                      /* 1: a value outside the formatter's range */
+    int pad0[14];
     int error, pad1[15];
     unsigned long long stats[kNumStats];
     unsigned long long dcount[2], pad2[6];
@@ -548,6 +551,7 @@ struct gsnp_context {
     uint8_t* d_ctl = nullptr;
     int ctl_segs = 0;               /* segments it has room for */
     int* d_gerror = nullptr;        /* its parts */
+    int* d_text_error = nullptr;
     int* d_error = nullptr;
     unsigned long long* d_stats = nullptr;
     unsigned long long* d_dcount = nullptr;  /* [2] requested sites, record words */
@@ -792,6 +796,7 @@ cudaError_t ensure_ctl(gsnp_context* c, int segs) {
     if (e != cudaSuccess) return e;
     c->ctl_segs = segs;
     c->d_gerror = reinterpret_cast<int*>(c->d_ctl + offsetof(Control, gerror));
+    c->d_text_error = reinterpret_cast<int*>(c->d_ctl + offsetof(Control, text_error));
     c->d_error = reinterpret_cast<int*>(c->d_ctl + offsetof(Control, error));
     c->d_stats = reinterpret_cast<unsigned long long*>(c->d_ctl + offsetof(Control, stats));
     c->d_dcount = reinterpret_cast<unsigned long long*>(c->d_ctl + offsetof(Control, dcount));
@@ -2654,14 +2659,14 @@ int emit_prepare(gsnp_context* c, const char* chr_name, int64_t sites, int* chr_
         if (!c->ev_text[i]) CK(cudaEventCreateWithFlags(&c->ev_text[i], cudaEventDisableTiming), "cudaEventCreate");
         if (!c->ev_copied[i]) CK(cudaEventCreateWithFlags(&c->ev_copied[i], cudaEventDisableTiming), "cudaEventCreate");
     }
-    CK(cudaMemsetAsync(c->d_error, 0, sizeof(int), c->stream), "memset");
+    CK(cudaMemsetAsync(c->d_text_error, 0, sizeof(int), c->stream), "memset");
     return GSNP_OK;
 }
 
 /* a cns value outside the formatter's range in any row since emit_prepare */
 int emit_finish(gsnp_context* c) {
     int err = 0;
-    CK(cudaMemcpyAsync(&err, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "error flag");
+    CK(cudaMemcpyAsync(&err, c->d_text_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "error flag");
     CK(cudaStreamSynchronize(c->stream), "cns text");
     if (err) return fail(c, GSNP_ERR_STATE, "a cns value is outside the text formatter's range");
     return GSNP_OK;
@@ -2730,7 +2735,7 @@ int emit_sites(gsnp_context* c, int chr_n, int64_t s_begin, int64_t s_end, const
     e.chr_n = chr_n;
     e.site0 = s_begin;
     e.n = std::max<int64_t>(0, s_end - s_begin);
-    e.error = c->d_error;
+    e.error = c->d_text_error;
     const int64_t pieces = emit_pieces(e.n);
     std::vector<uint64_t> at((size_t)pieces + 1);
     CK(emit_lengths(e, c->d_emit, c->stream), "cns text lengths");

@@ -49,3 +49,29 @@ def test_text_at_block_and_piece_edges(sites, tmp_path, oracle_bin, native_lib):
             c.format_cns("n" * 256)
     finally:
         c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("streamed", [False, True])
+def test_value_outside_the_formatter_is_an_error(streamed, tmp_path, native_lib):
+    """A rank-sum value that the exact formatter cannot print, in the first of
+    two chunks only, ends the text with an error however it is written."""
+    import dataclasses
+    from test_lean import edge_workload
+    w = edge_workload("plain")
+    ref = np.concatenate([w.ref, np.full(262144, ord("A"), dtype=np.uint8)])
+    w = dataclasses.replace(w, ref=ref, config=dataclasses.replace(w.config, genome_len=ref.size))
+    c, reads, pm = api.run_workload(w, list(w.config.flags))
+    try:
+        assert len(c.format_cns("chr1")) > 0
+        p = api.params_from_flags(w.config.flags)
+        c.load_tables(p, pm, c.prior_table(p), np.full(64 * 64 * 2048, 1e-30))
+        with pytest.raises(RuntimeError, match=r"\(3\).*formatter"):
+            if streamed:
+                c.set_option("stream_windows", 1)
+                c.call_streamed(reads, "chr1", None, str(tmp_path / "cns"))
+            else:
+                c.call(reads)
+                c.format_cns("chr1")
+    finally:
+        c.close()
