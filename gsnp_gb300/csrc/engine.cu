@@ -2502,7 +2502,7 @@ int gsnp_tune(gsnp_context* c, int sample_windows, char* report, size_t report_c
     c->bin_limit[0] = rc == GSNP_OK ? kLimits[best_lim][0] : saved0;
     c->bin_limit[1] = rc == GSNP_OK ? kLimits[best_lim][1] : saved1;
 
-    /* 3. the persistent kernel: slots, carveout, read mode (FP32 form) */
+    /* 3. the form's persistent kernel: slots, carveout, and in the FP32 form read mode */
     float best_pers = 1e30f;
     int best_slots = 48, best_cv = 0, best_mode = c->stream_mode;
     {
@@ -2548,7 +2548,7 @@ int gsnp_tune(gsnp_context* c, int sample_windows, char* report, size_t report_c
     snprintf(line, sizeof line, "bin_limit_32 %d\nbin_limit_40 %d\n", c->bin_limit[0], c->bin_limit[1]);
     opts += line;
     snprintf(line, sizeof line, "sample: windows %lld-%lld (%lld tiles); best binned %.3f ms, best persistent %.3f ms\n",
-             (long long)w0, (long long)w1, (long long)(g.t1 - g.t0), best_binned, fast ? best_pers : 0.f);
+             (long long)w0, (long long)w1, (long long)(g.t1 - g.t0), best_binned, best_pers);
     rep = opts + "# " + line + rep;
     if (const char* path = getenv("GSNP_TUNE_FILE")) {
         if (FILE* f = fopen(path, "w")) {
