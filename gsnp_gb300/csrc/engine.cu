@@ -3055,6 +3055,11 @@ int call_streamed(gsnp_context* c, const gsnp_reads* r, const char* chr_name, gs
         const int rc = ensure_call_streams(c);
         if (rc != GSNP_OK) return rc;
     }
+    /* what a streamed call holds is bounded by its chunks: the buffers of the
+     * calibration before it (some 200 MB) are given back */
+    if (c->d_calib) cudaFree(c->d_calib);
+    c->d_calib = nullptr;
+    c->calib_bytes = 0;
     const int L = c->params.read_length;
     c->called = false;
     c->streamed = false;

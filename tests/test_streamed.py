@@ -83,3 +83,26 @@ def test_streamed_fp64_form_and_no_resident_calls(tmp_path, native_lib):
         assert c.fetch(0, w.genome_len).tobytes() == want[0].tobytes()
     finally:
         c.close()
+
+
+@pytest.mark.gpu
+def test_calibration_buffers_are_given_back(native_lib):
+    """A calibration before a streamed call leaves nothing on the device beside
+    what the streamed call holds by itself; it runs again afterwards."""
+    import torch
+    w = synth.make_workload("c1", scale=0.02)
+    flags = [f for f in w.cli_flags() if f != "-C"]
+    with api.Caller() as c:
+        arrs = [np.ascontiguousarray(x) for x in (w.pos, w.length, w.hit, w.strand, w.seq, w.qual)]
+        reads = api.Caller.reads_struct(*arrs)
+        p = api.params_from_flags(flags, api.PRECISION_FP32_FIXUP)
+        c.load_reference(api.site_codes(w.ref))
+        pm = c.calibrate(p, reads)
+        c.load_tables(p, pm, c.prior_table(p), c.rank_table())
+        c.call_streamed(reads)
+        c.call_streamed(reads)
+        free0, _ = torch.cuda.mem_get_info()
+        assert (c.calibrate(p, reads) == pm).all()
+        assert torch.cuda.mem_get_info()[0] < free0
+        c.call_streamed(reads)
+        assert torch.cuda.mem_get_info()[0] == free0
