@@ -363,6 +363,7 @@ __device__ __forceinline__ bool lean_tile64(const CallArgs& a, int64_t tile, int
     const int32_t snp_row = tile_snp_row(a, tile, (ori & 8) != 0);
     LeanSums z;
     lean_walk<kTile, true>(a, recs, pile.num, ori & 3, &z);
+    lean_zeros(pile, &z);
     if (active) {
         if (wflags & kWinKeepCounts) store_counts(a, site, lean_counts(pile, z));
         CallWords call;

@@ -192,6 +192,7 @@ __device__ __forceinline__ bool lean_tile(const CallArgs& a, int64_t tile, int64
     const int32_t snp_row = tile_snp_row(a, tile, (ori & 8) != 0);
     LeanSums z;
     lean_walk<kTile>(a, recs, pile.num, ori & 3, &z);
+    lean_zeros(pile, &z);
     const SitePileup p = lean_counts(pile, z);
     finish_fast_site(a, site, active, ori, wflags, snp_row, p, recs,
                      [&](CallWords* call) { return lean_posterior(a, snp_row, ori, pile, z, call); },

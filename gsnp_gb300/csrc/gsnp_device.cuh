@@ -47,19 +47,24 @@ GSNP_HDI int rec_occ(uint32_t w) { return (int)(w & 0xffu); }
 
 /* A base and its quality in a packed read row (16 bits).  q = quality char -
  * q_min:
- *   1 <= q <= 63   base << 6 | (64 - q): bits 24:17 of its record word
- *   other q >= 0   kElemWide | base << 8 | q
+ *   1 <= q <= 64   base << 6 | (64 - q): bits 24:17 of its record word
+ *   q = 0          kElemZero | base << 8 | those bits of its record, in which 64
+ *                  spills into the base (make_record_of)
+ *   q > 64         kElemWide | base << 8 | q
  *   q < 0          kElemInvalid: never part of a pileup (nor are columns past
  *                  the read's end) */
-constexpr uint32_t kElemInvalid = 0x8000u, kElemWide = 0x4000u;
+constexpr uint32_t kElemInvalid = 0x8000u, kElemWide = 0x4000u, kElemZero = 0x2000u;
 
 GSNP_HDI uint32_t make_elem(uint32_t base, int q) {
     if (q < 0) return kElemInvalid;
-    return q >= 1 && q <= 63 ? base << 6 | (uint32_t)(kMaxQ - q) : kElemWide | base << 8 | (uint32_t)q;
+    if (q == 0) return kElemZero | base << 8 | (base | 1u) << 6;
+    return q <= 64 ? base << 6 | (uint32_t)(kMaxQ - q) : kElemWide | base << 8 | (uint32_t)q;
 }
 GSNP_HDI bool elem_valid(uint32_t e) { return (e & kElemInvalid) == 0; }
-GSNP_HDI int elem_base(uint32_t e) { return (int)((e & kElemWide ? e >> 8 : e >> 6) & 3u); }
-GSNP_HDI int elem_q(uint32_t e) { return e & kElemWide ? (int)(e & 0xffu) : kMaxQ - (int)(e & 63u); }
+GSNP_HDI int elem_base(uint32_t e) { return (int)((e & (kElemWide | kElemZero) ? e >> 8 : e >> 6) & 3u); }
+GSNP_HDI int elem_q(uint32_t e) {
+    return e & kElemWide ? (int)(e & 0xffu) : e & kElemZero ? 0 : kMaxQ - (int)(e & 63u);
+}
 
 /* genotype code (a1 << 2 | a2) of table column t, a1 <= a2 in ACTG order */
 GSNP_HDI int genotype_of(int t) {

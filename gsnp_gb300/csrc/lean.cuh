@@ -114,12 +114,19 @@ GSNP_HDI void lean_sort(uint32_t* recs, int num, int most) {
     }
 }
 
-/* what the pileup leaves besides the records */
+/* What the pileup leaves besides the records.  extra4 has 16 bits a base: in the
+ * low nine count_all beyond the records, in the high seven the records of
+ * quality 0 among the base's reads, which lie under base | 1 (lean_zeros). */
 struct LeanPile {
     uint32_t depth, repeat;
-    uint64_t extra4;   /* count_all beyond the records, 4 x 16 bits */
+    uint64_t extra4;
     int num;
 };
+constexpr int kLeanExtraBits = 9;
+constexpr uint64_t kLeanExtraOf4 = 0x01ff01ff01ff01ffull;
+GSNP_HDI uint32_t lean_extra(uint64_t extra4, int base) {
+    return (uint32_t)(extra4 >> (16 * base)) & ((1u << kLeanExtraBits) - 1u);
+}
 
 /* what the walk leaves of a site's column */
 struct LeanSums {
@@ -130,6 +137,18 @@ struct LeanSums {
     uint64_t qs4;      /* quality sums per base, 4 x 16 bits */
     int maj, n_minor;
 };
+
+/* The walk counts a record by the base of its word.  One of quality 0 lies
+ * under base | 1 with a score of 64: its count goes back to its read's base, its
+ * score away. */
+GSNP_HDI void lean_zeros(const LeanPile& pile, LeanSums* z) {
+    const uint64_t zeros = pile.extra4 & ~kLeanExtraOf4;
+    if (zeros == 0) return;
+    auto of = [&](int base) { return (uint32_t)(zeros >> (16 * base + kLeanExtraBits)) & 0x7fu; };
+    const uint32_t a = of(0), t = of(2);
+    z->cu4 += a - (a << 8) + (t << 16) - (t << 24);
+    z->qs4 -= (uint64_t)(kMaxQ * (a + of(1))) << 16 | (uint64_t)(kMaxQ * (t + of(3))) << 48;
+}
 
 /* The counts of one base group's walk: the earlier records of a record's key,
  * and 64 * (distinct keys so far - 1) */
@@ -278,7 +297,7 @@ __device__ __forceinline__ void lean_sums64(const CallArgs& a, const uint32_t* r
     const double* t1 = a.lik64 + col_of(lo, hi);
     const double2* rows = reinterpret_cast<const double2*>(a.lean2d) + (size_t)((maj * 4 + win) * a.qa_rows) * a.L;
     double s0 = 0.0, s1 = 0.0;
-    const int m = (int)((z.cu4 >> (8 * maj)) & 0xffu);
+    const int m = num - z.n_minor;
     /* the other bases' records before maj's, maj's, and those after: one loop
      * each, so that the lanes of a warp run maj's together */
     auto other = [&](int i) {
@@ -321,7 +340,7 @@ __device__ __forceinline__ SitePileup lean_counts(const LeanPile& pile, const Le
     for (int b = 0; b < 4; ++b) {
         p.cu[b] = (int)((z.cu4 >> (8 * b)) & 0xffu);
         p.qs[b] = (int)((z.qs4 >> (16 * b)) & 0xffffu);
-        p.ca[b] = (uint32_t)p.cu[b] + (uint32_t)((pile.extra4 >> (16 * b)) & 0xffffu);
+        p.ca[b] = (uint32_t)p.cu[b] + lean_extra(pile.extra4, b);
     }
     p.depth = pile.depth;
     p.repeat = pile.repeat;
@@ -344,8 +363,8 @@ __device__ __forceinline__ void lean_fill(CallWords* out, const LeanPile& pile, 
     const uint32_t cu1 = b1 ? (z.cu4 >> (8 * tb.base1)) & 0xffu : 0u, cu2 = b2 ? (z.cu4 >> (8 * tb.base2)) & 0xffu : 0u;
     const uint32_t qs1 = b1 ? (uint32_t)(z.qs4 >> (16 * tb.base1)) & 0xffffu : 0u;
     const uint32_t qs2 = b2 ? (uint32_t)(z.qs4 >> (16 * tb.base2)) & 0xffffu : 0u;
-    const uint32_t ca1 = cu1 + (b1 ? (uint32_t)(pile.extra4 >> (16 * tb.base1)) & 0xffffu : 0u);
-    const uint32_t ca2 = cu2 + (b2 ? (uint32_t)(pile.extra4 >> (16 * tb.base2)) & 0xffffu : 0u);
+    const uint32_t ca1 = cu1 + (b1 ? lean_extra(pile.extra4, tb.base1) : 0u);
+    const uint32_t ca2 = cu2 + (b2 ? lean_extra(pile.extra4, tb.base2) : 0u);
     out->a.x = (uint32_t)type1 | (uint32_t)tb.base1 << 8 | (uint32_t)tb.base2 << 16 | (uint32_t)q << 24;
     out->a.y = (qs1 ? avg(qs1, cu1) : 0u) | (qs2 ? avg(qs2, cu2) : 0u) << 8;
     out->a.z = cu1 | ca1 << 16;

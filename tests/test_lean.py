@@ -178,3 +178,31 @@ def test_matrix_entry_above_one_takes_the_general_form(precision, native_lib):
         assert got[0] == got[1]
     finally:
         c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [api.PRECISION_FP64, api.PRECISION_FP32_FIXUP])
+def test_qualities_zero_and_64_stay_in_the_short_form(precision, tmp_path, oracle_bin, native_lib):
+    """Records of quality 0, whose word lies under another base, and of 64: no
+    tile is left to the binned kernels, and the text is the oracle's."""
+    w = edge_workload("plain")
+    odd = np.random.default_rng(3).random(w.qual.shape)
+    q = w.qual.astype(np.int64) - 64
+    q = np.where(odd < 0.05, 0, np.where(odd < 0.08, 64, q))
+    w.qual = np.where(w.qual > 0, 33 + q, 0).astype(np.uint8)
+    w.config = dataclasses.replace(w.config, flags=w.config.flags + ["-z", "!", "-Q", "d"])
+    paths = synth.write_inputs(w, str(tmp_path))
+    flags = flags_for(w, paths)
+    ref = oracle_outputs(oracle_bin, w, flags, str(tmp_path))
+    assert ref["rc"] == 0, ref["stderr"]
+    c, _, _ = api.run_workload(w, flags, precision=precision)
+    try:
+        got = c.format_cns(w.chr_name)
+        left = sum(launch["tiles"] for launch in c.last_launches() if launch["kind"] in (1, 2, 6))
+        assert c.stats()["sample_mismatches"] == 0
+    finally:
+        c.close()
+    if got != ref["cns"]:
+        i, x, y = first_diff(got, ref["cns"])
+        pytest.fail(f"precision {precision}: first differing row {i}:\n gpu   : {x!r}\n oracle: {y!r}")
+    assert left == 0
