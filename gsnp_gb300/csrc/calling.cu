@@ -158,7 +158,8 @@ cudaError_t launch_empty_calls(const CallArgs& a, SiteCall* calls, uint8_t* vali
 
 /* Per tile: the deepest site's record need (reads starting in [site - L + 1,
  * site], capped at 255) picks the depth bin; the window's mode picks the FP64
- * kernel (bins 0 .. kNumBins-1) or the fast one (the next kNumBins).  Each
+ * kernel (bins 0 .. kNumBins-1) or the fast one (the next kNumBins).  The bins
+ * start at min_bin, for a listed tile marked kTileGeneral at general_bin.  Each
  * warp's read range is stored for the calling kernels.  A CTA classifies
  * kClassifyTiles tiles and adds its bin counts to the global ones with one
  * atomic per bin. */
@@ -167,7 +168,8 @@ constexpr int kClassifyTiles = kClassifyThreads / kTile;
 constexpr int kClassifyStage = 256;   /* read starts staged in shared memory per tile */
 static_assert(kClassifyThreads % kTile == 0, "a classify CTA holds whole tiles");
 
-__global__ void __launch_bounds__(kClassifyThreads) classify_tiles_kernel(CallArgs a, int pass, int min_bin, int64_t t_begin,
+__global__ void __launch_bounds__(kClassifyThreads) classify_tiles_kernel(CallArgs a, int pass, int min_bin,
+                                                                          int general_bin, int64_t t_begin,
                                                                           int64_t t_end, int* bin_count,
                                                                           int32_t* bin_tiles,
                                                                           const int32_t* __restrict__ list,
@@ -186,7 +188,8 @@ __global__ void __launch_bounds__(kClassifyThreads) classify_tiles_kernel(CallAr
     const int64_t idx = gbase + lt;
     if (threadIdx.x < 2 * kNumBins) sbin_count[threadIdx.x] = 0;
     bool part = idx < end;
-    const int64_t tile = list ? (part ? (int64_t)list[idx] : 0) : idx;
+    const int32_t entry = list ? (part ? list[idx] : 0) : (int32_t)idx;
+    const int64_t tile = entry & ~kTileGeneral;
     const int64_t s0 = tile * kTile;
     uint8_t wflags = 0;
     if (part) {
@@ -220,7 +223,7 @@ __global__ void __launch_bounds__(kClassifyThreads) classify_tiles_kernel(CallAr
     if (part && tt == 0) {
         const int m = smax[lt];
         const bool fast = a.precision == 1 && !(wflags & (kWinKeepLik | kWinExternalLik));
-        int bin = min_bin;
+        int bin = entry & kTileGeneral ? general_bin : min_bin;
         while (bin < kNumBins - 1 && m > a.bin_limit[bin]) ++bin;
         my_bin = bin + (fast ? kNumBins : 0);
         my_rank = atomicAdd(&sbin_count[my_bin], 1);
@@ -231,7 +234,7 @@ __global__ void __launch_bounds__(kClassifyThreads) classify_tiles_kernel(CallAr
         sbin_base[threadIdx.x] = cnt ? atomicAdd(&bin_count[threadIdx.x], cnt) : 0;
     }
     __syncthreads();
-    if (my_bin >= 0) bin_tiles[(int64_t)my_bin * a.bin_stride + sbin_base[my_bin] + my_rank] = (int32_t)tile;
+    if (my_bin >= 0) bin_tiles[(int64_t)my_bin * a.bin_stride + sbin_base[my_bin] + my_rank] = entry;
     __syncthreads();
     }
 }
@@ -342,7 +345,7 @@ static __device__ __noinline__ void lean_general64(const CallArgs& a, int64_t si
 }
 
 /* A tile in the short form (lean.cuh) with FP64 sums; every lane of the warp
- * calls it.  False (for the warp, nothing written) when lean_pileup leaves it.
+ * calls it.  Nothing is written when lean_pileup leaves it.
  *
  * The FP64 pipe bounds the FP64 form (an FP64 instruction of a warp takes 16
  * cycles of the SM's pipe): the short form adds two terms a record instead of
@@ -351,14 +354,15 @@ static __device__ __noinline__ void lean_general64(const CallArgs& a, int64_t si
  * the general form, 1.73 with four FP64 sums (73% of the FP64 pipe), 1.35 with
  * two (44%). */
 template <int SLOTS>
-__device__ __forceinline__ bool lean_tile64(const CallArgs& a, int64_t tile, int64_t r_lo, int64_t r_hi, uint8_t wflags,
+__device__ __forceinline__ LeanTook lean_tile64(const CallArgs& a, int64_t tile, int64_t r_lo, int64_t r_hi, uint8_t wflags,
                                             uint32_t* recs_all, uint32_t* scratch) {
     const int t = threadIdx.x & 31;
     const int64_t s0 = tile * kTile, site = s0 + t;
     const bool active = site < a.chr_len;
     uint32_t* recs = recs_all + t;
     LeanPile pile;
-    if (!lean_columns<SLOTS>(a, s0, r_lo, r_hi, recs_all, scratch, &pile)) return false;
+    const LeanTook took = lean_columns<SLOTS>(a, s0, r_lo, r_hi, recs_all, scratch, &pile);
+    if (took != kLeanTook) return took;
     const uint8_t ori = active ? __ldg(a.ori + site) : 0;
     const int32_t snp_row = tile_snp_row(a, tile, (ori & 8) != 0);
     LeanSums z;
@@ -386,21 +390,22 @@ __device__ __forceinline__ bool lean_tile64(const CallArgs& a, int64_t tile, int
             lean_general64(a, site, ori, snp_row, pile, z.cu4, z.qs4, recs);
         }
     }
-    return true;
+    return kLeanTook;
 }
 
 /* One tile of the FP64 kernel; every lane of the warp calls it. */
 template <int SLOTS>
-__device__ __forceinline__ void fp64_tile(const CallArgs& a, int64_t tile, uint32_t* recs_all, uint32_t* seen_all) {
+__device__ __forceinline__ void fp64_tile(const CallArgs& a, int32_t entry, uint32_t* recs_all, uint32_t* seen_all) {
     const int t = threadIdx.x;
-    const int64_t s0 = tile * kTile;
+    const int64_t tile = entry & ~kTileGeneral, s0 = tile * kTile;
     const int win = (int)(s0 / kWin);
     const uint8_t wflags = a.win_flags[win];
     const int64_t r_lo = a.warp_rng[tile * 2];
     const int64_t r_hi = a.warp_rng[tile * 2 + 1];
     if constexpr (SLOTS <= kLeanG) {
-        if (a.lean_q && !(wflags & (kWinKeepLik | kWinExternalLik)) &&
-            lean_tile64<lean_slots(SLOTS)>(a, tile, r_lo, r_hi, wflags, recs_all, recs_all + lean_slots(SLOTS) * kTile))
+        if (a.lean_q && !(entry & kTileGeneral) && !(wflags & (kWinKeepLik | kWinExternalLik)) &&
+            lean_tile64<lean_slots(SLOTS)>(a, tile, r_lo, r_hi, wflags, recs_all,
+                                           recs_all + lean_slots(SLOTS) * kTile) == kLeanTook)
             return;
         __syncwarp();
     }
@@ -480,11 +485,13 @@ __global__ void __launch_bounds__(32 * kStreamWarps, kStream64Warps / kStreamWar
         for (int64_t i = (int64_t)first; i < end; ++i) {
             const int64_t tile = q.t_begin + i;
             const uint8_t wflags = a.win_flags[(int)(tile * kTile / kWin)];
-            const bool called =
-                !(wflags & (kWinKeepLik | kWinExternalLik)) &&
-                lean_tile64<SLOTS>(a, tile, a.tile_rng[tile * 2], a.tile_rng[tile * 2 + 1], wflags, recs_all,
-                                   recs_all + SLOTS * kTile);
-            if (!called && t == 0) q.leftover[atomicAdd(q.n_leftover, 1)] = (int32_t)tile;
+            const LeanTook took =
+                wflags & (kWinKeepLik | kWinExternalLik)
+                    ? kLeanNever
+                    : lean_tile64<SLOTS>(a, tile, a.tile_rng[tile * 2], a.tile_rng[tile * 2 + 1], wflags, recs_all,
+                                         recs_all + SLOTS * kTile);
+            if (took != kLeanTook && t == 0)
+                q.leftover[atomicAdd(q.n_leftover, 1)] = (int32_t)tile | (took == kLeanNever ? kTileGeneral : 0);
             __syncwarp();
         }
     }
@@ -507,16 +514,16 @@ static size_t fp64_smem_bytes(int slots, int L) {
 
 /* Classify tiles [t_begin, t_end) (with a list, list[t_begin, t_end); with
  * d_count, list[0, *d_count) read on the device, by a fixed grid of `grid`
- * CTAs) into the depth bins from min_bin on; d_bin_count's kBinCountInts ints
- * are zero. */
-cudaError_t launch_classify(const CallArgs& a, int pass, int min_bin, int64_t t_begin, int64_t t_end, int* d_bin_count,
-                            int32_t* d_bin_tiles, cudaStream_t stream, const int32_t* list, const int* d_count,
-                            int grid) {
+ * CTAs) into the depth bins from min_bin, marked tiles from general_bin on;
+ * d_bin_count's kBinCountInts ints are zero. */
+cudaError_t launch_classify(const CallArgs& a, int pass, int min_bin, int general_bin, int64_t t_begin, int64_t t_end,
+                            int* d_bin_count, int32_t* d_bin_tiles, cudaStream_t stream, const int32_t* list,
+                            const int* d_count, int grid) {
     const unsigned blocks =
         d_count ? (unsigned)grid : (unsigned)((t_end - t_begin + kClassifyTiles - 1) / kClassifyTiles);
     if (blocks == 0) return cudaSuccess;
-    classify_tiles_kernel<<<blocks, kClassifyThreads, 0, stream>>>(a, pass, min_bin, t_begin, t_end, d_bin_count,
-                                                                   d_bin_tiles, list, d_count);
+    classify_tiles_kernel<<<blocks, kClassifyThreads, 0, stream>>>(a, pass, min_bin, general_bin, t_begin, t_end,
+                                                                   d_bin_count, d_bin_tiles, list, d_count);
     return cudaGetLastError();
 }
 

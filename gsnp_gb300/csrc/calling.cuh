@@ -70,6 +70,21 @@ constexpr int kDeepSlots = 256;
 constexpr int kLeanG = 64;
 constexpr float kLeanGapUnit = 0x1p-5f;
 
+/* A tile number in a persistent kernel's leftover list and in a bin's list, with
+ * this bit where the short form cannot take the tile however many slots it gets
+ * (and in windows that need the general FP64 sums): the bin's kernel does not
+ * try it again. */
+constexpr int32_t kTileGeneral = 1 << 30;
+/* After a persistent kernel in the short form, the shallowest bins: 64 slots for
+ * the tiles that were too deep for its own, which try the short form again; 48,
+ * whose kernel keeps more warps an SM, for the marked ones of a segment with more
+ * tiles than the 64-slot kernel holds at once (in a smaller one the slots make no
+ * difference and a launch costs 3 us of a call's 330).  8 Mbp recalled with every
+ * tile marked (20 reads of one start and strand): 3.90 ms in the 64-slot bin
+ * after a second try, 3.15 in the 48-slot one, 3.02 and 2.90 with bins of 40 and
+ * of 32 slots, each a launch more in every segment. */
+constexpr int kGeneralBin = 2, kDeeperBin = 3;
+
 /* tiles a warp of a persistent kernel takes per counter increment */
 constexpr int kStreamChunk = 2;
 
@@ -92,7 +107,7 @@ constexpr int kBinCountInts = 4 * kNumBins;
 struct StreamQueue {
     int64_t t_begin, t_end;       /* the segment's tiles */
     unsigned long long* next;     /* tiles handed out so far (zero before the launch) */
-    int32_t* leftover;            /* tiles left to the binned kernels */
+    int32_t* leftover;            /* tiles left to the binned kernels (kTileGeneral) */
     int* n_leftover;              /* their count (zero before the launch) */
 };
 

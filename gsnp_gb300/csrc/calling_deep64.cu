@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(32 * kDeep64Warps, 1)
     const unsigned per = (unsigned)(kTile / sites), items = (unsigned)n * per;
     unsigned item = blockIdx.x * kDeep64Warps + w;
     while (item < items) {
-        deep_batch(a, tiles[item / per], (int)(item % per) * sites, sites, sm);
+        deep_batch(a, tiles[item / per] & ~kTileGeneral, (int)(item % per) * sites, sites, sm);
         unsigned nx = item + step;
         if (next) {
             if (lane == 0) nx = (unsigned)atomicAdd(next, 1) + step;

@@ -175,10 +175,10 @@ __device__ __forceinline__ void fast_site(const CallArgs& a, int64_t site, bool 
                      [](uint32_t w) { return (w & ~0xffu) | 1u; });
 }
 
-/* A tile in the short form; every lane of the warp calls it.  False (for the
- * warp, nothing written) when lean_pileup leaves it. */
+/* A tile in the short form; every lane of the warp calls it.  Nothing is written
+ * when lean_pileup leaves it. */
 template <int SLOTS>
-__device__ __forceinline__ bool lean_tile(const CallArgs& a, int64_t tile, int64_t r_lo, int64_t r_hi, uint8_t wflags,
+__device__ __forceinline__ LeanTook lean_tile(const CallArgs& a, int64_t tile, int64_t r_lo, int64_t r_hi, uint8_t wflags,
                                           uint32_t* recs_all, uint32_t* scratch) {
     const int t = threadIdx.x & 31;
     const int64_t s0 = tile * kTile, site = s0 + t;
@@ -187,7 +187,8 @@ __device__ __forceinline__ bool lean_tile(const CallArgs& a, int64_t tile, int64
     LeanPile pile;
     /* a read's columns end before the chromosome does, so sites past the end
      * have no covering read */
-    if (!lean_columns<SLOTS>(a, s0, r_lo, r_hi, recs_all, scratch, &pile)) return false;
+    const LeanTook took = lean_columns<SLOTS>(a, s0, r_lo, r_hi, recs_all, scratch, &pile);
+    if (took != kLeanTook) return took;
     const uint8_t ori = active ? __ldg(a.ori + site) : 0;
     const int32_t snp_row = tile_snp_row(a, tile, (ori & 8) != 0);
     LeanSums z;
@@ -197,7 +198,7 @@ __device__ __forceinline__ bool lean_tile(const CallArgs& a, int64_t tile, int64
     finish_fast_site(a, site, active, ori, wflags, snp_row, p, recs,
                      [&](CallWords* call) { return lean_posterior(a, snp_row, ori, pile, z, call); },
                      [](uint32_t w) { return lean_to_record(w); });
-    return true;
+    return kLeanTook;
 }
 
 /* Sites whose call is not proven in FP32 (and every 4096th site, sampled for
@@ -206,16 +207,17 @@ __device__ __forceinline__ bool lean_tile(const CallArgs& a, int64_t tile, int64
  * keep counting past the capacities so that the host can size the pool and
  * run the pass again. */
 template <int SLOTS>
-__device__ __forceinline__ void fast_tile(const CallArgs& a, int64_t tile, uint32_t* recs_all, uint32_t* seen_all) {
+__device__ __forceinline__ void fast_tile(const CallArgs& a, int32_t entry, uint32_t* recs_all, uint32_t* seen_all) {
     const int t = threadIdx.x;
-    const int64_t s0 = tile * kTile;
+    const int64_t tile = entry & ~kTileGeneral, s0 = tile * kTile;
     const int win = (int)(s0 / kWin);
     const uint8_t wflags = a.win_flags[win];
     const int64_t r_lo = a.warp_rng[tile * 2];
     const int64_t r_hi = a.warp_rng[tile * 2 + 1];
     if constexpr (SLOTS <= kLeanG) {
-        if (a.lean_q && lean_tile<lean_slots(SLOTS)>(a, tile, r_lo, r_hi, wflags, recs_all,
-                                                     recs_all + lean_slots(SLOTS) * kTile))
+        if (a.lean_q && !(entry & kTileGeneral) &&
+            lean_tile<lean_slots(SLOTS)>(a, tile, r_lo, r_hi, wflags, recs_all, recs_all + lean_slots(SLOTS) * kTile) ==
+                kLeanTook)
             return;
         __syncwarp();
     }
@@ -410,7 +412,7 @@ __global__ void __launch_bounds__(kDeepThreads, 1) call_deep_kernel(const __grid
     const unsigned per = (unsigned)(kTile / sites), items = (unsigned)n * per;
     unsigned item = blockIdx.x * (kDeepThreads / 32) + w;
     while (item < items) {
-        deep_batch(a, tiles[item / per], (int)(item % per) * sites, sites, sm);
+        deep_batch(a, tiles[item / per] & ~kTileGeneral, (int)(item % per) * sites, sites, sm);
         unsigned nx = item + step;
         if (next) {
             if (lane == 0) nx = (unsigned)atomicAdd(next, 1) + step;
@@ -588,13 +590,13 @@ __global__ void __launch_bounds__(32 * kStreamWarps, kFastCtasPerSm / kStreamWar
         const int64_t nxt = next_tile();
         prefetch_l2(nxt);
         if (wflags & (kWinKeepLik | kWinExternalLik)) {
-            if (t == 0) q.leftover[atomicAdd(q.n_leftover, 1)] = (int32_t)tile;
+            if (t == 0) q.leftover[atomicAdd(q.n_leftover, 1)] = (int32_t)tile | kTileGeneral;
             tile = nxt;
             staged_n = stage(tile);
             continue;
         }
         int staged_next = -1;
-        bool called;
+        LeanTook took;
         if (STAGED) {
             const int64_t site = s0 + t;
             const bool active = site < a.chr_len;
@@ -618,17 +620,18 @@ __global__ void __launch_bounds__(32 * kStreamWarps, kFastCtasPerSm / kStreamWar
             /* the staging buffers are free: stage the next tile now, so that its
              * copies run while this one is sorted, walked and summed */
             staged_next = stage(nxt);
-            called = !__any_sync(kFull, overflow);
-            if (called) {
+            took = __any_sync(kFull, overflow) ? kLeanDeep : kLeanTook;
+            if (took == kLeanTook) {
                 /* one sort network for every tile: specialised networks per
                  * tile depth made the kernel's code larger and it ran slower */
                 if (active) sort_column<SLOTS>(recs, p.num);
                 fast_site<SLOTS>(a, site, active, ori, wflags, snp_row, p, recs, seen);
             }
         } else {
-            called = lean_tile<SLOTS>(a, tile, a.tile_rng[tile * 2], a.tile_rng[tile * 2 + 1], wflags, recs_all, seen_all);
+            took = lean_tile<SLOTS>(a, tile, a.tile_rng[tile * 2], a.tile_rng[tile * 2 + 1], wflags, recs_all, seen_all);
         }
-        if (!called && t == 0) q.leftover[atomicAdd(q.n_leftover, 1)] = (int32_t)tile;
+        if (took != kLeanTook && t == 0)
+            q.leftover[atomicAdd(q.n_leftover, 1)] = (int32_t)tile | (took == kLeanNever ? kTileGeneral : 0);
         tile = nxt;
         staged_n = staged_next;
         __syncwarp();

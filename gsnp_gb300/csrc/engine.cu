@@ -42,8 +42,8 @@
 
 namespace gsnp {
 
-cudaError_t launch_classify(const CallArgs& a, int pass, int min_bin, int64_t t_begin, int64_t t_end, int* d_bin_count,
-                            int32_t* d_bin_tiles, cudaStream_t stream, const int32_t* list = nullptr,
+cudaError_t launch_classify(const CallArgs& a, int pass, int min_bin, int general_bin, int64_t t_begin, int64_t t_end,
+                            int* d_bin_count, int32_t* d_bin_tiles, cudaStream_t stream, const int32_t* list = nullptr,
                             const int* d_count = nullptr, int grid = 0);
 cudaError_t launch_stream(const CallArgs& a, const StreamQueue& q, int slots, int mode, int ctas, int carveout,
                           cudaStream_t stream);
@@ -1214,10 +1214,10 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
             const int k = begin(kKindClassify, 0, use_stream ? n_left : g.t1 - g.t0);
             CK(cudaMemsetAsync(d_bins, 0, sizeof(int) * kBinCountInts, c->stream), "memset");
             if (use_stream)
-                CK(launch_classify(a, pass, 0, 0, n_left, d_bins, c->d_bin_tiles, c->stream, c->d_leftover),
+                CK(launch_classify(a, pass, 0, 0, 0, n_left, d_bins, c->d_bin_tiles, c->stream, c->d_leftover),
                    "classify kernel");
             else
-                CK(launch_classify(a, pass, 0, g.t0, g.t1, d_bins, c->d_bin_tiles, c->stream), "classify kernel");
+                CK(launch_classify(a, pass, 0, 0, g.t0, g.t1, d_bins, c->d_bin_tiles, c->stream), "classify kernel");
             end(k);
             CK(fetch_pass(), "classify");
             memcpy(c->h_bin_count, host_pc.bins[0], sizeof(c->h_bin_count));
@@ -1340,10 +1340,9 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
     cudaStream_t const side = several && use_stream ? c->bin_stream[0] : c->stream;
     /* after the persistent kernel in the general form (staged reads), the fast
      * bins get only tiles deeper than its record slots; the short form leaves
-     * shallow tiles too, so few that the 64-slot bin takes them all */
-    int min_bin = 0;
-    if (use_stream && !(fast && c->stream_mode == 2))
-        while (kSlotsOf(min_bin) < kLeanG) ++min_bin;
+     * shallow tiles too (kGeneralBin) */
+    const bool short_form = use_stream && !(fast && c->stream_mode == 2);
+    const int min_bin = short_form ? kDeeperBin : 0;
     /* With several segments the deferred sites of all of them go to one pool
      * and one deferred pass runs after the last segment, whose calls then are
      * put into the host copy (patch_deferred_calls). */
@@ -1355,6 +1354,8 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
             if (rc != GSNP_OK) return rc;
         }
         const WindowModes modes = window_modes(c, g);
+        const bool small = g.t1 - g.t0 <= c->bin_grid[fast ? 1 : 0][kDeeperBin];
+        const int first_bin = short_form && !small ? kGeneralBin : min_bin;
         CallArgs a = make_args(c);
         a.n_reads = c->n_gathered;
         PassCtl* const pc = pass_ctl(c, si);
@@ -1370,7 +1371,7 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
                 for (int i = 1; i < gsnp_context::kBinStreams; ++i)
                     CK(cudaStreamWaitEvent(c->bin_stream[i], c->ev_join[0], 0), "wait");
             }
-            for (int b = pass == 0 ? min_bin : 0; b < kNumBins; ++b) {
+            for (int b = pass == 0 ? first_bin : 0; b < kNumBins; ++b) {
                 if (kind == kKindFast && use_stream && min_bin == 0 && kSlotsOf(b) <= c->stream_slots) continue;
                 int* const cnt = pc->bins[pass] + ki * kNumBins + b;
                 const BinLaunch bl{0, cnt, c->bin_grid[ki][b], c->bin_carveout[ki][b], cnt + 2 * kNumBins};
@@ -1402,11 +1403,11 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
                 CK(cudaStreamWaitEvent(side, c->ev_fork, 0), "wait");
             }
             k = begin(kKindClassify, 0, 0, side);
-            CK(launch_classify(a, 0, min_bin, 0, 0, pc->bins[0], c->d_bin_tiles, side, left, &pc->n_leftover,
+            CK(launch_classify(a, 0, min_bin, first_bin, 0, 0, pc->bins[0], c->d_bin_tiles, side, left, &pc->n_leftover,
                                c->classify_grid),
                "classify kernel");
         } else {
-            CK(launch_classify(a, 0, 0, g.t0, g.t1, pc->bins[0], c->d_bin_tiles, side), "classify kernel");
+            CK(launch_classify(a, 0, 0, 0, g.t0, g.t1, pc->bins[0], c->d_bin_tiles, side), "classify kernel");
         }
         end(k, side);
         if (!fast || modes.keep_lik) {
@@ -1421,11 +1422,11 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
         if (modes.external) {
             const int kc = begin(kKindClassify, 0, 0, side);
             if (use_stream)
-                CK(launch_classify(a, 1, 0, 0, 0, pc->bins[1], c->d_bin_tiles, side, left, &pc->n_leftover,
+                CK(launch_classify(a, 1, 0, 0, 0, 0, pc->bins[1], c->d_bin_tiles, side, left, &pc->n_leftover,
                                    c->classify_grid),
                    "classify kernel");
             else
-                CK(launch_classify(a, 1, 0, g.t0, g.t1, pc->bins[1], c->d_bin_tiles, side), "classify kernel");
+                CK(launch_classify(a, 1, 0, 0, g.t0, g.t1, pc->bins[1], c->d_bin_tiles, side), "classify kernel");
             end(kc, side);
             const int rc = bins(kKindFP64, 1);
             if (rc != GSNP_OK) return rc;

@@ -34,10 +34,14 @@ __host__ __device__ constexpr size_t lean_smem_bytes(int slots, int L) {
 }
 constexpr int kLeanGroups = 15;   /* most groups, and most reads of one (a 4-bit count each) */
 
-/* The pileup of a warp's tile (as warp_pileup) in the short form: false, for
+/* Whether the short form took a tile: else a site deeper than its slots, or
+ * something that no number of slots mends. */
+enum LeanTook : int { kLeanTook = 0, kLeanDeep = 1, kLeanNever = 2 };
+
+/* The pileup of a warp's tile (as warp_pileup) in the short form: not taken, for
  * the whole warp, when the tile needs the general one - a site deeper than
- * SLOTS records, more reads than the lists hold, a quality above 64, or more
- * repeated keys than the walk's counts hold.
+ * SLOTS records, more reads than the lists hold (both kLeanDeep), a quality above
+ * 64, or more repeated keys than the walk's counts hold (kLeanNever).
  *
  * What bounds it is the number of instructions per read, since every lane
  * looks at every read of the tile.  What depends on the read only is worked
@@ -55,7 +59,7 @@ constexpr int kLeanGroups = 15;   /* most groups, and most reads of one (a 4-bit
  * one base in 100 of quality 0, recalled: FP32 6.04 ms (3.68 without the short
  * form) -> 2.34, FP64 8.58 (7.01) -> 3.45. */
 template <int SLOTS>
-__device__ __forceinline__ bool lean_pileup(const CallArgs& a, int64_t s0, int64_t r_lo, int64_t r_hi,
+__device__ __forceinline__ LeanTook lean_pileup(const CallArgs& a, int64_t s0, int64_t r_lo, int64_t r_hi,
                                             uint32_t* recs_all, LeanRead* reads, LeanPile* out) {
     constexpr int kReads = lean_reads(SLOTS);
     const int lane = threadIdx.x & 31;
@@ -63,7 +67,7 @@ __device__ __forceinline__ bool lean_pileup(const CallArgs& a, int64_t s0, int64
     const int L = a.L;
     uint32_t* const recs = recs_all + lane;
     uint32_t* const table = recs_all;
-    if (r_hi - r_lo > kReads - 8) return false;
+    if (r_hi - r_lo > kReads - 8) return kLeanDeep;
     const int n = (int)(r_hi - r_lo);
     for (int i = lane; i < lean_table_words(L); i += 32) table[i] = 0u;
     __syncwarp();
@@ -124,7 +128,7 @@ __device__ __forceinline__ bool lean_pileup(const CallArgs& a, int64_t s0, int64
         }
         __syncwarp();
     }
-    if (__any_sync(kFull, bad) || groups > kLeanGroups) return false;
+    if (__any_sync(kFull, bad) || groups > kLeanGroups) return kLeanNever;
     /* each read's group; both lists are padded to whole steps of four */
     if (lane < 4) {
         reads[fwd + lane].len = 0;
@@ -177,26 +181,28 @@ __device__ __forceinline__ bool lean_pileup(const CallArgs& a, int64_t s0, int64
             }
         }
     }
-    if (__any_sync(kFull, num > SLOTS || (seen_bits & kElemWide))) return false;
+    if (__any_sync(kFull, num > SLOTS || (seen_bits & kElemWide)))
+        return __any_sync(kFull, (seen_bits & kElemWide) != 0) ? kLeanNever : kLeanDeep;
     out->depth = depth;
     out->repeat = depth + extra_hits;
     out->extra4 = extra4;
     out->num = num;
-    return true;
+    return kLeanTook;
 }
 
-/* The sorted columns of a tile: lean_pileup, padded and sorted.  False, for
- * the warp, when lean_pileup leaves the tile. */
+/* The sorted columns of a tile: lean_pileup, padded and sorted, when that takes
+ * it. */
 template <int SLOTS>
-__device__ __forceinline__ bool lean_columns(const CallArgs& a, int64_t s0, int64_t r_lo, int64_t r_hi,
+__device__ __forceinline__ LeanTook lean_columns(const CallArgs& a, int64_t s0, int64_t r_lo, int64_t r_hi,
                                              uint32_t* recs_all, uint32_t* scratch, LeanPile* pile) {
     static_assert(SLOTS <= kLeanG && SLOTS % 16 == 0, "a walk counts at most kLeanG distinct keys; chunks of 16");
-    if (!lean_pileup<SLOTS>(a, s0, r_lo, r_hi, recs_all, reinterpret_cast<LeanRead*>(scratch), pile)) return false;
+    const LeanTook took = lean_pileup<SLOTS>(a, s0, r_lo, r_hi, recs_all, reinterpret_cast<LeanRead*>(scratch), pile);
+    if (took != kLeanTook) return took;
     uint32_t* recs = recs_all + (threadIdx.x & 31);
     const int most = __reduce_max_sync(kFull, pile->num);
     for (int i = pile->num; i < ((most + 15) & ~15); ++i) recs[i * kTile] = kLeanPad;
     lean_sort<kTile>(recs, pile->num, most);
-    return true;
+    return kLeanTook;
 }
 
 }  // namespace gsnp

@@ -209,6 +209,7 @@ constexpr int kStreamWarps = 4;
 
 /* record-slot capacity of each depth bin */
 constexpr int kSlots[kNumBins] = {32, 40, 48, 64, 96, 128, 256};
+static_assert(kSlots[kDeeperBin] == kLeanG && kSlots[kGeneralBin] == 48, "the bins after a persistent kernel");
 
 /* 32-bit words of shared memory a bin's kernel keeps its pcr counts in */
 __host__ __device__ constexpr int pcr_smem_words(int slots, int L, bool fast) {

@@ -206,3 +206,40 @@ def test_qualities_zero_and_64_stay_in_the_short_form(precision, tmp_path, oracl
         i, x, y = first_diff(got, ref["cns"])
         pytest.fail(f"precision {precision}: first differing row {i}:\n gpu   : {x!r}\n oracle: {y!r}")
     assert left == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sites,slots", [(30013, 64), (300013, 48)])
+def test_tiles_it_can_never_take_go_to_one_shallow_bin(sites, slots, tmp_path, oracle_bin, native_lib):
+    """Twenty reads of one start and strand everywhere: no tile of the short form
+    but too deep for none of its slots.  A segment of more tiles than the 64-slot
+    kernel holds at once gives them to the 48-slot one."""
+    w = edge_workload("plain")
+    rng = np.random.default_rng(9)
+    L, code = 100, rng.integers(0, 4, sites)
+    acgt = np.frombuffer(b"ACTG", dtype=np.uint8)
+    pos = np.repeat(np.arange(0, sites - L - 1, L), 20)
+    R = pos.size
+    base = code[pos[:, None] + np.arange(L)]
+    seq = acgt[np.where(rng.random((R, L)) < 0.01, rng.integers(0, 4, (R, L)), base)]
+    w = dataclasses.replace(w, ref=acgt[code], config=dataclasses.replace(w.config, genome_len=sites),
+                            pos=pos.astype(np.int32), length=np.full(R, L, dtype=np.int32),
+                            hit=np.ones(R, dtype=np.int32),
+                            strand=np.where(pos // L % 2 == 0, ord("+"), ord("-")).astype(np.uint8), seq=seq,
+                            qual=(64 + rng.integers(2, 41, (R, L))).astype(np.uint8),
+                            mismatch=np.zeros(R, dtype=np.int32))
+    paths = synth.write_inputs(w, str(tmp_path))
+    flags = flags_for(w, paths)
+    ref = oracle_outputs(oracle_bin, w, flags, str(tmp_path))
+    assert ref["rc"] == 0, ref["stderr"]
+    for prec in (api.PRECISION_FP64, api.PRECISION_FP32_FIXUP):
+        c, _, _ = api.run_workload(w, flags, precision=prec)
+        try:
+            got = c.format_cns(w.chr_name)
+            bins = {launch["slots"] for launch in c.last_launches() if launch["kind"] in (1, 2, 6) and launch["tiles"]}
+        finally:
+            c.close()
+        if got != ref["cns"]:
+            i, x, y = first_diff(got, ref["cns"])
+            pytest.fail(f"{sites}, precision {prec}: first differing row {i}:\n gpu   : {x!r}\n oracle: {y!r}")
+        assert bins == {slots}
