@@ -792,7 +792,8 @@ cudaError_t ensure_ctl(gsnp_context* c, int segs) {
     c->d_ctl = nullptr;
     c->ctl_segs = 0;
     cudaError_t e = cudaMalloc((void**)&c->d_ctl, ctl_bytes(segs));
-    if (e == cudaSuccess) e = cudaMemset(c->d_ctl, 0, ctl_bytes(segs));
+    /* on the call's stream: the default stream does not wait for it, nor it for that */
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_ctl, 0, ctl_bytes(segs), c->stream);
     if (e != cudaSuccess) return e;
     c->ctl_segs = segs;
     c->d_gerror = reinterpret_cast<int*>(c->d_ctl + offsetof(Control, gerror));

@@ -133,3 +133,18 @@ def test_recall_after_a_call_with_other_gap_windows(precision, native_lib):
         got = c.fetch().tobytes()
         c.call(reads["gap"])
         assert got == c.fetch().tobytes() != before
+
+
+@pytest.mark.gpu
+def test_more_segments_than_any_call_before(native_lib, monkeypatch):
+    """The control block grows in the middle of a call, between its uploads and
+    its passes."""
+    small, w = edge_workload("plain"), gap_workload(30)
+    with api.Caller() as c:
+        c.call(load(c, small))
+        reads = load(c, w)
+        monkeypatch.setenv("GSNP_SEGMENTS", "25")
+        out = np.zeros(w.config.genome_len, dtype=api.SITE_DTYPE)
+        c.call_into(reads, out.ctypes.data)
+        monkeypatch.setenv("GSNP_SEGMENTS", "1")
+        assert out.tobytes() == own_context(w)
