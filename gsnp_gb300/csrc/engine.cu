@@ -2062,9 +2062,14 @@ int gsnp_load_tables(gsnp_context* c, const gsnp_params* p, const double* p_matr
     if (!c || !p || !p_matrix || !p_prior || !p_rank) return fail(c, GSNP_ERR_ARG, "null argument");
     if (p->read_length <= 0 || p->read_length > 255) return fail(c, GSNP_ERR_ARG, "read_length must be 1..255");
     cudaSetDevice(c->device);
-    c->params = *p;
+    /* the tables of before stay as they are when these cannot be made, and are
+     * gone when these cannot be put on the device */
+    HostTables made;
     std::string err;
-    if (build_tables(*p, p_matrix, p_prior, &c->tables, &err) != 0) return fail(c, GSNP_ERR_ARG, err);
+    if (build_tables(*p, p_matrix, p_prior, &made, &err) != 0) return fail(c, GSNP_ERR_ARG, err);
+    c->have_tables = false;
+    c->params = *p;
+    c->tables = std::move(made);
     const HostTables& t = c->tables;
     /* one device buffer and one copy for all of them: an allocation and a
      * pageable copy each took longer than building the tables */
@@ -2095,7 +2100,6 @@ int gsnp_load_tables(gsnp_context* c, const gsnp_params* p, const double* p_matr
     for (const Part& q : parts)
         if (q.src) memcpy(blob.data() + q.at, q.src, q.bytes);
     if (total > c->tables_bytes) {
-        c->have_tables = false;
         c->tables_bytes = 0;
         CK(dev_alloc(&c->d_tables, total), "cudaMalloc tables");
         c->tables_bytes = total;

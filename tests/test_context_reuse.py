@@ -148,3 +148,23 @@ def test_more_segments_than_any_call_before(native_lib, monkeypatch):
         c.call_into(reads, out.ctypes.data)
         monkeypatch.setenv("GSNP_SEGMENTS", "1")
         assert out.tobytes() == own_context(w)
+
+
+@pytest.mark.gpu
+def test_tables_that_cannot_be_made_change_nothing(native_lib):
+    """A dependency coefficient above 1 is refused; the context goes on with the
+    parameters and tables it has."""
+    w, long = edge_workload("plain"), edge_workload("lengths")
+    with api.Caller() as c:
+        reads = load(c, w)
+        c.call(reads)
+        want = c.fetch().tobytes()
+        p = api.params_from_flags(long.config.flags, api.PRECISION_FP64)
+        pm = c.calibrate(p, reads)
+        p.pcr_dependency = 0.1
+        with pytest.raises(RuntimeError, match=r"\(2\).*dependency"):
+            c.load_tables(p, pm, c.prior_table(p), c.rank_table())
+        c.recall_resident()
+        assert c.fetch().tobytes() == want
+        c.call(reads)
+        assert c.fetch().tobytes() == want
