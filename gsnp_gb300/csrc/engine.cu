@@ -2121,11 +2121,6 @@ int gsnp_load_reference(gsnp_context* c, const uint8_t* codes, int64_t length, c
                         int64_t n_snp) {
     if (!c || !codes || length <= 0 || (n_snp > 0 && !snp)) return fail(c, GSNP_ERR_ARG, "bad reference");
     if (length > 0x7fffffffLL) return fail(c, GSNP_ERR_CAPACITY, "chromosome longer than 2^31-1");
-    cudaSetDevice(c->device);
-    c->chr_len = length;
-    c->h_codes.assign(codes, codes + length);
-    CK(dev_alloc(&c->d_codes, (size_t)length), "cudaMalloc codes");
-    CK(cudaMemcpy(c->d_codes, codes, (size_t)length, cudaMemcpyHostToDevice), "upload codes");
     static_assert(sizeof(gsnp_snp) == sizeof(DbSnpEntry), "dbSNP row layout");
     /* the rows are the flagged sites in position order: the kernels find a
      * site's row from the rows before its tile */
@@ -2141,18 +2136,32 @@ int gsnp_load_reference(gsnp_context* c, const uint8_t* codes, int64_t length, c
         tile_snp[(size_t)(pos / kTile) + 1] += 1;
     }
     for (int64_t t = 0; t < n_tiles; ++t) tile_snp[(size_t)t + 1] += tile_snp[(size_t)t];
-    CK(dev_alloc(&c->d_tile_snp, (size_t)n_tiles + 1), "cudaMalloc tiles");
-    CK(cudaMemcpy(c->d_tile_snp, tile_snp.data(), ((size_t)n_tiles + 1) * 4, cudaMemcpyHostToDevice), "upload");
-    c->n_snp = n_snp;
-    CK(dev_alloc(&c->d_snp, (size_t)std::max<int64_t>(n_snp, 1)), "cudaMalloc dbsnp");
-    if (n_snp > 0) CK(cudaMemcpy(c->d_snp, snp, sizeof(gsnp_snp) * n_snp, cudaMemcpyHostToDevice), "upload dbsnp");
+    /* nothing of the context has changed so far; from here on the reference
+     * before is gone, and this one is loaded once all of it is there */
+    cudaSetDevice(c->device);
+    c->called = false;
+    c->resident_L = 0;
+    c->snp_lp_ready = false;
+    c->chr_len = 0;
+    if (c->d_codes) cudaFree(c->d_codes);
+    c->d_codes = nullptr;
     /* the resident calls are allocated by the first resident call */
     if (c->d_out) cudaFree(c->d_out);
     c->d_out = nullptr;
     c->out_sites = 0;
-    c->resident_L = 0;
-    c->snp_lp_ready = false;
-    c->called = false;
+    c->h_codes.assign(codes, codes + length);
+    CK(dev_alloc(&c->d_tile_snp, (size_t)n_tiles + 1), "cudaMalloc tiles");
+    CK(cudaMemcpy(c->d_tile_snp, tile_snp.data(), ((size_t)n_tiles + 1) * 4, cudaMemcpyHostToDevice), "upload");
+    CK(dev_alloc(&c->d_snp, (size_t)std::max<int64_t>(n_snp, 1)), "cudaMalloc dbsnp");
+    if (n_snp > 0) CK(cudaMemcpy(c->d_snp, snp, sizeof(gsnp_snp) * n_snp, cudaMemcpyHostToDevice), "upload dbsnp");
+    uint8_t* d_codes = nullptr;
+    CK(cudaMalloc((void**)&d_codes, (size_t)length), "cudaMalloc codes");
+    const cudaError_t e = cudaMemcpy(d_codes, codes, (size_t)length, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) cudaFree(d_codes);
+    CK(e, "upload codes");
+    c->d_codes = d_codes;
+    c->chr_len = length;
+    c->n_snp = n_snp;
     return GSNP_OK;
 }
 

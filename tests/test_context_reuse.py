@@ -168,3 +168,27 @@ def test_tables_that_cannot_be_made_change_nothing(native_lib):
         assert c.fetch().tobytes() == want
         c.call(reads)
         assert c.fetch().tobytes() == want
+
+
+@pytest.mark.gpu
+def test_reference_that_is_refused_changes_nothing(native_lib):
+    """dbSNP rows that do not match the site codes, of a longer chromosome: the
+    context keeps the reference and the calls it has."""
+    w, longer = edge_workload("plain"), gap_workload(2)
+    with api.Caller() as c:
+        reads = load(c, w)
+        c.call(reads)
+        want, text = c.fetch().tobytes(), c.format_cns("chr1")
+        codes = api.site_codes(longer.ref, np.array([7, 100000]))
+        length = c.length
+        rows = np.zeros(2, dtype=api.SNP_DTYPE)
+        for pos in ((7,), (100000, 7), (7, 100001)):
+            rows["pos"][:len(pos)] = pos
+            with pytest.raises(RuntimeError, match=r"\(2\).*dbSNP"):
+                c.load_reference(codes, rows[:len(pos)])
+            c.length = length
+            assert c.fetch().tobytes() == want and c.format_cns("chr1") == text
+        c.recall_resident()
+        assert c.fetch().tobytes() == want
+        c.call(reads)
+        assert c.fetch().tobytes() == want
