@@ -736,6 +736,7 @@ int fail(gsnp_context* c, int code, const std::string& msg) {
 }
 
 int cuda_fail(gsnp_context* c, cudaError_t e, const char* what) {
+    (void)cudaGetLastError();   /* reported here: not for the next launch check to find */
     return fail(c, GSNP_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
@@ -745,6 +746,9 @@ int cuda_fail(gsnp_context* c, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail(c, e_, what); \
     } while (0)
 
+/* a new buffer in the place of *p; a capacity kept beside it is set to nothing
+ * before and to the new one after, so that a failure leaves no size to a buffer
+ * that is gone */
 template <class T>
 cudaError_t dev_alloc(T** p, size_t count) {
     if (*p) cudaFree(*p);
@@ -752,23 +756,6 @@ cudaError_t dev_alloc(T** p, size_t count) {
     if (count == 0) count = 1;
     return cudaMalloc((void**)p, count * sizeof(T));
 }
-
-/* device buffers of one call, freed when it returns, on every path */
-struct CallTemps {
-    std::vector<void*> ptrs;
-    CallTemps() = default;
-    CallTemps(const CallTemps&) = delete;
-    CallTemps& operator=(const CallTemps&) = delete;
-    ~CallTemps() {
-        for (void* q : ptrs) cudaFree(q);
-    }
-    template <class T>
-    cudaError_t alloc(T** q, size_t bytes) {
-        const cudaError_t e = cudaMalloc((void**)q, bytes);
-        if (e == cudaSuccess) ptrs.push_back(*q);
-        return e;
-    }
-};
 
 /* host threads for the per-alignment pass of the window replay:
  * GSNP_HOST_THREADS, else every hardware thread (at most 64) */
@@ -958,6 +945,17 @@ struct Segment {
     int64_t next_pos;    /* start of deposited read dhi, kNoRead when there is none */
 };
 
+/* the deferred pool (its capacities 0 while it has no memory) */
+cudaError_t alloc_deferred(gsnp_context* c, int64_t sites, int64_t words) {
+    c->dsite_cap = c->dpool_cap = 0;
+    cudaError_t e = dev_alloc(&c->d_dsites, (size_t)sites);
+    if (e == cudaSuccess) e = dev_alloc(&c->d_dpool, (size_t)words);
+    if (e != cudaSuccess) return e;
+    c->dsite_cap = sites;
+    c->dpool_cap = words;
+    return cudaSuccess;
+}
+
 /* The calling pass, segment by segment.  before(s) runs first for each
  * segment (the call gathers the reads there: those of segments 0 .. s must be
  * on the device), after(s) once its calls are queued. */
@@ -974,7 +972,7 @@ int prepare_calling(gsnp_context* c, size_t segs) {
     if (!c->snp_lp_ready) {
         CK(dev_alloc(&c->d_snp_lp, (size_t)std::max<int64_t>(c->n_snp, 1) * 16), "cudaMalloc dbSNP priors");
         CK(dev_alloc(&c->d_snp_lp32, (size_t)std::max<int64_t>(c->n_snp, 1) * 12), "cudaMalloc dbSNP priors");
-        if (!c->d_empty_calls) {
+        if (!c->d_empty_valid) {
             CK(dev_alloc(&c->d_empty_calls, 16), "cudaMalloc");
             CK(dev_alloc(&c->d_empty_valid, 16), "cudaMalloc");
         }
@@ -984,6 +982,7 @@ int prepare_calling(gsnp_context* c, size_t segs) {
         c->snp_lp_ready = true;
     }
     if (n_tiles > c->tiles_cap) {
+        c->tiles_cap = 0;
         CK(dev_alloc(&c->d_bin_tiles, (size_t)n_tiles * 2 * kNumBins), "cudaMalloc bins");
         CK(dev_alloc(&c->d_warp_rng, (size_t)n_tiles * 2), "cudaMalloc ranges");
         CK(dev_alloc(&c->d_tile_rng, (size_t)n_tiles * 2), "cudaMalloc ranges");
@@ -1002,10 +1001,8 @@ int prepare_calling(gsnp_context* c, size_t segs) {
     }
     if (c->dsite_cap == 0) {
         /* deferred sites: about 0.1% of a 30x genome; grown on demand */
-        c->dsite_cap = std::max<int64_t>(1 << 16, (c->view.on ? n_tiles * kTile : c->chr_len) / 256);
-        c->dpool_cap = c->dsite_cap * 48;
-        CK(dev_alloc(&c->d_dsites, (size_t)c->dsite_cap), "cudaMalloc deferred");
-        CK(dev_alloc(&c->d_dpool, (size_t)c->dpool_cap), "cudaMalloc deferred");
+        const int64_t sites = std::max<int64_t>(1 << 16, (c->view.on ? n_tiles * kTile : c->chr_len) / 256);
+        CK(alloc_deferred(c, sites, sites * 48), "cudaMalloc deferred");
     }
     if (!c->ev[0])
         for (int i = 0; i < 2 * gsnp_context::kMaxLaunches; ++i) CK(cudaEventCreate(&c->ev[i]), "cudaEventCreate");
@@ -1059,10 +1056,8 @@ int finish_device(gsnp_context* c, size_t segs) {
     if (err) return fail(c, GSNP_ERR_STATE, "record slots of a tile overflowed its depth bin");
     const int64_t ns = (int64_t)c->h_dcount[0], nw = (int64_t)c->h_dcount[1];
     if (ns > c->dsite_cap || nw > c->dpool_cap) {
-        c->dsite_cap = std::max(c->dsite_cap, ns + ns / 8 + 1024);
-        c->dpool_cap = std::max(c->dpool_cap, nw + nw / 8 + 65536);
-        CK(dev_alloc(&c->d_dsites, (size_t)c->dsite_cap), "cudaMalloc deferred");
-        CK(dev_alloc(&c->d_dpool, (size_t)c->dpool_cap), "cudaMalloc deferred");
+        CK(alloc_deferred(c, std::max(c->dsite_cap, ns + ns / 8 + 1024), std::max(c->dpool_cap, nw + nw / 8 + 65536)),
+           "cudaMalloc deferred");
         return kRedoDeferred;
     }
     c->stats[0] = (uint64_t)c->chr_len;
@@ -1261,10 +1256,9 @@ int run_calling(gsnp_context* c, const std::vector<Segment>& segs, const std::fu
                 /* grow the pool to what the segment asked for and run its fast
                  * kernels again (their sampled-site statistics were not yet
                  * counted: that happens in the deferred pass) */
-                c->dsite_cap = std::max(c->dsite_cap, ns + ns / 8 + 1024);
-                c->dpool_cap = std::max(c->dpool_cap, nw + nw / 8 + 65536);
-                CK(dev_alloc(&c->d_dsites, (size_t)c->dsite_cap), "cudaMalloc deferred");
-                CK(dev_alloc(&c->d_dpool, (size_t)c->dpool_cap), "cudaMalloc deferred");
+                CK(alloc_deferred(c, std::max(c->dsite_cap, ns + ns / 8 + 1024),
+                                  std::max(c->dpool_cap, nw + nw / 8 + 65536)),
+                   "cudaMalloc deferred");
                 c->n_launches = first;
             }
         }
@@ -1472,6 +1466,7 @@ int patch_deferred_calls(gsnp_context* c, gsnp_site_call* out) {
     }
     (void)cudaGetLastError();
     if (n > c->patch_cap) {
+        c->patch_cap = 0;
         CK(dev_alloc(&c->d_patch, (size_t)n), "cudaMalloc deferred calls");
         c->patch_cap = n;
     }
@@ -1621,6 +1616,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
     c->resident_L = 0;
     if (!c->d_out || c->out_sites < c->chr_len) {
         /* the resident calls of the chromosome (a streamed call keeps none) */
+        c->out_sites = 0;
         CK(dev_alloc(&c->d_out, (size_t)c->chr_len), "cudaMalloc calls");
         c->out_sites = c->chr_len;
     }
@@ -1638,6 +1634,8 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
     const size_t raw = (size_t)n * r->pitch;
     if (n > c->raw_cap || raw > c->raw_bytes) {
         const int64_t cap = std::max<int64_t>(n, 1);
+        c->raw_cap = 0;
+        c->raw_bytes = 0;
         CK(dev_alloc(&c->d_raw_pos, (size_t)cap), "cudaMalloc raw");
         CK(dev_alloc(&c->d_raw_len, (size_t)cap), "cudaMalloc raw");
         CK(dev_alloc(&c->d_raw_hit, (size_t)cap), "cudaMalloc raw");
@@ -1751,14 +1749,17 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
     }
     c->have_counts = need_counts;
     if (need_counts && c->counts_sites < c->chr_len) {
+        c->counts_sites = 0;
         CK(dev_alloc(&c->d_counts, (size_t)c->chr_len), "cudaMalloc counts");
         c->counts_sites = c->chr_len;
     }
     if (need_lik && c->lik_sites < c->chr_len) {
+        c->lik_sites = 0;
         CK(dev_alloc(&c->d_lik_keep, (size_t)c->chr_len * 10), "cudaMalloc likelihood");
         c->lik_sites = c->chr_len;
     }
     if (nd > c->cap_dep) {
+        c->cap_dep = 0;
         CK(dev_alloc(&c->d_pos, (size_t)nd), "cudaMalloc reads");
         CK(dev_alloc(&c->d_lenhit, (size_t)nd), "cudaMalloc reads");
         CK(dev_alloc(&c->d_len, (size_t)nd), "cudaMalloc reads");
@@ -1768,6 +1769,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
     /* 64 elements of slack: the staging bulk copies of the persistent kernel
      * round a row window up to 16 bytes past the last row */
     if (nd * L + 64 > c->cap_bq) {
+        c->cap_bq = 0;
         CK(dev_alloc(&c->d_bq, (size_t)nd * L + 64), "cudaMalloc reads");
         c->cap_bq = nd * L + 64;
     }
@@ -1788,6 +1790,7 @@ int call_chromosome(gsnp_context* c, const gsnp_reads* r, gsnp_site_call* out) {
     if (nd > 0) {
         const int64_t n_chunks = (n + kDepChunk - 1) / kDepChunk;
         if (n_chunks > c->dep_chunk_cap) {
+            c->dep_chunk_cap = 0;
             CK(dev_alloc(&c->d_dep_off, (size_t)n_chunks), "cudaMalloc index");
             c->dep_chunk_cap = n_chunks;
         }
@@ -2973,6 +2976,7 @@ int ring_ensure(gsnp_context* c, StreamRing* g, int64_t raw_rows, int64_t raw_by
         const int64_t rr = std::max(raw_rows, g->raw_rows), rb = std::max(raw_bytes, g->raw_bytes);
         const int64_t dr = std::max(dep_rows, g->dep_rows), ns = std::max(sites, g->sites);
         const int64_t nw = std::max(windows, g->windows), dc = std::max<int64_t>(1, (rr + kDepChunk - 1) / kDepChunk);
+        g->L = 0;   /* no chunk fits until all of it is there */
         for (auto& s : g->slot) {
             void* p[] = {s.raw_pos, s.raw_len, s.raw_hit, s.raw_strand, s.raw_seq, s.raw_qual, s.idx, s.dep_off,
                          s.pos, s.lenhit, s.len, s.strand, s.bq, s.out, s.win_flags, s.win_lik_src, s.win_host_src};

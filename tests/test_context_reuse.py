@@ -192,3 +192,28 @@ def test_reference_that_is_refused_changes_nothing(native_lib):
         assert c.fetch().tobytes() == want
         c.call(reads)
         assert c.fetch().tobytes() == want
+
+
+@pytest.mark.gpu
+def test_call_after_one_that_found_no_memory(native_lib):
+    """Rows that no device holds (200 of 2 GB, never touched: no alignment has a
+    base) end the call with an error; the next one allocates what it needs."""
+    w = edge_workload("plain")
+    with api.Caller() as c:
+        reads = load(c, w)
+        c.call(reads)
+        want = c.fetch().tobytes()
+        a = [x[:200].copy() for x in arrays(w)]
+        a[1][:] = 0
+        a[2][:] = 2
+        huge = api.Caller.reads_struct(*a)
+        huge.pitch = 2**31 - 1
+        with pytest.raises(RuntimeError, match=r"\(1\).*memory"):
+            c.call(huge)
+        with pytest.raises(RuntimeError, match=r"\(1\).*memory"):
+            c.call_streamed(huge)
+        c.call(reads)
+        assert c.fetch().tobytes() == want
+        out = np.zeros(c.length, dtype=api.SITE_DTYPE)
+        c.call_streamed(reads, None, out.ctypes.data)
+        assert out.tobytes() == want
