@@ -53,11 +53,11 @@ enum LeanTook : int { kLeanTook = 0, kLeanDeep = 1, kLeanNever = 2 };
  * taken in any order: forward ones from a list at the front, reverse ones from
  * one at the back, and the few reads of several hits, which leave no record,
  * as they are met.  A base of quality 0 makes its record like any other (its
- * element has the spilled base's bits); a tile that has one goes over its reads
+ * element has the spilled base's bits); the sites that have one go over the reads
  * once more to count them by their own base.  Left to the general form, tiles
  * with such a base cost more than before there was a short one: 8 Mbp at 30x,
  * one base in 100 of quality 0, recalled: FP32 6.04 ms (3.68 without the short
- * form) -> 2.34, FP64 8.58 (7.01) -> 3.45. */
+ * form) -> 2.55, FP64 8.58 (7.01) -> 3.57. */
 template <int SLOTS>
 __device__ __forceinline__ LeanTook lean_pileup(const CallArgs& a, int64_t s0, int64_t r_lo, int64_t r_hi,
                                             uint32_t* recs_all, LeanRead* reads, LeanPile* out) {
@@ -171,18 +171,21 @@ __device__ __forceinline__ LeanTook lean_pileup(const CallArgs& a, int64_t s0, i
                 }
             }
         }
-        if (__any_sync(kFull, (seen_bits & kElemZero) != 0)) {
-#pragma unroll 1
-            for (int k = 0; k < ((cnt + 3) & ~3); ++k) {
-                const int4 rd = list[k];
-                uint32_t x = kElemInvalid;
-                if ((uint32_t)(rd.x + lane) < (uint32_t)rd.w) x = __ldg(row + rd.y);
-                if ((x & (kElemInvalid | kElemZero)) == kElemZero) extra4 += 1ull << (elem_base(x) * 16 + kLeanExtraBits);
-            }
-        }
     }
     if (__any_sync(kFull, num > SLOTS || (seen_bits & kElemWide)))
         return __any_sync(kFull, (seen_bits & kElemWide) != 0) ? kLeanNever : kLeanDeep;
+    if (seen_bits & kElemZero) {
+        /* all slots of the two lists, the unused ones skipped: a loop over the
+         * used ones ran a tenth shorter here but cost every other tile of the
+         * FP64 kernel, which has no register to spare, another half percent */
+#pragma unroll 1
+        for (int i = 0; i < kReads; ++i) {
+            const int4 rd = reinterpret_cast<const int4*>(reads)[i];
+            uint32_t x = kElemInvalid;
+            if ((i < fwd || i >= kReads - rev) && (uint32_t)(rd.x + lane) < (uint32_t)rd.w) x = __ldg(row + rd.y);
+            if ((x & (kElemInvalid | kElemZero)) == kElemZero) extra4 += 1ull << (elem_base(x) * 16 + kLeanExtraBits);
+        }
+    }
     out->depth = depth;
     out->repeat = depth + extra_hits;
     out->extra4 = extra4;
