@@ -78,8 +78,9 @@ constexpr int32_t kTileGeneral = 1 << 30;
 /* After a persistent kernel in the short form, the shallowest bins: 64 slots for
  * the tiles that were too deep for its own, which try the short form again; 48,
  * whose kernel keeps more warps an SM, for the marked ones of a segment with more
- * tiles than the 64-slot kernel holds at once (in a smaller one the slots make no
- * difference and a launch costs 3 us of a call's 330).  8 Mbp recalled with every
+ * than eight times the tiles that the 64-slot kernel holds at once (some 0.8 Mbp;
+ * ordinary data has hardly a marked tile, and the launch costs it 3 us of each
+ * segment: a 30 kb recall 159 us instead of 156).  8 Mbp recalled with every
  * tile marked (20 reads of one start and strand): 3.90 ms in the 64-slot bin
  * after a second try, 3.15 in the 48-slot one, 3.02 and 2.90 with bins of 40 and
  * of 32 slots, each a launch more in every segment. */

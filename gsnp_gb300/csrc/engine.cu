@@ -1349,7 +1349,7 @@ int enqueue_device(gsnp_context* c, const std::vector<Segment>& segs, const std:
             if (rc != GSNP_OK) return rc;
         }
         const WindowModes modes = window_modes(c, g);
-        const bool small = g.t1 - g.t0 <= c->bin_grid[fast ? 1 : 0][kDeeperBin];
+        const bool small = g.t1 - g.t0 <= 8 * (int64_t)c->bin_grid[fast ? 1 : 0][kDeeperBin];
         const int first_bin = short_form && !small ? kGeneralBin : min_bin;
         CallArgs a = make_args(c);
         a.n_reads = c->n_gathered;

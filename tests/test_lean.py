@@ -209,11 +209,12 @@ def test_qualities_zero_and_64_stay_in_the_short_form(precision, tmp_path, oracl
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("sites,slots", [(30013, 64), (300013, 48)])
-def test_tiles_it_can_never_take_go_to_one_shallow_bin(sites, slots, tmp_path, oracle_bin, native_lib):
+@pytest.mark.parametrize("sites,slots", [(30013, 64), (1200013, 48)])
+def test_tiles_it_can_never_take_go_to_one_shallow_bin(sites, slots, tmp_path, oracle_bin, native_lib, monkeypatch):
     """Twenty reads of one start and strand everywhere: no tile of the short form
-    but too deep for none of its slots.  A segment of more tiles than the 64-slot
-    kernel holds at once gives them to the 48-slot one."""
+    but too deep for none of its slots.  A segment of many times the tiles that the
+    64-slot kernel holds at once gives them to the 48-slot one."""
+    monkeypatch.setenv("GSNP_SEGMENTS", "1")
     w = edge_workload("plain")
     rng = np.random.default_rng(9)
     L, code = 100, rng.integers(0, 4, sites)
