@@ -165,6 +165,10 @@ __device__ __forceinline__ void lik32_row(const CallArgs& a, int qa, int coord, 
     x[9] = t.y;
 }
 
+/* The grouping of the kernels' FP32 sums (fast_site, lean_walk, deferred_sum):
+ * four terms pairwise, then one compensated step.  The kernels each have it in
+ * their own form; this one states it for a whole column, for the host check of
+ * its error bound. */
 template <int BITS = 1>
 __device__ __forceinline__ void likelihood_fp32(const CallArgs& a, const uint32_t* recs, uint32_t* seen, int stride,
                                                 int num, double* tl, double* eps) {
